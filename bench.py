@@ -644,9 +644,9 @@ def main():
     clk = clocks.summary()
 
     # ---- dominant kernel roofline (FP64 DMMA bound) ----
-    # the FMM products launches: the direct variant (pre-summed operands) or the folding kernel
-    kinds = [k for k in ("fmm_gemm_direct_kernel[fmm products]", "fmm_gemm_kernel[fmm products]") if kt.count.get(k)]
-    core_name = max(kinds, key=lambda k: kt.ms[k]) if kinds else "fmm_gemm_direct_kernel[fmm products]"
+    # the FMM products launches
+    kinds = [k for k in ("fmm_products_kernel",) if kt.count.get(k)]
+    core_name = "fmm_products_kernel"
     core_ms = sum(kt.ms[k] for k in kinds)
     core_launches = sum(kt.count[k] for k in kinds)
     cflops = core_flops(plan.algebra, SHAPES) * args.steps

@@ -17,7 +17,6 @@
 #include <atomic>
 #include <cmath>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -26,6 +25,7 @@
 #include "../../include/fmm_b200.h"
 #include "fmm_kernels.cuh"
 #include "fmm_split_bf16.cuh"
+#include "fmm_tile.cuh"
 
 namespace {
 
@@ -47,27 +47,22 @@ thread_local long long t_last_ws = 0;
 // Optional per-kernel timing: when enabled, every launch is bracketed by CUDA events on
 // its own stream; fmm_profile_end() sums the durations per kernel kind.
 enum KernelKind {
-  K_GEMM_FMM = 0,
-  K_GEMM_CLASSICAL = 1,
-  K_LINCOMB = 2,
+  K_PRODUCTS = 0,
+  K_TILE_GEMM = 1,
+  K_PRESUM = 2,
   K_SCATTER = 3,
   K_SPLIT_OPERANDS = 4,
   K_GEMM_SPLIT = 5,
-  K_GEMM_BATCH = 6,
-  K_LINCOMB_BATCH = 7,
+  K_PRODUCTS_BATCH = 6,
+  K_PRESUM_BATCH = 7,
   K_PITCH_COPY = 8,
   K_COMBINE = 9,
-  K_GEMM_FMM_DIRECT = 10,        // the same launches when they run the direct variant
-  K_GEMM_CLASSICAL_DIRECT = 11,
-  K_NUM = 12
+  K_NUM = 10
 };
-const char* const kKernelNames[K_NUM] = {"fmm_gemm_kernel[fmm products]", "fmm_gemm_kernel[classical]",
-                                         "fmm_lincomb_kernel", "fmm_scatter_kernel",
-                                         "fmm_split_operands_kernel", "fmm_split_gemm_kernel",
-                                         "fmm_gemm_batch_kernel", "fmm_lincomb_batch_kernel",
-                                         "fmm_pitch_copy_kernel", "fmm_combine_kernel",
-                                         "fmm_gemm_direct_kernel[fmm products]",
-                                         "fmm_gemm_direct_kernel[classical]"};
+const char* const kKernelNames[K_NUM] = {"fmm_products_kernel",       "fmm_tile_gemm_kernel",    "fmm_presum_kernel",
+                                         "fmm_scatter_kernel",        "fmm_split_operands_kernel", "fmm_split_gemm_kernel",
+                                         "fmm_products_batch_kernel", "fmm_presum_batch_kernel", "fmm_pitch_copy_kernel",
+                                         "fmm_combine_kernel"};
 struct ProfRec {
   int kind;
   cudaEvent_t e0, e1;
@@ -117,14 +112,16 @@ struct DevTables {
   fmm::Prod* prods_all = nullptr;  // every product over pre-summed slots (slot r = product r)
   fmm::Term* terms_all = nullptr;
   int* plist_all = nullptr;        // 0 .. R-1
+  int* ps_first[2] = {nullptr, nullptr};         // presum tables of the A and B side
+  fmm::PTerm* ps_terms[2] = {nullptr, nullptr};
   bool ready = false;
 };
 
-// Tables of a k split (see ksplit_tables): base tables (one of the TableBase forms) with
-// every product r split into S products (r, p) over k range p of its operands.
-enum TableBase : int { BASE_ORIG = 0, BASE_PS = 1, BASE_ALL = 2, BASE_GROUP = 3 };
+// Tables derived from a plan on first use: the classical plan's k split into S parts
+// (ksplit_build) or the products [S, g1) of a workspace group (group_build).
+enum TableBase : int { BASE_SPLIT = 0, BASE_GROUP = 1 };
 struct KSplitTables {
-  int base = 0, S = 0, g1 = 0, dev = -1;  // BASE_GROUP: products [S, g1) (see group_build)
+  int base = 0, S = 0, g1 = 0, dev = -1;
   fmm::Prod* prods = nullptr;
   fmm::Term* terms = nullptr;
 };
@@ -159,6 +156,9 @@ struct fmm_plan {
   // k step, so that zero-padded workspaces keep each k step inside its operand block.
   std::vector<fmm::Prod> prods_all;
   std::vector<fmm::Term> terms_all;
+  // A (0) and B (1) terms of every product, product r's from ps_first[r] on.
+  std::vector<int> ps_first[2];
+  std::vector<fmm::PTerm> ps_terms[2];
   std::mutex mu;
   DevTables dev[kMaxDevices];
   std::vector<KSplitTables> ksplit;  // uploaded k-split tables (any device), built on first use
@@ -211,6 +211,10 @@ int upload_tables(fmm_plan* p, DevTables& d) {
     FMM_CUDA_TRY(up(&d.ch_r, p->ch_r));
     FMM_CUDA_TRY(up(&d.ch_m, p->ch_m));
     FMM_CUDA_TRY(up(&d.ch_c, p->ch_c));
+    for (int side = 0; side < 2; ++side) {
+      FMM_CUDA_TRY(up(&d.ps_first[side], p->ps_first[side]));
+      FMM_CUDA_TRY(up(&d.ps_terms[side], p->ps_terms[side]));
+    }
   }
   FMM_CUDA_TRY(cudaMalloc(&d.prods_ps, sizeof(fmm::Prod) * p->prods_ps.size()));
   FMM_CUDA_TRY(cudaMalloc(&d.terms_ps, sizeof(fmm::Term) * p->terms_ps.size()));
@@ -252,46 +256,16 @@ int device_tables(const fmm_plan* cp, DevTables** out) {
   return FMM_OK;
 }
 
-// k split of a plan's products: product r (k extent ks) becomes S products (r, p), p = 0..S-1,
-// each over k range [p ks/S, (p+1) ks/S) of r's operands, with r's C terms.  A work unit then
-// covers a product's k range part, so a launch with too few units for whole waves of the
-// SMs gets S times as many, shorter ones.  The C update is linear in the product, so the
-// parts' updates, applied in order (r, 0), (r, 1), ... under the same tickets, sum to r's.
-// With the part depth ks' = ks / S every operand term keeps its block and indexes part p by
-// its k block coordinate: an A term (row, col) becomes (row, col S + p) (A column offset
-// col ks + p ks' = (col S + p) ks'), a B term (row, col) becomes (row S + p, col); this holds
-// for blocks of A and B and for the slots of the pre-summed workspaces alike.  C terms keep
-// their block; their per-block ticket position (pad) counts the split products.
-void ksplit_build(const fmm_plan* p, int base, int S, std::vector<fmm::Prod>* op, std::vector<fmm::Term>* ot) {
-  const std::vector<fmm::Prod>& prods = base == BASE_PS ? p->prods_ps : base == BASE_ALL ? p->prods_all : p->prods;
-  const std::vector<fmm::Term>& terms = base == BASE_PS ? p->terms_ps : base == BASE_ALL ? p->terms_all : p->terms;
-  std::vector<int> cnt((size_t)p->dims[0] * p->dims[2], 0);
-  // part-major: split product (r, q) is q * R + r, so the S parts of one (tile, product) are
-  // R tiles' worth of units apart and do not run at the same time (their C updates are
-  // ordered by tickets, so parts claimed together would wait on each other)
+// k split of the classical plan: S products over k parts of depth d, part q at block
+// coordinate q (the products kernel addresses operand blocks by multiples of the product's k
+// depth, so part q starts at q d), all added to the one C block in order.
+void ksplit_build(int S, std::vector<fmm::Prod>* op, std::vector<fmm::Term>* ot) {
   for (int q = 0; q < S; ++q) {
-    for (const fmm::Prod& pr : prods) {
-      fmm::Prod v = pr;
-      v.a0 = (int)ot->size();
-      for (int t = 0; t < pr.na; ++t) {
-        fmm::Term x = terms[pr.a0 + t];
-        x.col = x.col * S + q;
-        ot->push_back(x);
-      }
-      v.b0 = (int)ot->size();
-      for (int t = 0; t < pr.nb; ++t) {
-        fmm::Term x = terms[pr.b0 + t];
-        x.row = x.row * S + q;
-        ot->push_back(x);
-      }
-      v.c0 = (int)ot->size();
-      for (int t = 0; t < pr.nc; ++t) {
-        fmm::Term x = terms[pr.c0 + t];
-        x.pad = cnt[(size_t)x.row * p->dims[2] + x.col]++;
-        ot->push_back(x);
-      }
-      op->push_back(v);
-    }
+    const int t = (int)ot->size();
+    ot->push_back(fmm::Term{0, q, 1.0, 0, 0});
+    ot->push_back(fmm::Term{q, 0, 1.0, 0, 0});
+    ot->push_back(fmm::Term{0, 0, 1.0, 0, q});
+    op->push_back(fmm::Prod{t, 1, t + 1, 1, t + 2, 1});
   }
 }
 
@@ -320,8 +294,8 @@ void group_build(const fmm_plan* p, int g0, int g1, std::vector<fmm::Prod>* op, 
   }
 }
 
-// Derived tables of a plan on the current device (uploaded on first use): the k split S of a
-// base form (ksplit_build), or with base == BASE_GROUP the group [S, g1) (group_build).
+// Derived tables of a plan on the current device (uploaded on first use): the classical plan's
+// k split into S parts, or with base == BASE_GROUP the group [S, g1) (group_build).
 int ksplit_tables(const fmm_plan* cp, int base, int S, const fmm::Prod** prods, const fmm::Term** terms,
                   int g1 = 0) {
   fmm_plan* p = const_cast<fmm_plan*>(cp);
@@ -339,7 +313,7 @@ int ksplit_tables(const fmm_plan* cp, int base, int S, const fmm::Prod** prods, 
   if (base == BASE_GROUP)
     group_build(p, S, g1, &vp, &vt);
   else
-    ksplit_build(p, base, S, &vp, &vt);
+    ksplit_build(S, &vp, &vt);
   KSplitTables t;
   t.base = base;
   t.S = S;
@@ -597,7 +571,16 @@ int build_plan(const int dims[3], int rank, const int* nterms, const int* rows, 
     qa.nc = pr.nc;
     for (int c = 0; c < pr.nc; ++c) p->terms_all.push_back(p->terms[pr.c0 + c]);
     p->prods_all.push_back(qa);
+    for (int side = 0; side < 2; ++side) {
+      const int t0 = side == 0 ? pr.a0 : pr.b0, nt = side == 0 ? pr.na : pr.nb;
+      p->ps_first[side].push_back((int)p->ps_terms[side].size());
+      for (int t = 0; t < nt; ++t) {
+        const fmm::Term& tm = p->terms[t0 + t];
+        p->ps_terms[side].push_back(fmm::PTerm{tm.row, tm.col, tm.coef});
+      }
+    }
   }
+  for (int side = 0; side < 2; ++side) p->ps_first[side].push_back((int)p->ps_terms[side].size());
   *out = p;
   return FMM_OK;
 }
@@ -628,12 +611,15 @@ int configure_kernel(int* dev_out) {
   if (dev < 0 || dev >= kMaxDevices) return FMM_E_UNSUPPORTED;
   std::lock_guard<std::mutex> lk(g_attr_mu);
   if (!smem_configured[dev]) {
-    FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)fmm::smem_bytes(false)));
-    FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)fmm::smem_bytes(true)));
-    FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_gemm_direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)fmm::SMEM_BYTES_DIRECT));
+    auto smem = [](auto kernel, size_t bytes) {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    FMM_CUDA_TRY(smem(fmmt::fmm_tile_gemm_kernel<64, 64>, fmmt::TileShape<64, 64>::SMEM));
+    FMM_CUDA_TRY(smem(fmmt::fmm_tile_gemm_kernel<32, 32>, fmmt::TileShape<32, 32>::SMEM));
+    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<64>, fmmt::ProdShape<64>::SMEM));
+    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<32>, fmmt::ProdShape<32>::SMEM));
+    FMM_CUDA_TRY(smem(fmmt::fmm_products_batch_kernel<false>, fmmt::ProdShape<64>::SMEM));
+    FMM_CUDA_TRY(smem(fmmt::fmm_products_batch_kernel<true>, fmmt::ProdShape<64>::SMEM));
     if (!g_encode_tiled) {
       cudaDriverEntryPointQueryResult q;
       void* fn = nullptr;
@@ -661,7 +647,7 @@ int configure_kernel(int* dev_out) {
 // Column-major FP64 matrix (rows x cols, leading dimension ld) as a 2-D tensor map with
 // the given box.  Returns false when TMA cannot address it (then cp.async staging runs).
 bool make_tensor_map(CUtensorMap* map, const double* base, long long rows, long long cols, long long ld,
-                     unsigned box_rows, unsigned box_cols) {
+                     unsigned box_rows, unsigned box_cols, bool swizzle = false) {
   if (!g_encode_tiled) return false;
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (ld & 1) != 0) return false;
   if (rows <= 0 || cols <= 0 || rows >= (1LL << 31) || cols >= (1LL << 31) || ld * 8 >= (1LL << 40)) return false;
@@ -670,87 +656,210 @@ bool make_tensor_map(CUtensorMap* map, const double* base, long long rows, long 
   cuuint32_t box[2] = {box_rows, box_cols};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(base), dims, strides, box,
-                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
-// Work units take one product each (product-major order): the CTAs running at one time
-// then work on one or two products, whose operand panels stay in L2, and the per-tile
-// tickets keep the C updates in product order.  Measured on B200 against units of many
-// products: 16384^3 222-1 x 333-1 35.6 -> 36.5 TFLOP/s, 222-2 41.0 -> 41.3.
-int choose_chunks(int ntiles, int nprod, int nsm) {
-  (void)ntiles;
-  (void)nsm;
-  return nprod;
+// The maps the tile kernels read their operands with (see fmm_tile.cuh's stage layout).
+bool make_a_map(CUtensorMap* map, const double* A, long long m, long long k, long long lda) {
+  return make_tensor_map(map, A, m, k, lda, 16, fmmt::BK, true);
+}
+bool make_b_map(CUtensorMap* map, const double* B, long long k, long long n, long long ldb, int tile) {
+  return make_tensor_map(map, B, k, n, ldb, 8, tile);
 }
 
-// k split (ksplit_build) for a launch of `units` work units of ks deep products on nsm SMs.
-// A launch of few units spends its last wave partly idle: 222-1 at 2048^3 has 448 units
-// on 148 SMs, 3.03 waves whose last holds 4 units.  Splitting every product's k range into S
-// parts gives S times the units, each S times shorter; the modelled time
-// ceil(units S / nsm) (ks / (8 S) + kUnitOverheadSteps) k steps picks S in 1..8 (parts of
-// whole k steps, at least kMinPartSteps deep; a split must gain 3 %).  Launches of many waves
-// keep S = 1.
-constexpr int kUnitOverheadSteps = 4;  // per-unit cost beyond its k steps (hand-off, C tile traffic)
-constexpr int kMinPartSteps = 16;
-std::atomic<int> g_split_form{0};     // fmm_debug_set FMM_DEBUG_SPLIT_OPERANDS: 1 = one product per CTA
-std::atomic<int> g_force_ksplit{0};  // fmm_debug_set FMM_DEBUG_KSPLIT: S for every split launch (0: model)
-int choose_ksplit(long long units, int ks, int nsm) {
-  if (units <= 0 || nsm <= 0 || units >= 8LL * nsm || ks % fmm::BK != 0) return 1;
-  const long long nks = ks / fmm::BK;
-  const int forced = g_force_ksplit.load();
-  if (forced > 0) return (nks % forced == 0 && nks / forced >= kMinPartSteps) ? forced : 1;
-  auto cost = [&](int S) { return ((units * S + nsm - 1) / nsm) * (double)(nks / S + kUnitOverheadSteps); };
-  int best = 1;
-  double best_cost = cost(1);
-  for (int S = 2; S <= 8; ++S) {
-    if (nks % S != 0 || nks / S < kMinPartSteps) continue;
-    const double c = cost(S);
-    if (c < 0.97 * best_cost) {
-      best = S;
-      best_cost = c;
-    }
+// Launch with programmatic stream serialization (the kernel waits for its predecessors itself,
+// griddepcontrol.wait, so its set-up overlaps their end) and an optional cluster.
+template <class... Params, class... Args>
+int launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster,
+                     Args... args) {
+  cudaLaunchAttribute at[2];
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 1;
+  if (cluster > 1) {
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)cluster;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
   }
-  return best;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cuda_status(e);
 }
 
-// Launch the persistent DMMA GEMM over sub-blocks of size ms x ks x ns.
-// Workspaces of pre-summed operands (slot j of S: ms x ks, of T: ks x ns, block columns).
+std::atomic<int> g_split_form{0};    // fmm_debug_set FMM_DEBUG_SPLIT_OPERANDS: 1 = one product per CTA
+std::atomic<int> g_force_ksplit{0};  // fmm_debug_set FMM_DEBUG_KSPLIT: S for every classical launch (0: the rule)
+
+long long tiles_of(int m, int n, int t) { return (long long)((m + t - 1) / t) * ((n + t - 1) / t); }
+
+// Tile side for u64 units of 64 x 64 or u32 of 32 x 32: the modelled time, SM-seconds over the
+// SMs plus half a unit for the last, partly filled round, the small tile at 6 % lower rate
+// (more shared-memory reads per DMMA).  Measured us with 64 / 32: stored 222-1 512^3 44.9 /
+// 30.7, 1024^3 103.9 / 97.3, 1488^3 242 / 264, 2048^3 544 / 572; 222-1 x 333-1 1200^3 247 / 228,
+// 2016 x 2016 x 8064 2443 / 2327, 3024^3 1722 / 1862; plain 1024^3 77.1 / 75.8, 4096^3 3857 / 4022.
+int tile_side(long long u64, long long u32, int nsm) {
+  const double c64 = ((double)u64 / nsm + 0.5) * 4096, c32 = ((double)u32 / nsm + 0.5) * 1024 * 1.06;
+  return c64 <= c32 ? 64 : 32;
+}
+
+// k parts of a classical update: S parts of depth d (a multiple of 8), part s covering
+// [s d, min(k, (s + 1) d)).  The result of an update depends on S (each part is summed on its
+// own and added to C in order), so S is a function of the sizes alone and batches use the
+// same one.
+constexpr int kMinPartDepth = 64;
+constexpr int kPartCtas = 460;
+void classical_parts(int m, int n, int k, int* S, int* d) {
+  auto depth = [&](int s) { return ((k + s - 1) / s + 7) / 8 * 8; };
+  const long long t32 = tiles_of(m, n, 32);
+  int s = 1;
+  while (2 * s <= fmmt::MAX_SPLIT && t32 * 2 * s <= kPartCtas && k >= 2 * s * kMinPartDepth) s *= 2;
+  const int forced = g_force_ksplit.load();
+  if (forced > 0 && (long long)(forced - 1) * depth(forced) < k) s = forced;
+  *S = s;
+  *d = s == 1 ? k : depth(s);
+}
+
+// One classical update of a tile_gemm launch.
+struct GemmJob {
+  int m, n, k;
+  const double* A;
+  long long lda;
+  const double* B;
+  long long ldb;
+  double* C;
+  long long ldc;
+};
+
+template <int T>
+int launch_tile_gemm(const GemmJob* jobs, int njob, unsigned* status, cudaStream_t st) {
+  fmmt::TileArgs g{};
+  int cluster = 1;
+  for (int q = 0; q < njob; ++q) {
+    fmmt::TileJob& J = g.job[q];
+    classical_parts(jobs[q].m, jobs[q].n, jobs[q].k, &J.S, &J.d);
+    cluster = std::max(cluster, J.S);
+  }
+  long long first = 0;
+  for (int q = 0; q < njob; ++q) {
+    const GemmJob& b = jobs[q];
+    fmmt::TileJob& J = g.job[q];
+    J.A = b.A;
+    J.lda = b.lda;
+    J.B = b.B;
+    J.ldb = b.ldb;
+    J.C = b.C;
+    J.ldc = b.ldc;
+    J.m = b.m;
+    J.n = b.n;
+    J.k = b.k;
+    J.tiles_m = (b.m + T - 1) / T;
+    J.tiles_n = (b.n + T - 1) / T;
+    J.a_tma = make_a_map(&J.tmA, b.A, b.m, b.k, b.lda);
+    J.b_tma = make_b_map(&J.tmB, b.B, b.k, b.n, b.ldb, T);
+    const long long units = (long long)J.tiles_m * J.tiles_n * J.S;
+    if (first + units > INT32_MAX - fmmt::MAX_SPLIT) return FMM_E_UNSUPPORTED;
+    J.first = (int)first;
+    J.units = (int)units;
+    first += (units + cluster - 1) / cluster * cluster;
+  }
+  g.njob = njob;
+  g.status = status;
+  ProfScope ps(K_TILE_GEMM, st);
+  return launch_dependent(fmmt::fmm_tile_gemm_kernel<T, T>, dim3((unsigned)first), fmmt::NT, fmmt::TileShape<T, T>::SMEM,
+                          st, cluster, g);
+}
+
+int tile_gemm(const GemmJob* jobs, int njob, cudaStream_t st) {
+  int dev = 0;
+  const int rc = configure_kernel(&dev);
+  if (rc != FMM_OK) return rc;
+  // parts of one tile are a cluster: jobs of one launch share S or have one part
+  GemmJob todo[fmmt::MAX_JOBS];
+  int n = 0, S = 1;
+  for (int q = 0; q < njob; ++q) {
+    if (jobs[q].m <= 0 || jobs[q].n <= 0 || jobs[q].k <= 0) continue;
+    int s, d;
+    classical_parts(jobs[q].m, jobs[q].n, jobs[q].k, &s, &d);
+    if (s > 1 && S > 1 && s != S) {  // another cluster size: a launch of its own
+      const int r = launch_tile_gemm<32>(jobs + q, 1, dev_status[dev], st);
+      if (r != FMM_OK) return r;
+      continue;
+    }
+    S = std::max(S, s);
+    todo[n++] = jobs[q];
+  }
+  if (n == 0) return FMM_OK;
+  if (n == 1 && S == 1 && tile_side(tiles_of(todo[0].m, todo[0].n, 64), tiles_of(todo[0].m, todo[0].n, 32), sm_count[dev]) == 64)
+    return launch_tile_gemm<64>(todo, n, dev_status[dev], st);
+  return launch_tile_gemm<32>(todo, n, dev_status[dev], st);
+}
+
+// Workspaces of pre-summed operands: slot j of S is ms x kslot, of T kslot x ns (block
+// columns); nslot = 0: every operand of that side is a block of A / B.
 struct PresumOps {
-  const int* plistA = nullptr;  // products of the slots (device); nullptr: the plan's lists
+  const int* plistA = nullptr;  // products of the slots (device)
   const int* plistB = nullptr;
-  int kslot = 0;                // columns per S slot and rows per T slot; 0: ks
-  const double* S = nullptr;
+  int kslot = 0;                // columns per S slot and rows per T slot
+  double* S = nullptr;
   long long ldS = 0;
   int nslotA = 0;
-  const double* T = nullptr;
+  double* T = nullptr;
   long long ldT = 0;
   int nslotB = 0;
 };
 
-// Every k step of a product reads only its own operand blocks: ks is a multiple of BK, or
-// the block grid is 1 x 1 x 1, where the tensor maps end at the operands' last k column / row
-// and a partial last step reads TMA's zero fill.
-bool whole_k_steps(const int grid_dims[3], int ks) {
-  return ks % fmm::BK == 0 || (grid_dims[0] == 1 && grid_dims[1] == 1 && grid_dims[2] == 1);
+// Every k group of a product reads only its own operand blocks: ks is a multiple of eight, or
+// the plan is one product of whole operands, where the tensor maps end at their last k column
+// / row and a partial last group reads TMA's zero fill.
+bool whole_k_steps(const fmm_plan* plan, int ks) {
+  return ks % 8 == 0 || (plan->rank == 1 && plan->dims[0] == 1 && plan->dims[1] == 1 && plan->dims[2] == 1);
 }
 
-// direct_ok: every product's operands are single unit-coefficient blocks (pre-summed
-// products, the classical plan), so with TMA staging and whole k steps the direct variant
-// (epilogue on the otherwise idle folding warps, overlapping the next product) can run.
-// ksplit > 1: prods / terms are k-split tables (ksplit_tables) with nprod = R * ksplit products
-// of depth ks / ksplit, a whole number of k steps; ks is the operands' full depth.
-int launch_gemm(int kind, const fmm::Prod* prods, const fmm::Term* terms, const int grid_dims[3], int nprod,
-                int mode, const double* A, long long lda, const double* B, long long ldb, const PresumOps& ps,
-                double* C, long long ldc, double* M, long long ldm, long long m_stride, int ms, int ns, int ks,
-                cudaStream_t st, bool direct_ok = false, int ks_orig = -1, int ksplit = 1) {
-  if (ms <= 0 || ns <= 0 || ks <= 0 || nprod <= 0) return FMM_OK;
-  if (ksplit < 1 || ks % ksplit != 0 || (ksplit > 1 && (ks / ksplit) % fmm::BK != 0)) return FMM_E_INVALID;
+constexpr int kResident64 = fmmt::TileShape<64, 64>::CTAS;  // 64 x 64 CTAs per SM
+
+// Tile side of a products launch and its tickets: per (tile, C block) where a product has no
+// more tiles than CTAs run at a time (the units of one tile then run together, and one ticket
+// per tile would chain all R updates), else per tile.
+struct ProdLaunch {
+  int tile = 64;
+  size_t tickets = 0;
+  int nbt = 0, nbc = 0;
+};
+
+ProdLaunch plan_products(const int grid_dims[3], int nprod, int mode, int ms, int ns, int nsm) {
+  ProdLaunch L;
+  L.tile = tile_side(tiles_of(ms, ns, 64) * nprod, tiles_of(ms, ns, 32) * nprod, nsm);
+  if (mode == fmm::MODE_ACCUM_C && nprod > 1) {
+    const long long ntiles = tiles_of(ms, ns, L.tile);
+    if (ntiles <= kResident64 * (long long)nsm) {
+      L.nbt = grid_dims[0] * grid_dims[2];
+      L.nbc = grid_dims[2];
+    }
+    L.tickets = 4 * (size_t)ntiles * (L.nbt > 0 ? L.nbt : 1);
+  }
+  return L;
+}
+
+// The products of a plan over sub-blocks ms x ns with k depth kk (kk: the slots' depth, ks:
+// the operands' own); counter: the launch's work-unit counter and then its tickets, zeroed.
+int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int grid_dims[3], int nprod, int mode,
+                    const double* A, long long lda, const double* B, long long ldb, const PresumOps& ps, double* C,
+                    long long ldc, double* M, int ms, int ns, int ks, int kk, const ProdLaunch& L, int* counter,
+                    cudaStream_t st) {
   int dev = 0;
   int rc = configure_kernel(&dev);
   if (rc != FMM_OK) return rc;
-  fmm::GemmArgs a{};
+  fmmt::ProdArgs a{};
   a.A = A;
   a.lda = lda;
   a.B = B;
@@ -758,99 +867,41 @@ int launch_gemm(int kind, const fmm::Prod* prods, const fmm::Term* terms, const 
   a.C = C;
   a.ldc = ldc;
   a.M = M;
-  a.ldm = ldm;
-  a.m_stride = m_stride;
-  a.ms = ms;
-  a.ns = ns;
-  a.ks = ks / ksplit;
+  a.m_stride = (long long)ms * ns;
   a.prods = prods;
   a.terms = terms;
-  a.Aw = ps.S ? ps.S : A;
-  a.ldaw = ps.S ? ps.ldS : lda;
-  a.Bw = ps.T ? ps.T : B;
-  a.ldbw = ps.T ? ps.ldT : ldb;
+  a.ms = ms;
+  a.ns = ns;
+  a.ks = kk;
   a.nprod = nprod;
-  a.tiles_m = (ms + fmm::BM - 1) / fmm::BM;
-  a.tiles_n = (ns + fmm::BN - 1) / fmm::BN;
+  a.tiles_m = (ms + L.tile - 1) / L.tile;
+  a.tiles_n = (ns + L.tile - 1) / L.tile;
+  a.chunks = nprod;
   a.mode = mode;
   a.status = dev_status[dev];
-  const int ntiles = a.tiles_m * a.tiles_n;
-  a.chunks = (mode == fmm::MODE_ACCUM_C) ? choose_chunks(ntiles, nprod, sm_count[dev]) : 1;
-  const long long units = (long long)ntiles * (mode == fmm::MODE_STORE_M ? nprod : a.chunks);
+  a.counter = counter;
+  a.tickets = L.tickets ? counter + 1 : nullptr;
+  a.nbt = L.nbt;
+  a.nbc = L.nbc;
+  a.a_tma = a.b_tma = 1;
+  const long long units = (long long)a.tiles_m * a.tiles_n * nprod;
   if (units > INT32_MAX) return FMM_E_UNSUPPORTED;
-  const unsigned grid = (unsigned)(units < sm_count[dev] ? units : sm_count[dev]);
-  // A spans grid_dims[0] x grid_dims[1] blocks of ms x ks; B grid_dims[1] x grid_dims[2] of ks x ns
-  // the operands' own maps cover the operands (their k extent is the real one when the
-  // products read zero-padded pre-summed slots)
-  const long long am = (long long)grid_dims[0] * ms, ak = (long long)grid_dims[1] * (ks_orig >= 0 ? ks_orig : ks),
-                  bn = (long long)grid_dims[2] * ns;
-  bool tma = make_tensor_map(&a.tmA, A, am, ak, lda, fmm::BM, fmm::BK) &&
-             make_tensor_map(&a.tmA64, A, am, ak, lda, fmm::BM / 2, fmm::BK) &&
-             make_tensor_map(&a.tmB, B, ak, bn, ldb, fmm::BK, fmm::BN) &&
-             make_tensor_map(&a.tmB2, B, ak, bn, ldb, fmm::TB_K, fmm::BN);
-  if (tma) {
-    if (ps.S && ps.nslotA > 0)
-      tma = make_tensor_map(&a.tmAw, ps.S, ms, (long long)ps.nslotA * ks, ps.ldS, fmm::BM, fmm::BK) &&
-            make_tensor_map(&a.tmAw64, ps.S, ms, (long long)ps.nslotA * ks, ps.ldS, fmm::BM / 2, fmm::BK);
-    else
-      a.tmAw = a.tmA, a.tmAw64 = a.tmA64;
-  }
-  if (tma) {
-    if (ps.T && ps.nslotB > 0)
-      tma = make_tensor_map(&a.tmBw, ps.T, ks, (long long)ps.nslotB * ns, ps.ldT, fmm::BK, fmm::BN) &&
-            make_tensor_map(&a.tmBw2, ps.T, ks, (long long)ps.nslotB * ns, ps.ldT, fmm::TB_K, fmm::BN);
-    else
-      a.tmBw = a.tmB, a.tmBw2 = a.tmB2;
-  }
-  const bool direct = direct_ok && tma && whole_k_steps(grid_dims, a.ks);
-  // Per-tile tickets keep a tile's C updates in product order.  With few tile positions
-  // (at most half as many as SMs) the units of one position run at the same time and their
-  // epilogues form one chain of all R products; there the direct variant (one product per
-  // unit) orders the updates per (tile, C block) instead, so only products that update the
-  // same C block wait for one another.  Each C element still receives its products'
-  // updates in product order (same results).  Measured on B200, per tile -> per block:
-  // 222-1 x 333-1 3000^3 3.21 -> 2.13 ms, 4000 x 3840 x 2000 3.29 -> 2.67 ms, 4096^3 5.42
-  // -> 5.08 ms; 222-2 2048^3 0.88 -> 0.60 ms; 222-1 1024^3 0.17 -> 0.14 ms.  With more
-  // positions the extra barrier per C term costs more than it frees (14400^2 x 480, 361
-  // positions: 12.5 -> 14.0 ms; 4000 x 16000 x 2000, 126 positions: 9.5 -> 9.9 ms).
-  // [0]: the launch's work-unit counter; then the tickets
-  size_t nt = 0;
-  if (mode == fmm::MODE_ACCUM_C && a.chunks > 1) {
-    if (direct && a.chunks == nprod && 2 * ntiles <= sm_count[dev]) {
-      a.nbt = grid_dims[0] * grid_dims[2];
-      a.nbc = grid_dims[2];
-    }
-    nt = (size_t)ntiles * (a.nbt > 0 ? a.nbt : 1);
-  }
-  int* tickets = nullptr;
-  FMM_CUDA_TRY(cudaMallocAsync((void**)&tickets, sizeof(int) * (nt + 1), st));
-  FMM_CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(int) * (nt + 1), st));
-  if (nt > 0 && g_ticket_fill != 0)
-    FMM_CUDA_TRY(cudaMemsetAsync(tickets + 1, g_ticket_fill, sizeof(int) * nt, st));
-  a.counter = tickets;
-  a.tickets = nt > 0 ? tickets + 1 : nullptr;
-  {
-    const int pkind = !direct ? kind : (kind == K_GEMM_FMM ? K_GEMM_FMM_DIRECT : K_GEMM_CLASSICAL_DIRECT);
-    ProfScope ps(pkind, st);
-    if (direct)
-      fmm::fmm_gemm_direct_kernel<<<grid, fmm::NTHREADS, fmm::SMEM_BYTES_DIRECT, st>>>(a);
-    else if (tma)
-      fmm::fmm_gemm_kernel<true><<<grid, fmm::NTHREADS, fmm::smem_bytes(true), st>>>(a);
-    else
-      fmm::fmm_gemm_kernel<false><<<grid, fmm::NTHREADS, fmm::smem_bytes(false), st>>>(a);
-  }
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  rc = cuda_status(cudaGetLastError());
-  if (tickets) {
-    cudaError_t fe = cudaFreeAsync(tickets, st);
-    if (rc == FMM_OK) rc = cuda_status(fe);
-  }
-  return rc;
+  const long long am = (long long)grid_dims[0] * ms, ak = (long long)grid_dims[1] * ks, bn = (long long)grid_dims[2] * ns;
+  bool ok = true;
+  if (ps.nslotA < nprod) ok = ok && make_a_map(&a.tmA, A, am, ak, lda);
+  if (ps.nslotB < nprod) ok = ok && make_b_map(&a.tmB, B, ak, bn, ldb, L.tile);
+  if (ps.nslotA > 0) ok = ok && make_a_map(&a.tmAw, ps.S, ms, (long long)ps.nslotA * kk, ps.ldS);
+  if (ps.nslotB > 0) ok = ok && make_b_map(&a.tmBw, ps.T, kk, (long long)ps.nslotB * ns, ps.ldT, L.tile);
+  if (!ok) return FMM_E_UNSUPPORTED;
+  const int per_sm = L.tile == 64 ? fmmt::TileShape<64, 64>::CTAS : fmmt::TileShape<32, 32>::CTAS;
+  const unsigned grid = (unsigned)std::min<long long>(units, (long long)sm_count[dev] * per_sm);
+  ProfScope pf(K_PRODUCTS, st);
+  if (L.tile == 64)
+    return launch_dependent(fmmt::fmm_products_kernel<64>, dim3(grid), fmmt::NT, fmmt::ProdShape<64>::SMEM, st, 1, a);
+  return launch_dependent(fmmt::fmm_products_kernel<32>, dim3(grid), fmmt::NT, fmmt::ProdShape<32>::SMEM, st, 1, a);
 }
 
 const int kUnitGrid[3] = {1, 1, 1};
-
-int call_ksplit(const fmm_plan* plan, int ms, int ns, int ks, bool presum, int kk, int nsm);  // below
 
 int sm_count_current() {
   int dev = 0;
@@ -860,24 +911,8 @@ int sm_count_current() {
 
 int plain_gemm(int m, int n, int k, const double* A, long long lda, const double* B, long long ldb, double* C,
                long long ldc, cudaStream_t st) {
-  if (m <= 0 || n <= 0 || k <= 0) return FMM_OK;
-  DevTables* d = nullptr;
-  int rc = device_tables(classical_plan(), &d);
-  if (rc != FMM_OK) return rc;
-  int dev = 0;
-  rc = configure_kernel(&dev);
-  if (rc != FMM_OK) return rc;
-  const int S = call_ksplit(classical_plan(), m, n, k, false, k, sm_count[dev]);
-  if (S > 1) {
-    const fmm::Prod* vp = nullptr;
-    const fmm::Term* vt = nullptr;
-    rc = ksplit_tables(classical_plan(), BASE_ORIG, S, &vp, &vt);
-    if (rc != FMM_OK) return rc;
-    return launch_gemm(K_GEMM_CLASSICAL, vp, vt, kUnitGrid, S, fmm::MODE_ACCUM_C, A, lda, B, ldb, PresumOps{}, C,
-                       ldc, nullptr, 0, 0, m, n, k, st, true, -1, S);
-  }
-  return launch_gemm(K_GEMM_CLASSICAL, d->prods, d->terms, kUnitGrid, 1, fmm::MODE_ACCUM_C, A, lda, B, ldb,
-                     PresumOps{}, C, ldc, nullptr, 0, 0, m, n, k, st, true);
+  const GemmJob j{m, n, k, A, lda, B, ldb, C, ldc};
+  return tile_gemm(&j, 1, st);
 }
 
 int grid_for(long long total, int threads) {
@@ -887,32 +922,17 @@ int grid_for(long long total, int threads) {
   return (int)b;
 }
 
-// Blocks along the element dimension of fmm_lincomb_kernel (each covers LINCOMB_CHUNK
-// row pairs; beyond the grid limit the blocks loop).
-unsigned lincomb_chunks(long long pairs) {
-  const long long c = (pairs + fmm::LINCOMB_CHUNK - 1) / fmm::LINCOMB_CHUNK;
-  return (unsigned)std::max<long long>(1, std::min<long long>(c, 65535));
-}
-
-// Fringe GEMMs, same regions and order as the reference's dynamic peeling.
+// Fringe GEMMs, the regions of the reference's dynamic peeling: the k strip updates the core's
+// C, the n strip the last columns, the m strip the last rows; the three are disjoint in C, so
+// one launch covers them.
 int peel(int m, int n, int k, const double* A, long long lda, const double* B, long long ldb, double* C,
          long long ldc, int dim1, int dim2, int dim3, cudaStream_t st) {
   const int mr = m % dim1, kr = k % dim2, nr = n % dim3;
   const int ms = m - mr, ns = n - nr, ks = k - kr;
-  int rc = FMM_OK;
-  if (kr > 0 && ms > 0 && ns > 0) {
-    rc = plain_gemm(ms, ns, kr, A + (long long)ks * lda, lda, B + ks, ldb, C, ldc, st);
-    if (rc != FMM_OK) return rc;
-  }
-  if (nr > 0) {
-    rc = plain_gemm(m, nr, k, A, lda, B + (long long)ns * ldb, ldb, C + (long long)ns * ldc, ldc, st);
-    if (rc != FMM_OK) return rc;
-  }
-  if (mr > 0 && ns > 0) {
-    rc = plain_gemm(mr, ns, k, A + ms, lda, B, ldb, C + ms, ldc, st);
-    if (rc != FMM_OK) return rc;
-  }
-  return FMM_OK;
+  const GemmJob jobs[3] = {{m, nr, k, A, lda, B + (long long)ns * ldb, ldb, C + (long long)ns * ldc, ldc},
+                           {mr, ns, k, A + ms, lda, B, ldb, C + ms, ldc},
+                           {ms, ns, kr, A + (long long)ks * lda, lda, B + ks, ldb, C, ldc}};
+  return tile_gemm(jobs, 3, st);
 }
 
 // C_l += sum_r W[l,r] * M_r for every C block at once (fmm_combine_kernel); false when the
@@ -975,10 +995,9 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(ntile, (long long)sm_count[dev] * 3));
     {
       ProfScope pf(K_COMBINE, st);
-      fmm::fmm_combine_staged_kernel<<<grid, fmm::CST_THREADS + 32, ssm, st>>>(ga, dev_status[dev]);
+      return launch_dependent(fmm::fmm_combine_staged_kernel, dim3(grid), fmm::CST_THREADS + 32, ssm, st, 1, ga,
+                              dev_status[dev]);
     }
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    return cuda_status(cudaGetLastError());
   }
   const int P = g_combine_positions.load() == 2 ? 2 : 1;
   const size_t smem = fmm::combine_group_smem_bytes(ga.ngroup, ga.nent, ga.ncoef);
@@ -996,35 +1015,29 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
   return cuda_status(cudaGetLastError());
 }
 
-// Pre-summing pays off once the sub-blocks are large enough that the extra pass over HBM
-// (each operand sum written once, then read by every tile that uses it) costs less than
-// folding the sums while staging, which limits the producer warps, and it lets the
-// direct kernel variant run.  Measured on B200 (pre-summed vs folded): 222-1 x 333-1
-// 4096^3 11.7 -> 5.4 ms, 4000 x 3840 x 2000 5.6 -> 3.3 ms, 14400 x 14400 x 480 22.5 ->
-// 19.1 ms; 222-2 2048^3 1.34 -> 0.88 ms; 222-1 1024^3 0.24 -> 0.17 ms (ms * ns = 2^18).
-bool use_presum(const fmm_plan* plan, int ms, int ns, int ks) {
-  if (plan->plistA.empty() && plan->plistB.empty()) return false;
-  return (long long)ms * ns >= (1LL << 17) && ks >= 64;
-}
-
-// ABC schedule for pre-summed products: the multi-destination epilogue (C_l += W[l,r] M_r
-// straight from each product tile) or, when that C traffic dominates, the products stored
-// to a workspace and one combine pass (every M_r and C element crossing HBM once).  The
-// epilogue moves 16 nnz(W) ms ns bytes of C while the DMMAs run; the stored schedule writes
-// 8 R ms ns bytes of product tiles (also during the DMMAs), then the combine pass moves
-// 8 (R + 2 blocks) ms ns bytes.  Model fitted to B200 measurements (222-1 x 333-1, DMMA
-// products 33 TFLOP/s executed, epilogue C traffic 4.6 TB/s, product stores 6 TB/s, combine
-// 2.6 TB/s): the direct launch takes max(t_mma, t_epi) + 1.05 min^2 / max (the two overlap
-// less as they approach each other: 4000 x 16000 x 2000 7.76 ms for t_mma 5.75 and t_epi
-// 3.32, 14400 x 14400 x 480 12.4 ms, 8192^3 24.2 ms), the storing launch 1.08 max(t_mma,
-// t_store) (6.16 and 4.92 ms).  The stored schedule must gain 3 % and its product workspace
-// (8 R ms ns bytes) must fit the workspace cap.  It is the reference's own trade between its
-// ABC and AB variants (meta/model_gen.py:87-95 counts the C memory operations of each).
-bool prefer_stored_products(const fmm_plan* plan, int ms, int ns, int ks) {
+// ABC schedule: the multi-destination epilogue (C_l += W[l,r] M_r straight from each product
+// tile, ordered by tickets) or the products stored to a workspace and one combine pass (every
+// M_r and C element crossing HBM once).
+//   * Few tiles: when a product has no more tiles than CTAs run at a time, the units of one
+//     tile run together and their ordered C updates form a chain; storing has none.  Measured
+//     us direct / stored: 222-1 1024^3 119 / 97, 2048^3 542 / 544; 222-2 1024^3 189 / 112, 4096^3
+//     3484 / 3456; 222-1 x 333-1 528^3 200 / 67, 2016^3 1165 / 673, 4128^3 4248 / 3982.
+//   * C traffic: the epilogue moves 16 nnz(W) ms ns bytes of C while the DMMAs run, the stored
+//     schedule 8 R ms ns while they run and 8 (R + 2 blocks) ms ns in the combine.  Model
+//     (products 35 TFLOP/s, epilogue C traffic 4.6 TB/s, product stores 6 TB/s, combine 2.6
+//     TB/s): the direct launch takes max(t_mma, t_epi) + 1.05 min^2 / max, the storing launch
+//     1.08 max(t_mma, t_store); storing must gain 3 %.  Measured ms direct / stored: 222-1 x
+//     333-1 4000 x 16000 x 2000 8.83 / 7.81, 222-1 8192 x 8192 x 512 2.12 / 2.22, 8192^3 27.7 /
+//     28.0.
+// The product workspace (8 R ms ns bytes) must fit the workspace cap.  It is the reference's
+// own trade between its ABC and AB variants (meta/model_gen.py:87-95 counts the C memory
+// operations of each).  Both schedules give the same bits.
+bool prefer_stored_products(const fmm_plan* plan, int ms, int ns, int ks, int nsm) {
   const double mn = (double)ms * ns;
   const int nblk = plan->dims[0] * plan->dims[2];
-  if (8.0 * plan->rank * mn > (double)g_ws_limit.load()) return false;
-  const double t_mma = 2.0 * plan->rank * mn * ks / 33e12;
+  if (plan->rank < 2 || 8.0 * plan->rank * mn > (double)g_ws_limit.load()) return false;
+  if (tiles_of(ms, ns, 64) <= kResident64 * (long long)nsm) return true;
+  const double t_mma = 2.0 * plan->rank * mn * ks / 35e12;
   const double t_epi = 16.0 * plan->n_cterms * mn / 4.6e12;
   const double t_store = 8.0 * plan->rank * mn / 6.0e12;
   const double t_comb = 8.0 * (plan->rank + 2.0 * nblk) * mn / 2.6e12;
@@ -1033,217 +1046,135 @@ bool prefer_stored_products(const fmm_plan* plan, int ms, int ns, int ks) {
   return 1.08 * std::max(t_mma, t_store) + t_comb < 0.97 * t_direct;
 }
 
-// One operand's sums (fmm_lincomb_kernel): output j = blockIdx.x, element chunks over y.
-int launch_lincomb(const fmm_plan* plan, const fmm::LincombArgs& la, int nout, cudaStream_t st) {
-  (void)plan;
-  if (nout <= 0) return FMM_OK;
-  const long long pairs = (long long)(la.rows + 1) / 2 * la.cols;
-  {
-    ProfScope pf(K_LINCOMB, st);
-    fmm::fmm_lincomb_kernel<<<dim3((unsigned)nout, lincomb_chunks(pairs)), 256, 0, st>>>(la);
-  }
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cuda_status(cudaGetLastError());
-}
-
-int presum(const fmm_plan* plan, const DevTables& d, const double* A, long long lda, const double* B, long long ldb,
-           const PresumOps& ps, int ms, int ns, int ks, cudaStream_t st) {
-  if (ps.nslotA > 0) {
-    fmm::LincombArgs la{};
-    la.X = A;
-    la.ldx = lda;
-    la.rows = ms;
-    la.cols = ks;
-    la.blk_row_stride = ms;
-    la.blk_col_stride = ks;
-    la.out = const_cast<double*>(ps.S);
-    la.ldo = ps.ldS;
-    la.out_stride = ps.ldS * (ps.kslot ? ps.kslot : ks);
-    la.prods = d.prods;
-    la.terms = d.terms;
-    la.plist = ps.plistA ? ps.plistA : d.plistA;
-    la.side = 0;
-    const int rc = launch_lincomb(plan, la, ps.nslotA, st);
-    if (rc != FMM_OK) return rc;
-  }
-  if (ps.nslotB > 0) {
-    fmm::LincombArgs lb{};
-    lb.X = B;
-    lb.ldx = ldb;
-    lb.rows = ks;
-    lb.cols = ns;
-    lb.blk_row_stride = ks;
-    lb.blk_col_stride = ns;
-    lb.out = const_cast<double*>(ps.T);
-    lb.ldo = ps.ldT;
-    lb.out_stride = ps.ldT * ns;
-    lb.prods = d.prods;
-    lb.terms = d.terms;
-    lb.plist = ps.plistB ? ps.plistB : d.plistB;
-    lb.side = 1;
-    const int rc = launch_lincomb(plan, lb, ps.nslotB, st);
-    if (rc != FMM_OK) return rc;
-  }
-  return cuda_status(cudaGetLastError());
-}
-
-// Pre-summed operands for the products of one call: the workspace, the operand sums and the
-// tables the products kernel reads them with.  When ks is not a multiple of the k step every
-// product gets its own slot whose k extent is padded with zeros (kk = ks rounded up), so all
-// k steps stay inside the slot and the direct variant can run.
+// The pre-summed form of one call: which operands get slots, the tables the products kernel
+// reads them with, and the workspace.  With k per product a whole number of k groups and both
+// operands readable by tensor copies, single-block operands are read in place and only sums
+// get slots; otherwise (or when every sum is wanted) every product gets a slot of its own,
+// whose k extent is rounded up with zeros.
 struct PresumPlan {
-  PresumOps ps;
-  const fmm::Prod* prods = nullptr;
-  const fmm::Term* terms = nullptr;
-  int kk = 0;
-  char* ws = nullptr;
+  bool all = false;
+  int kk = 0;                // k depth of the products
+  int nA = 0, nB = 0;        // slots
+  long long ldS = 0, ldT = 0;
+  size_t s_bytes = 0, t_bytes = 0;
 };
 
-int presum_prepare(const fmm_plan* plan, const DevTables& d, const double* A, long long lda, const double* B,
-                   long long ldb, int ms, int ns, int ks, cudaStream_t st, PresumPlan* out) {
-  const int R = plan->rank;
-  PresumOps& ps = out->ps;
-  int rc = FMM_OK;
-  if (ks % fmm::BK != 0) {
-    const int kp = (ks + fmm::BK - 1) / fmm::BK * fmm::BK;
-    ps.plistA = d.plist_all;
-    ps.plistB = d.plist_all;
-    ps.kslot = kp;
-    const size_t sbytes = sizeof(double) * (size_t)ms * kp * R;
-    const size_t tbytes = sizeof(double) * (size_t)kp * ns * R;
-    FMM_CUDA_TRY(cudaMallocAsync((void**)&out->ws, sbytes + tbytes + 16, st));
-    ps.S = reinterpret_cast<double*>(out->ws);
-    ps.ldS = ms;
-    ps.nslotA = R;
-    ps.T = reinterpret_cast<double*>(out->ws + sbytes);
-    ps.ldT = kp;
-    ps.nslotB = R;
-    // zero padding: S slot r columns [ks, kp); T rows [ks, kp) of every column
-    rc = cuda_status(cudaMemset2DAsync(out->ws + sizeof(double) * (size_t)ms * ks, sizeof(double) * (size_t)ms * kp,
-                                       0, sizeof(double) * (size_t)ms * (kp - ks), R, st));
-    if (rc == FMM_OK)
-      rc = cuda_status(cudaMemset2DAsync(out->ws + sbytes + sizeof(double) * ks, sizeof(double) * kp, 0,
-                                         sizeof(double) * (kp - ks), (size_t)R * ns, st));
-    out->prods = d.prods_all;
-    out->terms = d.terms_all;
-    out->kk = kp;
-  } else {
-    const int nA = (int)plan->plistA.size(), nB = (int)plan->plistB.size();
-    const long long ldT = ks + (ks & 1);
-    const size_t sbytes = sizeof(double) * (size_t)ms * ks * nA;
-    const size_t tbytes = sizeof(double) * (size_t)ldT * ns * nB;
-    FMM_CUDA_TRY(cudaMallocAsync((void**)&out->ws, sbytes + tbytes + 16, st));
-    ps.S = reinterpret_cast<double*>(out->ws);
-    ps.ldS = ms;
-    ps.nslotA = nA;
-    ps.T = reinterpret_cast<double*>(out->ws + sbytes);
-    ps.ldT = ldT;
-    ps.nslotB = nB;
-    out->prods = d.prods_ps;
-    out->terms = d.terms_ps;
-    out->kk = ks;
-  }
-  if (rc == FMM_OK) rc = presum(plan, d, A, lda, B, ldb, ps, ms, ns, ks, st);
-  return rc;
+PresumPlan presum_plan(const fmm_plan* plan, int ms, int ns, int ks, bool all) {
+  PresumPlan pp;
+  pp.all = all || !whole_k_steps(plan, ks);
+  pp.kk = pp.all ? (ks + 7) / 8 * 8 : ks;
+  pp.nA = pp.all ? plan->rank : (int)plan->plistA.size();
+  pp.nB = pp.all ? plan->rank : (int)plan->plistB.size();
+  pp.ldS = (ms + 1) / 2 * 2;
+  pp.ldT = (pp.kk + 1) / 2 * 2;
+  pp.s_bytes = (sizeof(double) * (size_t)pp.ldS * pp.kk * pp.nA + 255) & ~(size_t)255;
+  pp.t_bytes = (sizeof(double) * (size_t)pp.ldT * ns * pp.nB + 255) & ~(size_t)255;
+  return pp;
 }
 
-// Bytes presum_prepare would allocate for one call.
-size_t presum_bytes(const fmm_plan* plan, int ms, int ns, int ks) {
-  if (ks % fmm::BK != 0) {
-    const size_t kp = (ks + fmm::BK - 1) / fmm::BK * fmm::BK;
-    return sizeof(double) * kp * ((size_t)ms + ns) * plan->rank + 16;
-  }
-  return sizeof(double) * ((size_t)ms * ks * plan->plistA.size() + (size_t)(ks + (ks & 1)) * ns * plan->plistB.size()) +
-         16;
+// One side's sums of products plist[0 .. n) into `out`.
+fmm::PresumSide presum_side(const DevTables& d, int side, const double* X, long long ldx, int ms, int ns, int ks, int kk,
+                            double* out, long long ldo, const int* plist, int n) {
+  fmm::PresumSide p{};
+  p.X = X;
+  p.ldx = ldx;
+  p.rows = side == 0 ? ms : ks;
+  p.cols = side == 0 ? ks : ns;
+  p.orows = (int)ldo;  // even; the pitch element of an odd row count is a zero
+  p.ocols = side == 0 ? kk : ns;
+  p.blk_row_stride = p.rows;
+  p.blk_col_stride = p.cols;
+  p.out = out;
+  p.ldo = ldo;
+  p.out_stride = ldo * p.ocols;
+  p.plist = plist;
+  p.first = d.ps_first[side];
+  p.terms = d.ps_terms[side];
+  p.nout = n;
+  return p;
 }
 
-// The k split a single call gives products of ms x ks x ns: the pre-summed direct launch
-// (unless the call stores its products or runs them in workspace groups) and the classical
-// plan split as choose_ksplit decides; other forms keep S = 1.  Batches apply the same split
-// per job.
-int call_ksplit(const fmm_plan* plan, int ms, int ns, int ks, bool presum, int kk, int nsm) {
-  const long long tiles = (long long)((ms + fmm::BM - 1) / fmm::BM) * ((ns + fmm::BN - 1) / fmm::BN);
-  if (plan->rank == 1) return choose_ksplit(tiles, ks, nsm);
-  if (!presum) return 1;
-  if (combine_fits(plan) && prefer_stored_products(plan, ms, ns, ks)) return 1;
-  if ((long long)presum_bytes(plan, ms, ns, ks) > g_ws_limit.load()) return 1;
-  return choose_ksplit(tiles * plan->rank, kk, nsm);
+// Terms of the larger side and the output ranges per position chunk: enough CTAs to fill the
+// SMs several times, else one CTA walks all its outputs so that they share its input values.
+int presum_cap(const fmm_plan* plan) {
+  return (int)std::min<size_t>(fmm::PS_TERMS, std::max(plan->ps_terms[0].size(), plan->ps_terms[1].size()));
 }
+unsigned presum_ranges(long long chunks, int nout, int nsm) {
+  long long y = (8LL * nsm + chunks - 1) / std::max<long long>(1, chunks);
+  return (unsigned)std::max<long long>(1, std::min<long long>(y, nout));
+}
+
+// Both sides' sums; zero[0 .. nzero) is cleared too (with no sums to make, by a memset).
+int launch_presum(const fmm_plan* plan, const fmm::PresumSide& a, const fmm::PresumSide& b, int* zero, long long nzero,
+                  int nsm, cudaStream_t st) {
+  if (a.nout == 0 && b.nout == 0)
+    return nzero > 0 ? cuda_status(cudaMemsetAsync(zero, 0, sizeof(int) * nzero, st)) : FMM_OK;
+  if (nzero > INT32_MAX) return FMM_E_UNSUPPORTED;
+  fmm::PresumArgs g{};
+  g.s[0] = a;
+  g.s[1] = b;
+  g.zero = zero;
+  g.nzero = (int)nzero;
+  g.cap = presum_cap(plan);
+  const long long ca = (long long)(a.orows / 2) * a.ocols, cb = (long long)(b.orows / 2) * b.ocols;
+  const long long nc = (std::max(a.nout ? ca : 0, b.nout ? cb : 0) + fmm::PS_THREADS - 1) / fmm::PS_THREADS;
+  const unsigned gx = (unsigned)std::max<long long>(1, std::min<long long>(nc, INT32_MAX));
+  ProfScope pf(K_PRESUM, st);
+  return launch_dependent(fmm::fmm_presum_kernel, dim3(gx, presum_ranges(nc, std::max(a.nout, b.nout), nsm), 2),
+                          fmm::PS_THREADS, sizeof(fmm::PresumOff) * g.cap, st, 1, g);
+}
+
+// Bytes of the pre-summed workspace of one call.
+size_t presum_bytes(const PresumPlan& pp) { return pp.s_bytes + pp.t_bytes; }
 
 // Pre-summed products in groups, when one call's whole operand workspace would exceed the
 // workspace limit: the R products run as groups of G consecutive products, each group's
-// operand sums (one slot per product, k extent padded to whole k steps) formed into one of
-// two workspace halves while the previous group's products run.  The sums go on a second
-// stream, which waits for the products that last read that half; each group's products
-// wait for their sums.  Groups run in product order on the caller's stream, so every C
-// element still receives its products' updates in order r = 0..R-1 (results are those of
-// the ungrouped call).  Workspace 2 G (ms + ns) kk 8 bytes, within the limit for G >= 1.
+// operand sums (one slot per product, k extent padded to whole k groups) formed in the one
+// workspace before its products run.  (Two half-size buffers with the next group's sums on a
+// second stream measured slower: the products' CTAs fill the SMs, so the sums ran between the
+// products launches all the same, and twice the groups read A and B twice as often: 16384^3
+// 222-1 x 333-1 200.6 ms.)  Groups run in product order, so every C element still receives its
+// products' updates in order r = 0..R-1 (results are those of the ungrouped call).  Workspace
+// G (ms + ns) kk 8 bytes, within the limit for G >= 1.
 int run_presum_groups(const fmm_plan* plan, const DevTables& d, const double* A, long long lda, const double* B,
-                      long long ldb, double* C, long long ldc, int ms, int ns, int ks, cudaStream_t st) {
+                      long long ldb, double* C, long long ldc, int ms, int ns, int ks, int nsm, cudaStream_t st) {
   const int R = plan->rank;
-  const int kk = (ks + fmm::BK - 1) / fmm::BK * fmm::BK;
-  const size_t sb = sizeof(double) * (size_t)ms * kk, tb = sizeof(double) * (size_t)kk * ns;
-  long long G = g_ws_limit.load() / (long long)(2 * (sb + tb));
+  const int kk = (ks + 7) / 8 * 8;
+  const long long ldS = (ms + 1) / 2 * 2;
+  const size_t sb = sizeof(double) * (size_t)ldS * kk, tb = sizeof(double) * (size_t)kk * ns;
+  long long G = g_ws_limit.load() / (long long)(sb + tb);
   G = std::max<long long>(1, std::min<long long>(G, R));
   const int ng = (int)((R + G - 1) / G);
-  const int nbuf = ng > 1 ? 2 : 1;
-  const size_t half = (size_t)G * (sb + tb);
+  G = (R + ng - 1) / ng;  // even groups
+  const ProdLaunch L = plan_products(plan->dims, (int)G, fmm::MODE_ACCUM_C, ms, ns, nsm);
+  const size_t tk = (sizeof(int) * (1 + L.tickets) + 255) & ~(size_t)255;
   char* ws = nullptr;
-  FMM_CUDA_TRY(cudaMallocAsync((void**)&ws, nbuf * half + 16, st));
-  t_last_ws = (long long)(nbuf * half);
+  FMM_CUDA_TRY(cudaMallocAsync((void**)&ws, G * (sb + tb) + tk, st));
+  t_last_ws = (long long)(G * (sb + tb));
+  int* counter = reinterpret_cast<int*>(ws);
   int rc = FMM_OK;
-  auto ok = [&](cudaError_t e) {
-    if (rc == FMM_OK && e != cudaSuccess) rc = cuda_status(e);
-    return rc == FMM_OK;
-  };
-  // zero padding once per half: S slot columns [ks, kk), T slot rows [ks, kk) (the sums fill [0, ks))
-  for (int b = 0; b < nbuf && kk != ks; ++b) {
-    char* S = ws + b * half;
-    ok(cudaMemset2DAsync(S + sizeof(double) * (size_t)ms * ks, sb, 0, sizeof(double) * (size_t)ms * (kk - ks), G,
-                         st)) &&
-        ok(cudaMemset2DAsync(S + G * sb + sizeof(double) * ks, sizeof(double) * kk, 0, sizeof(double) * (kk - ks),
-                             (size_t)G * ns, st));
-  }
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_start = nullptr, ev_sum[2] = {nullptr, nullptr}, ev_done[2] = {nullptr, nullptr};
-  ok(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking)) &&
-      ok(cudaEventCreateWithFlags(&ev_start, cudaEventDisableTiming)) &&
-      ok(cudaEventCreateWithFlags(&ev_sum[0], cudaEventDisableTiming)) &&
-      ok(cudaEventCreateWithFlags(&ev_sum[1], cudaEventDisableTiming)) &&
-      ok(cudaEventCreateWithFlags(&ev_done[0], cudaEventDisableTiming)) &&
-      ok(cudaEventCreateWithFlags(&ev_done[1], cudaEventDisableTiming)) && ok(cudaEventRecord(ev_start, st)) &&
-      ok(cudaStreamWaitEvent(side, ev_start, 0));
-  for (int g = 0; g < ng && rc == FMM_OK; ++g) {
-    const int g0 = (int)(g * G), g1 = (int)std::min<long long>(R, (g + 1) * G), n = g1 - g0, b = g % 2;
-    char* S = ws + b * half;
+  for (int g0 = 0; g0 < R && rc == FMM_OK; g0 += (int)G) {
+    const int g1 = (int)std::min<long long>(R, g0 + G), n = g1 - g0;
     PresumOps ps;
-    ps.plistA = d.plist_all + g0;
-    ps.plistB = d.plist_all + g0;
     ps.kslot = kk;
-    ps.S = reinterpret_cast<const double*>(S);
-    ps.ldS = ms;
+    ps.S = reinterpret_cast<double*>(ws + tk);
+    ps.ldS = ldS;
     ps.nslotA = n;
-    ps.T = reinterpret_cast<const double*>(S + G * sb);
+    ps.T = reinterpret_cast<double*>(ws + tk + G * sb);
     ps.ldT = kk;
     ps.nslotB = n;
-    if (g >= 2 && !ok(cudaStreamWaitEvent(side, ev_done[b], 0))) break;
-    rc = presum(plan, d, A, lda, B, ldb, ps, ms, ns, ks, side);
-    if (!ok(cudaEventRecord(ev_sum[b], side)) || !ok(cudaStreamWaitEvent(st, ev_sum[b], 0))) break;
+    rc = launch_presum(plan, presum_side(d, 0, A, lda, ms, ns, ks, kk, ps.S, ps.ldS, d.plist_all + g0, n),
+                       presum_side(d, 1, B, ldb, ms, ns, ks, kk, ps.T, ps.ldT, d.plist_all + g0, n), counter,
+                       1 + (long long)L.tickets, nsm, st);
     const fmm::Prod* gp = nullptr;
     const fmm::Term* gt = nullptr;
     if (rc == FMM_OK) rc = ksplit_tables(plan, BASE_GROUP, g0, &gp, &gt, g1);
     if (rc == FMM_OK)
-      rc = launch_gemm(K_GEMM_FMM, gp, gt, plan->dims, n, fmm::MODE_ACCUM_C, A, lda, B, ldb, ps, C, ldc, nullptr, 0,
-                       0, ms, ns, kk, st, true, ks);
-    if (rc == FMM_OK) ok(cudaEventRecord(ev_done[b], st));
+      rc = launch_products(gp, gt, plan->dims, n, fmm::MODE_ACCUM_C, A, lda, B, ldb, ps, C, ldc, nullptr, ms, ns, ks,
+                           kk, L, counter, st);
   }
-  // every sum was waited for by the caller's stream, so freeing there comes after all uses
   cudaError_t fe = cudaFreeAsync(ws, st);
-  if (rc == FMM_OK) rc = cuda_status(fe);
-  for (cudaEvent_t e : {ev_start, ev_sum[0], ev_sum[1], ev_done[0], ev_done[1]})
-    if (e) cudaEventDestroy(e);
-  if (side) cudaStreamDestroy(side);
-  return rc;
+  return rc == FMM_OK ? cuda_status(fe) : rc;
 }
 
 int check_args(int m, int n, int k, const void* A, long long lda, const void* B, long long ldb, const void* C,
@@ -1255,6 +1186,87 @@ int check_args(int m, int n, int k, const void* A, long long lda, const void* B,
   return FMM_OK;
 }
 
+bool is_classical(const fmm_plan* p) {
+  return p->rank == 1 && p->dims[0] == 1 && p->dims[1] == 1 && p->dims[2] == 1 && p->plistA.empty() &&
+         p->plistB.empty() && p->prods[0].nc == 1 && p->terms[p->prods[0].c0].coef == 1.0;
+}
+
+// The FMM core: sub-blocks ms x ks x ns, every dimension a whole number of them.
+//   abc: operand sums in HBM, then every product either added to its C blocks as it is made
+//        (tickets keep each C element's updates in product order) or, where that C traffic or
+//        the launch's few units dominate, stored and applied by one combine pass;
+//   ab, naive: the products stored, W applied by the combine pass (naive makes a temporary
+//        of every operand).
+int run_core(const fmm_plan* plan, int pack, const double* A, long long lda, const double* B, long long ldb, double* C,
+             long long ldc, int ms, int ns, int ks, cudaStream_t st) {
+  DevTables* d = nullptr;
+  int rc = device_tables(plan, &d);
+  if (rc != FMM_OK) return rc;
+  int dev = 0;
+  rc = configure_kernel(&dev);
+  if (rc != FMM_OK) return rc;
+  const int R = plan->rank, nsm = sm_count[dev];
+  // operands a tensor copy cannot read in place (odd leading dimension, unaligned base) all get slots
+  CUtensorMap probe;
+  const bool in_place = make_a_map(&probe, A, (long long)plan->dims[0] * ms, (long long)plan->dims[1] * ks, lda) &&
+                        make_b_map(&probe, B, (long long)plan->dims[1] * ks, (long long)plan->dims[2] * ns, ldb, 64);
+  const PresumPlan pp = presum_plan(plan, ms, ns, ks, pack == FMM_PACK_NAIVE || !in_place);
+  const bool stored = pack != FMM_PACK_ABC || (g_ticket_fill == 0 && combine_fits(plan) && prefer_stored_products(plan, ms, ns, ks, nsm));
+  if (!stored && (long long)presum_bytes(pp) > g_ws_limit.load())
+    return run_presum_groups(plan, *d, A, lda, B, ldb, C, ldc, ms, ns, ks, nsm, st);  // workspace within the limit
+  const int mode = stored ? fmm::MODE_STORE_M : fmm::MODE_ACCUM_C;
+  const ProdLaunch L = plan_products(plan->dims, R, mode, ms, ns, nsm);
+  const size_t tk = (sizeof(int) * (1 + L.tickets) + 255) & ~(size_t)255;
+  const size_t mb = stored ? sizeof(double) * (size_t)ms * ns * R : 0;
+  char* ws = nullptr;
+  FMM_CUDA_TRY(cudaMallocAsync((void**)&ws, tk + presum_bytes(pp) + mb, st));
+  t_last_ws = (long long)presum_bytes(pp);
+  int* counter = reinterpret_cast<int*>(ws);
+  double* M = stored ? reinterpret_cast<double*>(ws + tk + presum_bytes(pp)) : nullptr;
+  PresumOps ps;
+  ps.plistA = pp.all ? d->plist_all : d->plistA;
+  ps.plistB = pp.all ? d->plist_all : d->plistB;
+  ps.kslot = pp.kk;
+  ps.S = reinterpret_cast<double*>(ws + tk);
+  ps.ldS = pp.ldS;
+  ps.nslotA = pp.nA;
+  ps.T = reinterpret_cast<double*>(ws + tk + pp.s_bytes);
+  ps.ldT = pp.ldT;
+  ps.nslotB = pp.nB;
+  rc = launch_presum(plan, presum_side(*d, 0, A, lda, ms, ns, ks, pp.kk, ps.S, ps.ldS, ps.plistA, ps.nslotA),
+                     presum_side(*d, 1, B, ldb, ms, ns, ks, pp.kk, ps.T, ps.ldT, ps.plistB, ps.nslotB), counter,
+                     1 + (long long)L.tickets, nsm, st);
+  if (rc == FMM_OK && g_ticket_fill != 0 && L.tickets > 0)
+    rc = cuda_status(cudaMemsetAsync(counter + 1, g_ticket_fill, sizeof(int) * L.tickets, st));
+  if (rc == FMM_OK)
+    rc = launch_products(pp.all ? d->prods_all : d->prods_ps, pp.all ? d->terms_all : d->terms_ps, plan->dims, R, mode, A,
+                         lda, B, ldb, ps, C, ldc, M, ms, ns, ks, pp.kk, L, counter, st);
+  if (rc == FMM_OK && stored && combine_fits(plan)) {
+    rc = launch_combine(plan, *d, C, ldc, ms, ns, M, ms, (long long)ms * ns, st);
+  } else if (rc == FMM_OK && stored) {
+    fmm::ScatterArgs sa{};
+    sa.C = C;
+    sa.ldc = ldc;
+    sa.ms = ms;
+    sa.ns = ns;
+    sa.M = M;
+    sa.ldm = ms;
+    sa.m_stride = (long long)ms * ns;
+    sa.cblk = d->cblk;
+    sa.ent_r = d->ent_r;
+    sa.ent_w = d->ent_w;
+    const dim3 gs((unsigned)grid_for(sa.m_stride, 256), (unsigned)plan->n_cblk);
+    {
+      ProfScope pf(K_SCATTER, st);
+      fmm::fmm_scatter_kernel<<<gs, 256, 0, st>>>(sa);
+    }
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    rc = cuda_status(cudaGetLastError());
+  }
+  cudaError_t fe = cudaFreeAsync(ws, st);
+  return rc == FMM_OK ? cuda_status(fe) : rc;
+}
+
 int run_fmm(const fmm_plan* plan, int pack, int m, int n, int k, const double* A, long long lda, const double* B,
             long long ldb, double* C, long long ldc, cudaStream_t st) {
   if (!plan) return FMM_E_NOPLAN;
@@ -1262,154 +1274,13 @@ int run_fmm(const fmm_plan* plan, int pack, int m, int n, int k, const double* A
   int rc = check_args(m, n, k, A, lda, B, ldb, C, ldc);
   if (rc != FMM_OK) return rc;
   if (m == 0 || n == 0 || k == 0) return FMM_OK;
+  t_last_ws = 0;
+  if (is_classical(plan)) return plain_gemm(m, n, k, A, lda, B, ldb, C, ldc, st);
   const int pm = plan->dims[0] * kMR, pk = plan->dims[1], pn = plan->dims[2] * kNR;
   const int md = m - m % pm, kd = k - k % pk, nd = n - n % pn;
-  const int ms = md / plan->dims[0], ks = kd / plan->dims[1], ns = nd / plan->dims[2];
-  DevTables* d = nullptr;
-  rc = device_tables(plan, &d);
-  if (rc != FMM_OK) return rc;
-  const int R = plan->rank;
-  t_last_ws = 0;
-  if (ms > 0 && ns > 0 && ks > 0) {
-    if (pack == FMM_PACK_ABC) {
-      const int nA = (int)plan->plistA.size(), nB = (int)plan->plistB.size();
-      if (use_presum(plan, ms, ns, ks) && combine_fits(plan) && prefer_stored_products(plan, ms, ns, ks)) {
-        // C-traffic-bound shapes (small k per product): operand sums in HBM, each product
-        // stored by the direct variant, W applied by one combine pass
-        const long long mstride = (long long)ms * ns;
-        char* mws = nullptr;
-        FMM_CUDA_TRY(cudaMallocAsync((void**)&mws, sizeof(double) * (size_t)mstride * R, st));
-        double* M = reinterpret_cast<double*>(mws);
-        PresumPlan pp;
-        t_last_ws = (long long)presum_bytes(plan, ms, ns, ks);
-        rc = presum_prepare(plan, *d, A, lda, B, ldb, ms, ns, ks, st, &pp);
-        if (rc == FMM_OK)
-          rc = launch_gemm(K_GEMM_FMM, pp.prods, pp.terms, plan->dims, R, fmm::MODE_STORE_M, A, lda, B, ldb, pp.ps,
-                           C, ldc, M, ms, mstride, ms, ns, pp.kk, st, true, ks);
-        if (rc == FMM_OK) rc = launch_combine(plan, *d, C, ldc, ms, ns, M, ms, mstride, st);
-        if (pp.ws) {
-          cudaError_t fe = cudaFreeAsync(pp.ws, st);
-          if (rc == FMM_OK) rc = cuda_status(fe);
-        }
-        cudaError_t fe = cudaFreeAsync(mws, st);
-        if (rc == FMM_OK) rc = cuda_status(fe);
-      } else if (use_presum(plan, ms, ns, ks) && (long long)presum_bytes(plan, ms, ns, ks) > g_ws_limit.load()) {
-        rc = run_presum_groups(plan, *d, A, lda, B, ldb, C, ldc, ms, ns, ks, st);  // workspace within the limit
-      } else if (use_presum(plan, ms, ns, ks)) {
-        // U/V sums formed once per product in HBM (bandwidth-bound), then every
-        // product reads single operands; products scattered into C in the epilogue.
-        t_last_ws = (long long)presum_bytes(plan, ms, ns, ks);
-        PresumPlan pp;
-        rc = presum_prepare(plan, *d, A, lda, B, ldb, ms, ns, ks, st, &pp);
-        const int S = call_ksplit(plan, ms, ns, ks, true, pp.kk, sm_count_current());
-        const fmm::Prod* vp = pp.prods;
-        const fmm::Term* vt = pp.terms;
-        if (rc == FMM_OK && S > 1) rc = ksplit_tables(plan, pp.kk != ks ? BASE_ALL : BASE_PS, S, &vp, &vt);
-        if (rc == FMM_OK)
-          rc = launch_gemm(K_GEMM_FMM, vp, vt, plan->dims, R * S, fmm::MODE_ACCUM_C, A, lda, B, ldb, pp.ps, C, ldc,
-                           nullptr, 0, 0, ms, ns, pp.kk, st, true, ks, S);
-        if (pp.ws) {
-          cudaError_t fe = cudaFreeAsync(pp.ws, st);
-          if (rc == FMM_OK) rc = cuda_status(fe);
-        }
-      } else {
-        rc = launch_gemm(K_GEMM_FMM, d->prods, d->terms, plan->dims, R, fmm::MODE_ACCUM_C, A, lda, B, ldb,
-                         PresumOps{}, C, ldc, nullptr, 0, 0, ms, ns, ks, st);
-      }
-      if (rc != FMM_OK) return rc;
-    } else {
-      const long long mstride = (long long)ms * ns;
-      size_t bytes = sizeof(double) * (size_t)mstride * R;
-      size_t s_bytes = 0, t_bytes = 0;
-      if (pack == FMM_PACK_NAIVE) {
-        s_bytes = sizeof(double) * (size_t)ms * ks * R;
-        t_bytes = sizeof(double) * (size_t)ks * ns * R;
-      }
-      char* ws = nullptr;
-      FMM_CUDA_TRY(cudaMallocAsync((void**)&ws, bytes + s_bytes + t_bytes, st));
-      double* M = reinterpret_cast<double*>(ws);
-      if (pack == FMM_PACK_AB && use_presum(plan, ms, ns, ks)) {
-        // large sub-blocks: operands pre-summed as for ABC, each product stored to M by the
-        // direct variant, W applied by the combine pass below
-        PresumPlan pp;
-        rc = presum_prepare(plan, *d, A, lda, B, ldb, ms, ns, ks, st, &pp);
-        if (rc == FMM_OK)
-          rc = launch_gemm(K_GEMM_FMM, pp.prods, pp.terms, plan->dims, R, fmm::MODE_STORE_M, A, lda, B, ldb, pp.ps,
-                           C, ldc, M, ms, mstride, ms, ns, pp.kk, st, true, ks);
-        if (pp.ws) {
-          cudaError_t fe = cudaFreeAsync(pp.ws, st);
-          if (rc == FMM_OK) rc = cuda_status(fe);
-        }
-      } else if (pack == FMM_PACK_AB) {
-        rc = launch_gemm(K_GEMM_FMM, d->prods, d->terms, plan->dims, R, fmm::MODE_STORE_M, A, lda, B, ldb,
-                         PresumOps{}, C, ldc, M, ms, mstride, ms, ns, ks, st);
-      } else {
-        double* S = reinterpret_cast<double*>(ws + bytes);
-        double* T = reinterpret_cast<double*>(ws + bytes + s_bytes);
-        fmm::LincombArgs la{};
-        la.X = A;
-        la.ldx = lda;
-        la.rows = ms;
-        la.cols = ks;
-        la.blk_row_stride = ms;
-        la.blk_col_stride = ks;
-        la.out = S;
-        la.ldo = ms;
-        la.out_stride = (long long)ms * ks;
-        la.prods = d->prods;
-        la.terms = d->terms;
-        la.side = 0;
-        la.plist = nullptr;
-        rc = launch_lincomb(plan, la, R, st);
-        fmm::LincombArgs lb = la;
-        lb.X = B;
-        lb.ldx = ldb;
-        lb.rows = ks;
-        lb.cols = ns;
-        lb.blk_row_stride = ks;
-        lb.blk_col_stride = ns;
-        lb.out = T;
-        lb.ldo = ks;
-        lb.out_stride = (long long)ks * ns;
-        lb.side = 1;
-        if (rc == FMM_OK) rc = launch_lincomb(plan, lb, R, st);
-        // Product r: M_r = S_r * T_r, with S_r the block (0, r) of an ms x (R*ks) matrix.
-        if (rc == FMM_OK) {
-          DevTables* dc = nullptr;
-          rc = device_tables(classical_plan(), &dc);
-          for (int r = 0; rc == FMM_OK && r < R; ++r) {
-            rc = launch_gemm(K_GEMM_FMM, dc->prods, dc->terms, kUnitGrid, 1, fmm::MODE_STORE_M,
-                             S + (long long)r * ms * ks, ms, T + (long long)r * ks * ns, ks, PresumOps{}, nullptr, 0,
-                             M + (long long)r * mstride, ms, 0, ms, ns, ks, st);
-          }
-        }
-      }
-      if (rc == FMM_OK && combine_fits(plan)) {
-        rc = launch_combine(plan, *d, C, ldc, ms, ns, M, ms, mstride, st);
-      } else if (rc == FMM_OK) {
-        fmm::ScatterArgs sa{};
-        sa.C = C;
-        sa.ldc = ldc;
-        sa.ms = ms;
-        sa.ns = ns;
-        sa.M = M;
-        sa.ldm = ms;
-        sa.m_stride = mstride;
-        sa.cblk = d->cblk;
-        sa.ent_r = d->ent_r;
-        sa.ent_w = d->ent_w;
-        const dim3 gs((unsigned)grid_for(mstride, 256), (unsigned)plan->n_cblk);
-        {
-          ProfScope ps(K_SCATTER, st);
-          fmm::fmm_scatter_kernel<<<gs, 256, 0, st>>>(sa);
-        }
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        rc = cuda_status(cudaGetLastError());
-      }
-      cudaError_t fe = cudaFreeAsync(ws, st);
-      if (rc == FMM_OK) rc = cuda_status(fe);
-      if (rc != FMM_OK) return rc;
-    }
+  if (md > 0 && kd > 0 && nd > 0) {
+    rc = run_core(plan, pack, A, lda, B, ldb, C, ldc, md / plan->dims[0], nd / plan->dims[2], kd / plan->dims[1], st);
+    if (rc != FMM_OK) return rc;
   }
   return peel(m, n, k, A, lda, B, ldb, C, ldc, pm, pk, pn, st);
 }
@@ -1548,56 +1419,6 @@ int run_host(const fmm_plan* plan, int pack, bool plain, int m, int n, int k, co
   return rc;
 }
 
-// Operands whose leading dimension is odd cannot be staged by tensor copies (columns
-// must start on 16 bytes) and fall back to per-thread copies at about half the speed.
-// Large ones are copied once, stream-ordered, into an even-pitch workspace instead
-// (bandwidth-bound, a few percent of the GEMM); small ones stay in place.
-constexpr long long kRepitchMinElems = 1LL << 18;
-
-struct Repitched {
-  const double* A;
-  long long lda;
-  const double* B;
-  long long ldb;
-  char* ws = nullptr;
-};
-
-int repitch(int m, int n, int k, const double* A, long long lda, const double* B, long long ldb, cudaStream_t st,
-            Repitched* out) {
-  out->A = A;
-  out->lda = lda;
-  out->B = B;
-  out->ldb = ldb;
-  const bool a_odd = (lda & 1) && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (long long)m * k >= kRepitchMinElems;
-  const bool b_odd = (ldb & 1) && (reinterpret_cast<uintptr_t>(B) & 15) == 0 && (long long)k * n >= kRepitchMinElems;
-  if (!a_odd && !b_odd) return FMM_OK;
-  const long long pa = m + (m & 1), pb = k + (k & 1);
-  const size_t sa = a_odd ? ((sizeof(double) * (size_t)pa * k + 255) & ~(size_t)255) : 0;
-  const size_t sb = b_odd ? sizeof(double) * (size_t)pb * n : 0;
-  FMM_CUDA_TRY(cudaMallocAsync((void**)&out->ws, sa + sb, st));
-  if (a_odd) {
-    double* dst = reinterpret_cast<double*>(out->ws);
-    fmm::fmm_pitch_copy1_kernel<<<256, 256, 0, st>>>(fmm::PitchCopy{A, lda, dst, pa, m, k});
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    out->A = dst;
-    out->lda = pa;
-  }
-  if (b_odd) {
-    double* dst = reinterpret_cast<double*>(out->ws + sa);
-    fmm::fmm_pitch_copy1_kernel<<<256, 256, 0, st>>>(fmm::PitchCopy{B, ldb, dst, pb, k, n});
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    out->B = dst;
-    out->ldb = pb;
-  }
-  return cuda_status(cudaGetLastError());
-}
-
-int release(Repitched& r, int rc, cudaStream_t st) {
-  if (!r.ws) return rc;
-  cudaError_t e = cudaFreeAsync(r.ws, st);
-  return rc == FMM_OK ? cuda_status(e) : rc;
-}
-
 }  // namespace
 
 extern "C" {
@@ -1634,6 +1455,10 @@ int fmm_plan_destroy(fmm_plan* plan) {
     cudaFree(d.prods_all);
     cudaFree(d.terms_all);
     cudaFree(d.plist_all);
+    for (int side = 0; side < 2; ++side) {
+      cudaFree(d.ps_first[side]);
+      cudaFree(d.ps_terms[side]);
+    }
   }
   for (auto& t : plan->ksplit) {
     cudaFree(t.prods);
@@ -1666,24 +1491,14 @@ fmm_plan* fmm_default_plan(void) {
 
 int fmm_dgemm_dev(const fmm_plan* plan, int pack_type, int m, int n, int k, const double* A, long lda,
                   const double* B, long ldb, double* C, long ldc, void* stream) {
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int rc = check_args(m, n, k, A, lda, B, ldb, C, ldc);
-  if (rc != FMM_OK || m == 0 || n == 0 || k == 0 || !plan) return run_fmm(plan, pack_type, m, n, k, A, lda, B, ldb, C, ldc, st);
-  Repitched r;
-  rc = repitch(m, n, k, A, lda, B, ldb, st, &r);
-  if (rc == FMM_OK) rc = run_fmm(plan, pack_type, m, n, k, r.A, r.lda, r.B, r.ldb, C, ldc, st);
-  return release(r, rc, st);
+  return run_fmm(plan, pack_type, m, n, k, A, lda, B, ldb, C, ldc, static_cast<cudaStream_t>(stream));
 }
 
 int fmm_plain_dgemm_dev(int m, int n, int k, const double* A, long lda, const double* B, long ldb, double* C,
                         long ldc, void* stream) {
   int rc = check_args(m, n, k, A, lda, B, ldb, C, ldc);
   if (rc != FMM_OK || m == 0 || n == 0 || k == 0) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  Repitched r;
-  rc = repitch(m, n, k, A, lda, B, ldb, st, &r);
-  if (rc == FMM_OK) rc = plain_gemm(m, n, k, r.A, r.lda, r.B, r.ldb, C, ldc, st);
-  return release(r, rc, st);
+  return plain_gemm(m, n, k, A, lda, B, ldb, C, ldc, static_cast<cudaStream_t>(stream));
 }
 
 int fmm_dgemm_host(const fmm_plan* plan, int pack_type, int m, int n, int k, const double* A, int lda,
@@ -1946,10 +1761,6 @@ int noalloc_launch(const fmm::Prod* prods, const fmm::Term* terms, const int gri
   a.lda = lda;
   a.B = B;
   a.ldb = ldb;
-  a.Aw = A;
-  a.ldaw = lda;
-  a.Bw = B;
-  a.ldbw = ldb;
   a.C = C;
   a.ldc = ldc;
   a.ms = ms;
@@ -1960,25 +1771,20 @@ int noalloc_launch(const fmm::Prod* prods, const fmm::Term* terms, const int gri
   a.nprod = nprod;
   a.tiles_m = (ms + fmm::BM - 1) / fmm::BM;
   a.tiles_n = (ns + fmm::BN - 1) / fmm::BN;
-  a.mode = fmm::MODE_ACCUM_C;
   a.status = status;
   const int ntiles = a.tiles_m * a.tiles_n;
-  a.chunks = choose_chunks(ntiles, nprod, nsm);
   a.tickets = tickets;
-  if (a.chunks > 1 && ntiles > kNoAllocMaxTiles) return FMM_E_TOO_LARGE;  // tickets of one launch must fit
-  if (a.chunks > 1) FMM_CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(int) * ntiles, st));
+  if (nprod > 1 && ntiles > kNoAllocMaxTiles) return FMM_E_TOO_LARGE;  // tickets of one launch must fit
+  if (nprod > 1) FMM_CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(int) * ntiles, st));
   a.counter = counter;
   FMM_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(int), st));
-  const long long units = (long long)ntiles * a.chunks;
+  const long long units = (long long)ntiles * nprod;
   const unsigned grid = (unsigned)(units < nsm ? units : nsm);
   const long long am = (long long)grid_dims[0] * ms, ak = (long long)grid_dims[1] * ks,
                   bn = (long long)grid_dims[2] * ns;
   const bool tma = make_tensor_map(&a.tmA, A, am, ak, lda, fmm::BM, fmm::BK) &&
                    make_tensor_map(&a.tmB, B, ak, bn, ldb, fmm::BK, fmm::BN) &&
                    make_tensor_map(&a.tmB2, B, ak, bn, ldb, fmm::TB_K, fmm::BN);
-  a.tmAw = a.tmA;
-  a.tmBw = a.tmB;
-  a.tmBw2 = a.tmB2;
   if (tma)
     fmm::fmm_gemm_kernel<true><<<grid, fmm::NTHREADS, fmm::smem_bytes(true), st>>>(a);
   else
@@ -2261,16 +2067,11 @@ struct fmm_batch {
     int grid[3];                   // plan dims (1,1,1 for classical)
     int ms, ns, ks;                // sub-block sizes
     int a_r, a_c, b_r, b_c, c_r, c_c;  // operand offsets (row, column) inside the problem
-    bool presum;
-    int kk;                        // k extent of the products: ks, or ks rounded up to the k step
-                                   // when every product reads a zero-padded slot (ks % 8 != 0)
-    int nA, nB;                    // pre-summed operand slots
+    PresumPlan pp;                 // its pre-summed operands (FMM jobs)
     size_t ws_off;                 // byte offset of S (then T) in the workspace
-    long long ldT;
     int chunks, tiles_m, tiles_n, units;
-    int bm;                        // tile height: fmm::BM, or BM / 2 (direct phases only)
-    int S;                         // k split of the job's products (the one a single call chooses)
-    const fmm::Prod* vprods;       // its k-split tables when S > 1
+    int S, d;                      // classical jobs: the k parts a single call makes (classical_parts)
+    const fmm::Prod* vprods;       // their tables when S > 1
     const fmm::Term* vterms;
     size_t ticket_off;             // int offset into the ticket array
     double cost;                   // estimated k steps per unit (scheduling order)
@@ -2280,17 +2081,16 @@ struct fmm_batch {
   std::vector<int> m, n, k;
   std::vector<const fmm_plan*> plans;
   std::vector<Job> jobs[2];        // phase 0: FMM cores and disjoint strips; phase 1: k strips
-  bool direct[2] = {true, true};   // every job of the phase can run the direct variant
   std::vector<int> unit_start[2];
-  int max_slots = 0;
-  unsigned max_lincomb_chunks = 1;
-  int n_lincomb = 0;
+  int max_slots = 0, presum_cap = 1;
+  long long max_presum_chunks = 1;
+  int n_presum = 0;
   size_t n_tickets = 0, ws_bytes = 0;
-  fmm::GemmArgs* d_jobs[2] = {nullptr, nullptr};
+  fmmt::ProdArgs* d_jobs[2] = {nullptr, nullptr};
   int* d_start[2] = {nullptr, nullptr};
-  fmm::GemmArgs* h_jobs[2] = {nullptr, nullptr};  // pinned staging of the job tables
-  fmm::LincombTask* d_lc = nullptr;
-  fmm::LincombTask* h_lc = nullptr;
+  fmmt::ProdArgs* h_jobs[2] = {nullptr, nullptr};  // pinned staging of the job tables
+  fmm::PresumSide* d_ps = nullptr;
+  fmm::PresumSide* h_ps = nullptr;
   int* d_tickets = nullptr;        // kBatchCounters work-unit counters (one per phase), then the tickets
   char* d_ws = nullptr;
   // Even-pitch copies of A / B for problems whose row count is odd (a dense operand then
@@ -2306,28 +2106,10 @@ struct fmm_batch {
 
 namespace {
 
-bool batch_configured[kMaxDevices];
-
-int batch_configure(int* dev) {
-  int rc = configure_kernel(dev);
-  if (rc != FMM_OK) return rc;
-  std::lock_guard<std::mutex> lk(g_attr_mu);
-  if (!batch_configured[*dev]) {
-    FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_gemm_batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)fmm::smem_bytes(true)));
-    FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_gemm_batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)fmm::smem_bytes(false)));
-    FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_gemm_direct_batch_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fmm::SMEM_BYTES_DIRECT));
-    batch_configured[*dev] = true;
-  }
-  return FMM_OK;
-}
-
-// Products per unit: units of about the work of a 128 x 128 x 4096 classical tile, so the
+// Products per unit: units of about the work of a 64 x 64 x 4096 classical tile, so the
 // persistent grid balances across problems of very different sizes.
 int batch_chunks(int nprod, int ks) {
-  const long long ksteps = (long long)nprod * ((ks + fmm::BK - 1) / fmm::BK);
+  const long long ksteps = (long long)nprod * ((ks + 7) / 8);
   long long c = (ksteps + 511) / 512;
   if (c < 1) c = 1;
   if (c > nprod) c = nprod;
@@ -2335,11 +2117,10 @@ int batch_chunks(int nprod, int ks) {
 }
 
 void batch_add_job(fmm_batch* b, int phase, int prob, const fmm_plan* plan, int ms, int ns, int ks, int a_r, int a_c,
-                   int b_r, int b_c, int c_r, int c_c, int bm) {
+                   int b_r, int b_c, int c_r, int c_c) {
   if (ms <= 0 || ns <= 0 || ks <= 0) return;
   fmm_batch::Job j{};
   j.prob = prob;
-  j.bm = bm;
   j.plan = plan;
   std::memcpy(j.grid, plan->dims, sizeof(j.grid));
   j.ms = ms;
@@ -2351,32 +2132,34 @@ void batch_add_job(fmm_batch* b, int phase, int prob, const fmm_plan* plan, int 
   j.b_c = b_c;
   j.c_r = c_r;
   j.c_c = c_c;
-  j.presum = plan->rank > 1 && use_presum(plan, ms, ns, ks);
-  j.kk = ks;
-  if (j.presum) {
-    // as in run_fmm: with ks not a multiple of the k step every product gets its own slot,
-    // zero-padded to whole k steps, so the phase keeps the direct variant
-    const bool padded = ks % fmm::BK != 0;
-    j.kk = padded ? (ks + fmm::BK - 1) / fmm::BK * fmm::BK : ks;
-    j.nA = padded ? plan->rank : (int)plan->plistA.size();
-    j.nB = padded ? plan->rank : (int)plan->plistB.size();
-    j.ldT = padded ? j.kk : ks + (ks & 1);
+  j.S = 1;
+  j.d = ks;
+  int nprod = plan->rank, depth = ks;
+  if (is_classical(plan)) {
+    classical_parts(ms, ns, ks, &j.S, &j.d);
+    nprod = j.S;
+    depth = j.d;
+    j.chunks = 1;  // one unit adds all its parts, in order
+  } else {
+    // operands with an odd row count or k get slots throughout, so that no pitch copy of them
+    // is needed for the core
+    j.pp = presum_plan(plan, ms, ns, ks, (b->m[prob] & 1) || (b->k[prob] & 1));
     j.ws_off = b->ws_bytes;
-    b->ws_bytes += sizeof(double) * ((size_t)ms * j.kk * j.nA + (size_t)j.ldT * ns * j.nB);
-    b->ws_bytes = (b->ws_bytes + 255) & ~(size_t)255;
-    b->max_slots = std::max(b->max_slots, std::max(j.nA, j.nB));
-    b->max_lincomb_chunks = std::max({b->max_lincomb_chunks, lincomb_chunks((long long)(ms + 1) / 2 * ks),
-                                      lincomb_chunks((long long)(ks + 1) / 2 * ns)});
-    b->n_lincomb += (j.nA > 0) + (j.nB > 0);
+    b->ws_bytes += presum_bytes(j.pp);
+    b->max_slots = std::max(b->max_slots, std::max(j.pp.nA, j.pp.nB));
+    b->presum_cap = std::max(b->presum_cap, presum_cap(plan));
+    const long long ca = j.pp.nA ? (j.pp.ldS / 2) * j.pp.kk : 0, cb = j.pp.nB ? (j.pp.ldT / 2) * ns : 0;
+    b->max_presum_chunks = std::max(b->max_presum_chunks, (std::max(ca, cb) + fmm::PS_THREADS - 1) / fmm::PS_THREADS);
+    b->n_presum += (j.pp.nA > 0) + (j.pp.nB > 0);
+    depth = j.pp.kk;
+    j.chunks = batch_chunks(nprod, depth);
   }
-  j.tiles_n = (ns + fmm::BN - 1) / fmm::BN;
-  // the k split a single call gives these products, so a batch computes each problem with the
-  // same arithmetic as a call of its own
-  j.S = call_ksplit(plan, ms, ns, ks, j.presum, j.kk, sm_count[b->dev]);
-  j.chunks = batch_chunks(plan->rank * j.S, j.kk / j.S);
-  // direct staging: operands are single unit-coefficient blocks (pre-summed or classical)
-  // and every k step stays inside them
-  if (!((j.presum || plan->rank == 1) && whole_k_steps(j.grid, j.kk))) b->direct[phase] = false;
+  j.tiles_m = (ms + 63) / 64;
+  j.tiles_n = (ns + 63) / 64;
+  j.units = j.tiles_m * j.tiles_n * j.chunks;
+  j.ticket_off = b->n_tickets;
+  if (j.chunks > 1) b->n_tickets += 4 * (size_t)j.tiles_m * j.tiles_n;
+  j.cost = (double)nprod / j.chunks * ((depth + 7) / 8);
   b->jobs[phase].push_back(j);
 }
 
@@ -2386,8 +2169,8 @@ void batch_free(fmm_batch* b) {
     if (b->d_start[ph]) cudaFree(b->d_start[ph]);
     if (b->h_jobs[ph]) cudaFreeHost(b->h_jobs[ph]);
   }
-  if (b->d_lc) cudaFree(b->d_lc);
-  if (b->h_lc) cudaFreeHost(b->h_lc);
+  if (b->d_ps) cudaFree(b->d_ps);
+  if (b->h_ps) cudaFreeHost(b->h_ps);
   if (b->d_tickets) cudaFree(b->d_tickets);
   if (b->d_ws) cudaFree(b->d_ws);
   if (b->d_pitch) cudaFree(b->d_pitch);
@@ -2405,10 +2188,10 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
   if (!out || count <= 0 || !m || !n || !k) return FMM_E_INVALID;
   for (int i = 0; i < count; ++i) {
     if (m[i] < 0 || n[i] < 0 || k[i] < 0) return FMM_E_INVALID;
-    if (tile_m && tile_m[i] != 0 && tile_m[i] != fmm::BM && tile_m[i] != fmm::BM / 2) return FMM_E_INVALID;
+    if (tile_m && tile_m[i] != 0 && tile_m[i] != 128 && tile_m[i] != 64) return FMM_E_INVALID;
   }
   int dev = 0;
-  int rc = batch_configure(&dev);
+  int rc = configure_kernel(&dev);
   if (rc != FMM_OK) return rc;
   fmm_batch* b = new (std::nothrow) fmm_batch();
   if (!b) return FMM_E_NOMEM;
@@ -2422,7 +2205,6 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
     const fmm_plan* p = (plans && plans[i]) ? plans[i] : nullptr;
     b->plans.push_back(p);
     const bool live = m[i] > 0 && n[i] > 0 && k[i] > 0;
-    const int bm = (tile_m && tile_m[i] != 0) ? tile_m[i] : fmm::BM;
     auto reserve = [&](int rows, int cols) {
       const size_t off = b->pitch_bytes;
       b->pitch_bytes += (sizeof(double) * (size_t)(rows + 1) * cols + 255) & ~(size_t)255;
@@ -2431,8 +2213,8 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
     b->pitch_a.push_back(live && (m[i] & 1) ? reserve(m[i], k[i]) : SIZE_MAX);
     b->pitch_b.push_back(live && (k[i] & 1) ? reserve(k[i], n[i]) : SIZE_MAX);
     if (!live) continue;
-    if (!p) {
-      batch_add_job(b, 0, i, cls, m[i], n[i], k[i], 0, 0, 0, 0, 0, 0, bm);
+    if (!p || is_classical(p)) {
+      batch_add_job(b, 0, i, cls, m[i], n[i], k[i], 0, 0, 0, 0, 0, 0);
       continue;
     }
     // same partition and fringe regions as the single-problem path (run_fmm + peel)
@@ -2440,22 +2222,11 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
     const int mr = m[i] % pm, kr = k[i] % pk, nr = n[i] % pn;
     const int md = m[i] - mr, kd = k[i] - kr, nd = n[i] - nr;
     if (md > 0 && nd > 0 && kd > 0)
-      batch_add_job(b, 0, i, p, md / p->dims[0], nd / p->dims[2], kd / p->dims[1], 0, 0, 0, 0, 0, 0, bm);
-    if (kr > 0 && md > 0 && nd > 0) batch_add_job(b, 1, i, cls, md, nd, kr, 0, kd, kd, 0, 0, 0, bm);
-    if (nr > 0) batch_add_job(b, 0, i, cls, m[i], nr, k[i], 0, 0, 0, nd, 0, nd, bm);
-    if (mr > 0 && nd > 0) batch_add_job(b, 0, i, cls, mr, nd, k[i], md, 0, 0, 0, md, 0, bm);
+      batch_add_job(b, 0, i, p, md / p->dims[0], nd / p->dims[2], kd / p->dims[1], 0, 0, 0, 0, 0, 0);
+    if (kr > 0 && md > 0 && nd > 0) batch_add_job(b, 1, i, cls, md, nd, kr, 0, kd, kd, 0, 0, 0);
+    if (nr > 0) batch_add_job(b, 0, i, cls, m[i], nr, k[i], 0, 0, 0, nd, 0, nd);
+    if (mr > 0 && nd > 0) batch_add_job(b, 0, i, cls, mr, nd, k[i], md, 0, 0, 0, md, 0);
   }
-  // Tile heights (64-row tiles only where the whole phase runs the direct variant), then
-  // each job's units and tickets.
-  for (int ph = 0; ph < 2; ++ph)
-    for (auto& j : b->jobs[ph]) {
-      if (!b->direct[ph]) j.bm = fmm::BM;
-      j.tiles_m = (j.ms + j.bm - 1) / j.bm;
-      j.units = j.tiles_m * j.tiles_n * j.chunks;
-      j.ticket_off = b->n_tickets;
-      if (j.chunks > 1) b->n_tickets += (size_t)j.tiles_m * j.tiles_n;
-      j.cost = (double)j.plan->rank / j.chunks * ((j.kk + fmm::BK - 1) / fmm::BK) * j.bm / fmm::BM;
-    }
   // Longest units first: the persistent grid takes units in order, so the short ones
   // fill in at the end.
   for (int ph = 0; ph < 2; ++ph) {
@@ -2474,9 +2245,7 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
     for (auto& j : b->jobs[ph]) {
       DevTables* d = nullptr;
       rc = device_tables(j.plan, &d);
-      if (rc == FMM_OK && j.S > 1)
-        rc = ksplit_tables(j.plan, j.plan->rank == 1 ? BASE_ORIG : (j.kk != j.ks ? BASE_ALL : BASE_PS), j.S,
-                           &j.vprods, &j.vterms);
+      if (rc == FMM_OK && j.S > 1) rc = ksplit_tables(j.plan, BASE_SPLIT, j.S, &j.vprods, &j.vterms);
       if (rc != FMM_OK) {
         batch_free(b);
         return rc;
@@ -2500,15 +2269,15 @@ int batch_create(int count, const fmm_plan* const* plans, const int* m, const in
   for (int ph = 0; ph < 2 && e == cudaSuccess; ++ph) {
     const size_t nj = b->jobs[ph].size();
     if (nj == 0) continue;
-    e = cudaMalloc((void**)&b->d_jobs[ph], sizeof(fmm::GemmArgs) * nj);
+    e = cudaMalloc((void**)&b->d_jobs[ph], sizeof(fmmt::ProdArgs) * nj);
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_start[ph], sizeof(int) * (nj + 1));
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_jobs[ph], sizeof(fmm::GemmArgs) * nj);
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_jobs[ph], sizeof(fmmt::ProdArgs) * nj);
     if (e == cudaSuccess)
       e = cudaMemcpy(b->d_start[ph], b->unit_start[ph].data(), sizeof(int) * (nj + 1), cudaMemcpyHostToDevice);
   }
-  if (e == cudaSuccess && b->n_lincomb > 0) {
-    e = cudaMalloc((void**)&b->d_lc, sizeof(fmm::LincombTask) * b->n_lincomb);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_lc, sizeof(fmm::LincombTask) * b->n_lincomb);
+  if (e == cudaSuccess && b->n_presum > 0) {
+    e = cudaMalloc((void**)&b->d_ps, sizeof(fmm::PresumSide) * b->n_presum);
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_ps, sizeof(fmm::PresumSide) * b->n_presum);
   }
   if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_tickets, sizeof(int) * (kBatchCounters + b->n_tickets));
   if (e == cudaSuccess && b->ws_bytes > 0) e = cudaMalloc((void**)&b->d_ws, b->ws_bytes);
@@ -2523,15 +2292,15 @@ int batch_create(int count, const fmm_plan* const* plans, const int* m, const in
   return FMM_OK;
 }
 
-// Fill the job table of one phase for this call's operands; false if a problem cannot
-// use TMA staging (the phase then runs with cp.async staging).
+// Fill the job table of one phase for this call's operands; false if some operand cannot be
+// read by tensor copies (the launch then carries the per-lane copies).
 bool batch_fill(fmm_batch* b, int ph, const double* const* A, const long* lda, const double* const* B,
-                const long* ldb, double* const* C, const long* ldc, int* n_lc) {
+                const long* ldb, double* const* C, const long* ldc, int* n_ps) {
   bool tma = true;
   for (size_t q = 0; q < b->jobs[ph].size(); ++q) {
     const fmm_batch::Job& j = b->jobs[ph][q];
     const DevTables& d = j.plan->dev[b->dev];
-    fmm::GemmArgs a{};
+    fmmt::ProdArgs a{};
     const long long la = lda[j.prob], lb = ldb[j.prob], lc = ldc[j.prob];
     a.A = A[j.prob] + j.a_r + (long long)j.a_c * la;
     a.lda = la;
@@ -2541,86 +2310,50 @@ bool batch_fill(fmm_batch* b, int ph, const double* const* A, const long* lda, c
     a.ldc = lc;
     a.ms = j.ms;
     a.ns = j.ns;
-    a.ks = j.ks;
+    a.ks = j.d;
+    a.kcap = j.grid[1] * j.ks;
     a.nprod = j.plan->rank;
     a.tiles_m = j.tiles_m;
-    a.bm = j.bm;
     a.tiles_n = j.tiles_n;
     a.chunks = j.chunks;
     a.mode = fmm::MODE_ACCUM_C;
     a.tickets = j.chunks > 1 ? b->d_tickets + kBatchCounters + j.ticket_off : nullptr;
     a.status = dev_status[b->dev];
+    const PresumPlan& pp = j.pp;
+    double* S = reinterpret_cast<double*>(b->d_ws + j.ws_off);
+    double* T = reinterpret_cast<double*>(b->d_ws + j.ws_off + pp.s_bytes);
+    if (is_classical(j.plan)) {
+      a.prods = j.S > 1 ? j.vprods : d.prods;
+      a.terms = j.S > 1 ? j.vterms : d.terms;
+      a.nprod = j.S;
+    } else {
+      a.ks = pp.kk;
+      a.prods = pp.all ? d.prods_all : d.prods_ps;
+      a.terms = pp.all ? d.terms_all : d.terms_ps;
+      if (pp.nA > 0)
+        b->h_ps[(*n_ps)++] = presum_side(d, 0, a.A, la, j.ms, j.ns, j.ks, pp.kk, S, pp.ldS,
+                                         pp.all ? d.plist_all : d.plistA, pp.nA);
+      if (pp.nB > 0)
+        b->h_ps[(*n_ps)++] = presum_side(d, 1, a.B, lb, j.ms, j.ns, j.ks, pp.kk, T, pp.ldT,
+                                         pp.all ? d.plist_all : d.plistB, pp.nB);
+    }
     const long long am = (long long)j.grid[0] * j.ms, ak = (long long)j.grid[1] * j.ks,
                     bn = (long long)j.grid[2] * j.ns;
-    if (j.presum) {
-      const bool padded = j.kk != j.ks;
-      const double* S = reinterpret_cast<const double*>(b->d_ws + j.ws_off);
-      const double* T = S + (size_t)j.ms * j.kk * j.nA;
-      a.ks = j.kk;
-      a.prods = padded ? d.prods_all : d.prods_ps;
-      a.terms = padded ? d.terms_all : d.terms_ps;
-      a.Aw = S;
-      a.ldaw = j.ms;
-      a.Bw = T;
-      a.ldbw = j.ldT;
-      for (int side = 0; side < 2; ++side) {
-        const int ns = side == 0 ? j.nA : j.nB;
-        if (ns == 0) continue;
-        fmm::LincombTask& t = b->h_lc[(*n_lc)++];
-        t = fmm::LincombTask{};
-        t.nout = ns;
-        fmm::LincombArgs& l = t.a;
-        l.X = side == 0 ? a.A : a.B;
-        l.ldx = side == 0 ? la : lb;
-        l.rows = side == 0 ? j.ms : j.ks;
-        l.cols = side == 0 ? j.ks : j.ns;
-        l.blk_row_stride = l.rows;
-        l.blk_col_stride = l.cols;
-        l.out = const_cast<double*>(side == 0 ? S : T);
-        l.ldo = side == 0 ? j.ms : j.ldT;
-        l.out_stride = l.ldo * (side == 0 ? j.kk : l.cols);
-        l.prods = d.prods;
-        l.terms = d.terms;
-        l.plist = padded ? d.plist_all : side == 0 ? d.plistA : d.plistB;
-        l.side = side;
-      }
-    } else {
-      a.prods = d.prods;
-      a.terms = d.terms;
-      a.Aw = a.A;
-      a.ldaw = la;
-      a.Bw = a.B;
-      a.ldbw = lb;
-    }
-    bool ok = make_tensor_map(&a.tmA, a.A, am, ak, la, fmm::BM, fmm::BK) &&
-              make_tensor_map(&a.tmA64, a.A, am, ak, la, fmm::BM / 2, fmm::BK) &&
-              make_tensor_map(&a.tmB, a.B, ak, bn, lb, fmm::BK, fmm::BN) &&
-              make_tensor_map(&a.tmB2, a.B, ak, bn, lb, fmm::TB_K, fmm::BN);
-    if (ok && j.presum && j.nA > 0)
-      ok = make_tensor_map(&a.tmAw, a.Aw, j.ms, (long long)j.nA * j.kk, j.ms, fmm::BM, fmm::BK) &&
-           make_tensor_map(&a.tmAw64, a.Aw, j.ms, (long long)j.nA * j.kk, j.ms, fmm::BM / 2, fmm::BK);
-    else
-      a.tmAw = a.tmA, a.tmAw64 = a.tmA64;
-    if (ok && j.presum && j.nB > 0)
-      ok = make_tensor_map(&a.tmBw, a.Bw, j.kk, (long long)j.nB * j.ns, j.ldT, fmm::BK, fmm::BN) &&
-           make_tensor_map(&a.tmBw2, a.Bw, j.kk, (long long)j.nB * j.ns, j.ldT, fmm::TB_K, fmm::BN);
-    else
-      a.tmBw = a.tmB, a.tmBw2 = a.tmB2;
-    if (j.S > 1) {  // the k-split tables (part depth kk / S); the tensor maps keep the full depth
-      a.ks /= j.S;
-      a.nprod *= j.S;
-      a.prods = j.vprods;
-      a.terms = j.vterms;
-    }
-    tma = tma && ok;
+    // an operand with slots throughout is never read in place
+    a.a_tma = pp.all || make_a_map(&a.tmA, a.A, am, ak, la);
+    a.b_tma = pp.all || make_b_map(&a.tmB, a.B, ak, bn, lb, 64);
+    bool ok = true;
+    if (pp.nA > 0) ok = make_a_map(&a.tmAw, S, j.ms, (long long)pp.nA * pp.kk, pp.ldS);
+    if (pp.nB > 0) ok = ok && make_b_map(&a.tmBw, T, pp.kk, (long long)pp.nB * j.ns, pp.ldT, 64);
+    tma = tma && ok && a.a_tma && a.b_tma;
     b->h_jobs[ph][q] = a;
   }
   return tma;
 }
 
 void batch_prepare(fmm_batch* b, const double* const* A, const long* lda, const double* const* B, const long* ldb,
-                   double* const* C, const long* ldc, int* n_lc_out, int* n_pc_out, bool tma[2]);
-int batch_launch(fmm_batch* b, cudaStream_t st, int n_lc, int n_pc, const bool tma[2]);
+                   double* const* C, const long* ldc, int* n_ps_out, int* n_pc_out, bool tma[2]);
+int batch_launch(fmm_batch* b, cudaStream_t st, int n_ps, int n_pc, const bool tma[2]);
 
 int batch_run(fmm_batch* b, const double* const* A, const long* lda, const double* const* B, const long* ldb,
               double* const* C, const long* ldc, cudaStream_t st) {
@@ -2638,25 +2371,25 @@ int batch_run(fmm_batch* b, const double* const* A, const long* lda, const doubl
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   FMM_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
   if (cap == cudaStreamCaptureStatusNone) FMM_CUDA_TRY(cudaEventSynchronize(b->staged));
-  int n_lc = 0, n_pc = 0;
+  int n_ps = 0, n_pc = 0;
   bool tma[2] = {true, true};
-  batch_prepare(b, A, lda, B, ldb, C, ldc, &n_lc, &n_pc, tma);
+  batch_prepare(b, A, lda, B, ldb, C, ldc, &n_ps, &n_pc, tma);
   for (int ph = 0; ph < 2; ++ph)
     if (!b->jobs[ph].empty())
-      FMM_CUDA_TRY(cudaMemcpyAsync(b->d_jobs[ph], b->h_jobs[ph], sizeof(fmm::GemmArgs) * b->jobs[ph].size(),
+      FMM_CUDA_TRY(cudaMemcpyAsync(b->d_jobs[ph], b->h_jobs[ph], sizeof(fmmt::ProdArgs) * b->jobs[ph].size(),
                                    cudaMemcpyHostToDevice, st));
-  if (n_lc > 0)
-    FMM_CUDA_TRY(cudaMemcpyAsync(b->d_lc, b->h_lc, sizeof(fmm::LincombTask) * n_lc, cudaMemcpyHostToDevice, st));
+  if (n_ps > 0)
+    FMM_CUDA_TRY(cudaMemcpyAsync(b->d_ps, b->h_ps, sizeof(fmm::PresumSide) * n_ps, cudaMemcpyHostToDevice, st));
   if (n_pc > 0)
     FMM_CUDA_TRY(cudaMemcpyAsync(b->d_pc, b->h_pc, sizeof(fmm::PitchCopy) * n_pc, cudaMemcpyHostToDevice, st));
   if (cap == cudaStreamCaptureStatusNone) FMM_CUDA_TRY(cudaEventRecord(b->staged, st));
-  return batch_launch(b, st, n_lc, n_pc, tma);
+  return batch_launch(b, st, n_ps, n_pc, tma);
 }
 
 // This call's job tables (host staging): even-pitch copies for odd leading dimensions,
 // per-job arguments and tensor maps, pre-sum tasks.
 void batch_prepare(fmm_batch* b, const double* const* A, const long* lda, const double* const* B, const long* ldb,
-                   double* const* C, const long* ldc, int* n_lc_out, int* n_pc_out, bool tma[2]) {
+                   double* const* C, const long* ldc, int* n_ps_out, int* n_pc_out, bool tma[2]) {
   // Operands with an odd leading dimension and a reserved even-pitch copy are staged
   // through it (rows + 1 pitch); the others are used in place.
   std::vector<const double*> eA(A, A + b->count), eB(B, B + b->count);
@@ -2676,16 +2409,16 @@ void batch_prepare(fmm_batch* b, const double* const* A, const long* lda, const 
       eldb[i] = b->k[i] + 1;
     }
   }
-  int n_lc = 0;
+  int n_ps = 0;
   for (int ph = 0; ph < 2; ++ph)
     if (!b->jobs[ph].empty())
-      tma[ph] = batch_fill(b, ph, eA.data(), elda.data(), eB.data(), eldb.data(), C, ldc, &n_lc);
-  *n_lc_out = n_lc;
+      tma[ph] = batch_fill(b, ph, eA.data(), elda.data(), eB.data(), eldb.data(), C, ldc, &n_ps);
+  *n_ps_out = n_ps;
   *n_pc_out = n_pc;
 }
 
 // Enqueue the launches of a prepared batch whose tables are (being) copied to the device.
-int batch_launch(fmm_batch* b, cudaStream_t st, int n_lc, int n_pc, const bool tma[2]) {
+int batch_launch(fmm_batch* b, cudaStream_t st, int n_ps, int n_pc, const bool tma[2]) {
   // the phases' work-unit counters and every ticket start at zero
   FMM_CUDA_TRY(cudaMemsetAsync(b->d_tickets, 0, sizeof(int) * (kBatchCounters + b->n_tickets), st));
   if (n_pc > 0) {
@@ -2694,46 +2427,30 @@ int batch_launch(fmm_batch* b, cudaStream_t st, int n_lc, int n_pc, const bool t
     g_launches.fetch_add(1, std::memory_order_relaxed);
     FMM_CUDA_TRY(cudaGetLastError());
   }
-  // zero padding of the padded slots (k columns [ks, kk) of every S slot, rows [ks, kk)
-  // of every T slot column): the sums fill only [0, ks)
-  for (int ph = 0; ph < 2; ++ph)
-    for (const auto& j : b->jobs[ph]) {
-      if (!j.presum || j.kk == j.ks) continue;
-      char* S = b->d_ws + j.ws_off;
-      char* T = S + sizeof(double) * (size_t)j.ms * j.kk * j.nA;
-      FMM_CUDA_TRY(cudaMemset2DAsync(S + sizeof(double) * (size_t)j.ms * j.ks, sizeof(double) * (size_t)j.ms * j.kk, 0,
-                                     sizeof(double) * (size_t)j.ms * (j.kk - j.ks), j.nA, st));
-      FMM_CUDA_TRY(cudaMemset2DAsync(T + sizeof(double) * j.ks, sizeof(double) * (size_t)j.kk, 0,
-                                     sizeof(double) * (j.kk - j.ks), (size_t)j.nB * j.ns, st));
-    }
-  if (n_lc > 0) {
-    ProfScope pf(K_LINCOMB_BATCH, st);
-    fmm::fmm_lincomb_batch_kernel<<<dim3((unsigned)b->max_slots, b->max_lincomb_chunks, (unsigned)n_lc), 256, 0, st>>>(
-        b->d_lc);
+  if (n_ps > 0) {
+    ProfScope pf(K_PRESUM_BATCH, st);
+    const long long nc = std::min<long long>(b->max_presum_chunks, 1 << 16);
+    fmm::fmm_presum_batch_kernel<<<dim3((unsigned)nc, presum_ranges(nc * n_ps, b->max_slots, sm_count[b->dev]),
+                                        (unsigned)n_ps),
+                                   fmm::PS_THREADS, sizeof(fmm::PresumOff) * b->presum_cap, st>>>(b->d_ps, b->presum_cap);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     FMM_CUDA_TRY(cudaGetLastError());
   }
   for (int ph = 0; ph < 2; ++ph) {
     if (b->jobs[ph].empty()) continue;
-    fmm::BatchArgs ba{};
+    fmmt::ProdBatchArgs ba{};
     ba.jobs = b->d_jobs[ph];
     ba.unit_start = b->d_start[ph];
     ba.njobs = (int)b->jobs[ph].size();
     ba.units = b->unit_start[ph].back();
     ba.status = dev_status[b->dev];
     ba.counter = b->d_tickets + ph;
-    const unsigned grid = (unsigned)std::min<long long>(ba.units, sm_count[b->dev]);
-    {
-      ProfScope pf(K_GEMM_BATCH, st);
-      if (tma[ph] && b->direct[ph])
-        fmm::fmm_gemm_direct_batch_kernel<<<grid, fmm::NTHREADS, fmm::SMEM_BYTES_DIRECT, st>>>(ba);
-      else if (tma[ph])
-        fmm::fmm_gemm_batch_kernel<true><<<grid, fmm::NTHREADS, fmm::smem_bytes(true), st>>>(ba);
-      else
-        fmm::fmm_gemm_batch_kernel<false><<<grid, fmm::NTHREADS, fmm::smem_bytes(false), st>>>(ba);
-    }
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    FMM_CUDA_TRY(cudaGetLastError());
+    const unsigned grid =
+        (unsigned)std::min<long long>(ba.units, (long long)sm_count[b->dev] * fmmt::TileShape<64, 64>::CTAS);
+    ProfScope pf(K_PRODUCTS_BATCH, st);
+    const int rc = launch_dependent(tma[ph] ? fmmt::fmm_products_batch_kernel<false> : fmmt::fmm_products_batch_kernel<true>,
+                                    dim3(grid), fmmt::NT, fmmt::ProdShape<64>::SMEM, st, 1, ba);
+    if (rc != FMM_OK) return rc;
   }
   return FMM_OK;
 }
@@ -2828,7 +2545,7 @@ int batch_submit(int count, const fmm_plan* const* plans, const int* m, const in
   for (int ph = 0; ph < 2; ++ph) {
     off = align_up(off, 64);
     o_jobs[ph] = off;
-    off += sizeof(fmm::GemmArgs) * b->jobs[ph].size();
+    off += sizeof(fmmt::ProdArgs) * b->jobs[ph].size();
   }
   for (int ph = 0; ph < 2; ++ph) {
     off = align_up(off, 16);
@@ -2836,8 +2553,8 @@ int batch_submit(int count, const fmm_plan* const* plans, const int* m, const in
     off += sizeof(int) * b->unit_start[ph].size();
   }
   off = align_up(off, 64);
-  const size_t o_lc = off;
-  off += sizeof(fmm::LincombTask) * b->n_lincomb;
+  const size_t o_ps = off;
+  off += sizeof(fmm::PresumSide) * b->n_presum;
   off = align_up(off, 64);
   const size_t o_pc = off;
   off += sizeof(fmm::PitchCopy) * 2 * count;
@@ -2856,30 +2573,30 @@ int batch_submit(int count, const fmm_plan* const* plans, const int* m, const in
     return rc;
   }
   for (int ph = 0; ph < 2; ++ph) {
-    b->h_jobs[ph] = reinterpret_cast<fmm::GemmArgs*>(stage + o_jobs[ph]);
-    b->d_jobs[ph] = reinterpret_cast<fmm::GemmArgs*>(blk + o_jobs[ph]);
+    b->h_jobs[ph] = reinterpret_cast<fmmt::ProdArgs*>(stage + o_jobs[ph]);
+    b->d_jobs[ph] = reinterpret_cast<fmmt::ProdArgs*>(blk + o_jobs[ph]);
     b->d_start[ph] = reinterpret_cast<int*>(blk + o_start[ph]);
     if (!b->unit_start[ph].empty())
       std::memcpy(stage + o_start[ph], b->unit_start[ph].data(), sizeof(int) * b->unit_start[ph].size());
   }
-  b->h_lc = reinterpret_cast<fmm::LincombTask*>(stage + o_lc);
-  b->d_lc = reinterpret_cast<fmm::LincombTask*>(blk + o_lc);
+  b->h_ps = reinterpret_cast<fmm::PresumSide*>(stage + o_ps);
+  b->d_ps = reinterpret_cast<fmm::PresumSide*>(blk + o_ps);
   b->h_pc = reinterpret_cast<fmm::PitchCopy*>(stage + o_pc);
   b->d_pc = reinterpret_cast<fmm::PitchCopy*>(blk + o_pc);
   b->d_tickets = reinterpret_cast<int*>(blk + o_tk);
   b->d_ws = b->ws_bytes ? blk + o_ws : nullptr;
   b->d_pitch = b->pitch_bytes ? blk + o_pt : nullptr;
-  int n_lc = 0, n_pc = 0;
+  int n_ps = 0, n_pc = 0;
   bool tma[2] = {true, true};
-  batch_prepare(b, A, lda, B, ldb, C, ldc, &n_lc, &n_pc, tma);
+  batch_prepare(b, A, lda, B, ldb, C, ldc, &n_ps, &n_pc, tma);
   rc = cuda_status(cudaMemcpyAsync(blk, stage, table_bytes, cudaMemcpyHostToDevice, st));
   if (rc == FMM_OK) rc = cuda_status(cudaEventRecord(stage_ev, st));
-  if (rc == FMM_OK) rc = batch_launch(b, st, n_lc, n_pc, tma);
+  if (rc == FMM_OK) rc = batch_launch(b, st, n_ps, n_pc, tma);
   cudaError_t fe = cudaFreeAsync(blk, st);
   if (rc == FMM_OK) rc = cuda_status(fe);
   // the buffers belong to the pool and the ring: detach them before freeing the host side
   for (int ph = 0; ph < 2; ++ph) b->h_jobs[ph] = nullptr, b->d_jobs[ph] = nullptr, b->d_start[ph] = nullptr;
-  b->h_lc = nullptr, b->d_lc = nullptr, b->h_pc = nullptr, b->d_pc = nullptr;
+  b->h_ps = nullptr, b->d_ps = nullptr, b->h_pc = nullptr, b->d_pc = nullptr;
   b->d_tickets = nullptr, b->d_ws = nullptr, b->d_pitch = nullptr;
   batch_free(b);
   return rc;

@@ -1,34 +1,28 @@
-// fmm_b200 device code: a persistent, warp-specialised FP64 DMMA GEMM whose producer
-// warpgroup forms the U/V linear combinations of A and B sub-blocks while staging them
-// into shared memory, and whose consumer warpgroups scatter each product into every C
-// block with a nonzero W coefficient; plus the elementwise kernels of the AB / NAIVE
-// pack types.  sm_100a only.
+// fmm_b200 device code shared by the FP64 kernels (barriers, bounded waits, work-unit claims,
+// DMMA), the operand sums and combine passes, and the folding GEMM of the no-allocation entry
+// point: a persistent, warp-specialised FP64 DMMA GEMM whose producer warpgroup forms the U/V
+// linear combinations of A and B sub-blocks while staging them into shared memory, and whose
+// consumer warpgroups scatter each product into every C block with a nonzero W coefficient.
+// The other FP64 launches run the tile kernels of fmm_tile.cuh.  sm_100a only.
 //
 // Mapping of the reference's CPU design (fmm-gen):
 //   * BLIS packing with fused sums (meta/abc_gen_mix.py:171-251, packA/B_add_stra_abc<r>)
-//     -> producer warpgroup: cp.async of every U/V term tile into thread-private
-//        shared-memory slots, folded into the operand stage (sum with coefficients),
-//        released to the consumers with an mbarrier.
+//     -> fmm_presum_kernel (operand sums formed in HBM; S_Add / T_Add of
+//        meta/naive_gen_mix.py:60-137 too), or the folding GEMM's producer warps (cp.async /
+//        TMA of every U/V term tile, folded into the operand stage).
 //   * AVX 8x4 micro-kernel (common/kernels/bl_dgemm_asm_8x4.c)
-//     -> 128x128 CTA tile of mma.sync.m16n8k4 FP64 (DMMA) fragments, 8 consumer warps
-//        with 64x32 warp tiles.
+//     -> mma.sync.m16n8k4 FP64 (DMMA) fragments.
 //   * multi-destination C update (meta/abc_micro_kernel_gen.py:147-244)
-//     -> epilogue C_l += W[l,r] * M_r for every nonzero W of product r.  A work unit
-//        owns one tile position in all C blocks for a range of products; when products
-//        are split over several units, tickets per tile (or, in the direct variant with
-//        few tile positions, per tile and C block) order the units' C updates (bounded
-//        spin, error flag on timeout), so no two CTAs ever update the same C element at
-//        once and every element receives its products in order r = 0..R-1.
-//   * M_Add / S_Add / T_Add (meta/ab_gen_mix.py:341-372, meta/naive_gen_mix.py:60-137)
-//     -> fmm_lincomb_kernel / fmm_lincomb_batch_kernel (operand sums formed in HBM, also
-//        used by the ABC pack type for large sub-blocks), fmm_combine_staged_kernel and
-//        fmm_combine_kernel (every C_l += W[l,r] M_r of the stored products in one pass, the
-//        C blocks in groups that share products, running values in registers; the staged
-//        form brings the M tiles in by bulk copies), fmm_scatter_kernel (one C block per
-//        launch row, beyond the combine's tables).
-//   * The direct variant (fmm_gemm_direct_kernel) runs when every operand is a single
-//     aligned term (pre-summed operands): a deeper TMA pipeline and an epilogue on the
-//     producer warps that overlaps the next product's DMMA.
+//     -> epilogue C_l += W[l,r] * M_r for every nonzero W of product r.  A work unit owns one
+//        tile position in all C blocks; tickets per tile (or per tile and C block) order the
+//        units' C updates (bounded spin, error flag on timeout), so no two CTAs ever update
+//        the same C element at once and every element receives its products in order
+//        r = 0..R-1.
+//   * M_Add (meta/ab_gen_mix.py:341-372)
+//     -> fmm_combine_staged_kernel and fmm_combine_kernel (every C_l += W[l,r] M_r of the
+//        stored products in one pass, the C blocks in groups that share products, running
+//        values in registers; the staged form brings the M tiles in by bulk copies),
+//        fmm_scatter_kernel (one C block per launch row, beyond the combine's tables).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -137,38 +131,20 @@ struct GemmArgs {
   CUtensorMap tmA;   // whole-matrix tensor maps (TMA path), FP64: A (m x k), box BM x BK
   CUtensorMap tmB;   // B (k x n), box BK x BN (direct loads)
   CUtensorMap tmB2;  // B (k x n), box (BK + 2) x BN (raw loads at even k)
-  CUtensorMap tmAw;  // the same three for the pre-summed workspaces S (A side) and T (B side)
-  CUtensorMap tmBw;
-  CUtensorMap tmBw2;
-  CUtensorMap tmA64;   // A and S again with a box of BM / 2 rows: the half-height units of the
-  CUtensorMap tmAw64;  // direct variant (see Unit)
   const double* A;
   long long lda;
   const double* B;
   long long ldb;
-  const double* Aw;  // pre-summed operands: S holds one ms x ks block per slot (block column),
-  long long ldaw;    // T one ks x ns block per slot (block column); terms with src = 1 point here
-  const double* Bw;
-  long long ldbw;
-  double* C;      // MODE_ACCUM_C: C blocks receive C_l += w * M_r
+  double* C;        // C blocks receive C_l += w * M_r
   long long ldc;
-  double* M;      // MODE_STORE_M: product r stored at M + r * m_stride (ld = ldm)
-  long long ldm;
-  long long m_stride;
   int ms, ns, ks;   // sub-block sizes
   const Prod* prods;
   const Term* terms;
-  int nprod;        // products [0, nprod)
+  int nprod;
   int tiles_m, tiles_n;
-  int chunks;       // products are split into `chunks` consecutive ranges per tile
-  int mode;
-  int* tickets;     // per tile (nbt = 0): chunks completed; zeroed before launch; used when chunks > 1
+  int* tickets;     // per tile: products whose C updates are done (zeroed before launch); used when nprod > 1
   unsigned* status; // device status word (StatusBits)
-  int nbt;          // > 0 (direct variant, one product per unit): tickets per (tile, C block),
-  int nbc;          // nbt = C blocks, index tile * nbt + row * nbc + col, counting the block's
-                    // updates in product order; 0: one ticket per tile
   int* counter;     // work units claimed so far in this launch (zeroed before launch)
-  int bm;           // tile height: BM, or BM / 2 (direct variant only); 0 means BM
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
@@ -295,57 +271,29 @@ __device__ __forceinline__ void dmma_16x8x4(double (&d)[4], const double (&a)[2]
 
 __device__ __forceinline__ int prod_T(const Prod& p) { return p.na > p.nb ? p.na : p.nb; }
 
-// Work unit u -> (tile position, product range).  Chunk-major order: the units of one tile
-// are a whole tile grid apart, so a later chunk is claimed well after the earlier one.
-// unit_rows: the tile's rows inside the block (at most the tile height).  unit_half: the tile
-// has at most BM / 2 rows (a job of half-height tiles, or the last tile row of a block whose
-// height leaves <= 64 rows there); the direct variant then stages a BM / 2-row box of A and
-// lets both rows of consumer warps cover those rows, each taking half of the column fragments
-// (every element still gets a full tile's DMMAs in the same order).
+// Work unit u -> (tile position, product).  Product-major order: the units of one tile are a
+// whole tile grid apart, so a later product is claimed well after the earlier one.
 struct Unit {
-  int m0, n0, tile, r0, r1;
+  int m0, n0, tile, r;
 };
 
-__device__ __forceinline__ int tile_height(const GemmArgs& a) { return a.bm > 0 ? a.bm : BM; }
-// rows of the unit's tile inside the block, and whether that makes it a half-height unit
-__device__ __forceinline__ int unit_rows(const GemmArgs& a, const Unit& w) { return min(tile_height(a), a.ms - w.m0); }
-__device__ __forceinline__ bool unit_half(const GemmArgs& a, const Unit& w) { return unit_rows(a, w) <= BM / 2; }
-
-// VARH: the job's tile height may be BM / 2 (direct variant); the other kernels use BM, known
-// at compile time.
-template <bool VARH = false>
 __device__ __forceinline__ Unit decode_unit(const GemmArgs& a, int u) {
   const int ntiles = a.tiles_m * a.tiles_n;
   Unit w;
-  int c, bid;
-  if (a.mode == MODE_STORE_M) {
-    c = u / ntiles;  // one product per unit
-    bid = u % ntiles;
-    w.r0 = c;
-    w.r1 = c + 1;
-  } else {
-    c = u / ntiles;
-    bid = u % ntiles;
-    w.r0 = (int)((long long)a.nprod * c / a.chunks);
-    w.r1 = (int)((long long)a.nprod * (c + 1) / a.chunks);
-  }
+  const int bid = u % ntiles;
+  w.r = u / ntiles;
   const int per_group = GROUP_M * a.tiles_n;
   const int grp = bid / per_group;
   const int first_m = grp * GROUP_M;
   const int rows_here = min(a.tiles_m - first_m, GROUP_M);
   const int in_grp = bid % per_group;
-  const int tile_m = first_m + in_grp % rows_here;
-  const int tile_n = in_grp / rows_here;
-  w.m0 = tile_m * (VARH ? tile_height(a) : BM);
-  w.n0 = tile_n * BN;
+  w.m0 = (first_m + in_grp % rows_here) * BM;
+  w.n0 = (in_grp / rows_here) * BN;
   w.tile = bid;
   return w;
 }
 
-__device__ __forceinline__ int num_units(const GemmArgs& a) {
-  const int ntiles = a.tiles_m * a.tiles_n;
-  return ntiles * (a.mode == MODE_STORE_M ? a.nprod : a.chunks);
-}
+__device__ __forceinline__ int num_units(const GemmArgs& a) { return a.tiles_m * a.tiles_n * a.nprod; }
 
 // ------------------------------------------------------------------------------------
 // Work-unit claims.  One thread of each CTA (the operand issuer) claims the launch's units
@@ -425,17 +373,6 @@ struct UnitReader {
   }
 };
 
-// Warp 0 of the per-thread-copy producer: lane 0 claims, the warp shares the index.
-template <class Src>
-struct WarpClaimer {
-  UnitClaimer<Src> c;
-  __device__ __forceinline__ int next() {
-    int u = 0;
-    if ((threadIdx.x & 31) == 0) u = c.next();
-    return __shfl_sync(0xffffffffu, u, 0);
-  }
-};
-
 __device__ __forceinline__ void unit_ring_init(const UnitRing& q, unsigned readers) {
   for (int s = 0; s < UQ_DEPTH; ++s) {
     mbar_init(q.full(s), 1);
@@ -447,117 +384,60 @@ __device__ __forceinline__ void unit_ring_init(const UnitRing& q, unsigned reade
 // Producer: flattened stream of load units (k step s, term t) over the CTA's work units.
 // ------------------------------------------------------------------------------------
 struct LoadIter {
-  int u;            // work unit index (global over the launch)
-  int j;            // problem of the unit (0 for a single-problem launch)
-  int nks;          // k steps per product of that problem
+  int u;            // work unit index
   Unit w;
-  int r;            // product
   Prod p;
   int T;
   int s, t;
   bool valid;
-  // term t of product r, fetched when the iterator moves so that the global loads are
+  // term t of the product, fetched when the iterator moves so that the global loads are
   // off the producer's critical path
   Term ta, tb;
 };
 
-// Where a launch's work units come from.  OneJob: one problem, the kernel parameter (its
-// fields stay in the parameter space).  JobBatch: many problems in global memory, problem
-// j owning the units [unit_start[j], unit_start[j + 1]).
+// What a launch's claims need (UnitClaimer).
 struct OneJob {
   const GemmArgs& a;
-  __device__ __forceinline__ const GemmArgs& get(int) const { return a; }
-  __device__ __forceinline__ int find(int) const { return 0; }
-  __device__ __forceinline__ int first_unit(int) const { return 0; }
   __device__ __forceinline__ int total() const { return num_units(a); }
   __device__ __forceinline__ unsigned* status() const { return a.status; }
   __device__ __forceinline__ int* counter() const { return a.counter; }
-  __device__ __forceinline__ void acquire_maps(int) const {}
 };
 
-struct JobBatch {
-  const GemmArgs* jobs;
-  const int* unit_start;
-  int njobs, units;
-  unsigned* st;
-  int* ctr;
-  __device__ __forceinline__ const GemmArgs& get(int j) const { return jobs[j]; }
-  __device__ __forceinline__ int find(int u) const {  // last j with unit_start[j] <= u
-    int lo = 0, hi = njobs - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(unit_start + mid) <= u)
-        lo = mid;
-      else
-        hi = mid - 1;
-    }
-    return lo;
-  }
-  __device__ __forceinline__ int first_unit(int j) const { return __ldg(unit_start + j); }
-  __device__ __forceinline__ int total() const { return units; }
-  __device__ __forceinline__ unsigned* status() const { return st; }
-  __device__ __forceinline__ int* counter() const { return ctr; }
-  // The tensor maps were written into global memory by a copy before the launch; order
-  // that write before the tensor-map proxy reads them.
-  __device__ __forceinline__ void acquire_maps(int j) const {
-    const CUtensorMap* m = &jobs[j].tmA;
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(m + q) : "memory");
-  }
-};
+__device__ __forceinline__ int num_ksteps(const GemmArgs& a) { return (a.ks + BK - 1) / BK; }
 
 __device__ __forceinline__ void load_terms(const GemmArgs& a, LoadIter& it) {
   if (it.t < it.p.na) it.ta = a.terms[it.p.a0 + it.t];
   if (it.t < it.p.nb) it.tb = a.terms[it.p.b0 + it.t];
 }
 
-template <bool VARH = false, class Src>
-__device__ __forceinline__ void iter_enter_unit(const Src& src, LoadIter& it) {
-  it.j = src.find(it.u);
-  const GemmArgs& a = src.get(it.j);
-  it.nks = (a.ks + BK - 1) / BK;
-  it.w = decode_unit<VARH>(a, it.u - src.first_unit(it.j));
-  it.r = it.w.r0;
-  it.p = a.prods[it.r];
+__device__ __forceinline__ void iter_enter_unit(const GemmArgs& a, LoadIter& it) {
+  it.w = decode_unit(a, it.u);
+  it.p = a.prods[it.w.r];
   it.T = prod_T(it.p);
   it.s = 0;
   it.t = 0;
   load_terms(a, it);
 }
 
-template <bool VARH = false, class Src, class Nx>
-__device__ __forceinline__ void load_iter_start(const Src& src, LoadIter& it, Nx& nx) {
+template <class Nx>
+__device__ __forceinline__ void load_iter_unit(const GemmArgs& a, LoadIter& it, Nx& nx) {
   it.u = nx.next();
   it.valid = it.u >= 0;
-  if (it.valid) iter_enter_unit<VARH>(src, it);
+  if (it.valid) iter_enter_unit(a, it);
 }
 
-template <class Src, class Nx>
-__device__ __forceinline__ void load_iter_next(const Src& src, LoadIter& it, Nx& nx) {
-  const GemmArgs& a = src.get(it.j);
+template <class Nx>
+__device__ __forceinline__ void load_iter_next(const GemmArgs& a, LoadIter& it, Nx& nx) {
   if (++it.t < it.T) {
     load_terms(a, it);
     return;
   }
   it.t = 0;
-  if (++it.s < it.nks) {
+  if (++it.s < num_ksteps(a)) {
     if (it.T > 1) load_terms(a, it);
     return;
   }
-  it.s = 0;
-  if (++it.r < it.w.r1) {
-    it.p = a.prods[it.r];
-    it.T = prod_T(it.p);
-    load_terms(a, it);
-    return;
-  }
-  it.u = nx.next();
-  if (it.u < 0) {
-    it.valid = false;
-    return;
-  }
-  iter_enter_unit(src, it);
+  load_iter_unit(a, it, nx);
 }
 
 // Raw slot layout (thread-private, conflict-free): pair e of A at [e][pt] (16 B each),
@@ -569,8 +449,8 @@ constexpr int PB = EB / 2;
 __device__ __forceinline__ void issue_unit(const GemmArgs& a, const LoadIter& it, double* raw_slot, int pt) {
   const unsigned sbase = smem_u32(raw_slot);
   if (it.t < it.p.na) {
-    const double* M0 = it.ta.src ? a.Aw : a.A;
-    const long long ld = it.ta.src ? a.ldaw : a.lda;
+    const double* M0 = a.A;
+    const long long ld = a.lda;
     const long long off = (long long)it.ta.row * a.ms + (long long)it.ta.col * a.ks * ld;
     const double* base = M0 + off;
     const bool al16 = ((off & 1) == 0) && ((ld & 1) == 0) && ((reinterpret_cast<uintptr_t>(M0) & 15) == 0);
@@ -591,8 +471,8 @@ __device__ __forceinline__ void issue_unit(const GemmArgs& a, const LoadIter& it
     }
   }
   if (it.t < it.p.nb) {
-    const double* M0 = it.tb.src ? a.Bw : a.B;
-    const long long ld = it.tb.src ? a.ldbw : a.ldb;
+    const double* M0 = a.B;
+    const long long ld = a.ldb;
     const long long off = (long long)it.tb.row * a.ks + (long long)it.tb.col * a.ns * ld;
     const double* base = M0 + off;
     const bool al16 = ((off & 1) == 0) && ((ld & 1) == 0) && ((reinterpret_cast<uintptr_t>(M0) & 15) == 0);
@@ -653,31 +533,40 @@ __device__ __forceinline__ void fold_unit(const LoadIter& it, const double* raw_
   }
 }
 
+// Warp 0 of the per-thread-copy producer: lane 0 claims, the warp shares the index.
+struct WarpClaimer {
+  UnitClaimer<OneJob> c;
+  __device__ __forceinline__ int next() {
+    int u = 0;
+    if ((threadIdx.x & 31) == 0) u = c.next();
+    return __shfl_sync(0xffffffffu, u, 0);
+  }
+};
+
 // The per-thread-copy producer's cursor that runs ahead (issuing copies): warp 0 claims the
 // units, the other producer warps read the ring without freeing entries; the trailing
 // cursor (folding) frees them.
-template <class Src>
 struct IssueCursor {
-  WarpClaimer<Src> c;
+  WarpClaimer c;
   UnitReader r;
   bool claim;  // warp-uniform
   __device__ __forceinline__ int next() { return claim ? c.next() : r.next(); }
 };
 
-template <class Src>
-__device__ __forceinline__ void producer(const Src& src, double* stages, double* raw, unsigned full0, unsigned empty0,
+__device__ __forceinline__ void producer(const GemmArgs& a, double* stages, double* raw, unsigned full0, unsigned empty0,
                                          int pt, const UnitRing& q) {
-  IssueCursor<Src> inx{WarpClaimer<Src>{UnitClaimer<Src>{src, q}}, UnitReader{q, src.status(), false}, pt < 32};
-  UnitReader cnx{q, src.status(), true};
+  const OneJob src{a};
+  IssueCursor inx{WarpClaimer{UnitClaimer<OneJob>{src, q}}, UnitReader{q, a.status, false}, pt < 32};
+  UnitReader cnx{q, a.status, true};
   LoadIter iss, con;
-  load_iter_start(src, iss, inx);
-  load_iter_start(src, con, cnx);
+  load_iter_unit(a, iss, inx);
+  load_iter_unit(a, con, cnx);
   // prologue: NRAW - 1 load units in flight
 #pragma unroll 1
   for (int i = 0; i < NRAW - 1; ++i) {
     if (iss.valid) {
-      issue_unit(src.get(iss.j), iss, raw + (size_t)(i % NRAW) * RAW_SZ, pt);
-      load_iter_next(src, iss, inx);
+      issue_unit(a, iss, raw + (size_t)(i % NRAW) * RAW_SZ, pt);
+      load_iter_next(a, iss, inx);
     }
     cp_async_commit();
   }
@@ -688,13 +577,13 @@ __device__ __forceinline__ void producer(const Src& src, double* stages, double*
     const int stage = (int)(kc % NSTAGE);
     double* opA = stages + (size_t)stage * STAGE_SZ;
     double* opB = opA + OPA_SZ;
-    if (con.t == 0) mbar_wait(empty0 + 8 * stage, (unsigned)(((kc / NSTAGE) & 1) ^ 1), src.status());
+    if (con.t == 0) mbar_wait(empty0 + 8 * stage, (unsigned)(((kc / NSTAGE) & 1) ^ 1), a.status);
     cp_async_wait<NRAW - 2>();
     fold_unit(con, raw + (size_t)(unit % NRAW) * RAW_SZ, opA, opB, pt);
     const bool last_term = (con.t == con.T - 1);
     if (iss.valid) {
-      issue_unit(src.get(iss.j), iss, raw + (size_t)((unit + NRAW - 1) % NRAW) * RAW_SZ, pt);
-      load_iter_next(src, iss, inx);
+      issue_unit(a, iss, raw + (size_t)((unit + NRAW - 1) % NRAW) * RAW_SZ, pt);
+      load_iter_next(a, iss, inx);
     }
     cp_async_commit();
     ++unit;
@@ -703,7 +592,7 @@ __device__ __forceinline__ void producer(const Src& src, double* stages, double*
       if ((pt & 31) == 0) mbar_arrive(full0 + 8 * stage);
       ++kc;
     }
-    load_iter_next(src, con, cnx);
+    load_iter_next(a, con, cnx);
   }
   cp_async_wait<0>();
 }
@@ -731,59 +620,37 @@ __device__ __forceinline__ KStep kstep_info(const GemmArgs& a, const LoadIter& i
   return k;
 }
 
-// Per-k-step iterator over (unit, product, k step); ta / tb hold the first A / B term.
-template <bool VARH = false, class Src, class Nx>
-__device__ __forceinline__ void kiter_next(const Src& src, LoadIter& it, Nx& nx) {
+// Per-k-step iterator over (unit, k step); ta / tb hold the first A / B term.
+template <class Nx>
+__device__ __forceinline__ void kiter_next(const GemmArgs& a, LoadIter& it, Nx& nx) {
   it.t = 0;
-  if (++it.s < it.nks) return;
-  it.s = 0;
-  const GemmArgs& a = src.get(it.j);
-  if (++it.r < it.w.r1) {
-    it.p = a.prods[it.r];
-    it.T = prod_T(it.p);
-    load_terms(a, it);
-    return;
-  }
-  it.u = nx.next();
-  if (it.u < 0) {
-    it.valid = false;
-    return;
-  }
-  iter_enter_unit<VARH>(src, it);
+  if (++it.s >= num_ksteps(a)) load_iter_unit(a, it, nx);
 }
 
-template <class Src>
-__device__ __forceinline__ void tma_issuer(const Src& src, double* stages, double* raw, SlotMeta* meta, unsigned full0,
+__device__ __forceinline__ void tma_issuer(const GemmArgs& a, double* stages, double* raw, SlotMeta* meta, unsigned full0,
                                            unsigned empty0, unsigned rfull0, unsigned rempty0, const UnitRing& q) {
-  UnitClaimer<Src> nx{src, q};
+  const OneJob src{a};
+  UnitClaimer<OneJob> nx{src, q};
   LoadIter it;
-  load_iter_start(src, it, nx);
+  load_iter_unit(a, it, nx);
   long long kc = 0, rc = 0;
-  int mapped = -1;  // problem whose tensor maps were last acquired
 #pragma unroll 1
   while (it.valid) {
-    const GemmArgs& a = src.get(it.j);
-    if (it.j != mapped) {
-      src.acquire_maps(it.j);
-      mapped = it.j;
-    }
     const int stage = (int)(kc % NSTAGE);
     double* opA = stages + (size_t)stage * STAGE_SZ;
     const KStep ks = kstep_info(a, it);
     const int k0 = it.s * BK;
-    mbar_wait(empty0 + 8 * stage, (unsigned)(((kc / NSTAGE) & 1) ^ 1), src.status());
+    mbar_wait(empty0 + 8 * stage, (unsigned)(((kc / NSTAGE) & 1) ^ 1), a.status);
     const unsigned fb = full0 + 8 * stage;
     mbar_arrive_expect_tx(fb, (ks.dirA ? TMA_BYTES_A : 0u) + (ks.dirB ? TMA_BYTES_B8 : 0u));
     if (ks.dirA)
-      tma_load_2d(smem_u32(opA), it.ta.src ? &a.tmAw : &a.tmA, it.ta.row * a.ms + it.w.m0, it.ta.col * a.ks + k0,
-                  fb);
+      tma_load_2d(smem_u32(opA), &a.tmA, it.ta.row * a.ms + it.w.m0, it.ta.col * a.ks + k0, fb);
     if (ks.dirB)
-      tma_load_2d(smem_u32(opA + OPA_SZ), it.tb.src ? &a.tmBw : &a.tmB, it.tb.row * a.ks + k0,
-                  it.tb.col * a.ns + it.w.n0, fb);
+      tma_load_2d(smem_u32(opA + OPA_SZ), &a.tmB, it.tb.row * a.ks + k0, it.tb.col * a.ns + it.w.n0, fb);
 #pragma unroll 1
     for (int t = 0; t < ks.T; ++t, ++rc) {
       const int slot = (int)(rc % NRAW_TMA);
-      if (rc >= NRAW_TMA) mbar_wait(rempty0 + 8 * slot, (unsigned)(((rc / NRAW_TMA) - 1) & 1), src.status());
+      if (rc >= NRAW_TMA) mbar_wait(rempty0 + 8 * slot, (unsigned)(((rc / NRAW_TMA) - 1) & 1), a.status);
       const bool hasA = !ks.dirA && t < it.p.na, hasB = !ks.dirB && t < it.p.nb;
       const unsigned rb = rfull0 + 8 * slot;
       double* rs = raw + (size_t)slot * TRAW_SZ;
@@ -795,11 +662,11 @@ __device__ __forceinline__ void tma_issuer(const Src& src, double* stages, doubl
       meta[slot].shift = xk & 1;
       mbar_arrive_expect_tx(rb, (hasA ? TMA_BYTES_A : 0u) + (hasB ? TMA_BYTES_B : 0u));
       if (hasA)
-        tma_load_2d(smem_u32(rs), tA.src ? &a.tmAw : &a.tmA, tA.row * a.ms + it.w.m0, tA.col * a.ks + k0, rb);
-      if (hasB) tma_load_2d(smem_u32(rs + TRAW_A), tB.src ? &a.tmBw2 : &a.tmB2, xk & ~1, tB.col * a.ns + it.w.n0, rb);
+        tma_load_2d(smem_u32(rs), &a.tmA, tA.row * a.ms + it.w.m0, tA.col * a.ks + k0, rb);
+      if (hasB) tma_load_2d(smem_u32(rs + TRAW_A), &a.tmB2, xk & ~1, tB.col * a.ns + it.w.n0, rb);
     }
     ++kc;
-    kiter_next(src, it, nx);
+    kiter_next(a, it, nx);
   }
   // raw-slot copies still in flight (only on an error path) land before the CTA exits
   for (long long q = rc - NRAW_TMA; q < rc; ++q)
@@ -842,18 +709,16 @@ __device__ __forceinline__ void fold_slot(const double* rs, const SlotMeta& m, b
   }
 }
 
-template <class Src>
-__device__ __forceinline__ void tma_folder(const Src& src, double* stages, const double* raw, const SlotMeta* meta,
+__device__ __forceinline__ void tma_folder(const GemmArgs& a, double* stages, const double* raw, const SlotMeta* meta,
                                            unsigned full0, unsigned empty0, unsigned rfull0, unsigned rempty0, int ft,
                                            const UnitRing& q) {
-  UnitReader nx{q, src.status(), true};
+  UnitReader nx{q, a.status, true};
   LoadIter it;
-  load_iter_start(src, it, nx);
+  load_iter_unit(a, it, nx);
   long long kc = 0, rc = 0;
   const int lane = ft & 31;
 #pragma unroll 1
   while (it.valid) {
-    const GemmArgs& a = src.get(it.j);
     const int stage = (int)(kc % NSTAGE);
     double* opA = stages + (size_t)stage * STAGE_SZ;
     double* opB = opA + OPA_SZ;
@@ -863,14 +728,14 @@ __device__ __forceinline__ void tma_folder(const Src& src, double* stages, const
     // stage's full barrier, even when it has nothing to fold: an arrival made earlier
     // could land in the barrier's previous phase (whose issuer arrival and bytes may
     // still be outstanding) and break that phase's transaction accounting.
-    mbar_wait(empty0 + 8 * stage, (unsigned)(((kc / NSTAGE) & 1) ^ 1), src.status());
+    mbar_wait(empty0 + 8 * stage, (unsigned)(((kc / NSTAGE) & 1) ^ 1), a.status);
     if (ks.T > 0) {
       double2 accA[FPAIRS];
       double accB[FELEMS];
 #pragma unroll 1
       for (int t = 0; t < ks.T; ++t, ++rc) {
         const int slot = (int)(rc % NRAW_TMA);
-        mbar_wait(rfull0 + 8 * slot, (unsigned)((rc / NRAW_TMA) & 1), src.status());
+        mbar_wait(rfull0 + 8 * slot, (unsigned)((rc / NRAW_TMA) & 1), a.status);
         const double* rs = raw + (size_t)slot * TRAW_SZ;
         const bool hasA = !ks.dirA && t < it.p.na, hasB = !ks.dirB && t < it.p.nb;
         if (kvalid >= BK)
@@ -905,7 +770,7 @@ __device__ __forceinline__ void tma_folder(const Src& src, double* stages, const
     __syncwarp();
     if (lane == 0) mbar_arrive(full0 + 8 * stage);
     ++kc;
-    kiter_next(src, it, nx);
+    kiter_next(a, it, nx);
   }
 }
 
@@ -913,100 +778,33 @@ __device__ __forceinline__ void tma_folder(const Src& src, double* stages, const
 // Consumers: DMMA over the stages, then the multi-destination epilogue.
 //
 // Consumer warp (wm, wn) owns tile rows wm*64 + 16i + 0..15 and tile columns
-// frag_col(wn, j) + 0..7 for fragments i, j = 0..3.  The columns are interleaved (warp wn
-// owns wn*8 + 32j) so that a tile cut short by the block edge still spreads its column
-// fragments over all four warps of a row half; with the warp-to-scheduler mapping (warp
-// % 4, i.e. wn) every SM sub-partition then skips about the same share of an edge tile.
+// frag_col(wn, j) + 0..7 for fragments i, j = 0..3.
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ int frag_col(int wn, int j) { return wn * 8 + j * 32; }
 
-// Fragments of warp (wm, wn) that hold rows < vr and columns < vc of the tile: i < im, j < jn.
-__device__ __forceinline__ void frag_counts(int vr, int vc, int wm, int wn, int& im, int& jn) {
-  const int rrem = vr - wm * 64, crem = vc - wn * 8;
-  im = rrem <= 0 ? 0 : min(4, (rrem + 15) >> 4);
-  jn = crem <= 0 ? 0 : min(4, (crem + 31) >> 5);
-}
-
-// One operand stage into the fragments i < IM, j < JN of the accumulator (IM = JN = 4:
-// the whole 64 x 32 warp tile; fewer for the warps of an edge tile, whose other
-// fragments stay as they were and are never written out).  Compile-time counts keep each
-// form straight-line code: shared-memory loads and DMMAs with no predicates.
-// jb: first column fragment (the half-height form gives each row of warps two of the four).
-template <int IM, int JN, int LDA = LDA_S>
-__device__ __forceinline__ void mma_stage_t(const double* opA, const double* opB, double (&acc)[4][4][4], int wm,
-                                            int wn, int g, int t4, int jb = 0) {
+// One operand stage into the 64 x 32 warp tile.
+__device__ __forceinline__ void mma_stage(const double* opA, const double* opB, double (&acc)[4][4][4], int wm, int wn,
+                                          int g, int t4) {
 #pragma unroll
   for (int kq = 0; kq < BK / 4; ++kq) {
     double af[4][2], bf[4];
 #pragma unroll
-    for (int i = 0; i < IM; ++i) {
+    for (int i = 0; i < 4; ++i) {
       const int row = wm * 64 + i * 16 + g;
-      af[i][0] = opA[(kq * 4 + t4) * LDA + row];
-      af[i][1] = opA[(kq * 4 + t4) * LDA + row + 8];
+      af[i][0] = opA[(kq * 4 + t4) * LDA_S + row];
+      af[i][1] = opA[(kq * 4 + t4) * LDA_S + row + 8];
     }
 #pragma unroll
-    for (int j = 0; j < JN; ++j) bf[j] = opB[(frag_col(wn, jb + j) + g) * LDB_S + kq * 4 + t4];
-#pragma unroll
-    for (int i = 0; i < IM; ++i)
-#pragma unroll
-      for (int j = 0; j < JN; ++j) dmma_16x8x4(acc[i][j], af[i], bf[j]);
-  }
-}
-
-template <int IM_, int JN_>
-struct Frags {
-  static constexpr int IM = IM_, JN = JN_;
-};
-
-// Calls f(Frags<IM, JN>{}) with IM >= im, JN >= jn, so that a k loop written once is
-// compiled for the edge shapes: full tiles (4, 4), bottom-edge (1..3, 4), right-edge
-// (4, 1..3) and idle warps (0, 0); a corner takes the cheaper of its two edge forms.
-// Extra fragments are harmless, and eight forms instead of all seventeen keep the
-// consumer code small: on B200 the full set cost 1.5 % on short-k shapes.
-template <class F>
-__device__ __forceinline__ void with_frags(int im, int jn, F&& f) {
-  if (im == 4 && jn == 4) {
-    f(Frags<4, 4>{});
-    return;
-  }
-  if (im <= 0 || jn <= 0) {
-    f(Frags<0, 0>{});
-    return;
-  }
-  if (jn < 4 && (im == 4 || jn < im)) {
-    switch (jn) {
-      case 1: f(Frags<4, 1>{}); break;
-      case 2: f(Frags<4, 2>{}); break;
-      default: f(Frags<4, 3>{}); break;
-    }
-    return;
-  }
-  switch (im) {
-    case 1: f(Frags<1, 4>{}); break;
-    case 2: f(Frags<2, 4>{}); break;
-    case 3: f(Frags<3, 4>{}); break;
-    default: f(Frags<4, 4>{}); break;
-  }
-}
-
-__device__ __forceinline__ void epilogue(const GemmArgs& a, const Prod& p, int r, const double (&acc)[4][4][4],
-                                         int m0, int n0, int wm, int wn, int g, int t4) {
-  if (a.mode == MODE_STORE_M) {
-    double* Mr = a.M + (long long)r * a.m_stride;
+    for (int j = 0; j < 4; ++j) bf[j] = opB[(frag_col(wn, j) + g) * LDB_S + kq * 4 + t4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int rr = m0 + wm * 64 + i * 16 + g + 8 * h;
-            const int cc = n0 + frag_col(wn, j) + t4 * 2 + q;
-            if (rr < a.ms && cc < a.ns) Mr[rr + (long long)cc * a.ldm] = acc[i][j][2 * h + q];
-          }
-    return;
+      for (int j = 0; j < 4; ++j) dmma_16x8x4(acc[i][j], af[i], bf[j]);
   }
+}
+
+__device__ __forceinline__ void epilogue(const GemmArgs& a, const Prod& p, const double (&acc)[4][4][4],
+                                         int m0, int n0, int wm, int wn, int g, int t4) {
   // C_l += w * M_r, 4 * C_BATCH_J elements at a time: all loads of a batch are issued before
   // any store, so a batch costs one memory round trip instead of one per element.
 #pragma unroll 1
@@ -1046,7 +844,6 @@ __device__ __forceinline__ void epilogue(const GemmArgs& a, const Prod& p, int r
 
 // Pull the C tiles an epilogue will update into L2 while the product's last k steps run.
 __device__ __forceinline__ void prefetch_c_tiles(const GemmArgs& a, const Prod& p, int m0, int n0, int ct) {
-  if (a.mode != MODE_ACCUM_C) return;
   for (int c = 0; c < p.nc; ++c) {
     const Term tm = a.terms[p.c0 + c];
     const double* Cb = a.C + (long long)tm.row * a.ms + (long long)tm.col * a.ns * a.ldc;
@@ -1072,62 +869,53 @@ __device__ __forceinline__ void ticket_release(const GemmArgs& a, int tile, int 
   if (ct == 0) st_release(a.tickets + tile, chunk + 1);
 }
 
-template <class Src>
-__device__ __forceinline__ void consumer(const Src& src, const double* stages, unsigned full0, unsigned empty0,
+__device__ __forceinline__ void consumer(const GemmArgs& a, const double* stages, unsigned full0, unsigned empty0,
                                          int ct, const UnitRing& q) {
   const int warp = ct >> 5, lane = ct & 31;
   const int g = lane >> 2, t4 = lane & 3;
   const int wm = warp >> 2, wn = warp & 3;
-  UnitReader nx{q, src.status(), true};
+  UnitReader nx{q, a.status, true};
   long long kc = 0;
   double acc[4][4][4];
+  const int nks = num_ksteps(a);
+  const bool ordered = a.nprod > 1;
 #pragma unroll 1
   for (int u = nx.next(); u >= 0; u = nx.next()) {
-    const int job = src.find(u);
-    const GemmArgs& a = src.get(job);
-    const int ul = u - src.first_unit(job);
-    const int ntiles = a.tiles_m * a.tiles_n;
-    const bool ordered = (a.mode == MODE_ACCUM_C) && a.chunks > 1;
-    const int nks = (a.ks + BK - 1) / BK;
-    const Unit w = decode_unit(a, ul);
-    const int chunk = ul / ntiles;
+    const Unit w = decode_unit(a, u);
+    const Prod p = a.prods[w.r];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
 #pragma unroll 1
-    for (int r = w.r0; r < w.r1; ++r) {
-      const Prod p = a.prods[r];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
-#pragma unroll 1
-      for (int s = 0; s < nks; ++s) {
-        const int stage = (int)(kc % NSTAGE);
-        const double* opA = stages + (size_t)stage * STAGE_SZ;
-        const double* opB = opA + OPA_SZ;
-        mbar_wait(full0 + 8 * stage, (unsigned)((kc / NSTAGE) & 1), src.status());
-        if (s == (nks > C_PREFETCH_STEPS ? nks - C_PREFETCH_STEPS : 0)) prefetch_c_tiles(a, p, w.m0, w.n0, ct);
-        mma_stage_t<4, 4>(opA, opB, acc, wm, wn, g, t4);
-        // The stage is refilled by TMA as soon as every warp has arrived; the fence
-        // makes this warp's shared-memory fragment loads complete before its arrival
-        // (measured: without it a refill could overwrite fragments still in flight).
-        __threadfence_block();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(empty0 + 8 * stage);
-        ++kc;
-      }
-      if (ordered && r == w.r0) ticket_wait(a, w.tile, chunk, ct);
-      epilogue(a, p, r, acc, w.m0, w.n0, wm, wn, g, t4);
+    for (int s = 0; s < nks; ++s) {
+      const int stage = (int)(kc % NSTAGE);
+      const double* opA = stages + (size_t)stage * STAGE_SZ;
+      const double* opB = opA + OPA_SZ;
+      mbar_wait(full0 + 8 * stage, (unsigned)((kc / NSTAGE) & 1), a.status);
+      if (s == (nks > C_PREFETCH_STEPS ? nks - C_PREFETCH_STEPS : 0)) prefetch_c_tiles(a, p, w.m0, w.n0, ct);
+      mma_stage(opA, opB, acc, wm, wn, g, t4);
+      // The stage is refilled by TMA as soon as every warp has arrived; the fence
+      // makes this warp's shared-memory fragment loads complete before its arrival
+      // (measured: without it a refill could overwrite fragments still in flight).
+      __threadfence_block();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty0 + 8 * stage);
+      ++kc;
     }
-    if (ordered) ticket_release(a, w.tile, chunk, ct);
+    if (ordered) ticket_wait(a, w.tile, w.r, ct);
+    epilogue(a, p, acc, w.m0, w.n0, wm, wn, g, t4);
+    if (ordered) ticket_release(a, w.tile, w.r, ct);
   }
 }
 
 // Persistent: one CTA per SM takes work units in claim order (UnitClaimer) until none is left.
 // TMA = true stages operands with tensor copies (A, B 16-byte aligned, even leading
 // dimensions); TMA = false with per-thread cp.async (any alignment).
-template <bool TMA, class Src>
-__device__ __forceinline__ void gemm_cta(const Src& src) {
+template <bool TMA>
+__global__ void __launch_bounds__(NTHREADS, 1) fmm_gemm_kernel(const __grid_constant__ GemmArgs a) {
   extern __shared__ __align__(128) double smem[];
   double* stages = smem;                                  // [NSTAGE][STAGE_SZ]
   double* raw = stages + (size_t)NSTAGE * STAGE_SZ;       // [NRAW][RAW_SZ] or [NRAW_TMA][TRAW_SZ]
@@ -1160,435 +948,170 @@ __device__ __forceinline__ void gemm_cta(const Src& src) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(PROD_REGS));
     if (TMA) {
       if (tid == 0)
-        tma_issuer(src, stages, raw, meta, full0, empty0, rfull0, rempty0, q);
+        tma_issuer(a, stages, raw, meta, full0, empty0, rfull0, rempty0, q);
       else if (tid >= 32)
-        tma_folder(src, stages, raw, meta, full0, empty0, rfull0, rempty0, tid - 32, q);
+        tma_folder(a, stages, raw, meta, full0, empty0, rfull0, rempty0, tid - 32, q);
     } else {
-      producer(src, stages, raw, full0, empty0, tid, q);
+      producer(a, stages, raw, full0, empty0, tid, q);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(CONS_REGS));
-    consumer(src, stages, full0, empty0, tid - NPROD, q);
+    consumer(a, stages, full0, empty0, tid - NPROD, q);
   }
 }
 
-template <bool TMA>
-__global__ void __launch_bounds__(NTHREADS, 1) fmm_gemm_kernel(const __grid_constant__ GemmArgs a) {
-  gemm_cta<TMA>(OneJob{a});
-}
-
-// Many independent problems (each with its own plan tables, operands, sizes, tensor maps
-// and tickets) in one persistent launch: the units of all problems form one sequence,
-// problem j owning [unit_start[j], unit_start[j + 1]).
-struct BatchArgs {
-  const GemmArgs* jobs;    // global memory, 64-byte aligned (tensor maps inside)
-  const int* unit_start;   // njobs + 1 entries
-  int njobs;
-  int units;
-  unsigned* status;
-  int* counter;            // work units claimed so far (zeroed before launch)
+// Operand sums in HBM: slot j = sum_t coef_t * X_{blk_t} over the A (or B) terms of product
+// plist[j], the slot's k extent rounded up with zeros.  HBM bound: every input element once,
+// every slot element once; an input element feeds nnz(U) / blocks sums (15 for 222-1 x 333-1),
+// which come from L1 and L2.  A CTA owns a range of element positions and walks all its
+// outputs, so that the blocks' values at those positions stay close; the terms' offsets and
+// coefficients are in shared memory.
+struct PTerm {
+  int row, col;  // block
+  double coef;
 };
 
-template <bool TMA>
-__global__ void __launch_bounds__(NTHREADS, 1) fmm_gemm_batch_kernel(const BatchArgs b) {
-  gemm_cta<TMA>(JobBatch{b.jobs, b.unit_start, b.njobs, b.units, b.status, b.counter});
-}
-
-// ------------------------------------------------------------------------------------
-// Direct variant: every operand of every product is one unit-coefficient block staged by
-// TMA straight into the stage (the pre-summed ABC path and the classical plan) and ks is a
-// multiple of BK, so no term is folded.  The seven folding warps then run the
-// multi-destination C epilogue instead: the consumers write each finished product tile
-// into shared memory (one 128 x 128 FP64 buffer, in place of the raw slots and two of the
-// stages) and go straight on with the next product, while warps 1..7 add W[l,r] * M_r into
-// the C blocks from it.  The epilogue overlaps the DMMAs of the next product.
-// ------------------------------------------------------------------------------------
-constexpr int NSTAGE_D = 4;
-constexpr int MS_LD = BM + 1;  // product tile in shared memory: column-major, padded
-constexpr int NEPI_D = NFOLD;  // epilogue threads (warps 1..7)
-static_assert((size_t)(NSTAGE_D * STAGE_SZ + BN * (BM + 1)) * sizeof(double) + 80 <= 232448, "direct variant shared memory");
-constexpr size_t SMEM_BYTES_DIRECT = (size_t)(NSTAGE_D * STAGE_SZ + BN * MS_LD) * sizeof(double) +
-                                     (2 * NSTAGE_D + 2) * sizeof(unsigned long long) + RING_BYTES;
-
-template <class Src>
-__device__ __forceinline__ void direct_issuer(const Src& src, double* stages, unsigned full0, unsigned empty0,
-                                              const UnitRing& q) {
-  UnitClaimer<Src> nx{src, q};
-  LoadIter it;
-  load_iter_start<true>(src, it, nx);
-  long long kc = 0;
-  int mapped = -1;
-#pragma unroll 1
-  while (it.valid) {
-    const GemmArgs& a = src.get(it.j);
-    if (it.j != mapped) {
-      src.acquire_maps(it.j);
-      mapped = it.j;
-    }
-    const int stage = (int)(kc % NSTAGE_D);
-    double* opA = stages + (size_t)stage * STAGE_SZ;
-    const int k0 = it.s * BK;
-    mbar_wait(empty0 + 8 * stage, (unsigned)(((kc / NSTAGE_D) & 1) ^ 1), src.status());
-    const unsigned fb = full0 + 8 * stage;
-    const bool half = unit_half(a, it.w);  // half-height unit: a BM / 2-row A box, dense [k][BM / 2]
-    mbar_arrive_expect_tx(fb, (half ? TMA_BYTES_A / 2 : TMA_BYTES_A) + TMA_BYTES_B8);
-    const CUtensorMap* ma = it.ta.src ? (half ? &a.tmAw64 : &a.tmAw) : (half ? &a.tmA64 : &a.tmA);
-    tma_load_2d(smem_u32(opA), ma, it.ta.row * a.ms + it.w.m0, it.ta.col * a.ks + k0, fb);
-    tma_load_2d(smem_u32(opA + OPA_SZ), it.tb.src ? &a.tmBw : &a.tmB, it.tb.row * a.ks + k0,
-                it.tb.col * a.ns + it.w.n0, fb);
-    ++kc;
-    kiter_next<true>(src, it, nx);
-  }
-  // copies still in flight (only on an error path) land before the CTA exits
-  for (long long q = kc - NSTAGE_D; q < kc; ++q)
-    if (q >= 0) mbar_wait_drain(full0 + 8 * (int)(q % NSTAGE_D), (unsigned)((q / NSTAGE_D) & 1));
-}
-
-template <class Src>
-__device__ __forceinline__ void direct_consumer(const Src& src, const double* stages, double* Ms, unsigned full0,
-                                                unsigned empty0, unsigned mfull, unsigned mempty, int ct,
-                                                const UnitRing& uq) {
-  const int warp = ct >> 5, lane = ct & 31;
-  const int g = lane >> 2, t4 = lane & 3;
-  const int wm = warp >> 2, wn = warp & 3;
-  UnitReader nx{uq, src.status(), true};
-  long long kc = 0, q = 0;
-  double acc[4][4][4];
-#pragma unroll 1
-  for (int u = nx.next(); u >= 0; u = nx.next()) {
-    const int job = src.find(u);
-    const GemmArgs& a = src.get(job);
-    const int nks = (a.ks + BK - 1) / BK;
-    const Unit w = decode_unit<true>(a, u - src.first_unit(job));
-    const bool half = unit_half(a, w);
-    int im, jn;
-    frag_counts(a.ms - w.m0, a.ns - w.n0, wm, wn, im, jn);
-#pragma unroll 1
-    for (int r = w.r0; r < w.r1; ++r, ++q) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
-      if (half) {
-        // both rows of warps on the tile's BM / 2 rows, warp row wm taking the column
-        // fragments 2 wm, 2 wm + 1 of its warp column: each element gets the DMMAs of a full
-        // tile in the same order (results equal a full tile's bit for bit), in half the time
-#pragma unroll 1
-        for (int s = 0; s < nks; ++s, ++kc) {
-          const int stage = (int)(kc % NSTAGE_D);
-          const double* opA = stages + (size_t)stage * STAGE_SZ;
-          mbar_wait(full0 + 8 * stage, (unsigned)((kc / NSTAGE_D) & 1), src.status());
-          mma_stage_t<4, 2, BM / 2>(opA, opA + OPA_SZ, acc, 0, wn, g, t4, 2 * wm);
-          __threadfence_block();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(empty0 + 8 * stage);
-        }
-      } else {
-        with_frags(im, jn, [&](auto fr) {
-          using FR = decltype(fr);
-#pragma unroll 1
-          for (int s = 0; s < nks; ++s, ++kc) {
-            const int stage = (int)(kc % NSTAGE_D);
-            const double* opA = stages + (size_t)stage * STAGE_SZ;
-            mbar_wait(full0 + 8 * stage, (unsigned)((kc / NSTAGE_D) & 1), src.status());
-            mma_stage_t<FR::IM, FR::JN>(opA, opA + OPA_SZ, acc, wm, wn, g, t4);
-            __threadfence_block();  // fragment loads complete before the stage can be refilled
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty0 + 8 * stage);
-          }
-        });
-      }
-      // hand the product tile to the epilogue warps once they are done with the previous one
-      mbar_wait(mempty, (unsigned)((q & 1) ^ 1), src.status());
-      if (half) {  // rows 0..63, this warp's two column fragments
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int e = 0; e < 2; ++e)
-                Ms[(frag_col(wn, 2 * wm + j) + t4 * 2 + e) * MS_LD + i * 16 + g + 8 * h] = acc[i][j][2 * h + e];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int rr = wm * 64 + i * 16 + g + 8 * h;
-                const int cc = frag_col(wn, j) + t4 * 2 + e;
-                Ms[cc * MS_LD + rr] = acc[i][j][2 * h + e];
-              }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(mfull);
-    }
-  }
-}
-
-template <class Src>
-__device__ __forceinline__ void direct_epilogue(const Src& src, const double* Ms, unsigned mfull, unsigned mempty,
-                                                int et, const UnitRing& uq) {
-  const int ew = et >> 5, lane = et & 31;
-  constexpr int NW = NEPI_D / 32;  // 7 warps
-  UnitReader nx{uq, src.status(), true};
-  long long q = 0;
-#pragma unroll 1
-  for (int u = nx.next(); u >= 0; u = nx.next()) {
-    const int job = src.find(u);
-    const GemmArgs& a = src.get(job);
-    const int ul = u - src.first_unit(job);
-    const int ntiles = a.tiles_m * a.tiles_n;
-    const bool ordered = (a.mode == MODE_ACCUM_C) && a.chunks > 1;
-    const Unit w = decode_unit<true>(a, ul);
-    const int rows = unit_rows(a, w);
-    const int chunk = ul / ntiles;
-#pragma unroll 1
-    for (int r = w.r0; r < w.r1; ++r, ++q) {
-      const Prod p = a.prods[r];
-      // the unit's C tiles into L2 while its product is still being computed
-      for (int c = 0; a.mode == MODE_ACCUM_C && c < p.nc; ++c) {
-        const Term tm = a.terms[p.c0 + c];
-        const double* Cb = a.C + (long long)tm.row * a.ms + (long long)tm.col * a.ns * a.ldc;
-        for (int l = et; l < (BM / 16) * BN; l += NEPI_D) {
-          const int ri = (l % (BM / 16)) * 16, cc = w.n0 + l / (BM / 16);
-          if (ri < rows && cc < a.ns)
-            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(Cb + w.m0 + ri + (long long)cc * a.ldc));
-        }
-      }
-      mbar_wait(mfull, (unsigned)(q & 1), src.status());
-      if (a.mode == MODE_STORE_M) {  // the product tile to its workspace (the AB pack type)
-        double* Mr = a.M + (long long)r * a.m_stride + w.m0 + lane;
-        const int rmax = rows - lane;
-#pragma unroll 1
-        for (int col = ew; col < BN; col += NW) {
-          if (w.n0 + col >= a.ns) continue;
-          double* mp = Mr + (long long)(w.n0 + col) * a.ldm;
-#pragma unroll
-          for (int ch = 0; ch < 4; ++ch)
-            if (ch * 32 < rmax) mp[ch * 32] = Ms[col * MS_LD + lane + ch * 32];
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(mempty);
-        continue;
-      }
-      const bool per_block = ordered && a.nbt > 0;
-      if (ordered && !per_block && r == w.r0) {
-        if (et == 0) ticket_spin(a.tickets + w.tile, chunk, a.status, 256);
-        named_bar_sync(2, NEPI_D);
-      }
-      // C_l += w * M_r: warp ew takes columns ew, ew + 7, ... four at a time; a lane owns rows
-      // lane, lane + 32, lane + 64, lane + 96, so loads and stores are 256-byte coalesced and
-      // 16 loads are in flight per lane before the stores
-#pragma unroll 1
-      for (int c = 0; c < p.nc; ++c) {
-        const Term tm = a.terms[p.c0 + c];
-        const double wgt = tm.coef;
-        int* tk = nullptr;
-        if (per_block) {  // wait for the previous product that updates this C block
-          tk = a.tickets + (long long)w.tile * a.nbt + tm.row * a.nbc + tm.col;
-          if (et == 0) ticket_spin(tk, tm.pad, a.status, 128);
-          named_bar_sync(2, NEPI_D);
-        }
-        double* Cb = a.C + (long long)tm.row * a.ms + (long long)tm.col * a.ns * a.ldc + w.m0 + lane;
-        const int rmax = rows - lane;  // rows of this lane inside the tile: rr < rmax
-#pragma unroll 1
-        for (int col0 = ew; col0 < BN; col0 += NW * 4) {
-          double cv[4][4];
-#pragma unroll
-          for (int cb = 0; cb < 4; ++cb) {
-            const int col = col0 + cb * NW;
-            const bool cok = col < BN && w.n0 + col < a.ns;
-            const double* cp = Cb + (long long)(w.n0 + col) * a.ldc;
-#pragma unroll
-            for (int ch = 0; ch < 4; ++ch) cv[cb][ch] = (cok && ch * 32 < rmax) ? cp[ch * 32] : 0.0;
-          }
-#pragma unroll
-          for (int cb = 0; cb < 4; ++cb) {
-            const int col = col0 + cb * NW;
-            if (!(col < BN && w.n0 + col < a.ns)) continue;
-            double* cp = Cb + (long long)(w.n0 + col) * a.ldc;
-            const double* mp = Ms + col * MS_LD + lane;
-#pragma unroll
-            for (int ch = 0; ch < 4; ++ch)
-              if (ch * 32 < rmax) cp[ch * 32] = fma(wgt, mp[ch * 32], cv[cb][ch]);
-          }
-        }
-        if (tk) {  // this block's update is visible before the next product may start its own
-          __threadfence();
-          named_bar_sync(2, NEPI_D);
-          if (et == 0) st_release(tk, tm.pad + 1);
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(mempty);  // the buffer can take the next product
-    }
-    if (ordered && a.nbt == 0) {
-      __threadfence();
-      named_bar_sync(2, NEPI_D);
-      if (et == 0) st_release(a.tickets + w.tile, chunk + 1);
-    }
-  }
-}
-
-template <class Src>
-__device__ __forceinline__ void gemm_cta_direct(const Src& src) {
-  extern __shared__ __align__(128) double smem[];
-  double* stages = smem;                                        // [NSTAGE_D][STAGE_SZ]
-  double* Ms = stages + (size_t)NSTAGE_D * STAGE_SZ;            // [BN][MS_LD]
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(Ms + (size_t)BN * MS_LD);
-  const unsigned full0 = smem_u32(bars);
-  const unsigned empty0 = smem_u32(bars + NSTAGE_D);
-  const unsigned mfull = smem_u32(bars + 2 * NSTAGE_D);
-  const unsigned mempty = smem_u32(bars + 2 * NSTAGE_D + 1);
-  const UnitRing q{smem_u32(bars + 2 * NSTAGE_D + 2)};
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    for (int s = 0; s < NSTAGE_D; ++s) {
-      mbar_init(full0 + 8 * s, 1);             // the issuer's arrival + TMA bytes
-      mbar_init(empty0 + 8 * s, NCONS / 32);
-    }
-    mbar_init(mfull, NCONS / 32);
-    mbar_init(mempty, NEPI_D / 32);
-    unit_ring_init(q, (NEPI_D + NCONS) / 32);  // ring readers: epilogue + consumer warps
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncthreads();
-  if (tid < NPROD) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(PROD_REGS));
-    if (tid == 0)
-      direct_issuer(src, stages, full0, empty0, q);
-    else if (tid >= 32)
-      direct_epilogue(src, Ms, mfull, mempty, tid - 32, q);
-  } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(CONS_REGS));
-    direct_consumer(src, stages, Ms, full0, empty0, mfull, mempty, tid - NPROD, q);
-  }
-}
-
-__global__ void __launch_bounds__(NTHREADS, 1) fmm_gemm_direct_kernel(const __grid_constant__ GemmArgs a) {
-  gemm_cta_direct(OneJob{a});
-}
-
-__global__ void __launch_bounds__(NTHREADS, 1) fmm_gemm_direct_batch_kernel(const BatchArgs b) {
-  gemm_cta_direct(JobBatch{b.jobs, b.unit_start, b.njobs, b.units, b.status, b.counter});
-}
-
-// Operand sums in HBM: out_j = sum_t coef_t * X_{blk_t} for the A terms (side 0) or the
-// B terms (side 1) of product plist[j] (j = blockIdx.y).  Used for the NAIVE pack
-// type's S_r / T_r temporaries and for the pre-summed operands of the ABC pack type.
-// Each thread handles two consecutive rows of a column (16-byte loads and stores when
-// the addresses allow).
-struct LincombArgs {
+struct PresumSide {
   const double* X;
   long long ldx;
-  int rows, cols;          // sub-block size
+  int rows, cols;          // block size
+  int orows, ocols;        // slot size (orows even)
   int blk_row_stride;      // rows per block row (ms for A, ks for B)
   int blk_col_stride;      // cols per block column (ks for A, ns for B)
   double* out;
-  long long ldo;
-  long long out_stride;    // per output
-  const Prod* prods;
-  const Term* terms;
+  long long ldo;           // even
+  long long out_stride;
   const int* plist;        // product of each output; nullptr = output j is product j
-  int side;
-};
-
-// Elements per block: output j = blockIdx.x varies fastest in the grid, so the blocks
-// resident at one time cover the same element range for many outputs and read each input
-// element from HBM about once (the other reads hit L2).
-constexpr int LINCOMB_CHUNK = 256 * 16;  // row pairs per block
-
-__device__ __forceinline__ long long lincomb_pairs(const LincombArgs& a) {
-  return (long long)((a.rows + 1) / 2) * a.cols;
-}
-
-__device__ __forceinline__ void lincomb_body(const LincombArgs& a, int j, long long chunk) {
-  const int r = a.plist ? a.plist[j] : j;
-  const Prod p = a.prods[r];
-  const int t0 = a.side == 0 ? p.a0 : p.b0;
-  const int nt = a.side == 0 ? p.na : p.nb;
-  double* out = a.out + (long long)j * a.out_stride;
-  const int hr = (a.rows + 1) / 2;  // row pairs per column
-  const long long total = lincomb_pairs(a);
-  const long long e1 = min(total, (chunk + 1) * LINCOMB_CHUNK);
-  long long e = chunk * LINCOMB_CHUNK + threadIdx.x;
-  int ip = (int)(e % hr);  // row pair and column of element e, then stepped without division
-  long long c = e / hr;
-  for (; e < e1; e += blockDim.x) {
-    const int i = 2 * ip;
-    const bool two = i + 1 < a.rows;
-    double v0 = 0.0, v1 = 0.0;
-    // terms in groups of four: the group's loads are issued before its fmas, so a thread
-    // keeps several loads in flight (the sum order is unchanged)
-    for (int tg = 0; tg < nt; tg += 4) {
-      double x0[4], x1[4], cf[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        x0[q] = x1[q] = cf[q] = 0.0;
-        if (tg + q < nt) {
-          const Term tm = a.terms[t0 + tg + q];
-          cf[q] = tm.coef;
-          const double* x =
-              a.X + (long long)tm.row * a.blk_row_stride + i + ((long long)tm.col * a.blk_col_stride + c) * a.ldx;
-          if (two && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-            const double2 xx = *reinterpret_cast<const double2*>(x);
-            x0[q] = xx.x;
-            x1[q] = xx.y;
-          } else {
-            x0[q] = x[0];
-            if (two) x1[q] = x[1];
-          }
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int t = tg + q;
-        if (t < nt) {
-          v0 = (t == 0) ? cf[q] * x0[q] : fma(cf[q], x0[q], v0);
-          v1 = (t == 0) ? cf[q] * x1[q] : fma(cf[q], x1[q], v1);
-        }
-      }
-    }
-    double* o = out + i + c * a.ldo;
-    if (two && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-      *reinterpret_cast<double2*>(o) = make_double2(v0, v1);
-    } else {
-      o[0] = v0;
-      if (two) o[1] = v1;
-    }
-    ip += blockDim.x;
-    while (ip >= hr) {
-      ip -= hr;
-      ++c;
-    }
-  }
-}
-
-__global__ void fmm_lincomb_kernel(const LincombArgs a) {
-  const long long nchunk = (lincomb_pairs(a) + LINCOMB_CHUNK - 1) / LINCOMB_CHUNK;
-  for (long long c = blockIdx.y; c < nchunk; c += gridDim.y) lincomb_body(a, blockIdx.x, c);
-}
-
-// The operand sums of many problems in one launch: task blockIdx.z, output blockIdx.x
-// (tasks with fewer outputs return at once), element chunks over blockIdx.y.
-struct LincombTask {
-  LincombArgs a;
+  const int* first;        // per product its first term (R + 1 entries)
+  const PTerm* terms;
   int nout;
   int pad;
 };
 
-__global__ void fmm_lincomb_batch_kernel(const LincombTask* tasks) {
-  const LincombTask& tk = tasks[blockIdx.z];
-  if ((int)blockIdx.x >= tk.nout) return;
-  const long long nchunk = (lincomb_pairs(tk.a) + LINCOMB_CHUNK - 1) / LINCOMB_CHUNK;
-  for (long long c = blockIdx.y; c < nchunk; c += gridDim.y) lincomb_body(tk.a, blockIdx.x, c);
+constexpr int PS_THREADS = 256;
+constexpr int PS_TERMS = 2048;  // terms of one pass over the outputs (32 KB of shared memory at most)
+
+struct PresumOff {
+  long long off;
+  double coef;
+};
+
+__device__ __forceinline__ PresumOff presum_term(const PresumSide& a, const PTerm& t) {
+  return PresumOff{(long long)t.row * a.blk_row_stride + (long long)t.col * a.blk_col_stride * a.ldx, t.coef};
+}
+
+// Two rows of one column of the sum of terms [0, n): loads four terms at a time before their
+// fmas, so that several loads are in flight (the sum order is the term order).
+template <bool VEC, class Tm>
+__device__ __forceinline__ double2 presum_sum(const double* x0, int n, bool v0, bool v1, Tm&& term) {
+  double2 v = make_double2(0.0, 0.0);
+#pragma unroll 1
+  for (int tg = 0; tg < n; tg += 4) {
+    double2 x[4];
+    double cf[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      x[q] = make_double2(0.0, 0.0);
+      cf[q] = 0.0;
+      if (tg + q < n) {
+        const PresumOff o = term(tg + q);
+        cf[q] = o.coef;
+        if (VEC) {
+          if (v1) x[q] = __ldg(reinterpret_cast<const double2*>(x0 + o.off));
+        } else {
+          if (v0) x[q].x = __ldg(x0 + o.off);
+          if (v1) x[q].y = __ldg(x0 + o.off + 1);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (tg + q < n) {
+        v.x = (tg + q == 0) ? cf[q] * x[q].x : fma(cf[q], x[q].x, v.x);
+        v.y = (tg + q == 0) ? cf[q] * x[q].y : fma(cf[q], x[q].y, v.y);
+      }
+  }
+  return v;
+}
+
+// Outputs [j0, j1) at the positions of chunk `chunk`.
+__device__ __forceinline__ void presum_body(const PresumSide& a, PresumOff* tab, int cap, long long chunk, int j0, int j1) {
+  const int hr = a.orows / 2;
+  const long long e = chunk * PS_THREADS + threadIdx.x;
+  const bool live = e < (long long)hr * a.ocols;
+  const long long c = live ? e / hr : 0;
+  const int i = live ? 2 * (int)(e - c * hr) : 0;
+  const bool v0 = live && c < a.cols && i < a.rows, v1 = live && c < a.cols && i + 1 < a.rows;
+  const double* x0 = a.X + i + c * a.ldx;
+  double* o = a.out + i + c * a.ldo;
+  // pairs are 16-byte aligned and whole: even strides, base aligned, even row count
+  const bool vec = ((reinterpret_cast<uintptr_t>(a.X) & 15) == 0) && ((a.ldx | a.blk_row_stride | a.rows) & 1) == 0;
+  auto prod = [&](int j) { return a.plist ? __ldg(a.plist + j) : j; };
+  for (int j = j0; j < j1;) {
+    // as many outputs as the table holds (usually all of them)
+    const int t0 = __ldg(a.first + prod(j));
+    int je = j1;
+    if (__ldg(a.first + prod(je - 1) + 1) - t0 > cap) {
+      je = j;
+      while (je < j1 && __ldg(a.first + prod(je) + 1) - t0 <= cap) ++je;
+    }
+    if (je == j) {  // one output with more terms than the table: from global memory
+      const PTerm* tg = a.terms + t0;
+      const double2 v = presum_sum<false>(x0, __ldg(a.first + prod(j) + 1) - t0, v0, v1,
+                                          [&](int t) { return presum_term(a, tg[t]); });
+      if (live) *reinterpret_cast<double2*>(o + j * a.out_stride) = v;
+      ++j;
+      continue;
+    }
+    const int nt = __ldg(a.first + prod(je - 1) + 1) - t0;
+    __syncthreads();
+    for (int t = threadIdx.x; t < nt; t += PS_THREADS) tab[t] = presum_term(a, a.terms[t0 + t]);
+    __syncthreads();
+    for (; j < je; ++j) {
+      const int r = prod(j), f = __ldg(a.first + r), n = __ldg(a.first + r + 1) - f;
+      const PresumOff* tp = tab + (f - t0);
+      const double2 v = vec ? presum_sum<true>(x0, n, v0, v1, [&](int t) { return tp[t]; })
+                            : presum_sum<false>(x0, n, v0, v1, [&](int t) { return tp[t]; });
+      if (live) *reinterpret_cast<double2*>(o + j * a.out_stride) = v;
+    }
+  }
+}
+
+__device__ __forceinline__ long long presum_chunks(const PresumSide& a) {
+  return ((long long)(a.orows / 2) * a.ocols + PS_THREADS - 1) / PS_THREADS;
+}
+
+// Both sides of one call (blockIdx.z); blockIdx.x position chunks, blockIdx.y output ranges.
+// Also zeroes the products launch's tickets and work-unit counter (zero[0 .. nzero)).
+struct PresumArgs {
+  PresumSide s[2];
+  int* zero;
+  int nzero;
+  int cap;  // terms the dynamic shared memory holds
+};
+
+__global__ void __launch_bounds__(PS_THREADS) fmm_presum_kernel(const __grid_constant__ PresumArgs g) {
+  extern __shared__ __align__(16) PresumOff ptab[];
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  const PresumSide& a = g.s[blockIdx.z];
+  if (blockIdx.z == 0 && blockIdx.y == 0)
+    for (long long q = (long long)blockIdx.x * PS_THREADS + threadIdx.x; q < g.nzero; q += (long long)gridDim.x * PS_THREADS)
+      g.zero[q] = 0;
+  const int j0 = (int)((long long)a.nout * blockIdx.y / gridDim.y), j1 = (int)((long long)a.nout * (blockIdx.y + 1) / gridDim.y);
+  if (j0 == j1) return;
+  const long long nc = presum_chunks(a);
+  for (long long c = blockIdx.x; c < nc; c += gridDim.x) presum_body(a, ptab, g.cap, c, j0, j1);
+}
+
+// The operand sums of many problems in one launch (task blockIdx.z).
+__global__ void __launch_bounds__(PS_THREADS) fmm_presum_batch_kernel(const PresumSide* tasks, int cap) {
+  extern __shared__ __align__(16) PresumOff ptab[];
+  const PresumSide a = tasks[blockIdx.z];
+  const int j0 = (int)((long long)a.nout * blockIdx.y / gridDim.y), j1 = (int)((long long)a.nout * (blockIdx.y + 1) / gridDim.y);
+  if (j0 == j1) return;
+  const long long nc = presum_chunks(a);
+  for (long long c = blockIdx.x; c < nc; c += gridDim.x) presum_body(a, ptab, cap, c, j0, j1);
 }
 
 // Column-major copies between pitches, many in one launch (task blockIdx.y): used to give
@@ -1789,6 +1312,8 @@ __global__ void __launch_bounds__(CST_THREADS + 32) fmm_combine_staged_kernel(co
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the products (the tables above never change)
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const long long total = (long long)a.ms * a.ns;
   const long long ntile = (total + CST_TILE - 1) / CST_TILE;
   long long k = 0;  // stage step of this CTA

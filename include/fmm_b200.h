@@ -116,10 +116,10 @@ int fmm_device_status(int clear);
  * reference's counterpart is its packing pool (common/dgemm/bl_dgemm_util.c:375-394),
  * sized by the first call and never bounded.  One call's workspace is capped at `bytes`
  * (default 8 GiB; bytes <= 0 restores it): a call whose sums would need more runs its
- * products in groups over two halves of a capped workspace, the next group's sums formed
- * while the current group runs; results are unchanged.  The groups' workspace is
- * 2 G (ms + ns) kk 8 bytes for groups of G >= 1 products (kk: the k extent per product
- * rounded up to 8), so a cap below two products' sums is exceeded by that much.  Returns
+ * products in groups, one group's sums in the workspace at a time; results are unchanged.
+ * The groups' workspace is G (ms + ns) kk 8 bytes for groups of G >= 1 products (kk: the k
+ * extent per product rounded up to 8), so a cap below one product's sums is exceeded by that
+ * much.  Returns
  * the previous cap.
  * fmm_last_workspace_bytes: pre-summed workspace bytes of the calling thread's last
  * fmm_dgemm_dev / host call (0 when it used none).  The stored products of a call whose C
@@ -131,7 +131,8 @@ long long fmm_last_workspace_bytes(void);
  *   FMM_DEBUG_WAIT_LIMIT_NS: time limit of every bounded device-side wait on the current
  *     device, in ns (default 4e9; value <= 0 restores the default).
  *   FMM_DEBUG_TICKET_FILL: byte written into every ticket of a single-problem FMM launch
- *     before it runs (default 0).  0xFF starts every ticket at -1, which no launch ever
+ *     before it runs (default 0).  While it is set, ABC calls of any size take the schedule
+ *     whose products wait on tickets (else small ones store their products).  0xFF starts every ticket at -1, which no launch ever
  *     releases, so the launch's first ticket waits run out: the kernel records
  *     FMM_E_TIMEOUT after the limit, stops waiting for tickets, and finishes (its result
  *     is then unreliable); fmm_device_status() reports it.  Lets a test check the
@@ -139,9 +140,9 @@ long long fmm_last_workspace_bytes(void);
  *   FMM_DEBUG_COMBINE_POSITIONS: form of the stored-products combine pass: 0 (default) the
  *     shared-memory-staged form where the operands allow it, 1 or 2 the register form with
  *     that many element positions per thread; results are unchanged, for sweeps.
- *   FMM_DEBUG_KSPLIT: k split S (1..8) of every launch the model would consider splitting
- *     (launches of few waves); 0 restores the model's choice.  For sweeps; results change
- *     within rounding.
+ *   FMM_DEBUG_KSPLIT: k parts S (1..8) of every classical update (the plain GEMM and the
+ *     fringe strips) deep enough for them; 0 restores the library's choice by size.  For
+ *     sweeps; results change within rounding.
  *   FMM_DEBUG_SPLIT_OPERANDS: how the split-BF16 path forms its operand planes: 0 (default)
  *     every product's sums from one staged read of each operand, 1 one product per CTA (the
  *     two give identical planes; for tests and sweeps).
@@ -197,7 +198,7 @@ int fmm_split_gemm_dev(const fmm_plan *plan, int m, int n, int k, const float *A
  * fmm_dgemm_dev partitions it (FMM core plus fringe strips), so results are identical
  * to calling fmm_dgemm_dev per problem.  A second launch handles the k-fringe strips
  * (they update the same C region as their core), and a launch before them forms the
- * pre-summed operands of the large FMM problems.
+ * pre-summed operands of the FMM problems.
  *
  * fmm_batch_create fixes the shapes and plans and allocates (cudaMalloc) the job tables,
  * tickets and workspaces; the plans must outlive the batch.  fmm_batch_dgemm takes this
@@ -209,12 +210,9 @@ int fmm_split_gemm_dev(const fmm_plan *plan, int m, int n, int k, const float *A
 typedef struct fmm_batch fmm_batch;
 int fmm_batch_create(int count, const fmm_plan *const *plans, const int *m, const int *n, const int *k,
                      fmm_batch **out);
-/* The same with a tile height per problem: tile_m[i] = 128 (the default, also 0) or 64 rows per
- * work unit (problem i's FMM core and fringe strips).  64-row tiles halve a problem's unit
- * length and double its unit count (a finer split of the batch's work over the SMs); they run
- * in phases of the direct variant (pre-summed or classical jobs) and fall back to 128 rows
- * elsewhere.  Results of a 64-row problem equal a single call's up to rounding (two partial k
- * sums per tile), not bit for bit. */
+/* The same with a tile height per problem, tile_m[i] = 128 (the default, also 0) or 64.  Every
+ * problem's work units are 64 x 64 tiles, so both heights run alike; other values are
+ * refused. */
 int fmm_batch_create_tiled(int count, const fmm_plan *const *plans, const int *m, const int *n, const int *k,
                            const int *tile_m, fmm_batch **out);
 int fmm_batch_dgemm(fmm_batch *batch, const double *const *A, const long *lda, const double *const *B,
