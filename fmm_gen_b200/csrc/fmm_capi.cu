@@ -1865,6 +1865,7 @@ extern "C" int fmm_dgemm_dev_noalloc(const fmm_plan* plan, int m, int n, int k, 
 namespace {
 
 bool split_configured[kMaxDevices];
+constexpr int kPlaneSmem = 200 * 1024;
 
 int split_configure(int* dev_out) {
   int rc = configure_kernel(dev_out);
@@ -1873,10 +1874,9 @@ int split_configure(int* dev_out) {
   if (!split_configured[*dev_out]) {
     FMM_CUDA_TRY(cudaFuncSetAttribute(fmms::fmm_split_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)fmms::SMEM_BYTES));
-    FMM_CUDA_TRY(cudaFuncSetAttribute(fmms::fmm_split_all_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      100 * 1024));
-    FMM_CUDA_TRY(cudaFuncSetAttribute(fmms::fmm_split_all_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      100 * 1024));
+    for (auto kernel : {fmms::fmm_split_planes_kernel<16, 2>, fmms::fmm_split_planes_kernel<16, 1>,
+                        fmms::fmm_split_planes_kernel<8, 1>})
+      FMM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPlaneSmem));
     split_configured[*dev_out] = true;
   }
   return g_encode_tiled ? FMM_OK : FMM_E_UNSUPPORTED;
@@ -1896,156 +1896,273 @@ bool make_plane_map(CUtensorMap* map, const __nv_bfloat16* base, long long rows,
   return r == CUDA_SUCCESS;
 }
 
-// One split-BF16 launch pair over sub-blocks ms x ks x ns of a plan (R products):
-// operand planes into a stream-ordered workspace, then the persistent tcgen05 GEMM.
-int split_core(const fmm_plan* plan, const DevTables& d, const float* A, long long lda, const float* B,
-               long long ldb, double* C, long long ldc, int ms, int ns, int ks, cudaStream_t st) {
-  if (ms <= 0 || ns <= 0 || ks <= 0) return FMM_OK;
-  const int R = plan->rank;
-  // several products: store each M_r, then one combine pass applies W (no C loads in the
-  // tensor-core kernel's epilogue); a single product goes straight into C
-  const bool use_m = R > 1 && combine_fits(plan);
-  int dev = 0;
-  int rc = split_configure(&dev);
-  if (rc != FMM_OK) return rc;
-  static_assert(fmms::BM == fmms::BN, "one box shape for both plane maps");
-  const long long kpad = ((long long)ks + fmms::KPAD - 1) / fmms::KPAD * fmms::KPAD;
-  const long long rows_a = 3LL * R * ms, rows_b = 3LL * R * ns;
-  const int tiles_m = (ms + fmms::BM - 1) / fmms::BM, tiles_n = (ns + fmms::BN - 1) / fmms::BN;
-  const long long ntiles = (long long)tiles_m * tiles_n;
-  if (ntiles * R > INT32_MAX || (ms + fmms::SPLIT_ROWS - 1) / fmms::SPLIT_ROWS > 65535 ||
-      (ns + fmms::SPLIT_ROWS - 1) / fmms::SPLIT_ROWS > 65535 || kpad / fmms::SPLIT_K > 65535)
-    return FMM_E_UNSUPPORTED;
-  const size_t bytes_a = sizeof(__nv_bfloat16) * (size_t)(rows_a * kpad);
-  const size_t bytes_b = sizeof(__nv_bfloat16) * (size_t)(rows_b * kpad);
-  const size_t bytes_m = use_m ? sizeof(double) * (size_t)R * ms * ns : 0;
-  const size_t bytes_t = (R > 1 && !use_m) ? sizeof(int) * (size_t)ntiles : 0;
-  char* ws = nullptr;
-  // planes, product tiles, then the work-unit counter and the tickets
-  FMM_CUDA_TRY(cudaMallocAsync((void**)&ws, bytes_a + bytes_b + bytes_m + sizeof(int) + bytes_t + 16, st));
-  __nv_bfloat16* PA = reinterpret_cast<__nv_bfloat16*>(ws);
-  __nv_bfloat16* PB = reinterpret_cast<__nv_bfloat16*>(ws + bytes_a);
-  double* Mws = use_m ? reinterpret_cast<double*>(ws + bytes_a + bytes_b) : nullptr;
-  int* counter = reinterpret_cast<int*>(ws + bytes_a + bytes_b + bytes_m);
-  int* tickets = bytes_t ? counter + 1 : nullptr;
-  rc = cuda_status(cudaMemsetAsync(counter, 0, sizeof(int) + bytes_t, st));
+// One GEMM of a split-BF16 call: sub-blocks ms x ks x ns of a plan (the classical plan: a fringe
+// strip or the whole problem).
+struct SplitPart {
+  const fmm_plan* plan;
+  const float* A;
+  const float* B;
+  double* C;
+  int ms, ns, ks;
+  // workspace of its planes, tickets (ints from the counter on) and stored products
+  size_t off_a = 0, off_b = 0, off_m = 0;
+  long long ticket = 0;
+  long long kpad = 0;
+  int parts = 1, part_stages = 0;
+  bool use_m = false;
+  bool planes_done = false;
+};
 
-  fmms::SplitArgs sa{};
-  sa.X = A;
-  sa.ldx = lda;
-  sa.rows = ms;
-  sa.ks = ks;
-  sa.kpad = (int)kpad;
-  sa.blk_row_stride = ms;
-  sa.blk_col_stride = ks;
-  sa.out = PA;
-  sa.prods = d.prods;
-  sa.terms = d.terms;
-  sa.side = 0;
-  fmms::SplitArgs sb = sa;
-  sb.X = B;
-  sb.ldx = ldb;
-  sb.rows = ns;
-  sb.blk_row_stride = ks;
-  sb.blk_col_stride = ns;
-  sb.out = PB;
-  sb.side = 1;
-  // every product's sums from one read of each operand, where the staged tiles fit
-  int nta = 0, ntb = 0;
-  for (const auto& pr : plan->prods) nta += pr.na, ntb += pr.nb;
-  const int nblk_a = plan->dims[0] * plan->dims[1], nblk_b = plan->dims[1] * plan->dims[2];
-  const size_t sm_a = fmms::split_all_smem_bytes(0, nblk_a, R, nta), sm_b = fmms::split_all_smem_bytes(1, nblk_b, R, ntb);
-  const bool all_form = g_split_form.load() == 0 && sm_a <= 100 * 1024 && sm_b <= 100 * 1024 && kpad % 64 == 0;
-  if (rc == FMM_OK && all_form) {
-    fmms::SplitAllArgs ga{sa, nblk_a, plan->dims[1], R, nta};
-    fmms::SplitAllArgs gb{sb, nblk_b, plan->dims[2], R, ntb};
-    ProfScope pf(K_SPLIT_OPERANDS, st);
-    fmms::fmm_split_all_kernel<0><<<dim3((unsigned)(kpad / 32), (unsigned)((ms + 15) / 16)), 256, sm_a, st>>>(ga);
-    fmms::fmm_split_all_kernel<1><<<dim3((unsigned)(kpad / 64), (unsigned)((ns + 7) / 8)), 256, sm_b, st>>>(gb);
-    g_launches.fetch_add(2, std::memory_order_relaxed);
-    rc = cuda_status(cudaGetLastError());
-  } else if (rc == FMM_OK) {
-    ProfScope pf(K_SPLIT_OPERANDS, st);
-    const dim3 blk(32, 8);
-    const unsigned kt = (unsigned)(kpad / fmms::SPLIT_K);
-    fmms::fmm_split_operands_kernel<<<dim3((unsigned)R, kt, (unsigned)((ms + fmms::SPLIT_ROWS - 1) / fmms::SPLIT_ROWS)),
-                                      blk, 0, st>>>(sa);
-    fmms::fmm_split_operands_kernel<<<dim3((unsigned)R, kt, (unsigned)((ns + fmms::SPLIT_ROWS - 1) / fmms::SPLIT_ROWS)),
-                                      blk, 0, st>>>(sb);
-    g_launches.fetch_add(2, std::memory_order_relaxed);
-    rc = cuda_status(cudaGetLastError());
-  }
-  fmms::SplitGemmArgs g{};
-  if (rc == FMM_OK && (!make_plane_map(&g.tmA, PA, rows_a, kpad) || !make_plane_map(&g.tmB, PB, rows_b, kpad)))
-    rc = FMM_E_UNSUPPORTED;
-  if (rc == FMM_OK) {
-    g.C = C;
-    g.ldc = ldc;
-    g.ms = ms;
-    g.ns = ns;
-    g.kpad = (int)kpad;
-    g.prods = d.prods;
-    g.terms = d.terms;
-    g.nprod = R;
-    g.tiles_m = tiles_m;
-    g.tiles_n = tiles_n;
-    g.tickets = tickets;
-    g.counter = counter;
-    g.M = Mws;
-    g.ldm = ms;
-    g.m_stride = (long long)ms * ns;
-    g.status = dev_status[dev];
-    const long long units = ntiles * R;
-    const unsigned grid = (unsigned)(units < sm_count[dev] ? units : sm_count[dev]);
-    {
-      ProfScope pf(K_GEMM_SPLIT, st);
-      fmms::fmm_split_gemm_kernel<<<grid, fmms::NTHREADS, fmms::SMEM_BYTES, st>>>(g);
+// k parts of a single product: rounds of the SMs times chunks per unit (4.6 us each) against the
+// parts' C updates, which follow one another (kPartUpdateUs each).  Measured us with 1 / as many
+// parts as chunks: 512 x 512 x 2048 50 / 75, 512 x 512 x 8192 156 / 92, 258^3 21 / 29.
+constexpr double kChunkUs = 4.6, kPartUpdateUs = 6.0;
+void split_parts(SplitPart* p, int nsm) {
+  const int nks = (int)(p->kpad / fmms::BK);
+  const int chunks = (nks + fmms::DRAIN_STAGES - 1) / fmms::DRAIN_STAGES;
+  const long long tiles = tiles_of(p->ms, p->ns, fmms::BM);
+  int best = 1;
+  double cost = 1e300;
+  for (int s = 1; s <= std::min(chunks, 16); ++s) {
+    const double c = (double)((tiles * s + nsm - 1) / nsm) * ((chunks + s - 1) / s) * kChunkUs + s * kPartUpdateUs;
+    if (c < 0.97 * cost) {
+      best = s;
+      cost = c;
     }
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    rc = cuda_status(cudaGetLastError());
   }
-  if (rc == FMM_OK && use_m) rc = launch_combine(plan, d, C, ldc, ms, ns, Mws, ms, (long long)ms * ns, st);
-  cudaError_t fe = cudaFreeAsync(ws, st);
-  if (rc == FMM_OK) rc = cuda_status(fe);
-  return rc;
+  p->part_stages = (chunks + best - 1) / best * fmms::DRAIN_STAGES;
+  p->parts = (nks + p->part_stages - 1) / p->part_stages;
 }
 
-int split_plain(int m, int n, int k, const float* A, long long lda, const float* B, long long ldb, double* C,
-                long long ldc, cudaStream_t st) {
-  if (m <= 0 || n <= 0 || k <= 0) return FMM_OK;
+// The tile of a planes CTA by the operand's blocks: 16 rows x 64 k for few blocks (and several
+// k tiles per CTA, so that a thread has at least 16 loads in flight), x 32 k beyond, 8 rows for
+// more than 16.
+struct PlaneTile {
+  int tr, np, kts;
+};
+PlaneTile plane_tile(int maxblk, int nblk) {
+  if (maxblk <= 4) return PlaneTile{16, 2, std::max(1, 4 / nblk)};
+  return PlaneTile{maxblk <= 16 ? 16 : 8, 1, std::max(1, 8 / nblk)};
+}
+
+// The operand planes of several GEMMs (fmm_split_planes_kernel); zero[0 .. nzero) is cleared.
+int launch_planes(SplitPart* ps, int np, char* ws, long long lda, long long ldb, int* zero, long long nzero,
+                  cudaStream_t st) {
+  fmms::PlaneArgs g{};
+  int maxblk = 1;
+  for (int q = 0; q < np; ++q)
+    if (!ps[q].planes_done)
+      maxblk = std::max({maxblk, ps[q].plan->dims[0] * ps[q].plan->dims[1], ps[q].plan->dims[1] * ps[q].plan->dims[2]});
+  const int tr = plane_tile(maxblk, 1).tr, np2 = plane_tile(maxblk, 1).np;
+  long long ctas = 0;
+  size_t smem = 0;
+  for (int q = 0; q < np; ++q) {
+    SplitPart& p = ps[q];
+    if (p.planes_done) continue;
+    DevTables* d = nullptr;
+    const int rc = device_tables(p.plan, &d);
+    if (rc != FMM_OK) return rc;
+    for (int side = 0; side < 2; ++side) {
+      fmms::PlaneJob& j = g.job[g.njob++];
+      j.X = side == 0 ? p.A : p.B;
+      j.ldx = side == 0 ? lda : ldb;
+      j.out = reinterpret_cast<__nv_bfloat16*>(ws + (side == 0 ? p.off_a : p.off_b));
+      j.first = d->ps_first[side];
+      j.terms = d->ps_terms[side];
+      j.rows = side == 0 ? p.ms : p.ns;
+      j.ks = p.ks;
+      j.kpad = (int)p.kpad;
+      j.blk_row_stride = side == 0 ? p.ms : p.ks;
+      j.blk_col_stride = side == 0 ? p.ks : p.ns;
+      j.nblk = side == 0 ? p.plan->dims[0] * p.plan->dims[1] : p.plan->dims[1] * p.plan->dims[2];
+      j.block_cols = side == 0 ? p.plan->dims[1] : p.plan->dims[2];
+      j.nprod = p.plan->rank;
+      j.nterm = (int)p.plan->ps_terms[side].size();
+      j.side = side;
+      j.kt = (int)(p.kpad / (32 * np2));
+      j.kts = plane_tile(maxblk, j.nblk).kts;
+      j.cta0 = (int)ctas;
+      ctas += (long long)((j.rows + tr - 1) / tr) * ((j.kt + j.kts - 1) / j.kts);
+      smem = std::max(smem, fmms::plane_smem_bytes(tr, np2, j.nblk, j.kts, j.nprod, j.nterm));
+    }
+  }
+  if (ctas > INT32_MAX || nzero > INT32_MAX) return FMM_E_UNSUPPORTED;
+  if (g.njob == 0) return cuda_status(cudaMemsetAsync(zero, 0, sizeof(int) * nzero, st));
+  g.zero = zero;
+  g.nzero = (int)nzero;
+  ProfScope pf(K_SPLIT_OPERANDS, st);
+  return launch_dependent(np2 == 2   ? fmms::fmm_split_planes_kernel<16, 2>
+                          : tr == 16 ? fmms::fmm_split_planes_kernel<16, 1>
+                                     : fmms::fmm_split_planes_kernel<8, 1>,
+                          dim3((unsigned)ctas), 16 * tr, smem, st, 1, g);
+}
+
+// A core whose staged tiles do not fit (or the test hook): one product per CTA.
+int launch_operands(const SplitPart& p, char* ws, long long lda, long long ldb, cudaStream_t st) {
   DevTables* d = nullptr;
-  int rc = device_tables(classical_plan(), &d);
+  const int rc = device_tables(p.plan, &d);
   if (rc != FMM_OK) return rc;
-  return split_core(classical_plan(), *d, A, lda, B, ldb, C, ldc, m, n, k, st);
+  for (int side = 0; side < 2; ++side) {
+    fmms::SplitArgs a{};
+    a.X = side == 0 ? p.A : p.B;
+    a.ldx = side == 0 ? lda : ldb;
+    a.rows = side == 0 ? p.ms : p.ns;
+    a.ks = p.ks;
+    a.kpad = (int)p.kpad;
+    a.blk_row_stride = side == 0 ? p.ms : p.ks;
+    a.blk_col_stride = side == 0 ? p.ks : p.ns;
+    a.out = reinterpret_cast<__nv_bfloat16*>(ws + (side == 0 ? p.off_a : p.off_b));
+    a.prods = d->prods;
+    a.terms = d->terms;
+    a.side = side;
+    ProfScope pf(K_SPLIT_OPERANDS, st);
+    fmms::fmm_split_operands_kernel<<<dim3((unsigned)p.plan->rank, (unsigned)(p.kpad / fmms::SPLIT_K),
+                                           (unsigned)((a.rows + fmms::SPLIT_ROWS - 1) / fmms::SPLIT_ROWS)),
+                                      dim3(32, 8), 0, st>>>(a);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    FMM_CUDA_TRY(cudaGetLastError());
+  }
+  return FMM_OK;
 }
 
+// The GEMMs [p0, p1) in one launch; `counter` is the launch's own.
+int launch_split_gemm(const SplitPart* ps, int p0, int p1, char* ws, long long ldc, int* counter, int* tickets, int dev,
+                      cudaStream_t st) {
+  fmms::SplitGemmArgs g{};
+  long long units = 0;
+  for (int q = p1 - 1; q >= p0; --q) {  // the strips' long units first
+    const SplitPart& p = ps[q];
+    DevTables* d = nullptr;
+    const int rc = device_tables(p.plan, &d);
+    if (rc != FMM_OK) return rc;
+    fmms::SplitJob& j = g.job[g.njob++];
+    const int R = p.plan->rank;
+    if (!make_plane_map(&j.tmA, reinterpret_cast<const __nv_bfloat16*>(ws + p.off_a), 3LL * R * p.ms, p.kpad) ||
+        !make_plane_map(&j.tmB, reinterpret_cast<const __nv_bfloat16*>(ws + p.off_b), 3LL * R * p.ns, p.kpad))
+      return FMM_E_UNSUPPORTED;
+    j.C = p.C;
+    j.ldc = ldc;
+    j.prods = d->prods;
+    j.terms = d->terms;
+    j.tickets = tickets + p.ticket;
+    j.M = p.use_m ? reinterpret_cast<double*>(ws + p.off_m) : nullptr;
+    j.m_stride = (long long)p.ms * p.ns;
+    j.ms = p.ms;
+    j.ns = p.ns;
+    j.nks = (int)(p.kpad / fmms::BK);
+    j.nprod = R;
+    j.parts = p.parts;
+    j.part_stages = p.part_stages;
+    j.tiles_m = (p.ms + fmms::BM - 1) / fmms::BM;
+    j.tiles_n = (p.ns + fmms::BN - 1) / fmms::BN;
+    j.first = (int)units;
+    units += (long long)j.tiles_m * j.tiles_n * (p.parts > 1 ? p.parts : R);
+    if (units > INT32_MAX) return FMM_E_UNSUPPORTED;
+  }
+  g.units = (int)units;
+  g.status = dev_status[dev];
+  g.counter = counter;
+  const unsigned grid = (unsigned)std::min<long long>(units, sm_count[dev]);
+  ProfScope pf(K_GEMM_SPLIT, st);
+  return launch_dependent(fmms::fmm_split_gemm_kernel, dim3(grid), fmms::NTHREADS, fmms::SMEM_BYTES, st, 1, g);
+}
+
+// Same partition as the FP64 path: the FMM core, then the fringe strips (classical).  The n
+// and m strips lie outside the core's C and run in its launch; the k strip updates the core's
+// C and follows the combine pass.
 int run_split(const fmm_plan* plan, int m, int n, int k, const float* A, long long lda, const float* B,
               long long ldb, double* C, long long ldc, cudaStream_t st) {
   int rc = check_args(m, n, k, A, lda, B, ldb, C, ldc);
   if (rc != FMM_OK || m == 0 || n == 0 || k == 0) return rc;
-  if (!plan) return split_plain(m, n, k, A, lda, B, ldb, C, ldc, st);
-  const int pm = plan->dims[0] * kMR, pk = plan->dims[1], pn = plan->dims[2] * kNR;
-  const int mr = m % pm, kr = k % pk, nr = n % pn;
-  const int md = m - mr, kd = k - kr, nd = n - nr;
-  if (md > 0 && nd > 0 && kd > 0) {
+  const fmm_plan* cls = classical_plan();
+  if (!plan || is_classical(plan)) plan = cls;
+  int dev = 0;
+  rc = split_configure(&dev);
+  if (rc != FMM_OK) return rc;
+  static_assert(fmms::BM == fmms::BN, "one box shape for both plane maps");
+  SplitPart ps[4];
+  int np = 0;
+  auto add = [&](const fmm_plan* p, const float* a, const float* b, double* c, int ms, int ns, int ks) {
+    if (ms <= 0 || ns <= 0 || ks <= 0) return;
+    ps[np] = SplitPart{};
+    ps[np].plan = p;
+    ps[np].A = a;
+    ps[np].B = b;
+    ps[np].C = c;
+    ps[np].ms = ms;
+    ps[np].ns = ns;
+    ps[np].ks = ks;
+    ++np;
+  };
+  int last = 0;  // the k strip's index when it needs a launch of its own
+  if (plan == cls) {
+    add(cls, A, B, C, m, n, k);
+    last = np;
+  } else {
+    const int pm = plan->dims[0] * kMR, pk = plan->dims[1], pn = plan->dims[2] * kNR;
+    const int md = m - m % pm, kd = k - k % pk, nd = n - n % pn;
+    const bool core = md > 0 && nd > 0 && kd > 0;
+    if (core) add(plan, A, B, C, md / plan->dims[0], nd / plan->dims[2], kd / plan->dims[1]);
+    add(cls, A, B + (long long)nd * ldb, C + (long long)nd * ldc, m, n - nd, k);
+    add(cls, A + md, B, C + md, m - md, nd, k);
+    last = np;
+    add(cls, A + (long long)kd * lda, B + kd, C, md, nd, k - kd);
+    if (!core) last = np;  // no core: the three strips are disjoint
+  }
+  // workspace: planes, stored products, the launches' counters (2) and the tickets
+  size_t bytes = 0;
+  long long tickets = 0;
+  auto take = [&](size_t b) {
+    const size_t at = bytes;
+    bytes += (b + 255) & ~(size_t)255;
+    return at;
+  };
+  for (int q = 0; q < np; ++q) {
+    SplitPart& p = ps[q];
+    const int R = p.plan->rank;
+    p.kpad = ((long long)p.ks + fmms::KPAD - 1) / fmms::KPAD * fmms::KPAD;
+    const long long tiles = tiles_of(p.ms, p.ns, fmms::BM);
+    if (tiles * R > INT32_MAX || (p.ms + fmms::SPLIT_ROWS - 1) / fmms::SPLIT_ROWS > 65535 ||
+        (p.ns + fmms::SPLIT_ROWS - 1) / fmms::SPLIT_ROWS > 65535 || p.kpad / fmms::SPLIT_K > 65535)
+      return FMM_E_UNSUPPORTED;
+    // several products: store each M_r, then one combine pass applies W (no C loads in the
+    // tensor-core kernel's epilogue); a single product goes straight into C
+    p.use_m = R > 1 && combine_fits(p.plan);
+    p.part_stages = (int)(p.kpad / fmms::BK);
+    if (R == 1) split_parts(&p, sm_count[dev]);
+    p.off_a = take(sizeof(__nv_bfloat16) * 3 * (size_t)R * p.ms * p.kpad);
+    p.off_b = take(sizeof(__nv_bfloat16) * 3 * (size_t)R * p.ns * p.kpad);
+    if (p.use_m) p.off_m = take(sizeof(double) * (size_t)R * p.ms * p.ns);
+    p.ticket = tickets;
+    if (!p.use_m && (R > 1 || p.parts > 1)) tickets += tiles * (fmms::NEPI / 32);
+  }
+  const size_t off_c = take(sizeof(int) * (2 + (size_t)tickets));
+  char* ws = nullptr;
+  FMM_CUDA_TRY(cudaMallocAsync((void**)&ws, bytes, st));
+  int* counter = reinterpret_cast<int*>(ws + off_c);
+  for (int q = 0; q < np && rc == FMM_OK; ++q) {  // cores whose staged tiles do not fit
+    SplitPart& p = ps[q];
+    const int na = p.plan->dims[0] * p.plan->dims[1], nb = p.plan->dims[1] * p.plan->dims[2];
+    const PlaneTile t = plane_tile(std::max(na, nb), std::max(na, nb));
+    const bool fits =
+        fmms::plane_smem_bytes(t.tr, t.np, na, t.kts, p.plan->rank, (int)p.plan->ps_terms[0].size()) <= kPlaneSmem &&
+        fmms::plane_smem_bytes(t.tr, t.np, nb, t.kts, p.plan->rank, (int)p.plan->ps_terms[1].size()) <= kPlaneSmem;
+    if (fits && (g_split_form.load() == 0 || p.plan->rank == 1)) continue;
+    rc = launch_operands(p, ws, lda, ldb, st);
+    p.planes_done = true;
+  }
+  if (rc == FMM_OK) rc = launch_planes(ps, np, ws, lda, ldb, counter, 2 + tickets, st);
+  if (rc == FMM_OK && last > 0) rc = launch_split_gemm(ps, 0, last, ws, ldc, counter, counter + 2, dev, st);
+  if (rc == FMM_OK && ps[0].use_m) {
     DevTables* d = nullptr;
-    rc = device_tables(plan, &d);
-    if (rc != FMM_OK) return rc;
-    rc = split_core(plan, *d, A, lda, B, ldb, C, ldc, md / plan->dims[0], nd / plan->dims[2], kd / plan->dims[1],
-                    st);
-    if (rc != FMM_OK) return rc;
+    rc = device_tables(ps[0].plan, &d);
+    if (rc == FMM_OK)
+      rc = launch_combine(ps[0].plan, *d, ps[0].C, ldc, ps[0].ms, ps[0].ns, reinterpret_cast<double*>(ws + ps[0].off_m),
+                          ps[0].ms, (long long)ps[0].ms * ps[0].ns, st);
   }
-  // fringe strips: the same regions, in the same order, as the FP64 path's peeling
-  if (kr > 0 && md > 0 && nd > 0) {
-    rc = split_plain(md, nd, kr, A + (long long)kd * lda, lda, B + kd, ldb, C, ldc, st);
-    if (rc != FMM_OK) return rc;
-  }
-  if (nr > 0) {
-    rc = split_plain(m, nr, k, A, lda, B + (long long)nd * ldb, ldb, C + (long long)nd * ldc, ldc, st);
-    if (rc != FMM_OK) return rc;
-  }
-  if (mr > 0 && nd > 0) rc = split_plain(mr, nd, k, A + md, lda, B, ldb, C + md, ldc, st);
-  return rc;
+  if (rc == FMM_OK && last < np) rc = launch_split_gemm(ps, last, np, ws, ldc, counter + 1, counter + 2, dev, st);
+  cudaError_t fe = cudaFreeAsync(ws, st);
+  return rc == FMM_OK ? cuda_status(fe) : rc;
 }
 
 }  // namespace

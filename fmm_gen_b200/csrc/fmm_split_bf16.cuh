@@ -2,7 +2,7 @@
 // FP32-level accuracy.  The reference is FP64 only; this path keeps its algebra (products r
 // in order, C_l += W[l,r] * M_r, fringes peeled the same way) and changes the arithmetic:
 //
-//   1. fmm_split_operands_kernel: for every product r the operand sum
+//   1. fmm_split_planes_kernel: for every product r the operand sum
 //      S_r = sum_i U[i,r] A_i is formed in FP64 from the FP32 inputs and split exactly into
 //      three bf16 planes, S = hi + mid + lo (hi = bf16(S), mid = bf16(S - hi),
 //      lo = bf16(S - hi - mid)), stored K-major (k contiguous, row pitch kpad, a multiple
@@ -17,10 +17,12 @@
 //      products the epilogue stores M_r (FP64) to a workspace and fmm_combine_kernel adds
 //      W[l,r] * M_r into C afterwards; a single product is added into C directly.
 //
-// Work unit = (128 x 128 tile position, product r), claimed in order from a launch-wide
-// counter (fmm::UnitClaimer); a unit owns its tile position in every C block, and per-tile
-// tickets order the products' C updates (no atomics on C, the result does not depend on
-// scheduling).  Warp roles (384 threads, one CTA per SM, persistent):
+// A launch runs up to three jobs: the FMM core and the fringe strips beside it (they update
+// disjoint parts of C), each a set of products over tiles, or one product whose k chunks are
+// cut into parts so that a job of few tiles still fills the SMs.  Work unit = (128 x 128 tile
+// position, product or part), claimed in order from a launch-wide counter (fmm::UnitClaimer);
+// a unit owns its tile position in every C block, and per-tile tickets order the products' or
+// parts' C updates (no atomics on C, the result does not depend on scheduling).  Warp roles (384 threads, one CTA per SM, persistent):
 // warp 0 lane 0 issues TMA (128-byte swizzle, each CTA loads its own tiles), warp 1 owns tensor memory and
 // its lane 0 issues the MMAs, warps 4..11 drain the accumulator and run the epilogue.
 // Every wait is bounded; tensor memory is freed on every path.
@@ -32,11 +34,13 @@
 #include <cstdint>
 
 #include "fmm_kernels.cuh"
+#include "fmm_tile.cuh"
 
 namespace fmms {
 
 using fmm::Prod;
 using fmm::Term;
+using fmm::PTerm;
 
 constexpr int BM = 128;        // tile rows (m) = tensor-memory lanes
 constexpr int BN = 128;        // tile columns (n) = accumulator columns
@@ -68,20 +72,31 @@ constexpr int EPI_REGS = 224;
 static_assert(128 * CTL_REGS + NEPI * EPI_REGS <= NTHREADS * LAUNCH_REGS, "register split exceeds the launch budget");
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 
-struct SplitGemmArgs {
+struct SplitJob {
   CUtensorMap tmA;   // A planes: row (3 r + p) ms + i, column k (pitch kpad); bf16, box 64 x 128, 128-byte swizzle
   CUtensorMap tmB;   // B planes: row (3 r + p) ns + j
   double* C;
   long long ldc;
-  int ms, ns, kpad;
   const Prod* prods;  // C terms of product r: terms[c0 .. c0+nc)
   const Term* terms;
+  int* tickets;      // per tile and epilogue warp: products (or parts) whose C updates are done (zeroed
+                     // before the launch); the warps of a CTA do not wait for one another
+  double* M;         // when set: product r's tile is stored to M + r * m_stride (ld ms) instead
+  long long m_stride;  // of being added into C; a combine pass applies W afterwards
+  int ms, ns;
+  int nks;           // stages (of BK) of a product
   int nprod;
+  int parts;         // k parts of the one product (1 when nprod > 1), each of
+  int part_stages;   // part_stages stages, a multiple of DRAIN_STAGES (the last may be shorter)
   int tiles_m, tiles_n;
-  int* tickets;      // per tile: products whose C updates are done (zeroed before launch)
-  double* M;         // when set: product r's tile is stored to M + r * m_stride (ld ldm) instead
-  long long ldm;     // of being added into C; a combine pass applies W afterwards
-  long long m_stride;
+  int first;         // first unit of the job
+};
+
+constexpr int MAX_SPLIT_JOBS = 3;
+struct SplitGemmArgs {
+  SplitJob job[MAX_SPLIT_JOBS];
+  int njob;
+  int units;
   unsigned* status;
   int* counter;      // work units claimed so far (zeroed before launch)
 };
@@ -89,7 +104,7 @@ struct SplitGemmArgs {
 // Where the split kernel's work units come from (for fmm::UnitClaimer).
 struct SplitSrc {
   const SplitGemmArgs& a;
-  __device__ __forceinline__ int total() const { return a.tiles_m * a.tiles_n * a.nprod; }
+  __device__ __forceinline__ int total() const { return a.units; }
   __device__ __forceinline__ unsigned* status() const { return a.status; }
   __device__ __forceinline__ int* counter() const { return a.counter; }
 };
@@ -149,7 +164,7 @@ using fmm::mbar_wait_drain;  // time-limited wait for copies and MMAs still in f
 
 // The unit's C tiles (every C block of product p) into L2: 128-byte lines of 16 rows of
 // one column, spread over the epilogue threads.
-__device__ __forceinline__ void prefetch_c_tiles(const SplitGemmArgs& a, const Prod& p, int m0, int n0, int et) {
+__device__ __forceinline__ void prefetch_c_tiles(const SplitJob& a, const Prod& p, int m0, int n0, int et) {
   for (int c = 0; c < p.nc; ++c) {
     const Term tm = a.terms[p.c0 + c];
     const double* Cb = a.C + (long long)tm.row * a.ms + (long long)tm.col * a.ns * a.ldc;
@@ -163,15 +178,29 @@ __device__ __forceinline__ void prefetch_c_tiles(const SplitGemmArgs& a, const P
 }
 
 struct SUnit {
-  int m0, n0, tile, r;
+  const SplitJob* j;
+  int m0, n0, tile;
+  int r, part;
+  int s0, ns;  // first stage, stages
 };
 
-// Units in product-major order; tiles rastered in groups of GROUP_M tile rows so that
-// concurrent units share operand panels in L2.
-__device__ __forceinline__ SUnit s_decode(const SplitGemmArgs& a, int u) {
+// Units of a job in product-major (part-major) order; tiles rastered in groups of GROUP_M tile
+// rows so that concurrent units share operand panels in L2.
+__device__ __forceinline__ SUnit s_decode(const SplitGemmArgs& g, int u) {
+  int ji = 0;
+#pragma unroll
+  for (int q = 1; q < MAX_SPLIT_JOBS; ++q)
+    if (q < g.njob && u >= g.job[q].first) ji = q;
+  const SplitJob& a = g.job[ji];
+  u -= a.first;
   const int ntiles = a.tiles_m * a.tiles_n;
   SUnit w;
-  w.r = u / ntiles;
+  w.j = &a;
+  const int idx = u / ntiles;
+  w.r = a.parts > 1 ? 0 : idx;
+  w.part = a.parts > 1 ? idx : 0;
+  w.s0 = w.part * a.part_stages;
+  w.ns = min(a.part_stages, a.nks - w.s0);
   const int bid = u % ntiles;
   const int per_group = GROUP_M * a.tiles_n;
   const int first_m = (bid / per_group) * GROUP_M;
@@ -183,7 +212,7 @@ __device__ __forceinline__ SUnit s_decode(const SplitGemmArgs& a, int u) {
   return w;
 }
 
-__global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __grid_constant__ SplitGemmArgs a) {
+__global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __grid_constant__ SplitGemmArgs g) {
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment for the 128-byte swizzle atoms
   unsigned char* smem = smem_raw + ((1024 - (fmm::smem_u32(smem_raw) & 1023)) & 1023);
@@ -196,7 +225,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __gri
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + NBARS);
   const fmm::UnitRing q{fmm::smem_u32(bars + NBARS + 2)};
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nks = a.kpad / BK;
 
   if (tid == 0) {
     for (int s = 0; s < NSTG; ++s) {
@@ -221,19 +249,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __gri
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = *reinterpret_cast<volatile unsigned*>(tmem_slot);
+  fmmt::grid_wait();  // the planes; nothing above touches what earlier launches write
+  fmmt::grid_launch();
 
   if (warp == 0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(CTL_REGS));
     if (lane == 0) {  // ---- TMA producer; claims the work units ----
-      const SplitSrc src{a};
+      const SplitSrc src{g};
       fmm::UnitClaimer<SplitSrc> nx{src, q};
       long long kc = 0;
       for (int u = nx.next(); u >= 0; u = nx.next()) {
-        const SUnit w = s_decode(a, u);
+        const SUnit w = s_decode(g, u);
+        const SplitJob& a = *w.j;
         const int ya = 3 * w.r * a.ms + w.m0, yb = 3 * w.r * a.ns + w.n0;
-        for (int s = 0; s < nks; ++s, ++kc) {
+        for (int s = w.s0; s < w.s0 + w.ns; ++s, ++kc) {
           const int stg = (int)(kc % NSTG);
-          fmm::mbar_wait(empty0 + 8 * stg, (unsigned)(((kc / NSTG) & 1) ^ 1), a.status);
+          fmm::mbar_wait(empty0 + 8 * stg, (unsigned)(((kc / NSTG) & 1) ^ 1), g.status);
           const unsigned fb = full0 + 8 * stg;
           fmm::mbar_arrive_expect_tx(fb, (unsigned)STAGE_BYTES);
           const unsigned base = fmm::smem_u32(smem + (size_t)stg * STAGE_BYTES);
@@ -255,15 +286,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __gri
       // plane pairs (A plane, B plane); the last, hi*hi, has an accumulator of its own
       constexpr int pa[NPAIR] = {2, 0, 1, 1, 0, 0};
       constexpr int pb[NPAIR] = {0, 2, 1, 0, 1, 0};
-      fmm::UnitReader nx{q, a.status, true, 0, true};
+      fmm::UnitReader nx{q, g.status, true, 0, true};
       long long kc = 0, ch = 0;
       for (int u = nx.next(); u >= 0; u = nx.next()) {
+        const int nks = s_decode(g, u).ns;
         for (int s = 0; s < nks; ++s, ++kc) {
           const int stg = (int)(kc % NSTG);
           const int b = (int)(ch % NACC);
           const bool first = s % DRAIN_STAGES == 0, last = s % DRAIN_STAGES == DRAIN_STAGES - 1 || s == nks - 1;
-          fmm::mbar_wait(full0 + 8 * stg, (unsigned)((kc / NSTG) & 1), a.status);
-          if (first) fmm::mbar_wait(acce0 + 8 * b, (unsigned)(((ch / NACC) & 1) ^ 1), a.status);
+          fmm::mbar_wait(full0 + 8 * stg, (unsigned)((kc / NSTG) & 1), g.status);
+          if (first) fmm::mbar_wait(acce0 + 8 * b, (unsigned)(((ch / NACC) & 1) ^ 1), g.status);
           tc_fence_after();
           const unsigned base = fmm::smem_u32(smem + (size_t)stg * STAGE_BYTES);
           const uint64_t dbase = smem_desc_sw128(base);
@@ -296,20 +328,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __gri
     const int et = tid - 128;
     const int quarter = warp & 3, half = (warp - 4) >> 2;
     const int row = quarter * 32 + lane;
-    const bool ordered = a.nprod > 1 && a.M == nullptr;
-    fmm::UnitReader nx{q, a.status, true};
+    fmm::UnitReader nx{q, g.status, true};
     long long ch = 0;
     for (int u = nx.next(); u >= 0; u = nx.next()) {
-      const SUnit w = s_decode(a, u);
+      const SUnit w = s_decode(g, u);
+      const SplitJob& a = *w.j;
+      const int seq = a.parts > 1 ? w.part : w.r;  // place in the order of the tile's C updates
+      const bool ordered = (a.nprod > 1 || a.parts > 1) && a.M == nullptr;
       double acc[64];
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = 0.0;
       const Prod p = a.prods[w.r];
-      const int nch = (nks + DRAIN_STAGES - 1) / DRAIN_STAGES;
+      const int nch = (w.ns + DRAIN_STAGES - 1) / DRAIN_STAGES;
       for (int c = 0; c < nch; ++c, ++ch) {
         if (!a.M && c == (nch > C_PREFETCH_CHUNKS ? nch - C_PREFETCH_CHUNKS : 0)) prefetch_c_tiles(a, p, w.m0, w.n0, et);
         const int b = (int)(ch % NACC);
-        fmm::mbar_wait(accf0 + 8 * b, (unsigned)((ch / NACC) & 1), a.status);
+        fmm::mbar_wait(accf0 + 8 * b, (unsigned)((ch / NACC) & 1), g.status);
         tc_fence_after();
         const unsigned taddr = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(b * ACC_COLS + half * 64);
 #pragma unroll
@@ -332,15 +366,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __gri
 #pragma unroll
           for (int j = 0; j < 64; ++j) {
             const int cc = w.n0 + half * 64 + j;
-            if (cc < a.ns) Mr[(long long)cc * a.ldm] = acc[j];
+            if (cc < a.ns) Mr[(long long)cc * a.ms] = acc[j];
           }
         }
         continue;
       }
-      // this tile position's updates from products < r are complete
-      if (ordered && w.r > 0) {
-        if (et == 0) fmm::ticket_spin(a.tickets + w.tile, w.r, a.status, 256);
-        fmm::named_bar_sync(1, NEPI);
+      // this tile position's earlier updates are complete
+      if (ordered && seq > 0) {
+        if (lane == 0) fmm::ticket_spin(a.tickets + w.tile * (NEPI / 32) + warp - 4, seq, g.status, 256);
+        __syncwarp();
       }
       // C_l += W[l, r] * M_r in FP64; a warp's lanes cover 32 consecutive rows of a column
       const int rr = w.m0 + row;
@@ -366,8 +400,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __gri
       }
       if (ordered) {
         __threadfence();
-        fmm::named_bar_sync(1, NEPI);
-        if (et == 0) fmm::st_release(a.tickets + w.tile, w.r + 1);
+        __syncwarp();
+        if (lane == 0) fmm::st_release(a.tickets + w.tile * (NEPI / 32) + warp - 4, seq + 1);
       }
     }
   }
@@ -380,11 +414,54 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_split_gemm_kernel(const __gri
   }
 }
 
+// Three bf16 planes of two values each, hi = bf16(x), mid = bf16(x - hi), lo = bf16(x - hi - mid),
+// every conversion rounding to nearest even.
+//
+// The conversions FP64 -> bf16 and FP32 -> FP64 run at an eighth of the issue rate and bound
+// the kernels below, so hi and mid go back to FP64 without one: their exponent and mantissa,
+// three bits lower in the upper word, are the value times 2^-896, and an FMA scales it back
+// while it subtracts (exact; a zero stays zero).  Values outside 2^-62 <= |x| < 2^127, where a
+// plane could leave bf16's normal range, take the plain conversions.
+__device__ __forceinline__ double sub_bf16(double x, unsigned h) {  // h: the bf16 in the upper 16 bits
+  return fma(__hiloint2double(((int)h >> 3) & (int)0x8fffffffu, 0), -0x1p896, x);
+}
+__device__ __forceinline__ unsigned to_bf16_pair(double x0, double x1) {
+  return (unsigned)__bfloat16_as_ushort(__double2bfloat16(x0)) |
+         ((unsigned)__bfloat16_as_ushort(__double2bfloat16(x1)) << 16);
+}
+__device__ __forceinline__ bool plane_range(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x3c100000u < 0x0bd00000u;
+}
+__device__ __forceinline__ void split3(double x, __nv_bfloat16& hi, __nv_bfloat16& mid, __nv_bfloat16& lo) {
+  hi = __double2bfloat16(x);
+  const double r1 = x - (double)__bfloat162float(hi);  // exact: hi is within 2^-9 |x| of x
+  mid = __double2bfloat16(r1);
+  const double r2 = r1 - (double)__bfloat162float(mid);
+  lo = __double2bfloat16(r2);
+}
+__device__ __forceinline__ void split3_pair(double x0, double x1, unsigned& hi, unsigned& mid, unsigned& lo) {
+  if (plane_range(x0) && plane_range(x1)) {
+    hi = to_bf16_pair(x0, x1);
+    x0 = sub_bf16(x0, hi << 16);
+    x1 = sub_bf16(x1, hi & 0xffff0000u);
+    mid = to_bf16_pair(x0, x1);
+    lo = to_bf16_pair(sub_bf16(x0, mid << 16), sub_bf16(x1, mid & 0xffff0000u));
+    return;
+  }
+  __nv_bfloat16 h0, m0, l0, h1, m1, l1;
+  split3(x0, h0, m0, l0);
+  split3(x1, h1, m1, l1);
+  hi = (unsigned)__bfloat16_as_ushort(h0) | ((unsigned)__bfloat16_as_ushort(h1) << 16);
+  mid = (unsigned)__bfloat16_as_ushort(m0) | ((unsigned)__bfloat16_as_ushort(m1) << 16);
+  lo = (unsigned)__bfloat16_as_ushort(l0) | ((unsigned)__bfloat16_as_ushort(l1) << 16);
+}
+
 // S_r (side 0) or T_r (side 1) of product r = blockIdx.x, summed in FP64 from FP32 inputs
 // and split into three bf16 planes, K-major: plane p of product r holds rows
 // (3 r + p) * rows .. + rows, row pitch kpad; columns k in [ks, kpad) are zeros.  A CTA
 // makes a 32-row x 64-k tile; products vary fastest in the grid, so the CTAs resident at
 // one time read the same input tiles and every input element comes from HBM about once.
+// Runs where fmm_split_planes_kernel's staged tiles do not fit.
 //   side 0: X = A (column-major, m x k), plane row i = row of A; the tile is transposed
 //           through shared memory so that both the reads and the writes coalesce.
 //   side 1: X = B (column-major, k x n), plane row j = column of B (k already contiguous).
@@ -402,25 +479,16 @@ struct SplitArgs {
 
 constexpr int SPLIT_ROWS = 32, SPLIT_K = 64;
 
-__device__ __forceinline__ void split3(double x, __nv_bfloat16& hi, __nv_bfloat16& mid, __nv_bfloat16& lo) {
-  hi = __double2bfloat16(x);
-  const double r1 = x - (double)__bfloat162float(hi);  // exact: hi is within 2^-9 |x| of x
-  mid = __double2bfloat16(r1);
-  const double r2 = r1 - (double)__bfloat162float(mid);
-  lo = __double2bfloat16(r2);
-}
-
 // Planes of two k-adjacent values, stored as bf16 pairs.
 __device__ __forceinline__ void store_split_pair(const SplitArgs& a, int r, int row, int kk, double x0, double x1) {
-  __nv_bfloat16 h0, m0, l0, h1, m1, l1;
-  split3(x0, h0, m0, l0);
-  split3(x1, h1, m1, l1);
+  unsigned hi, mid, lo;
+  split3_pair(x0, x1, hi, mid, lo);
   const size_t plane = (size_t)a.rows * a.kpad;
-  __nv_bfloat162* P = reinterpret_cast<__nv_bfloat162*>(a.out + (size_t)(3 * r) * plane + (size_t)row * a.kpad + kk);
+  unsigned* P = reinterpret_cast<unsigned*>(a.out + (size_t)(3 * r) * plane + (size_t)row * a.kpad + kk);
   const size_t step = plane / 2;  // plane size in bf16 pairs (kpad is even)
-  P[0] = __halves2bfloat162(h0, h1);
-  P[step] = __halves2bfloat162(m0, m1);
-  P[2 * step] = __halves2bfloat162(l0, l1);
+  P[0] = hi;
+  P[step] = mid;
+  P[2 * step] = lo;
 }
 
 __global__ void __launch_bounds__(256) fmm_split_operands_kernel(const SplitArgs a) {
@@ -466,112 +534,132 @@ __global__ void __launch_bounds__(256) fmm_split_operands_kernel(const SplitArgs
   }
 }
 
-// Every product's operand sum from one read of the operand: a CTA stages one tile position of
-// all the operand's blocks (side 0: 16 rows x 32 k of each A block, side 1: 8 columns x 64 k
-// of each B block) in shared memory in the output orientation (row, k), then makes all R
-// products' sums of that tile in FP64 in term order (the same arithmetic as
-// fmm_split_operands_kernel, so the planes are bit-identical) and stores their three bf16
-// planes.  Each input element is read from HBM once and no CTA waits on a global load per
-// term: the per-product kernel read each block once per product that uses it.
-//   tables (shared memory): per product its first term and term count; per term its block
-//   (row * block_cols + col of the operand's block grid) and coefficient.
-template <int SIDE>
-struct SplitAllShape;
-template <>
-struct SplitAllShape<0> {  // A: 16 rows x 32 k, loads coalesced along rows
-  static constexpr int TR = 16, TK = 32;
-};
-template <>
-struct SplitAllShape<1> {  // B: 8 columns x 64 k, loads coalesced along k
-  static constexpr int TR = 8, TK = 64;
+// Every product's operand planes from one read of the operand: a CTA stages 16 rows x 32 or 64 k
+// of all the operand's blocks (several such k tiles where the blocks are few) in shared memory in
+// the output orientation (row, k), then makes all R products' sums of that tile in FP64 in
+// term order (the arithmetic of fmm_split_operands_kernel, so the planes are the same bits) and
+// stores their three planes, 64-byte row segments at a time.  One launch covers the operands of
+// several GEMMs (an FMM core and its strips).  Bound by instruction issue (77 % of the cycles)
+// and the conversion pipe (56 %).  Measured us, both operands, against one launch per operand
+// that built its tables in every CTA and converted every plane back and forth: 6704 x 3320 x
+// 6256 classical 307 -> 168, 222-1 4096^3 168 -> 124, 222-2 2048^3 97 -> 82, 8192^3 1129 -> 1065;
+// with the strips of 222-1 1021 x 3007 x 1530, 92 -> 46.
+struct PlaneJob {
+  const float* X;
+  long long ldx;
+  __nv_bfloat16* out;
+  const int* first;        // per product its first term of this side (nprod + 1 entries)
+  const PTerm* terms;
+  int rows, ks, kpad;      // plane rows, k per product, row pitch
+  int blk_row_stride;      // A: ms (rows per block row), B: ks
+  int blk_col_stride;      // A: ks (columns per block column), B: ns
+  int nblk, block_cols;    // the operand's block grid: nblk blocks, block_cols per block row
+  int nprod, nterm;
+  int side;
+  int kt, kts;             // k tiles, and how many of them a CTA takes
+  int cta0;                // first CTA of the job
 };
 
-struct SplitAllArgs {
-  SplitArgs s;
-  int nblk, block_cols;  // the operand's block grid: nblk blocks, block_cols per block row
-  int nprod;
-  int nterm;             // sum of the products' term counts on this side
+constexpr int MAX_PLANE_JOBS = 8;
+struct PlaneArgs {
+  PlaneJob job[MAX_PLANE_JOBS];
+  int njob;
+  int nzero;
+  int* zero;               // cleared: the GEMM's work-unit counter and tickets
 };
 
-__host__ __device__ constexpr size_t split_all_smem_bytes(int side, int nblk, int nprod, int nterm) {
-  return sizeof(float) * (size_t)nblk * (side == 0 ? 16 * 33 : 8 * 65) + sizeof(int) * (2 * (size_t)nprod + nterm) +
-         sizeof(double) * (size_t)nterm + 16;
+__host__ __device__ constexpr int plane_ld(int np) { return 32 * np + 2; }  // floats per staged row
+struct PlaneTerm {
+  double coef;
+  int off;                 // the block's staged tile
+  int pad;
+};
+__host__ __device__ constexpr size_t plane_smem_bytes(int tr, int np, int nblk, int kts, int nprod, int nterm) {
+  return sizeof(PlaneTerm) * (size_t)nterm + sizeof(long long) * (size_t)nblk +
+         sizeof(float) * (size_t)nblk * kts * tr * plane_ld(np) + sizeof(int) * ((size_t)nprod + 1);
 }
 
-template <int SIDE>
-__global__ void __launch_bounds__(256) fmm_split_all_kernel(const SplitAllArgs g) {
-  constexpr int TR = SplitAllShape<SIDE>::TR, TK = SplitAllShape<SIDE>::TK, LD = TK + 1;
-  const SplitArgs& a = g.s;
-  extern __shared__ __align__(16) double sall[];
-  double* tcoef = sall;                                      // [nterm]
-  int* tblk = reinterpret_cast<int*>(tcoef + g.nterm);       // [nterm]
-  int* tfirst = tblk + g.nterm;                              // [nprod]
-  int* tcount = tfirst + g.nprod;                            // [nprod]
-  float* x = reinterpret_cast<float*>(tcount + g.nprod);     // [nblk][TR][LD]
+// TR rows x 32 NP k, 16 threads per row: thread q of a row makes the k pairs 2 q + 32 h, h < NP.
+template <int TR, int NP>
+__global__ void __launch_bounds__(16 * TR) fmm_split_planes_kernel(const __grid_constant__ PlaneArgs g) {
+  constexpr int NTH = 16 * TR, TK = 32 * NP, LD = plane_ld(NP), EL = 2 * NP;
+  extern __shared__ __align__(16) unsigned char psm[];
+  fmmt::grid_wait();
+  fmmt::grid_launch();
   const int tid = threadIdx.x;
-  // tables: term counts in parallel, offsets by one thread (shared memory only), terms in parallel
-  for (int r = tid; r < g.nprod; r += blockDim.x) {
-    const Prod p = a.prods[r];
-    tcount[r] = SIDE == 0 ? p.na : p.nb;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int acc = 0;
-    for (int r = 0; r < g.nprod; ++r) {
-      tfirst[r] = acc;
-      acc += tcount[r];
-    }
-  }
-  __syncthreads();
-  for (int r = tid; r < g.nprod; r += blockDim.x) {
-    const Prod p = a.prods[r];
-    const int t0 = SIDE == 0 ? p.a0 : p.b0, nt = tcount[r], f = tfirst[r];
-    for (int t = 0; t < nt; ++t) {
-      const Term tm = a.terms[t0 + t];
-      tcoef[f + t] = tm.coef;
-      tblk[f + t] = tm.row * g.block_cols + tm.col;
-    }
-  }
-  const int row0 = blockIdx.y * TR, k0 = blockIdx.x * TK;
-  // stage every block's tile, output orientation x[b][row][k]; zeros outside the block
-  for (int b = 0; b < g.nblk; ++b) {
-    const int br = b / g.block_cols, bc = b % g.block_cols;
-    float* xb = x + (size_t)b * TR * LD;
-    if (SIDE == 0) {  // A[(br ms + i) + (bc ks + k) lda]: lanes along i
-      const int i = tid % TR;
+  for (long long q = (long long)blockIdx.x * NTH + tid; q < g.nzero; q += (long long)gridDim.x * NTH) g.zero[q] = 0;
+  int ji = 0;
 #pragma unroll
-      for (int kk = tid / TR; kk < TK; kk += 256 / TR) {
-        const int row = row0 + i, k = k0 + kk;
-        xb[i * LD + kk] = (row < a.rows && k < a.ks)
-                              ? a.X[(long long)br * a.blk_row_stride + row + ((long long)bc * a.blk_col_stride + k) * a.ldx]
-                              : 0.0f;
-      }
-    } else {  // B[(br ks + k) + (bc ns + j) ldb]: lanes along k
-      const int kk = tid % TK;
+  for (int q = 1; q < MAX_PLANE_JOBS; ++q)
+    if (q < g.njob && (int)blockIdx.x >= g.job[q].cta0) ji = q;
+  const PlaneJob& a = g.job[ji];
+  const int bid = (int)blockIdx.x - a.cta0;
+  // k tiles vary fastest: the CTAs resident at one time write whole rows of the planes
+  const int kg = (a.kt + a.kts - 1) / a.kts;
+  const int row0 = (bid / kg) * TR, kt0 = (bid % kg) * a.kts, nkt = min(a.kts, a.kt - kt0);
+  PlaneTerm* tt = reinterpret_cast<PlaneTerm*>(psm);                        // [nterm]
+  long long* bo = reinterpret_cast<long long*>(tt + a.nterm);               // [nblk] block offsets
+  float* x = reinterpret_cast<float*>(bo + a.nblk);                         // [kts][nblk][TR][LD]
+  int* tf = reinterpret_cast<int*>(x + (size_t)a.kts * a.nblk * TR * LD);  // [nprod + 1]
+  for (int b = tid; b < a.nblk; b += NTH)
+    bo[b] = (long long)(b / a.block_cols) * a.blk_row_stride + (long long)(b % a.block_cols) * a.blk_col_stride * a.ldx;
+  for (int t = tid; t < a.nterm; t += NTH) {
+    const PTerm tm = a.terms[t];
+    tt[t] = PlaneTerm{tm.coef, (tm.row * a.block_cols + tm.col) * TR * LD, 0};
+  }
+  for (int r = tid; r <= a.nprod; r += NTH) tf[r] = a.first[r];
+  __syncthreads();
+  // the blocks' tiles, zeros outside the block; lanes along the operand's contiguous direction
+  const int lr = a.side == 0 ? tid % TR : tid / TK, lk = a.side == 0 ? tid / TR : tid % TK;
+  const int dr = a.side == 0 ? 0 : NTH / TK, dk = a.side == 0 ? 16 : 0;
+  const long long sr = a.side == 0 ? 1 : a.ldx, sk = a.side == 0 ? a.ldx : 1;
+  for (int kq = 0; kq < nkt; ++kq) {
+    const int k0 = (kt0 + kq) * TK + lk;
+    const float* xk = a.X + (row0 + lr) * sr + k0 * sk;
+    float* xs = x + ((size_t)kq * a.nblk * TR + lr) * LD + lk;
+    bool in[EL];
 #pragma unroll
-      for (int j = tid / TK; j < TR; j += 256 / TK) {
-        const int row = row0 + j, k = k0 + kk;
-        xb[j * LD + kk] = (row < a.rows && k < a.ks)
-                              ? a.X[(long long)br * a.blk_row_stride + k + ((long long)bc * a.blk_col_stride + row) * a.ldx]
-                              : 0.0f;
-      }
+    for (int e = 0; e < EL; ++e) in[e] = row0 + lr + e * dr < a.rows && k0 + e * dk < a.ks;
+#pragma unroll 4
+    for (int b = 0; b < a.nblk; ++b) {
+      const float* xb = xk + bo[b];
+#pragma unroll
+      for (int e = 0; e < EL; ++e) xs[(b * TR + e * dr) * LD + e * dk] = in[e] ? __ldg(xb + e * (dr * sr + dk * sk)) : 0.0f;
     }
   }
   __syncthreads();
-  // one k pair per thread: rows TR x TK / 2 pairs = 256
-  const int row = tid / (TK / 2), kk = 2 * (tid % (TK / 2));
+  const int q = tid % 16, row = tid / 16;
   if (row0 + row >= a.rows) return;
-  const float* xr = x + row * LD + kk;
-  for (int r = 0; r < g.nprod; ++r) {
-    double v0 = 0.0, v1 = 0.0;
-    const int f = tfirst[r], nt = tcount[r];
-    for (int t = 0; t < nt; ++t) {
-      const float* xp = xr + (size_t)tblk[f + t] * TR * LD;
-      const double w = tcoef[f + t];
-      v0 = fma(w, (double)xp[0], v0);
-      v1 = fma(w, (double)xp[1], v1);
+  const size_t step = (size_t)a.rows * a.kpad / 2;  // plane size in bf16 pairs
+  for (int kq = 0; kq < nkt; ++kq) {
+    const float* xr = x + ((size_t)kq * a.nblk * TR + row) * LD + 2 * q;
+    unsigned* P = reinterpret_cast<unsigned*>(a.out + (size_t)(row0 + row) * a.kpad + (kt0 + kq) * TK + 2 * q);
+    int f = 0;
+#pragma unroll 1
+    for (int r = 0; r < a.nprod; ++r, P += 3 * step) {
+      const int fe = tf[r + 1];
+      double v[2 * NP];
+#pragma unroll
+      for (int h = 0; h < 2 * NP; ++h) v[h] = 0.0;
+#pragma unroll 1
+      for (; f < fe; ++f) {
+        const PlaneTerm t = tt[f];
+#pragma unroll
+        for (int h = 0; h < NP; ++h) {
+          const float2 u = *reinterpret_cast<const float2*>(xr + t.off + 32 * h);
+          v[2 * h] = fma(t.coef, (double)u.x, v[2 * h]);
+          v[2 * h + 1] = fma(t.coef, (double)u.y, v[2 * h + 1]);
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < NP; ++h) {
+        unsigned hi, mid, lo;
+        split3_pair(v[2 * h], v[2 * h + 1], hi, mid, lo);
+        P[16 * h] = hi;
+        P[step + 16 * h] = mid;
+        P[2 * step + 16 * h] = lo;
+      }
     }
-    store_split_pair(a, r, row0 + row, k0 + kk, v0, v1);
   }
 }
 
