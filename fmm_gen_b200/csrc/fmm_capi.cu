@@ -103,8 +103,8 @@ struct DevTables {
   int* cg_m = nullptr;
   double* cg_c = nullptr;
   int* ch_r = nullptr;
-  unsigned long long* ch_m = nullptr;
-  double* ch_c = nullptr;
+  unsigned long long* ch_n = nullptr;
+  fmm::CombineOp* ch_op = nullptr;
   fmm::Prod* prods_ps = nullptr;  // products over pre-summed operands (one A and one B term each)
   fmm::Term* terms_ps = nullptr;
   int* plistA = nullptr;          // products whose A operand is pre-summed, in slot order
@@ -145,8 +145,8 @@ struct fmm_plan {
   std::vector<double> cg_c;
   int n_cgroup = 0;
   std::vector<int> ch_r;                 // staged kernel: CST_CHUNK products per chunk
-  std::vector<unsigned long long> ch_m;  // one byte of slot bits per member
-  std::vector<double> ch_c;              // COMBINE_GROUP x CST_CHUNK coefficients per chunk
+  std::vector<unsigned long long> ch_n;  // one byte per member: its operations in the chunk
+  std::vector<fmm::CombineOp> ch_op;     // the operations in the order they run
   // Pre-summed form: each product's A operand is either its single A block (src 0) or
   // slot j of the workspace S (src 1) that holds sum_i U[i,r] A_i; likewise for B / T.
   std::vector<fmm::Prod> prods_ps;
@@ -209,8 +209,8 @@ int upload_tables(fmm_plan* p, DevTables& d) {
     FMM_CUDA_TRY(up(&d.cg_m, p->cg_m));
     FMM_CUDA_TRY(up(&d.cg_c, p->cg_c));
     FMM_CUDA_TRY(up(&d.ch_r, p->ch_r));
-    FMM_CUDA_TRY(up(&d.ch_m, p->ch_m));
-    FMM_CUDA_TRY(up(&d.ch_c, p->ch_c));
+    FMM_CUDA_TRY(up(&d.ch_n, p->ch_n));
+    FMM_CUDA_TRY(up(&d.ch_op, p->ch_op));
     for (int side = 0; side < 2; ++side) {
       FMM_CUDA_TRY(up(&d.ps_first[side], p->ps_first[side]));
       FMM_CUDA_TRY(up(&d.ps_terms[side], p->ps_terms[side]));
@@ -392,8 +392,8 @@ void build_combine_groups(fmm_plan* p) {
   }
   p->cg_desc.clear();
   p->ch_r.clear();
-  p->ch_m.clear();
-  p->ch_c.clear();
+  p->ch_n.clear();
+  p->ch_op.clear();
   p->cg_r.clear();
   p->cg_m.clear();
   p->cg_c.clear();
@@ -416,14 +416,12 @@ void build_combine_groups(fmm_plan* p) {
       p->cg_m.push_back(mask | (k0 << 8));
     }
     // the group's entries in chunks of CST_CHUNK (the staged kernel's stage): per chunk the
-    // products, one byte per member (bit t: slot t updates it) and a member-major
-    // CST_CHUNK x CST_CHUNK coefficient block (0 where the bit is clear)
+    // products, and per member the operations on it, slots in increasing product order
     const int first_chunk = (int)(p->ch_r.size() / fmm::CST_CHUNK);
     {
       const int ne = (int)p->cg_r.size() - first;
       for (int q0 = 0; q0 < ne; q0 += fmm::CST_CHUNK) {
-        unsigned long long bits = 0;
-        std::vector<double> cf((size_t)fmm::COMBINE_GROUP * fmm::CST_CHUNK, 0.0);
+        std::vector<fmm::CombineOp> ops[fmm::COMBINE_GROUP];
         for (int t = 0; t < fmm::CST_CHUNK; ++t) {
           const int e = first + std::min(q0 + t, ne - 1);
           p->ch_r.push_back(p->cg_r[e]);
@@ -431,13 +429,15 @@ void build_combine_groups(fmm_plan* p) {
           const int mk = p->cg_m[e];
           int kc = mk >> 8;
           for (int q = 0; q < fmm::COMBINE_GROUP; ++q)
-            if (mk & (1 << q)) {
-              bits |= 1ULL << (8 * q + t);
-              cf[(size_t)q * fmm::CST_CHUNK + t] = p->cg_c[kc++];
-            }
+            if (mk & (1 << q))
+              ops[q].push_back(fmm::CombineOp{p->cg_c[kc++], (int)(t * fmm::CST_TILE * sizeof(double)), 0});
         }
-        p->ch_m.push_back(bits);
-        p->ch_c.insert(p->ch_c.end(), cf.begin(), cf.end());
+        unsigned long long n = 0;
+        for (int q = 0; q < fmm::COMBINE_GROUP; ++q) {
+          n |= (unsigned long long)ops[q].size() << (8 * q);
+          p->ch_op.insert(p->ch_op.end(), ops[q].begin(), ops[q].end());
+        }
+        p->ch_n.push_back(n);
       }
     }
     p->cg_desc.push_back(first);
@@ -452,15 +452,18 @@ void build_combine_groups(fmm_plan* p) {
   p->n_cgroup = (int)mem.size();
   // the kernels index their tables with these values: check them here (a plan whose tables
   // fail falls back to the per-block scatter)
-  bool ok = p->ch_r.size() == (size_t)fmm::CST_CHUNK * p->ch_m.size() &&
-            p->ch_c.size() == (size_t)fmm::COMBINE_GROUP * fmm::CST_CHUNK * p->ch_m.size();
+  size_t nop = 0;
+  for (unsigned long long n : p->ch_n)
+    for (int q = 0; q < fmm::COMBINE_GROUP; ++q) nop += (n >> (8 * q)) & 0xff;
+  bool ok = p->ch_r.size() == (size_t)fmm::CST_CHUNK * p->ch_n.size() && nop == p->ch_op.size();
+  for (const auto& o : p->ch_op) ok = ok && o.off >= 0 && o.off < (int)(fmm::CST_STAGE_DOUBLES * sizeof(double));
   for (int r : p->ch_r) ok = ok && r >= 0 && r < p->rank;
   for (int r : p->cg_r) ok = ok && r >= 0 && r < p->rank;
   for (int g = 0; ok && g < p->n_cgroup; ++g) {
     const int* gd = p->cg_desc.data() + (size_t)g * fmm::GDESC;
     const int nch = (gd[1] + fmm::CST_CHUNK - 1) / fmm::CST_CHUNK;
     ok = gd[1] > 0 && gd[0] + gd[1] <= (int)p->cg_r.size() && gd[2] >= 1 && gd[2] <= fmm::COMBINE_GROUP &&
-         gd[3] >= 0 && gd[3] + nch <= (int)p->ch_m.size();
+         gd[3] >= 0 && gd[3] + nch <= (int)p->ch_n.size();
     for (int q = 0; ok && q < fmm::COMBINE_GROUP; ++q) ok = gd[4 + q] >= 0 && gd[4 + q] < p->dims[0] * p->dims[2];
   }
   if (!ok) p->n_cgroup = 0;
@@ -982,13 +985,14 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
   ga.ec = d.cg_c;
   ga.nprod = plan->rank;
   const long long total = (long long)ms * ns;
-  ga.nchunk = (int)plan->ch_m.size();
+  ga.nchunk = (int)plan->ch_n.size();
+  ga.nop = (int)plan->ch_op.size();
   ga.chr = d.ch_r;
-  ga.chm = d.ch_m;
-  ga.chc = d.ch_c;
-  const size_t ssm = fmm::combine_staged_smem_bytes(ga.ngroup, ga.nchunk);
+  ga.chn = d.ch_n;
+  ga.op = d.ch_op;
+  const size_t ssm = fmm::combine_staged_smem_bytes(ga.ngroup, ga.nchunk, ga.nop);
   // staged form: the M tiles of a position range are contiguous 16-byte-aligned runs
-  const bool staged = g_combine_positions.load() == 0 && ldm == ms && m_stride % 2 == 0 && total % 2 == 0 &&
+  const bool staged = g_combine_positions.load() == 0 && ldm == ms && m_stride % 2 == 0 && ms % 2 == 0 &&
                       ((uintptr_t)M & 15) == 0 && ssm <= 200 * 1024 && total > 0;
   if (staged) {
     const long long ntile = (total + fmm::CST_TILE - 1) / fmm::CST_TILE;
@@ -1446,8 +1450,8 @@ int fmm_plan_destroy(fmm_plan* plan) {
     cudaFree(d.cg_m);
     cudaFree(d.cg_c);
     cudaFree(d.ch_r);
-    cudaFree(d.ch_m);
-    cudaFree(d.ch_c);
+    cudaFree(d.ch_n);
+    cudaFree(d.ch_op);
     cudaFree(d.prods_ps);
     cudaFree(d.terms_ps);
     cudaFree(d.plistA);
@@ -1474,7 +1478,7 @@ int fmm_plan_combine_info(const fmm_plan* plan, int* groups, int* entries, int* 
   if (!plan) return FMM_E_INVALID;
   if (groups) *groups = plan->n_cgroup;
   if (entries) *entries = plan->n_cgroup ? (int)plan->cg_r.size() : 0;
-  if (chunks) *chunks = plan->n_cgroup ? (int)plan->ch_m.size() : 0;
+  if (chunks) *chunks = plan->n_cgroup ? (int)plan->ch_n.size() : 0;
   return FMM_OK;
 }
 

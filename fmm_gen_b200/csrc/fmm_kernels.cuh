@@ -1169,10 +1169,17 @@ struct CombineGroupArgs {
   const double* ec;
   int nprod;  // products (slabs of M)
   // staged kernel: the entries of each group in chunks of CST_CHUNK
-  int nchunk;
+  int nchunk, nop;
   const int* chr;                 // [nchunk][CST_CHUNK] products (past a group's end: its last)
-  const unsigned long long* chm;  // [nchunk] byte q: slots that update member q
-  const double* chc;              // [nchunk][COMBINE_GROUP][CST_CHUNK] coefficients
+  const unsigned long long* chn;  // [nchunk] byte q: operations on member q
+  const struct CombineOp* op;     // the operations in the order they run: per chunk, per member
+};
+
+// c_member += coef * M of the chunk's slot at byte offset `off` of the stage.
+struct CombineOp {
+  double coef;
+  int off;
+  int pad;
 };
 
 __host__ __device__ constexpr size_t combine_group_smem_bytes(int ngroup, int nent, int ncoef) {
@@ -1262,22 +1269,27 @@ __global__ void __launch_bounds__(COMBINE_G_THREADS) fmm_combine_kernel(const Co
 // CST_TILE consecutive element positions (M_r[e0 .. e0 + CST_TILE) is contiguous when
 // ldm == ms), walked group by group and, within a group, CST_CHUNK products at a time; a
 // producer warp copies each chunk's M_r tiles (cp.async.bulk, 2 KB each) into a ring of
-// CST_STAGES stages while the compute warps apply earlier chunks, so the loads in flight per
-// SM are bounded by shared memory instead of registers.  A compute thread owns one position
-// of the tile and keeps its group's running C values in registers; the arithmetic per block
-// is the register kernel's (bit-identical).  Waits are bounded (status word on timeout).
-constexpr int CST_THREADS = 256;  // compute threads, one position each
-constexpr int CST_TILE = CST_THREADS;
+// CST_STAGES stages while the compute warps apply earlier chunks.  HBM bound: every M_r and C
+// element once, and the M_r tiles a later group reads again that have left L2 by then (222-1 x
+// 333-1: 1.3 x the algorithmic bytes; C goes past L2 with streaming hints so that fewer do).  A
+// compute thread owns two positions (16-byte loads) and keeps its group's running C values in
+// registers; what to do with a chunk is a list of operations per member in shared memory, so
+// an update of two values costs two loads, two FMAs and the loop.  The arithmetic per block is
+// the register kernel's (bit-identical).  Measured on B200 against one position per thread
+// with bit masks walked per chunk: 222-1 x 333-1 14400^2 x 480 2.65 -> 2.23 ms, 222-2 8192^3
+// split 0.58 -> 0.49 ms; fewer or single-position warps, a software pipeline over the
+// operations and loading the next group's C ahead were slower or the same.
+// Waits are bounded (status word on timeout).
+constexpr int CST_THREADS = 128;  // compute threads, two positions each
+constexpr int CST_TILE = 2 * CST_THREADS;
 constexpr int CST_CHUNK = 8;      // products per stage
-constexpr int CST_STAGES = 3;  // 48 KB of stages: three CTAs per SM (24 compute warps)
+constexpr int CST_STAGES = 3;     // 48 KB of stages: three CTAs per SM
 constexpr size_t CST_STAGE_DOUBLES = (size_t)CST_CHUNK * CST_TILE;
-static_assert(COMBINE_GROUP * CST_CHUNK <= 64, "one 64-bit word of slot bits per chunk");
 
-__host__ __device__ constexpr size_t combine_staged_smem_bytes(int ngroup, int nchunk) {
-  return sizeof(double) * CST_STAGE_DOUBLES * CST_STAGES + 16 * CST_STAGES +
-         (sizeof(double) * COMBINE_GROUP * CST_CHUNK + sizeof(unsigned long long) + sizeof(int) * CST_CHUNK) *
-             (size_t)nchunk +
-         sizeof(int) * GDESC * (size_t)ngroup + 16;
+__host__ __device__ constexpr size_t combine_staged_smem_bytes(int ngroup, int nchunk, int nop) {
+  return sizeof(double) * CST_STAGE_DOUBLES * CST_STAGES + 16 * CST_STAGES + sizeof(CombineOp) * (size_t)nop +
+         (sizeof(unsigned long long) + sizeof(int) * CST_CHUNK) * (size_t)nchunk +
+         (sizeof(long long) * COMBINE_GROUP + sizeof(int) * GDESC) * (size_t)ngroup + 16;
 }
 
 __device__ __forceinline__ void bulk_load_1d(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
@@ -1286,24 +1298,47 @@ __device__ __forceinline__ void bulk_load_1d(unsigned dst, const void* src, unsi
                : "memory");
 }
 
+// Two consecutive C values of every member of a group at element offset cofs.
+__device__ __forceinline__ void combine_load(const CombineGroupArgs& a, const long long* off, int nm, long long cofs,
+                                             bool live, bool vec, double2 (&c)[COMBINE_GROUP]) {
+#pragma unroll
+  for (int q = 0; q < COMBINE_GROUP; ++q) {
+    c[q] = make_double2(0.0, 0.0);
+    if (q < nm && live) {
+      const double* p = a.C + off[q] + cofs;
+      if (vec) {
+        c[q] = __ldcs(reinterpret_cast<const double2*>(p));
+      } else {
+        c[q].x = __ldcs(p);
+        c[q].y = __ldcs(p + 1);
+      }
+    }
+  }
+}
+
 // CombineGroupArgs plus the status word; requires ldm == ms, M and m_stride 16-byte
-// multiples (in doubles: m_stride even) and ms * ns even (every tile's byte count a multiple
-// of 16).
-__global__ void __launch_bounds__(CST_THREADS + 32) fmm_combine_staged_kernel(const CombineGroupArgs a,
-                                                                              unsigned* status) {
+// multiples (in doubles: m_stride even) and ms even (pairs of positions lie in one column, and
+// every tile's byte count is a multiple of 16).
+__global__ void __launch_bounds__(CST_THREADS + 32, 3) fmm_combine_staged_kernel(const CombineGroupArgs a,
+                                                                                 unsigned* status) {
   extern __shared__ __align__(128) double cst[];
   double* stages = cst;                                                    // [STAGES][CHUNK][TILE]
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(stages + CST_STAGE_DOUBLES * CST_STAGES);
-  double* sc = reinterpret_cast<double*>(bars + 2 * CST_STAGES);           // [nchunk][GROUP][CHUNK]
-  unsigned long long* smk = reinterpret_cast<unsigned long long*>(sc + (size_t)a.nchunk * COMBINE_GROUP * CST_CHUNK);
-  int* sr = reinterpret_cast<int*>(smk + a.nchunk);                        // [nchunk][CHUNK]
+  CombineOp* sop = reinterpret_cast<CombineOp*>(bars + 2 * CST_STAGES);    // [nop]
+  unsigned long long* scn = reinterpret_cast<unsigned long long*>(sop + a.nop);  // [nchunk]
+  long long* sgo = reinterpret_cast<long long*>(scn + a.nchunk);           // [ngroup][GROUP] block offsets in C
+  int* sr = reinterpret_cast<int*>(sgo + (size_t)a.ngroup * COMBINE_GROUP);  // [nchunk][CHUNK]
   int* sg = sr + (size_t)a.nchunk * CST_CHUNK;                             // [GDESC * ngroup]
   const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + CST_STAGES);
   const int tid = threadIdx.x;
-  for (int q = tid; q < a.nchunk * COMBINE_GROUP * CST_CHUNK; q += blockDim.x) sc[q] = a.chc[q];
-  for (int q = tid; q < a.nchunk; q += blockDim.x) smk[q] = a.chm[q];
+  for (int q = tid; q < a.nop; q += blockDim.x) sop[q] = a.op[q];
+  for (int q = tid; q < a.nchunk; q += blockDim.x) scn[q] = a.chn[q];
   for (int q = tid; q < a.nchunk * CST_CHUNK; q += blockDim.x) sr[q] = a.chr[q];
   for (int q = tid; q < GDESC * a.ngroup; q += blockDim.x) sg[q] = a.gdesc[q];
+  for (int q = tid; q < COMBINE_GROUP * a.ngroup; q += blockDim.x) {
+    const int b = a.gdesc[(q / COMBINE_GROUP) * GDESC + 4 + q % COMBINE_GROUP];
+    sgo[q] = (long long)(b / a.grid_n) * a.ms + (long long)(b % a.grid_n) * a.ns * a.ldc;
+  }
   if (tid == 0) {
     for (int s = 0; s < CST_STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
@@ -1348,40 +1383,38 @@ __global__ void __launch_bounds__(CST_THREADS + 32) fmm_combine_staged_kernel(co
     return;
   }
   const int lane = tid & 31;
+  const bool vec = ((reinterpret_cast<uintptr_t>(a.C) & 15) == 0) && (a.ldc & 1) == 0;
+  auto position = [&](long long t, bool& live) {  // element offset in a C block of this thread's pair
+    const long long e = t * CST_TILE + 2 * tid;
+    live = t < ntile && e < total;
+    const long long ee = live ? e : 0;
+    return (ee % a.ms) + (ee / a.ms) * a.ldc;
+  };
+  double2 c[COMBINE_GROUP];
   for (long long t = blockIdx.x; t < ntile; t += gridDim.x) {
-    const long long e = t * CST_TILE + tid;
-    const bool live = e < total;
-    const long long ee = live ? e : total - 1;
-    const long long cofs = (ee % a.ms) + (ee / a.ms) * a.ldc;
+    bool live;
+    const long long cofs = position(t, live);
+    const CombineOp* op = sop;
     for (int g = 0; g < a.ngroup; ++g) {
       const int* gd = sg + g * GDESC;
       const int ne = gd[1], nm = gd[2], c0 = gd[3];
-      double c[COMBINE_GROUP];
-      long long cb[COMBINE_GROUP];
-#pragma unroll
-      for (int q = 0; q < COMBINE_GROUP; ++q) {
-        const int b = gd[4 + (q < nm ? q : 0)];
-        cb[q] = (long long)(b / a.grid_n) * a.ms + (long long)(b % a.grid_n) * a.ns * a.ldc + cofs;
-        c[q] = q < nm ? a.C[cb[q]] : 0.0;
-      }
+      combine_load(a, sgo + g * COMBINE_GROUP, nm, cofs, live, vec, c);
       for (int q0 = 0; q0 < ne; q0 += CST_CHUNK, ++k) {
         const int s = (int)(k % CST_STAGES);
-        const int ch = c0 + q0 / CST_CHUNK;
-        const unsigned long long bits = smk[ch];
-        const double* cf = sc + (size_t)ch * COMBINE_GROUP * CST_CHUNK;
+        const unsigned long long cnt = scn[c0 + q0 / CST_CHUNK];
         mbar_wait(full0 + 8 * s, (unsigned)((k / CST_STAGES) & 1), status);
-        const double* st = stages + (size_t)s * CST_STAGE_DOUBLES + tid;
-        // per member only its set slots (warp-uniform bit loops): the M value and the
-        // coefficient come from shared memory at the slot's index, the running value stays in
-        // a register (members unrolled); slots past the group's end have no bits
+        const unsigned char* st = reinterpret_cast<const unsigned char*>(stages + (size_t)s * CST_STAGE_DOUBLES) + 16 * tid;
 #pragma unroll
         for (int b = 0; b < COMBINE_GROUP; ++b) {
-          unsigned bq = (unsigned)(bits >> (8 * b)) & 0xffu;
-          while (bq) {
-            const int q = __ffs(bq) - 1;
-            bq &= bq - 1;
-            c[b] = fma(cf[b * CST_CHUNK + q], st[(size_t)q * CST_TILE], c[b]);
+          const int n = (int)(cnt >> (8 * b)) & 0xff;
+#pragma unroll 2
+          for (int i = 0; i < n; ++i) {
+            const CombineOp o = op[i];
+            const double2 m = *reinterpret_cast<const double2*>(st + o.off);
+            c[b].x = fma(o.coef, m.x, c[b].x);
+            c[b].y = fma(o.coef, m.y, c[b].y);
           }
+          op += n;
         }
         __threadfence_block();  // the stage's loads complete before it can be refilled
         __syncwarp();
@@ -1390,7 +1423,15 @@ __global__ void __launch_bounds__(CST_THREADS + 32) fmm_combine_staged_kernel(co
       if (live) {
 #pragma unroll
         for (int q = 0; q < COMBINE_GROUP; ++q)
-          if (q < nm) a.C[cb[q]] = c[q];
+          if (q < nm) {
+            double* p = a.C + sgo[g * COMBINE_GROUP + q] + cofs;
+            if (vec) {
+              __stcs(reinterpret_cast<double2*>(p), c[q]);
+            } else {
+              __stcs(p, c[q].x);
+              __stcs(p + 1, c[q].y);
+            }
+          }
       }
     }
   }
