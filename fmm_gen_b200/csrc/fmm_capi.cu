@@ -1100,6 +1100,7 @@ fmm::PresumSide presum_side(const DevTables& d, int side, const double* X, long 
 
 // Terms of the larger side and the output ranges per position chunk: enough CTAs to fill the
 // SMs several times, else one CTA walks all its outputs so that they share its input values.
+constexpr int kPsChunk = fmm::PS_THREADS;  // positions of a presum CTA
 int presum_cap(const fmm_plan* plan) {
   return (int)std::min<size_t>(fmm::PS_TERMS, std::max(plan->ps_terms[0].size(), plan->ps_terms[1].size()));
 }
@@ -1121,11 +1122,12 @@ int launch_presum(const fmm_plan* plan, const fmm::PresumSide& a, const fmm::Pre
   g.nzero = (int)nzero;
   g.cap = presum_cap(plan);
   const long long ca = (long long)(a.orows / 2) * a.ocols, cb = (long long)(b.orows / 2) * b.ocols;
-  const long long nc = (std::max(a.nout ? ca : 0, b.nout ? cb : 0) + fmm::PS_THREADS - 1) / fmm::PS_THREADS;
-  const unsigned gx = (unsigned)std::max<long long>(1, std::min<long long>(nc, INT32_MAX));
+  const long long nca = a.nout ? (ca + kPsChunk - 1) / kPsChunk : 0, ncb = b.nout ? (cb + kPsChunk - 1) / kPsChunk : 0;
+  const long long nc = nca + ncb;
+  const unsigned gx = (unsigned)std::max<long long>(1, std::min<long long>(nc, 4LL * nsm));
   ProfScope pf(K_PRESUM, st);
-  return launch_dependent(fmm::fmm_presum_kernel, dim3(gx, presum_ranges(nc, std::max(a.nout, b.nout), nsm), 2),
-                          fmm::PS_THREADS, sizeof(fmm::PresumOff) * g.cap, st, 1, g);
+  return launch_dependent(fmm::fmm_presum_kernel, dim3(gx, presum_ranges(nc, std::max(a.nout, b.nout), nsm)),
+                          fmm::PS_THREADS, fmm::presum_smem_bytes(g.cap), st, 1, g);
 }
 
 // Bytes of the pre-summed workspace of one call.
@@ -2270,7 +2272,7 @@ void batch_add_job(fmm_batch* b, int phase, int prob, const fmm_plan* plan, int 
     b->max_slots = std::max(b->max_slots, std::max(j.pp.nA, j.pp.nB));
     b->presum_cap = std::max(b->presum_cap, presum_cap(plan));
     const long long ca = j.pp.nA ? (j.pp.ldS / 2) * j.pp.kk : 0, cb = j.pp.nB ? (j.pp.ldT / 2) * ns : 0;
-    b->max_presum_chunks = std::max(b->max_presum_chunks, (std::max(ca, cb) + fmm::PS_THREADS - 1) / fmm::PS_THREADS);
+    b->max_presum_chunks = std::max(b->max_presum_chunks, (std::max(ca, cb) + kPsChunk - 1) / kPsChunk);
     b->n_presum += (j.pp.nA > 0) + (j.pp.nB > 0);
     depth = j.pp.kk;
     j.chunks = batch_chunks(nprod, depth);
@@ -2553,7 +2555,7 @@ int batch_launch(fmm_batch* b, cudaStream_t st, int n_ps, int n_pc, const bool t
     const long long nc = std::min<long long>(b->max_presum_chunks, 1 << 16);
     fmm::fmm_presum_batch_kernel<<<dim3((unsigned)nc, presum_ranges(nc * n_ps, b->max_slots, sm_count[b->dev]),
                                         (unsigned)n_ps),
-                                   fmm::PS_THREADS, sizeof(fmm::PresumOff) * b->presum_cap, st>>>(b->d_ps, b->presum_cap);
+                                   fmm::PS_THREADS, fmm::presum_smem_bytes(b->presum_cap), st>>>(b->d_ps, b->presum_cap);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     FMM_CUDA_TRY(cudaGetLastError());
   }

@@ -963,9 +963,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_gemm_kernel(const __grid_cons
 // Operand sums in HBM: slot j = sum_t coef_t * X_{blk_t} over the A (or B) terms of product
 // plist[j], the slot's k extent rounded up with zeros.  HBM bound: every input element once,
 // every slot element once; an input element feeds nnz(U) / blocks sums (15 for 222-1 x 333-1),
-// which come from L1 and L2.  A CTA owns a range of element positions and walks all its
-// outputs, so that the blocks' values at those positions stay close; the terms' offsets and
-// coefficients are in shared memory.
+// which come from L1 and L2.  A CTA takes chunks of element positions (a row pair a thread) and
+// walks all its outputs for each, so that the blocks' values at those positions stay close;
+// the terms' offsets and coefficients and the outputs' places among them are in shared
+// memory, made once per CTA.  Measured on B200 at four CTAs per SM (the registers' limit) against
+// one chunk per CTA, tables per chunk and masked groups of four terms: 222-1 2048^3 50 -> 39 us,
+// 8192^3 644 -> 455 us; 222-2 8192^3 1050 -> 936 us; 222-1 x 333-1 16384^3 8.0 -> 7.7 ms.  One to
+// three CTAs per SM, whose positions would fit L1, took 1.1 to 2.3 times as long, two
+// positions per thread 1.1 to 1.3 times on plans of many blocks.
 struct PTerm {
   int row, col;  // block
   double coef;
@@ -990,99 +995,141 @@ struct PresumSide {
 
 constexpr int PS_THREADS = 256;
 constexpr int PS_TERMS = 2048;  // terms of one pass over the outputs (32 KB of shared memory at most)
+constexpr int PS_OUTS = 512;    // outputs of one pass
 
 struct PresumOff {
   long long off;
   double coef;
 };
+__host__ __device__ constexpr size_t presum_smem_bytes(int cap) {
+  return sizeof(PresumOff) * (size_t)cap + sizeof(int2) * PS_OUTS;
+}
 
 __device__ __forceinline__ PresumOff presum_term(const PresumSide& a, const PTerm& t) {
   return PresumOff{(long long)t.row * a.blk_row_stride + (long long)t.col * a.blk_col_stride * a.ldx, t.coef};
 }
 
-// Two rows of one column of the sum of terms [0, n): loads four terms at a time before their
-// fmas, so that several loads are in flight (the sum order is the term order).
-template <bool VEC, class Tm>
-__device__ __forceinline__ double2 presum_sum(const double* x0, int n, bool v0, bool v1, Tm&& term) {
-  double2 v = make_double2(0.0, 0.0);
-#pragma unroll 1
-  for (int tg = 0; tg < n; tg += 4) {
-    double2 x[4];
-    double cf[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      x[q] = make_double2(0.0, 0.0);
-      cf[q] = 0.0;
-      if (tg + q < n) {
-        const PresumOff o = term(tg + q);
-        cf[q] = o.coef;
-        if (VEC) {
-          if (v1) x[q] = __ldg(reinterpret_cast<const double2*>(x0 + o.off));
-        } else {
-          if (v0) x[q].x = __ldg(x0 + o.off);
-          if (v1) x[q].y = __ldg(x0 + o.off + 1);
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (tg + q < n) {
-        v.x = (tg + q == 0) ? cf[q] * x[q].x : fma(cf[q], x[q].x, v.x);
-        v.y = (tg + q == 0) ? cf[q] * x[q].y : fma(cf[q], x[q].y, v.y);
-      }
+// A thread's position: rows i, i + 1 of a column; v0, v1: inside the block.
+struct PresumPos {
+  const double* x;
+  bool v0, v1;
+};
+
+template <bool VEC>
+__device__ __forceinline__ double2 presum_load(const PresumPos& p, long long off) {
+  double2 x = make_double2(0.0, 0.0);
+  if (VEC) {
+    if (p.v1) x = __ldg(reinterpret_cast<const double2*>(p.x + off));
+  } else {
+    if (p.v0) x.x = __ldg(p.x + off);
+    if (p.v1) x.y = __ldg(p.x + off + 1);
   }
-  return v;
+  return x;
 }
 
-// Outputs [j0, j1) at the positions of chunk `chunk`.
-__device__ __forceinline__ void presum_body(const PresumSide& a, PresumOff* tab, int cap, long long chunk, int j0, int j1) {
-  const int hr = a.orows / 2;
-  const long long e = chunk * PS_THREADS + threadIdx.x;
-  const bool live = e < (long long)hr * a.ocols;
-  const long long c = live ? e / hr : 0;
-  const int i = live ? 2 * (int)(e - c * hr) : 0;
-  const bool v0 = live && c < a.cols && i < a.rows, v1 = live && c < a.cols && i + 1 < a.rows;
-  const double* x0 = a.X + i + c * a.ldx;
-  double* o = a.out + i + c * a.ldo;
-  // pairs are 16-byte aligned and whole: even strides, base aligned, even row count
-  const bool vec = ((reinterpret_cast<uintptr_t>(a.X) & 15) == 0) && ((a.ldx | a.blk_row_stride | a.rows) & 1) == 0;
-  auto prod = [&](int j) { return a.plist ? __ldg(a.plist + j) : j; };
-  for (int j = j0; j < j1;) {
-    // as many outputs as the table holds (usually all of them)
-    const int t0 = __ldg(a.first + prod(j));
-    int je = j1;
-    if (__ldg(a.first + prod(je - 1) + 1) - t0 > cap) {
-      je = j;
-      while (je < j1 && __ldg(a.first + prod(je) + 1) - t0 <= cap) ++je;
-    }
-    if (je == j) {  // one output with more terms than the table: from global memory
-      const PTerm* tg = a.terms + t0;
-      const double2 v = presum_sum<false>(x0, __ldg(a.first + prod(j) + 1) - t0, v0, v1,
-                                          [&](int t) { return presum_term(a, tg[t]); });
-      if (live) *reinterpret_cast<double2*>(o + j * a.out_stride) = v;
-      ++j;
-      continue;
-    }
-    const int nt = __ldg(a.first + prod(je - 1) + 1) - t0;
-    __syncthreads();
-    for (int t = threadIdx.x; t < nt; t += PS_THREADS) tab[t] = presum_term(a, a.terms[t0 + t]);
-    __syncthreads();
-    for (; j < je; ++j) {
-      const int r = prod(j), f = __ldg(a.first + r), n = __ldg(a.first + r + 1) - f;
-      const PresumOff* tp = tab + (f - t0);
-      const double2 v = vec ? presum_sum<true>(x0, n, v0, v1, [&](int t) { return tp[t]; })
-                            : presum_sum<false>(x0, n, v0, v1, [&](int t) { return tp[t]; });
-      if (live) *reinterpret_cast<double2*>(o + j * a.out_stride) = v;
-    }
+// v += N terms in order, all their loads issued first.
+template <bool VEC, int N, class Tm>
+__device__ __forceinline__ void presum_add(const PresumPos& p, Tm&& term, int t, double2& v) {
+  PresumOff o[N];
+  double2 x[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) o[q] = term(t + q);
+#pragma unroll
+  for (int q = 0; q < N; ++q) x[q] = presum_load<VEC>(p, o[q].off);
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    v.x = fma(o[q].coef, x[q].x, v.x);
+    v.y = fma(o[q].coef, x[q].y, v.y);
   }
+}
+
+template <bool VEC, class Tm>
+__device__ __forceinline__ double2 presum_sum(const PresumPos& p, int n, Tm&& term) {
+  double2 v = make_double2(0.0, 0.0);
+  int t = 0;
+#pragma unroll 1
+  for (; t + 4 <= n; t += 4) presum_add<VEC, 4>(p, term, t, v);
+  switch (n - t) {
+    case 1: presum_add<VEC, 1>(p, term, t, v); break;
+    case 2: presum_add<VEC, 2>(p, term, t, v); break;
+    case 3: presum_add<VEC, 3>(p, term, t, v); break;
+    default: break;
+  }
+  return v;
 }
 
 __device__ __forceinline__ long long presum_chunks(const PresumSide& a) {
   return ((long long)(a.orows / 2) * a.ocols + PS_THREADS - 1) / PS_THREADS;
 }
 
-// Both sides of one call (blockIdx.z); blockIdx.x position chunks, blockIdx.y output ranges.
-// Also zeroes the products launch's tickets and work-unit counter (zero[0 .. nzero)).
+// Outputs [j, je) (their terms in the table, or with tab == nullptr one output from global
+// memory) at the positions of chunks c0, c0 + cstep, ...
+template <bool VEC>
+__device__ __forceinline__ void presum_chunk_loop(const PresumSide& a, const PresumOff* tab, const int2* dsc, int j, int je,
+                                                  const PTerm* tg, int ntg, long long c0, long long cstep) {
+  const int hr = a.orows / 2;
+  const long long nc = presum_chunks(a);
+  for (long long ch = c0; ch < nc; ch += cstep) {
+    const long long e = ch * PS_THREADS + threadIdx.x;
+    if (e >= (long long)hr * a.ocols) continue;
+    const long long c = e / hr;
+    const int i = 2 * (int)(e - c * hr);
+    const bool in = c < a.cols;
+    const PresumPos p{a.X + i + c * a.ldx, in && i < a.rows, in && i + 1 < a.rows};
+    double* o = a.out + i + c * a.ldo + j * a.out_stride;
+    if (!tab) {
+      *reinterpret_cast<double2*>(o) = presum_sum<false>(p, ntg, [&](int t) { return presum_term(a, tg[t]); });
+      continue;
+    }
+#pragma unroll 1
+    for (int q = 0; q < je - j; ++q, o += a.out_stride) {
+      const int2 d = dsc[q];
+      const PresumOff* tp = tab + d.x;
+      *reinterpret_cast<double2*>(o) = presum_sum<VEC>(p, d.y, [&](int t) { return tp[t]; });
+    }
+  }
+}
+
+// Outputs [j0, j1) of one side at the position chunks c0, c0 + cstep, ...
+__device__ __forceinline__ void presum_side(const PresumSide& a, PresumOff* tab, int cap, int j0, int j1, long long c0,
+                                            long long cstep) {
+  int2* dsc = reinterpret_cast<int2*>(tab + cap);  // per output of a pass: first term in the table, terms
+  // pairs are 16-byte aligned and whole: even strides, base aligned, even row count
+  const bool vec = ((reinterpret_cast<uintptr_t>(a.X) & 15) == 0) && ((a.ldx | a.blk_row_stride | a.rows) & 1) == 0;
+  auto prod = [&](int j) { return a.plist ? __ldg(a.plist + j) : j; };
+  for (int j = j0; j < j1;) {
+    // as many outputs as the tables hold (usually all of them)
+    const int t0 = __ldg(a.first + prod(j));
+    int je = min(j1, j + PS_OUTS);
+    if (__ldg(a.first + prod(je - 1) + 1) - t0 > cap) {
+      const int lim = je;
+      je = j;
+      while (je < lim && __ldg(a.first + prod(je) + 1) - t0 <= cap) ++je;
+    }
+    if (je == j) {  // one output with more terms than the table
+      presum_chunk_loop<false>(a, nullptr, nullptr, j, j + 1, a.terms + t0, __ldg(a.first + prod(j) + 1) - t0, c0, cstep);
+      ++j;
+      continue;
+    }
+    const int nt = __ldg(a.first + prod(je - 1) + 1) - t0;
+    __syncthreads();
+    for (int t = threadIdx.x; t < nt; t += PS_THREADS) tab[t] = presum_term(a, a.terms[t0 + t]);
+    for (int q = threadIdx.x; q < je - j; q += PS_THREADS) {
+      const int r = prod(j + q), f = __ldg(a.first + r);
+      dsc[q] = make_int2(f - t0, __ldg(a.first + r + 1) - f);
+    }
+    __syncthreads();
+    if (vec)
+      presum_chunk_loop<true>(a, tab, dsc, j, je, nullptr, 0, c0, cstep);
+    else
+      presum_chunk_loop<false>(a, tab, dsc, j, je, nullptr, 0, c0, cstep);
+    j = je;
+  }
+}
+
+// Both sides of one call: CTA x takes chunks x, x + grid, ... of A's and then B's positions,
+// output range blockIdx.y of each.  Also zeroes the products launch's tickets and work-unit
+// counter (zero[0 .. nzero)).
 struct PresumArgs {
   PresumSide s[2];
   int* zero;
@@ -1094,14 +1141,20 @@ __global__ void __launch_bounds__(PS_THREADS) fmm_presum_kernel(const __grid_con
   extern __shared__ __align__(16) PresumOff ptab[];
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  const PresumSide& a = g.s[blockIdx.z];
-  if (blockIdx.z == 0 && blockIdx.y == 0)
+  if (blockIdx.y == 0)
     for (long long q = (long long)blockIdx.x * PS_THREADS + threadIdx.x; q < g.nzero; q += (long long)gridDim.x * PS_THREADS)
       g.zero[q] = 0;
-  const int j0 = (int)((long long)a.nout * blockIdx.y / gridDim.y), j1 = (int)((long long)a.nout * (blockIdx.y + 1) / gridDim.y);
-  if (j0 == j1) return;
-  const long long nc = presum_chunks(a);
-  for (long long c = blockIdx.x; c < nc; c += gridDim.x) presum_body(a, ptab, g.cap, c, j0, j1);
+  long long c0 = blockIdx.x;
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    const PresumSide& a = g.s[s];
+    if (a.nout == 0) continue;
+    const int j0 = (int)((long long)a.nout * blockIdx.y / gridDim.y), j1 = (int)((long long)a.nout * (blockIdx.y + 1) / gridDim.y);
+    const long long nc = presum_chunks(a);
+    if (j0 < j1 && c0 < nc) presum_side(a, ptab, g.cap, j0, j1, c0, gridDim.x);
+    // go on where this side's round robin ended
+    c0 = (c0 + gridDim.x - nc % gridDim.x) % gridDim.x;
+  }
 }
 
 // The operand sums of many problems in one launch (task blockIdx.z).
@@ -1109,9 +1162,7 @@ __global__ void __launch_bounds__(PS_THREADS) fmm_presum_batch_kernel(const Pres
   extern __shared__ __align__(16) PresumOff ptab[];
   const PresumSide a = tasks[blockIdx.z];
   const int j0 = (int)((long long)a.nout * blockIdx.y / gridDim.y), j1 = (int)((long long)a.nout * (blockIdx.y + 1) / gridDim.y);
-  if (j0 == j1) return;
-  const long long nc = presum_chunks(a);
-  for (long long c = blockIdx.x; c < nc; c += gridDim.x) presum_body(a, ptab, cap, c, j0, j1);
+  if (j0 < j1 && blockIdx.x < presum_chunks(a)) presum_side(a, ptab, cap, j0, j1, blockIdx.x, gridDim.x);
 }
 
 // Column-major copies between pitches, many in one launch (task blockIdx.y): used to give
