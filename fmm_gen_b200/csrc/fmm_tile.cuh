@@ -72,6 +72,12 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+
 __device__ __forceinline__ double2 ld_cluster_f64x2(unsigned addr, unsigned rank) {
   double2 v;
   asm volatile(
@@ -429,6 +435,8 @@ __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_k
               make_double2(acc[i][j][q], acc[i][j][2 + q]);
   }
   cluster_sync();
+  // the tile's parts are neighbours in the cluster, which may hold several tiles
+  const unsigned rank0 = cluster_rank() - (unsigned)part;
   constexpr int P = TM / 2 * TN;
   for (int q = P * part / J.S + tid; q < P * (part + 1) / J.S; q += NT) {
     const int rr = m0 + 2 * (q % (TM / 2)), cc = n0 + q / (TM / 2);
@@ -444,7 +452,7 @@ __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_k
     }
     const unsigned addr = s0 + (unsigned)q * 16;
     for (int s = 0; s < J.S; ++s) {
-      const double2 v = ld_cluster_f64x2(addr, (unsigned)s);
+      const double2 v = ld_cluster_f64x2(addr, rank0 + (unsigned)s);
       c.x += v.x;
       c.y += v.y;
     }

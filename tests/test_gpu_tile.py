@@ -49,7 +49,7 @@ def check(A, B, C0, C, extra=0.0):
 
 
 SHAPES = [(1, 1, 1), (31, 33, 7), (32, 32, 16), (33, 31, 17), (64, 64, 64), (65, 63, 65), (16, 8, 129), (17, 9, 8),
-          (240, 250, 600), (7, 700, 515), (700, 7, 515), (1000, 1100, 24), (2100, 1050, 129)]
+          (240, 250, 600), (7, 700, 515), (700, 7, 515), (1000, 1100, 24), (2100, 1050, 129), (1601, 1500, 1501)]
 
 
 @pytest.mark.parametrize("pad,off", [(0, 0), (1, 0), (0, 1), (3, 1)])
@@ -97,6 +97,32 @@ def test_fmm_edges(lib, alg, shape, pack, pad, off):
     assert lib.fmm_device_status(1) == 0
     check(A, B, C0, C, algebra.error_bound(plan.algebra, *shape, 1.0, 1.0, 1.0))
     plan.close()
+
+
+@pytest.mark.parametrize("alg", [None, "222"])
+@pytest.mark.parametrize("shape,pad", [((1030, 1100, 300), 0), ((1024, 2100, 257), 3), ((701, 511, 90), 0), ((2049, 700, 33), 1)],
+                         ids=str)
+def test_host_calls_in_column_panels(lib, alg, shape, pad):
+    """Host matrices whose copies run in column panels (C of at least 2^20 elements) or whole, dense
+    and with a padded leading dimension."""
+    m, n, k = shape
+    dev = operands(m, n, k, 0, 0, 3 * m + n)
+
+    def host(x):
+        flat = torch.full((x.shape[1], x.shape[0] + pad), 7.0, dtype=torch.float64)
+        flat[:, :x.shape[0]] = x.t().cpu()
+        return flat.numpy().T[:x.shape[0]], flat
+
+    (A, _), (B, _), (C, flat) = (host(x) for x in dev)
+    if alg is None:
+        rt.bl_dgemm_host(A, B, C)
+        extra = 0.0
+    else:
+        plan = rt.Plan.from_levels([alg], [1])
+        rt.fmm_gemm_host(plan, A, B, C)
+        extra = algebra.error_bound(plan.algebra, m, n, k, 1.0, 1.0, 1.0)
+    assert pad == 0 or bool((flat[:, m:] == 7.0).all())
+    check(dev[0], dev[1], dev[2], torch.from_numpy(C.copy()).cuda(), extra)
 
 
 def test_batch_reads_unaligned_operands_in_place(lib):
