@@ -417,7 +417,7 @@ void build_combine_groups(fmm_plan* p) {
     }
     // the group's entries in chunks of CST_CHUNK (the staged kernel's stage): per chunk the
     // products, and per member the operations on it, slots in increasing product order
-    const int first_chunk = (int)(p->ch_r.size() / fmm::CST_CHUNK);
+    const int first_chunk = (int)(p->ch_r.size() / fmm::CST_CHUNK), first_op = (int)p->ch_op.size();
     {
       const int ne = (int)p->cg_r.size() - first;
       for (int q0 = 0; q0 < ne; q0 += fmm::CST_CHUNK) {
@@ -444,6 +444,7 @@ void build_combine_groups(fmm_plan* p) {
     p->cg_desc.push_back((int)p->cg_r.size() - first);
     p->cg_desc.push_back((int)mem[g].size());
     p->cg_desc.push_back(first_chunk);
+    p->cg_desc.push_back(first_op);
     for (int q = 0; q < fmm::COMBINE_GROUP; ++q) {
       const int b = q < (int)mem[g].size() ? mem[g][q] : mem[g][0];
       p->cg_desc.push_back(p->cblk[4 * b] * p->dims[2] + p->cblk[4 * b + 1]);
@@ -463,8 +464,8 @@ void build_combine_groups(fmm_plan* p) {
     const int* gd = p->cg_desc.data() + (size_t)g * fmm::GDESC;
     const int nch = (gd[1] + fmm::CST_CHUNK - 1) / fmm::CST_CHUNK;
     ok = gd[1] > 0 && gd[0] + gd[1] <= (int)p->cg_r.size() && gd[2] >= 1 && gd[2] <= fmm::COMBINE_GROUP &&
-         gd[3] >= 0 && gd[3] + nch <= (int)p->ch_n.size();
-    for (int q = 0; ok && q < fmm::COMBINE_GROUP; ++q) ok = gd[4 + q] >= 0 && gd[4 + q] < p->dims[0] * p->dims[2];
+         gd[3] >= 0 && gd[3] + nch <= (int)p->ch_n.size() && gd[4] >= 0 && gd[4] <= (int)p->ch_op.size();
+    for (int q = 0; ok && q < fmm::COMBINE_GROUP; ++q) ok = gd[fmm::GD_MEMBERS + q] >= 0 && gd[fmm::GD_MEMBERS + q] < p->dims[0] * p->dims[2];
   }
   if (!ok) p->n_cgroup = 0;
 }
@@ -996,8 +997,10 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
   {
     std::lock_guard<std::mutex> lk(g_attr_mu);
     if (!combine_configured[dev]) {
-      FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_combine_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        200 * 1024));
+      FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_combine_staged_kernel<false>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+      FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_combine_staged_kernel<true>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_combine_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         200 * 1024));
       FMM_CUDA_TRY(cudaFuncSetAttribute(fmm::fmm_combine_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1033,12 +1036,14 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
   const bool staged = g_combine_positions.load() == 0 && ldm == ms && m_stride % 2 == 0 && ms % 2 == 0 &&
                       ((uintptr_t)M & 15) == 0 && ssm <= 200 * 1024 && total > 0;
   if (staged) {
-    const long long ntile = (total + fmm::CST_TILE - 1) / fmm::CST_TILE;
+    const long long tiles = (total + fmm::CST_TILE - 1) / fmm::CST_TILE;
+    const bool split = tiles < 3LL * sm_count[dev];  // too few tiles to fill the chip: a unit per group
+    const long long ntile = tiles * (split ? ga.ngroup : 1);
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(ntile, (long long)sm_count[dev] * 3));
     {
       ProfScope pf(K_COMBINE, st);
-      return launch_dependent(fmm::fmm_combine_staged_kernel, dim3(grid), fmm::CST_THREADS + 32, ssm, st, 1, ga,
-                              dev_status[dev]);
+      return launch_dependent(split ? fmm::fmm_combine_staged_kernel<true> : fmm::fmm_combine_staged_kernel<false>,
+                              dim3(grid), fmm::CST_THREADS + 32, ssm, st, 1, ga, dev_status[dev]);
     }
   }
   const int P = g_combine_positions.load() == 2 ? 2 : 1;

@@ -1196,12 +1196,13 @@ __global__ void fmm_pitch_copy1_kernel(const PitchCopy t) { pitch_copy_body(t); 
 // direct schedule.  The host groups blocks that share products (greedy by overlap), which
 // cuts the M loads per position from nnz(W) toward R (222-1 x 333-1: 540 -> 299 in 5
 // groups) with no shared-memory read-modify-write.  Tables (shared memory, per CTA):
-//   group g: gdesc[g * GDESC + 0..3] = first entry, #entries, #members, first chunk;
-//            gdesc[g * GDESC + 4 + q] = block id of member q (row * grid_n + col)
+//   group g: gdesc[g * GDESC + 0..4] = first entry, #entries, #members, first chunk, first
+//            operation; gdesc[g * GDESC + GD_MEMBERS + q] = block id of member q (row * grid_n + col)
 //   entry e: er[e] = product r, em[e] = member mask | (first coefficient of e) << 8,
 //            the coefficients of its set bits, member order, from ec[first coefficient]
 constexpr int COMBINE_GROUP = 8;
-constexpr int GDESC = 4 + COMBINE_GROUP;
+constexpr int GD_MEMBERS = 5;
+constexpr int GDESC = GD_MEMBERS + COMBINE_GROUP;
 constexpr int COMBINE_G_THREADS = 256;
 constexpr int COMBINE_G_BATCH = 16;
 
@@ -1277,7 +1278,7 @@ __global__ void __launch_bounds__(COMBINE_G_THREADS) fmm_combine_kernel(const Co
       long long cb[COMBINE_GROUP];
 #pragma unroll
       for (int q = 0; q < COMBINE_GROUP; ++q) {
-        const int b = gd[4 + (q < nm ? q : 0)];
+        const int b = gd[GD_MEMBERS + (q < nm ? q : 0)];
         cb[q] = (long long)(b / a.grid_n) * a.ms + (long long)(b % a.grid_n) * a.ns * a.ldc;
 #pragma unroll
         for (int p = 0; p < P; ++p) c[q][p] = q < nm ? a.C[cb[q] + cofs[p]] : 0.0;
@@ -1318,7 +1319,7 @@ __global__ void __launch_bounds__(COMBINE_G_THREADS) fmm_combine_kernel(const Co
 
 // The same combine with the M values staged in shared memory by bulk copies: a tile of
 // CST_TILE consecutive element positions (M_r[e0 .. e0 + CST_TILE) is contiguous when
-// ldm == ms), walked group by group and, within a group, CST_CHUNK products at a time; a
+// ldm == ms) and a group at a time, CST_CHUNK products per step; a
 // producer warp copies each chunk's M_r tiles (cp.async.bulk, 2 KB each) into a ring of
 // CST_STAGES stages while the compute warps apply earlier chunks.  HBM bound: every M_r and C
 // element once, and the M_r tiles a later group reads again that have left L2 by then (222-1 x
@@ -1329,7 +1330,9 @@ __global__ void __launch_bounds__(COMBINE_G_THREADS) fmm_combine_kernel(const Co
 // the register kernel's (bit-identical).  Measured on B200 against one position per thread
 // with bit masks walked per chunk: 222-1 x 333-1 14400^2 x 480 2.65 -> 2.23 ms, 222-2 8192^3
 // split 0.58 -> 0.49 ms; fewer or single-position warps, a software pipeline over the
-// operations and loading the next group's C ahead were slower or the same.
+// operations and loading the next group's C ahead were slower or the same.  Where tiles are
+// fewer than the CTAs of the chip each group is a unit of its own (528^3 42 -> 21 us); at
+// 14400^2 x 480 that takes 2.47 ms.
 // Waits are bounded (status word on timeout).
 constexpr int CST_THREADS = 128;  // compute threads, two positions each
 constexpr int CST_TILE = 2 * CST_THREADS;
@@ -1370,6 +1373,7 @@ __device__ __forceinline__ void combine_load(const CombineGroupArgs& a, const lo
 // CombineGroupArgs plus the status word; requires ldm == ms, M and m_stride 16-byte
 // multiples (in doubles: m_stride even) and ms even (pairs of positions lie in one column, and
 // every tile's byte count is a multiple of 16).
+template <bool SPLIT>
 __global__ void __launch_bounds__(CST_THREADS + 32, 3) fmm_combine_staged_kernel(const CombineGroupArgs a,
                                                                                  unsigned* status) {
   extern __shared__ __align__(128) double cst[];
@@ -1387,7 +1391,7 @@ __global__ void __launch_bounds__(CST_THREADS + 32, 3) fmm_combine_staged_kernel
   for (int q = tid; q < a.nchunk * CST_CHUNK; q += blockDim.x) sr[q] = a.chr[q];
   for (int q = tid; q < GDESC * a.ngroup; q += blockDim.x) sg[q] = a.gdesc[q];
   for (int q = tid; q < COMBINE_GROUP * a.ngroup; q += blockDim.x) {
-    const int b = a.gdesc[(q / COMBINE_GROUP) * GDESC + 4 + q % COMBINE_GROUP];
+    const int b = a.gdesc[(q / COMBINE_GROUP) * GDESC + GD_MEMBERS + q % COMBINE_GROUP];
     sgo[q] = (long long)(b / a.grid_n) * a.ms + (long long)(b % a.grid_n) * a.ns * a.ldc;
   }
   if (tid == 0) {
@@ -1401,14 +1405,15 @@ __global__ void __launch_bounds__(CST_THREADS + 32, 3) fmm_combine_staged_kernel
   asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the products (the tables above never change)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const long long total = (long long)a.ms * a.ns;
-  const long long ntile = (total + CST_TILE - 1) / CST_TILE;
+  const long long nunit = (total + CST_TILE - 1) / CST_TILE * (SPLIT ? a.ngroup : 1);
   long long k = 0;  // stage step of this CTA
   if (tid >= CST_THREADS) {  // producer warp: lane 0 issues the copies
     if (tid != CST_THREADS) return;
-    for (long long t = blockIdx.x; t < ntile; t += gridDim.x) {
-      const long long e0 = t * CST_TILE;
+    for (long long u = blockIdx.x; u < nunit; u += gridDim.x) {
+      const long long t = SPLIT ? u / a.ngroup : u, e0 = t * CST_TILE;
       const unsigned bytes = (unsigned)(8 * min((long long)CST_TILE, total - e0));
-      for (int g = 0; g < a.ngroup; ++g) {
+      const int g0 = SPLIT ? (int)(u - t * a.ngroup) : 0, g1 = SPLIT ? g0 + 1 : a.ngroup;
+      for (int g = g0; g < g1; ++g) {
         const int ne = sg[g * GDESC + 1], c0 = sg[g * GDESC + 3];
         for (int q0 = 0; q0 < ne; q0 += CST_CHUNK, ++k) {
           const int s = (int)(k % CST_STAGES);
@@ -1435,18 +1440,15 @@ __global__ void __launch_bounds__(CST_THREADS + 32, 3) fmm_combine_staged_kernel
   }
   const int lane = tid & 31;
   const bool vec = ((reinterpret_cast<uintptr_t>(a.C) & 15) == 0) && (a.ldc & 1) == 0;
-  auto position = [&](long long t, bool& live) {  // element offset in a C block of this thread's pair
-    const long long e = t * CST_TILE + 2 * tid;
-    live = t < ntile && e < total;
-    const long long ee = live ? e : 0;
-    return (ee % a.ms) + (ee / a.ms) * a.ldc;
-  };
   double2 c[COMBINE_GROUP];
-  for (long long t = blockIdx.x; t < ntile; t += gridDim.x) {
-    bool live;
-    const long long cofs = position(t, live);
-    const CombineOp* op = sop;
-    for (int g = 0; g < a.ngroup; ++g) {
+  for (long long u = blockIdx.x; u < nunit; u += gridDim.x) {
+    const long long t = SPLIT ? u / a.ngroup : u, e = t * CST_TILE + 2 * tid;  // this thread's pair of positions
+    const bool live = e < total;
+    const long long ee = live ? e : 0;
+    const long long cofs = (ee % a.ms) + (ee / a.ms) * a.ldc;  // element offset in a C block
+    const int g0 = SPLIT ? (int)(u - t * a.ngroup) : 0, g1 = SPLIT ? g0 + 1 : a.ngroup;
+    const CombineOp* op = sop + sg[g0 * GDESC + 4];  // runs on from group to group
+    for (int g = g0; g < g1; ++g) {
       const int* gd = sg + g * GDESC;
       const int ne = gd[1], nm = gd[2], c0 = gd[3];
       combine_load(a, sgo + g * COMBINE_GROUP, nm, cofs, live, vec, c);

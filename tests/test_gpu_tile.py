@@ -99,6 +99,21 @@ def test_fmm_edges(lib, alg, shape, pack, pad, off):
     plan.close()
 
 
+@pytest.mark.parametrize("side", [2, 66, 336, 338])
+def test_combine_units(lib, side):
+    """36 C blocks in five groups: a group per unit below three tiles of 256 positions per SM (blocks of
+    336 x 336 are the last on a 148-SM chip), every group of a tile in one unit from there on."""
+    plan = rt.Plan.from_levels(["222", "333"], [1, 1])
+    shape = (6 * side, 6 * side, 48)
+    A, B, C0 = operands(*shape, 0, 0, side)
+    _, _, C = operands(*shape, 0, 0, side)
+    rt.fmm_gemm(plan, A, B, C, "abc")
+    torch.cuda.synchronize()
+    assert lib.fmm_device_status(1) == 0
+    check(A, B, C0, C, algebra.error_bound(plan.algebra, *shape, 1.0, 1.0, 1.0))
+    plan.close()
+
+
 @pytest.mark.parametrize("alg", [None, "222"])
 @pytest.mark.parametrize("shape,pad", [((1030, 1100, 300), 0), ((1024, 2100, 257), 3), ((701, 511, 90), 0), ((2049, 700, 33), 1)],
                          ids=str)
