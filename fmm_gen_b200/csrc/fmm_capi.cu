@@ -620,8 +620,9 @@ int configure_kernel(int* dev_out) {
     };
     FMM_CUDA_TRY(smem(fmmt::fmm_tile_gemm_kernel<64, 64>, fmmt::TileShape<64, 64>::SMEM));
     FMM_CUDA_TRY(smem(fmmt::fmm_tile_gemm_kernel<32, 32>, fmmt::TileShape<32, 32>::SMEM));
-    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<64>, fmmt::ProdShape<64>::SMEM));
-    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<32>, fmmt::ProdShape<32>::SMEM));
+    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<64, false>, fmmt::ProdShape<64>::SMEM));
+    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<64, true>, fmmt::ProdShape<64>::SMEM));
+    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<32, false>, fmmt::ProdShape<32>::SMEM));
     FMM_CUDA_TRY(smem(fmmt::fmm_products_batch_kernel<false>, fmmt::ProdShape<64>::SMEM));
     FMM_CUDA_TRY(smem(fmmt::fmm_products_batch_kernel<true>, fmmt::ProdShape<64>::SMEM));
     if (!g_encode_tiled) {
@@ -706,13 +707,39 @@ std::atomic<int> g_force_ksplit{0};  // fmm_debug_set FMM_DEBUG_KSPLIT: S for ev
 
 long long tiles_of(int m, int n, int t) { return (long long)((m + t - 1) / t) * ((n + t - 1) / t); }
 
-// Tile side for u64 units of 64 x 64 or u32 of 32 x 32: the modelled time, SM-seconds over the
-// SMs plus half a unit for the last, partly filled round, the small tile at 6 % lower rate
-// (more shared-memory reads per DMMA).  Measured us with 64 / 32: stored 222-1 512^3 44.9 /
-// 30.7, 1024^3 103.9 / 97.3, 1488^3 242 / 264, 2048^3 544 / 572; 222-1 x 333-1 1200^3 247 / 228,
-// 2016 x 2016 x 8064 2443 / 2327, 3024^3 1722 / 1862; plain 1024^3 77.1 / 75.8, 4096^3 3857 / 4022.
+// Tile side of a plain update with u64 units of 64 x 64 or u32 of 32 x 32: the modelled time,
+// SM-seconds over the SMs plus half a unit for the last, partly filled round, the small tile at
+// 6 % lower rate (more shared-memory reads per DMMA, twice the operand bytes).  Measured us with
+// 64 / 32: 1024^3 77.1 / 75.8, 1200^3 139 / 124, 2048^3 503 / 528, 4096^3 3857 / 4022.
 int tile_side(long long u64, long long u32, int nsm) {
   const double c64 = ((double)u64 / nsm + 0.5) * 4096, c32 = ((double)u32 / nsm + 0.5) * 1024 * 1.06;
+  return c64 <= c32 ? 64 : 32;
+}
+
+// Units at the end of a launch of 64 x 64 products that are cut into row strips: those past the
+// last whole number per SM, when their strips are fewer per SM than the unit they replace (up to
+// 0.7 of the SMs; at three to four units per SM always, where an SM's last unit would run alone).
+// Below three per SM all run at once, from twelve on the last round is a small share.  Measured us
+// without / with: products of 222-1 1024^3 (448 units) 83.7 / 70.1, 1100^3 (567) 107 / 93, 1488 x 1200 x
+// 998 (840) 136 / 116, 1900 x 1800 x 2200 (1575) 452 / 415; past the lines 1280^3 (700) 123 / 125,
+// 2500^3 (2800) 827 / 836, 2048^3 (1792) 464 / 466.  Strips for one whole unit per SM more took 1488 x
+// 1200 x 998 to 123; plain updates gained at some sizes and lost as much at others.
+constexpr int kTailDepth = 128;  // k steps of a product worth cutting
+bool cut_tail(double units_per_sm) {
+  const double whole = std::floor(units_per_sm);
+  return whole >= 3 && whole < 12 && (whole < 4 || units_per_sm - whole <= 0.7);
+}
+
+// Tile side for nprod products of m x n: SM-seconds of the 16 x 8 fragments over the SMs, the last,
+// partly filled round in quarters where it runs as strips (half a unit for 32 x 32), the small
+// tile at 6 % lower rate.  Measured us with 64 / 32: products of 222-1 1024^3 70 / 76, 1100^3 93 / 95,
+// 1488 x 1200 x 998 116 / 124, 1900 x 1800 x 2200 415 / 444, 2500^3 827 / 872, of 222-1 x 333-1 1200^3
+// 116 / 116, 2016^3 406 / 431 (blocks of 336: partial tiles cost their fragments, not whole tiles).
+int product_tile(long long m, long long n, int nprod, int nsm) {
+  const double work = (double)((m + 15) / 16 * 16) * (double)((n + 7) / 8 * 8) * nprod / nsm;
+  const double u64 = work / 4096, whole = std::floor(u64), f = u64 - whole;
+  const double c64 = 4096 * (whole >= 12 ? u64 + 0.5 : whole + (cut_tail(u64) ? std::ceil(4 * f) / 4 : std::ceil(f)));
+  const double c32 = 1024 * 1.06 * (work / 1024 + 0.5);
   return c64 <= c32 ? 64 : 32;
 }
 
@@ -844,7 +871,7 @@ struct ProdLaunch {
 
 ProdLaunch plan_products(const int grid_dims[3], int nprod, int mode, int ms, int ns, int nsm) {
   ProdLaunch L;
-  L.tile = tile_side(tiles_of(ms, ns, 64) * nprod, tiles_of(ms, ns, 32) * nprod, nsm);
+  L.tile = product_tile(ms, ns, nprod, nsm);
   if (mode == fmm::MODE_ACCUM_C && nprod > 1) {
     const long long ntiles = tiles_of(ms, ns, L.tile);
     if (ntiles <= kResident64 * (long long)nsm) {
@@ -891,7 +918,13 @@ int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int gr
   a.nbc = L.nbc;
   a.a_tma = a.b_tma = 1;
   const long long units = (long long)a.tiles_m * a.tiles_n * nprod;
-  if (units > INT32_MAX) return FMM_E_UNSUPPORTED;
+  const int nsm = sm_count[dev];
+  const bool cut = L.tile == 64 && L.tickets == 0 && kk >= kTailDepth && cut_tail((double)units / nsm);
+  const long long tail = cut ? units % nsm : 0;
+  const long long claims = units + (64 / fmmt::TAIL_ROWS - 1) * tail;
+  if (claims > INT32_MAX) return FMM_E_UNSUPPORTED;
+  a.tail = (int)(units - tail);
+  a.claims = (int)claims;
   const long long am = (long long)grid_dims[0] * ms, ak = (long long)grid_dims[1] * ks, bn = (long long)grid_dims[2] * ns;
   bool ok = true;
   if (ps.nslotA < nprod) ok = ok && make_a_map(&a.tmA, A, am, ak, lda);
@@ -900,11 +933,12 @@ int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int gr
   if (ps.nslotB > 0) ok = ok && make_b_map(&a.tmBw, ps.T, kk, (long long)ps.nslotB * ns, ps.ldT, L.tile);
   if (!ok) return FMM_E_UNSUPPORTED;
   const int per_sm = L.tile == 64 ? fmmt::TileShape<64, 64>::CTAS : fmmt::TileShape<32, 32>::CTAS;
-  const unsigned grid = (unsigned)std::min<long long>(units, (long long)sm_count[dev] * per_sm);
+  const unsigned grid = (unsigned)std::min<long long>(claims, (long long)nsm * per_sm);
   ProfScope pf(K_PRODUCTS, st);
   if (L.tile == 64)
-    return launch_dependent(fmmt::fmm_products_kernel<64>, dim3(grid), fmmt::NT, fmmt::ProdShape<64>::SMEM, st, 1, a);
-  return launch_dependent(fmmt::fmm_products_kernel<32>, dim3(grid), fmmt::NT, fmmt::ProdShape<32>::SMEM, st, 1, a);
+    return launch_dependent(tail > 0 ? fmmt::fmm_products_kernel<64, true> : fmmt::fmm_products_kernel<64, false>,
+                            dim3(grid), fmmt::NT, fmmt::ProdShape<64>::SMEM, st, 1, a);
+  return launch_dependent(fmmt::fmm_products_kernel<32, false>, dim3(grid), fmmt::NT, fmmt::ProdShape<32>::SMEM, st, 1, a);
 }
 
 const int kUnitGrid[3] = {1, 1, 1};

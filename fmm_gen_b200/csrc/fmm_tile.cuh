@@ -31,6 +31,9 @@ constexpr int NT = NC + 32;   // + the producer warp
 constexpr int BK = 16;        // k depth of a stage: two groups of eight
 constexpr int MAX_JOBS = 3;   // a launch covers up to three independent GEMMs (the fringe strips)
 constexpr int MAX_SPLIT = 8;  // k parts = CTAs of a cluster
+// The last units of a products launch are cut into strips of TAIL_ROWS rows (64-row tiles only), so that
+// the SMs, which each hold three units at a time, finish closer together.
+constexpr int TAIL_ROWS = 16;
 
 // A classical update C += A * B.  The k range is cut into S parts of depth d (a multiple of 8;
 // S > 1: one CTA of a cluster each); every C element receives its parts' sums in increasing
@@ -65,6 +68,7 @@ struct TileShape {
   static constexpr int STAGES = TM == 64 ? 4 : 5;
   static constexpr int CTAS = TM == 64 ? 3 : 5;  // per SM
   static constexpr size_t SMEM = (size_t)STAGE * STAGES + 16 * STAGES + 1024;
+  static constexpr unsigned STRIP_ABYTES = sizeof(double) * BK * TAIL_ROWS;
   static_assert(sizeof(double) * TM * TN <= (size_t)STAGE * STAGES, "the part exchange reuses the stages");
 };
 
@@ -238,13 +242,13 @@ __device__ __forceinline__ void mma_group(const unsigned char* sa, const unsigne
 template <int TM, int TN, int IM, int JN>
 __device__ __forceinline__ void consume_loop(const unsigned char* smem, unsigned full0, unsigned empty0, unsigned* status,
                                              int kleft, double (&acc)[TileShape<TM, TN>::NI][TileShape<TM, TN>::NJ][4],
-                                             int wm, int wn, int lane, int& slot, unsigned& ph) {
+                                             int row, int col, int lane, int& slot, unsigned& ph) {
   using S = TileShape<TM, TN>;
   const int g = lane >> 2, t4 = lane & 3;
   const unsigned oa0 = (unsigned)(2 * t4 * 128 + ((g ^ (2 * t4)) * 16));
   const unsigned oa1 = (unsigned)((2 * t4 + 1) * 128 + ((g ^ (2 * t4 + 1)) * 16));
-  const unsigned char* a0 = smem + wm * S::NI * 16 * BK * 8;
-  const unsigned char* b0 = smem + S::ABYTES + (wn * S::WN + g) * 64 + t4 * 16;
+  const unsigned char* a0 = smem + row * BK * 8;
+  const unsigned char* b0 = smem + S::ABYTES + (col + g) * 64 + t4 * 16;
 #pragma unroll 1
   for (; kleft > 0; kleft -= BK) {
     fmm::mbar_wait(full0 + 8 * slot, ph, status);
@@ -269,19 +273,19 @@ __device__ __forceinline__ void consume_loop(const unsigned char* smem, unsigned
 // most of whose fragments are all needed.
 template <int TM, int TN>
 __device__ __forceinline__ void consume(const unsigned char* smem, unsigned full0, unsigned empty0, unsigned* status, int kleft,
-                                        double (&acc)[TileShape<TM, TN>::NI][TileShape<TM, TN>::NJ][4], int wm, int wn,
+                                        double (&acc)[TileShape<TM, TN>::NI][TileShape<TM, TN>::NJ][4], int row, int col,
                                         int lane, int im, int jn, int& slot, unsigned& ph) {
   constexpr int NI = TileShape<TM, TN>::NI, NJ = TileShape<TM, TN>::NJ;
   if (im == 0 || jn == 0)
-    consume_loop<TM, TN, 0, 0>(smem, full0, empty0, status, kleft, acc, wm, wn, lane, slot, ph);
+    consume_loop<TM, TN, 0, 0>(smem, full0, empty0, status, kleft, acc, row, col, lane, slot, ph);
   else if (jn <= NJ / 2 && im <= NI / 2)
-    consume_loop<TM, TN, (NI + 1) / 2, NJ / 2>(smem, full0, empty0, status, kleft, acc, wm, wn, lane, slot, ph);
+    consume_loop<TM, TN, (NI + 1) / 2, NJ / 2>(smem, full0, empty0, status, kleft, acc, row, col, lane, slot, ph);
   else if (jn <= NJ / 2)
-    consume_loop<TM, TN, NI, NJ / 2>(smem, full0, empty0, status, kleft, acc, wm, wn, lane, slot, ph);
+    consume_loop<TM, TN, NI, NJ / 2>(smem, full0, empty0, status, kleft, acc, row, col, lane, slot, ph);
   else if (im <= NI / 2)
-    consume_loop<TM, TN, (NI + 1) / 2, NJ>(smem, full0, empty0, status, kleft, acc, wm, wn, lane, slot, ph);
+    consume_loop<TM, TN, (NI + 1) / 2, NJ>(smem, full0, empty0, status, kleft, acc, row, col, lane, slot, ph);
   else
-    consume_loop<TM, TN, NI, NJ>(smem, full0, empty0, status, kleft, acc, wm, wn, lane, slot, ph);
+    consume_loop<TM, TN, NI, NJ>(smem, full0, empty0, status, kleft, acc, row, col, lane, slot, ph);
 }
 
 template <int TM, int TN>
@@ -417,7 +421,7 @@ __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_k
     int im, jn, slot = 0;
     unsigned ph = 0;
     frag_counts<TM, TN>(vr, vc, im, jn);
-    consume<TM, TN>(smem, full0, empty0, g.status, kend - kbeg, acc, wm, wn, lane, im, jn, slot, ph);
+    consume<TM, TN>(smem, full0, empty0, g.status, kend - kbeg, acc, wm * S::WM, wn * S::WN, lane, im, jn, slot, ph);
     if (J.S == 1) {
       update_c<TM, TN, false>(J.C + (m0 + wm * S::WM) + (long long)(n0 + wn * S::WN) * J.ldc, J.ldc, vr, vc, vec, 1.0, acc,
                               g4, t4);
@@ -495,7 +499,9 @@ struct ProdArgs {
   int mode;
   int nbt, nbc;           // > 0: tickets per C block too, nbt blocks in rows of nbc
   int a_tma, b_tma;
-  int pad[4];
+  int tail, claims;       // fmm_products_kernel: units from `tail` on are cut into row strips (only in launches
+                          // without tickets), and the claims that makes
+  int pad[2];
 };
 static_assert(sizeof(ProdArgs) % 64 == 0, "tensor maps in a job table start on 64 bytes");
 
@@ -504,7 +510,8 @@ struct OneProd {
   __device__ __forceinline__ const ProdArgs& get(int) const { return a; }
   __device__ __forceinline__ int find(int) const { return 0; }
   __device__ __forceinline__ int first_unit(int) const { return 0; }
-  __device__ __forceinline__ int total() const { return a.tiles_m * a.tiles_n * a.chunks; }
+  __device__ __forceinline__ int tail() const { return a.tail; }
+  __device__ __forceinline__ int claims() const { return a.claims; }
   __device__ __forceinline__ unsigned* status() const { return a.status; }
   __device__ __forceinline__ int* counter() const { return a.counter; }
   __device__ __forceinline__ void acquire_maps(int) const {}
@@ -533,7 +540,8 @@ struct ProdBatch {
     return lo;
   }
   __device__ __forceinline__ int first_unit(int j) const { return __ldg(b.unit_start + j); }
-  __device__ __forceinline__ int total() const { return b.units; }
+  __device__ __forceinline__ int tail() const { return b.units; }
+  __device__ __forceinline__ int claims() const { return b.units; }
   __device__ __forceinline__ unsigned* status() const { return b.status; }
   __device__ __forceinline__ int* counter() const { return b.counter; }
   // the maps were written by a copy before the launch; order it before the tensor-map proxy
@@ -545,12 +553,23 @@ struct ProdBatch {
   }
 };
 
+// A claim: a unit of a job, or a row strip of one (strip >= 0).
+struct PClaim {
+  int unit, strip;
+};
+template <int T, bool STRIPS>
+__device__ __forceinline__ PClaim decode_claim(int v, int tail) {
+  constexpr int N = T / TAIL_ROWS;
+  return STRIPS && v >= tail ? PClaim{tail + (v - tail) / N, (v - tail) % N} : PClaim{v, -1};
+}
+
 struct PUnit {
   int m0, n0, tile, chunk, r0, r1;
+  bool strip;
 };
 
 template <int T>
-__device__ __forceinline__ PUnit decode(const ProdArgs& a, int u) {
+__device__ __forceinline__ PUnit decode(const ProdArgs& a, int u, int strip) {
   const int ntiles = a.tiles_m * a.tiles_n;
   PUnit w;
   w.chunk = u / ntiles;  // chunk-major: the units of one tile are a whole tile grid apart
@@ -558,6 +577,11 @@ __device__ __forceinline__ PUnit decode(const ProdArgs& a, int u) {
   w.r0 = (int)((long long)a.nprod * w.chunk / a.chunks);
   w.r1 = (int)((long long)a.nprod * (w.chunk + 1) / a.chunks);
   tile_origin<T, T>(w.tile, a.tiles_m, a.tiles_n, w.m0, w.n0);
+  w.strip = strip >= 0;
+  if (w.strip) {
+    w.m0 += strip * TAIL_ROWS;
+    if (w.m0 >= a.ms) w.r1 = w.r0;  // a strip below the last row
+  }
   return w;
 }
 
@@ -581,7 +605,7 @@ __device__ __forceinline__ void prefetch_c(const ProdArgs& a, const fmm::Prod& p
   }
 }
 
-template <int T, bool LANES, class Src>
+template <int T, bool LANES, bool STRIPS, class Src>
 __device__ __forceinline__ void prod_producer(const Src& src, const fmm::UnitRing& q, unsigned s0, unsigned full0,
                                               unsigned empty0, int lane) {
   using S = TileShape<T, T>;
@@ -596,20 +620,21 @@ __device__ __forceinline__ void prod_producer(const Src& src, const fmm::UnitRin
       fmm::mbar_wait(q.empty(e), (unsigned)(((n / fmm::UQ_DEPTH) & 1) ^ 1), src.status());
       if ((*(volatile unsigned*)src.status() & fmm::STATUS_WAIT_TIMEOUT) == 0u) {
         u = src.counter() ? atomicAdd(src.counter(), 1) : (int)(blockIdx.x + (unsigned)n * gridDim.x);
-        if (u >= src.total()) u = -1;
+        if (u >= src.claims()) u = -1;
       }
       fmm::st_shared_s32(q.entry(e), u);
       fmm::mbar_arrive(q.full(e));
     }
     u = __shfl_sync(0xffffffffu, u, 0);
     if (u < 0) break;
-    const int job = src.find(u);
+    const PClaim cl = decode_claim<T, STRIPS>(u, src.tail());
+    const int job = src.find(cl.unit);
     const ProdArgs& a = src.get(job);
     if (job != mapped) {
       if (lane == 0) src.acquire_maps(job);
       mapped = job;
     }
-    const PUnit w = decode<T>(a, u - src.first_unit(job));
+    const PUnit w = decode<T>(a, cl.unit - src.first_unit(job), STRIPS ? cl.strip : -1);
     const int nst = (a.ks + BK - 1) / BK;
     const int spre = a.mode == fmm::MODE_ACCUM_C ? max(0, nst - C_PREFETCH_STAGES) : -1;
 #pragma unroll 1
@@ -621,11 +646,11 @@ __device__ __forceinline__ void prod_producer(const Src& src, const fmm::UnitRin
       const int xa = ta.row * a.ms + w.m0, ya = ta.col * a.ks;
       const int xb = tb.row * a.ks, yb = tb.col * a.ns + w.n0;
       const bool at = !LANES || ta.src || a.a_tma, bt = !LANES || tb.src || a.b_tma;
-      const unsigned tx = (at ? S::ABYTES : 0u) + (bt ? S::BBYTES : 0u);
+      const unsigned tx = (at ? (STRIPS && w.strip ? S::STRIP_ABYTES : S::ABYTES) : 0u) + (bt ? S::BBYTES : 0u);
       LaneCopy<T, T> lc;
       if (LANES && (!at || !bt))
-        lc.init(a.A + xa + (long long)ya * a.lda, a.lda, a.B + xb + (long long)yb * a.ldb, a.ldb, a.ms - w.m0,
-                a.ns - w.n0, lane);
+        lc.init(a.A + xa + (long long)ya * a.lda, a.lda, a.B + xb + (long long)yb * a.ldb, a.ldb,
+                a.ms - w.m0, a.ns - w.n0, lane);
 #pragma unroll 1
       for (int s = 0; s < nst; ++s, ++kc) {
         const int slot = (int)(kc % S::STAGES);
@@ -635,7 +660,10 @@ __device__ __forceinline__ void prod_producer(const Src& src, const fmm::UnitRin
         if (!ok) break;
         if (lane == 0) {
           fmm::mbar_arrive_expect_tx(fb, tx);
-          if (at) tma_stage_a<T>(st, ma, xa, ya + s * BK, fb);
+          if (STRIPS && w.strip)
+            tma_stage_a<TAIL_ROWS>(st, ma, xa, ya + s * BK, fb);
+          else if (at)
+            tma_stage_a<T>(st, ma, xa, ya + s * BK, fb);
           if (bt) tma_stage_b<T>(st + S::ABYTES, mb, xb + s * BK, yb, fb);
         }
         if (LANES) {
@@ -657,7 +685,7 @@ __device__ __forceinline__ void prod_producer(const Src& src, const fmm::UnitRin
     fmm::mbar_wait_drain(full0 + 8 * (int)(k % S::STAGES), (unsigned)((k / S::STAGES) & 1));
 }
 
-template <int T, class Src>
+template <int T, bool STRIPS, class Src>
 __device__ __forceinline__ void prod_consumer(const Src& src, const fmm::UnitRing& q, const unsigned char* smem,
                                               unsigned full0, unsigned empty0, int warp, int lane) {
   using S = TileShape<T, T>;
@@ -668,18 +696,23 @@ __device__ __forceinline__ void prod_consumer(const Src& src, const fmm::UnitRin
   double acc[S::NI][S::NJ][4];
 #pragma unroll 1
   for (int u = nx.next(); u >= 0; u = nx.next()) {
-    const int job = src.find(u);
+    const PClaim cl = decode_claim<T, STRIPS>(u, src.tail());
+    const int job = src.find(cl.unit);
     const ProdArgs& a = src.get(job);
-    const PUnit w = decode<T>(a, u - src.first_unit(job));
-    const int vr = a.ms - w.m0 - wm * S::WM, vc = a.ns - w.n0 - wn * S::WN;
+    const PUnit w = decode<T>(a, cl.unit - src.first_unit(job), STRIPS ? cl.strip : -1);
+    // two by two warps over a tile, four side by side over a row strip
+    const bool strip = STRIPS && w.strip;
+    const int wrow = strip ? 0 : wm * S::WM, wcol = strip ? warp * (T / 4) : wn * S::WN;
+    const int vr = strip ? min(a.ms - w.m0, TAIL_ROWS) : a.ms - w.m0 - wrow;
+    const int vc = strip ? min(a.ns - w.n0 - wcol, T / 4) : a.ns - w.n0 - wcol;
     int im, jn;
     frag_counts<T, T>(vr, vc, im, jn);
     const bool ordered = a.mode == fmm::MODE_ACCUM_C && a.chunks > 1;
 #pragma unroll 1
     for (int r = w.r0; r < w.r1; ++r) {
       zero_acc<T, T>(acc);
-      consume<T, T>(smem, full0, empty0, src.status(), a.ks, acc, wm, wn, lane, im, jn, slot, ph);
-      const long long row = w.m0 + wm * S::WM, col = w.n0 + wn * S::WN;
+      consume<T, T>(smem, full0, empty0, src.status(), a.ks, acc, wrow, wcol, lane, im, jn, slot, ph);
+      const long long row = w.m0 + wrow, col = w.n0 + wcol;
       if (a.mode == fmm::MODE_STORE_M) {
         update_c<T, T, true>(a.M + (long long)r * a.m_stride + row + col * a.ms, a.ms, vr, vc,
                              vec_ok(a.M + (long long)r * a.m_stride, a.ms), 1.0, acc, g4, t4);
@@ -702,8 +735,8 @@ __device__ __forceinline__ void prod_consumer(const Src& src, const fmm::UnitRin
           if (lane == 0) fmm::ticket_spin(tk, tm.pad, a.status, 64);
           __syncwarp();
         }
-        update_c<T, T, false>(a.C + (tm.row * (long long)a.ms + row) + (tm.col * (long long)a.ns + col) * a.ldc, a.ldc, vr,
-                              vc, vec && ((tm.row * a.ms) & 1) == 0, tm.coef, acc, g4, t4);
+        update_c<T, T, false>(a.C + (tm.row * (long long)a.ms + row) + (tm.col * (long long)a.ns + col) * a.ldc, a.ldc,
+                              vr, vc, vec && ((tm.row * a.ms) & 1) == 0, tm.coef, acc, g4, t4);
         if (tk) {  // this block's update is visible before the next product may start its own
           __threadfence();
           __syncwarp();
@@ -719,9 +752,11 @@ __device__ __forceinline__ void prod_consumer(const Src& src, const fmm::UnitRin
   }
 }
 
-template <int T, bool LANES, class Src>
+// LANES: some operands are read by per-lane copies; STRIPS: the last units run as row strips (not with LANES).
+template <int T, bool LANES, bool STRIPS, class Src>
 __device__ __forceinline__ void prod_cta(const Src& src) {
   using S = TileShape<T, T>;
+  static_assert(!(LANES && STRIPS), "per-lane copies fill whole tiles");
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024 - (fmm::smem_u32(smem_raw) & 1023)) & 1023);  // swizzle atoms
   const unsigned s0 = fmm::smem_u32(smem), full0 = s0 + S::STAGE * S::STAGES, empty0 = full0 + 8 * S::STAGES;
@@ -739,20 +774,20 @@ __device__ __forceinline__ void prod_cta(const Src& src) {
   grid_wait();
   grid_launch();
   if (warp == NC / 32)
-    prod_producer<T, LANES>(src, q, s0, full0, empty0, lane);
+    prod_producer<T, LANES, STRIPS>(src, q, s0, full0, empty0, lane);
   else
-    prod_consumer<T>(src, q, smem, full0, empty0, warp, lane);
+    prod_consumer<T, STRIPS>(src, q, smem, full0, empty0, warp, lane);
 }
 
-template <int T>
+template <int T, bool STRIPS>
 __global__ void __launch_bounds__(NT, (TileShape<T, T>::CTAS)) fmm_products_kernel(const __grid_constant__ ProdArgs a) {
-  prod_cta<T, false>(OneProd{a});
+  prod_cta<T, false, STRIPS>(OneProd{a});
 }
 
 template <bool LANES>
 __global__ void __launch_bounds__(NT, (TileShape<64, 64>::CTAS))
     fmm_products_batch_kernel(const __grid_constant__ ProdBatchArgs b) {
-  prod_cta<64, LANES>(ProdBatch{b});
+  prod_cta<64, LANES, false>(ProdBatch{b});
 }
 
 }  // namespace fmmt

@@ -114,6 +114,20 @@ def test_combine_units(lib, side):
     plan.close()
 
 
+@pytest.mark.parametrize("shape", [(1024, 1024, 256), (1072, 1000, 300), (1040, 1136, 264), (1504, 1216, 272)], ids=str)
+def test_product_strips(lib, shape):
+    """Stored products whose last 64 x 64 units run as 16-row strips (three to four units per SM on
+    148 SMs, and 0.7 past five): whole tiles, tiles of 24 and 8 rows whose lower strips are empty, and partial columns."""
+    plan = rt.Plan.from_levels(["222"], [1])
+    A, B, C0 = operands(*shape, 0, 0, sum(shape))
+    _, _, C = operands(*shape, 0, 0, sum(shape))
+    rt.fmm_gemm(plan, A, B, C, "abc")
+    torch.cuda.synchronize()
+    assert lib.fmm_device_status(1) == 0
+    check(A, B, C0, C, algebra.error_bound(plan.algebra, *shape, 1.0, 1.0, 1.0))
+    plan.close()
+
+
 @pytest.mark.parametrize("alg", [None, "222"])
 @pytest.mark.parametrize("shape,pad", [((1030, 1100, 300), 0), ((1024, 2100, 257), 3), ((701, 511, 90), 0), ((2049, 700, 33), 1)],
                          ids=str)
