@@ -609,6 +609,23 @@ std::mutex g_attr_mu;
 
 PFN_cuTensorMapEncodeTiled_v12000 g_encode_tiled = nullptr;
 
+// Dynamic shared memory of a launch of `ctas` CTAs that need `smem` each, so that no SM takes more
+// than its share of them (at least two: calls on other streams find room).  A dependent launch's
+// CTAs start as the previous kernel's leave, and an SM that empties early would otherwise be
+// filled up: 148 CTAs of the products kernel ran three each on 50 SMs.  Measured on B200 without /
+// with, whole calls: 222-1 240^3 17.9 / 14.4 us, 400^3 26.3 / 22.3, 512^3 32.6 / 29.1, 2000 x 100 x
+// 2000 94 / 83, plain 100 x 3000 x 100 7.8 / 6.5; on four streams 240^3 6.1 / 5.5 us a call, 400^3
+// 12.3 / 13.4.  Clusters are spread as it is (plain 256^3, four parts: 5.6 / 5.8).  Starting the
+// dependents at the end of the operand sums instead did as much for the products but took 0.3 to 1.3 us
+// more per call at other sizes.
+constexpr size_t kSmSmem = 228 * 1024, kCtaReserve = 1024;  // shared memory of an SM; the system's part of a CTA
+constexpr size_t kSpreadSmem = kSmSmem / 3;                 // the most that spread_smem asks for
+size_t spread_smem(size_t smem, long long ctas, int nsm) {
+  const long long per = std::max<long long>(2, (ctas + nsm - 1) / nsm);
+  if (per > 4) return smem;  // more than any of these kernels runs on an SM, or its own limit
+  return std::max<size_t>(smem, kSmSmem / (size_t)(per + 1) / 256 * 256 - kCtaReserve + 256);  // per + 1 do not fit
+}
+
 int configure_kernel(int* dev_out) {
   int dev = 0;
   FMM_CUDA_TRY(cudaGetDevice(&dev));
@@ -616,7 +633,8 @@ int configure_kernel(int* dev_out) {
   std::lock_guard<std::mutex> lk(g_attr_mu);
   if (!smem_configured[dev]) {
     auto smem = [](auto kernel, size_t bytes) {
-      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)std::max(bytes, kSpreadSmem));
     };
     FMM_CUDA_TRY(smem(fmmt::fmm_tile_gemm_kernel<64, 64>, fmmt::TileShape<64, 64>::SMEM));
     FMM_CUDA_TRY(smem(fmmt::fmm_tile_gemm_kernel<32, 32>, fmmt::TileShape<32, 32>::SMEM));
@@ -772,7 +790,7 @@ struct GemmJob {
 };
 
 template <int T>
-int launch_tile_gemm(const GemmJob* jobs, int njob, unsigned* status, cudaStream_t st) {
+int launch_tile_gemm(const GemmJob* jobs, int njob, int nsm, unsigned* status, cudaStream_t st) {
   fmmt::TileArgs g{};
   int cluster = 1;
   for (int q = 0; q < njob; ++q) {
@@ -785,7 +803,7 @@ int launch_tile_gemm(const GemmJob* jobs, int njob, unsigned* status, cudaStream
   for (int q = 0; q < njob; ++q)
     if (cluster % g.job[q].S != 0) {
       int rc = FMM_OK;
-      for (int j = 0; j < njob && rc == FMM_OK; ++j) rc = launch_tile_gemm<T>(jobs + j, 1, status, st);
+      for (int j = 0; j < njob && rc == FMM_OK; ++j) rc = launch_tile_gemm<T>(jobs + j, 1, nsm, status, st);
       return rc;
     }
   long long first = 0;
@@ -814,7 +832,8 @@ int launch_tile_gemm(const GemmJob* jobs, int njob, unsigned* status, cudaStream
   g.njob = njob;
   g.status = status;
   ProfScope ps(K_TILE_GEMM, st);
-  return launch_dependent(fmmt::fmm_tile_gemm_kernel<T, T>, dim3((unsigned)first), fmmt::NT, fmmt::TileShape<T, T>::SMEM,
+  return launch_dependent(fmmt::fmm_tile_gemm_kernel<T, T>, dim3((unsigned)first), fmmt::NT,
+                          cluster > 1 ? fmmt::TileShape<T, T>::SMEM : spread_smem(fmmt::TileShape<T, T>::SMEM, first, nsm),
                           st, cluster, g);
 }
 
@@ -833,8 +852,8 @@ int tile_gemm(const GemmJob* jobs, int njob, cudaStream_t st) {
   }
   if (n == 0) return FMM_OK;
   if (n == 1 && S == 1 && tile_side(tiles_of(todo[0].m, todo[0].n, 64), tiles_of(todo[0].m, todo[0].n, 32), sm_count[dev]) == 64)
-    return launch_tile_gemm<64>(todo, n, dev_status[dev], st);
-  return launch_tile_gemm<32>(todo, n, dev_status[dev], st);
+    return launch_tile_gemm<64>(todo, n, sm_count[dev], dev_status[dev], st);
+  return launch_tile_gemm<32>(todo, n, sm_count[dev], dev_status[dev], st);
 }
 
 // Workspaces of pre-summed operands: slot j of S is ms x kslot, of T kslot x ns (block
@@ -937,8 +956,9 @@ int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int gr
   ProfScope pf(K_PRODUCTS, st);
   if (L.tile == 64)
     return launch_dependent(tail > 0 ? fmmt::fmm_products_kernel<64, true> : fmmt::fmm_products_kernel<64, false>,
-                            dim3(grid), fmmt::NT, fmmt::ProdShape<64>::SMEM, st, 1, a);
-  return launch_dependent(fmmt::fmm_products_kernel<32, false>, dim3(grid), fmmt::NT, fmmt::ProdShape<32>::SMEM, st, 1, a);
+                            dim3(grid), fmmt::NT, spread_smem(fmmt::ProdShape<64>::SMEM, grid, nsm), st, 1, a);
+  return launch_dependent(fmmt::fmm_products_kernel<32, false>, dim3(grid), fmmt::NT,
+                          spread_smem(fmmt::ProdShape<32>::SMEM, grid, nsm), st, 1, a);
 }
 
 const int kUnitGrid[3] = {1, 1, 1};
@@ -1077,7 +1097,8 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
     {
       ProfScope pf(K_COMBINE, st);
       return launch_dependent(split ? fmm::fmm_combine_staged_kernel<true> : fmm::fmm_combine_staged_kernel<false>,
-                              dim3(grid), fmm::CST_THREADS + 32, ssm, st, 1, ga, dev_status[dev]);
+                              dim3(grid), fmm::CST_THREADS + 32, spread_smem(ssm, grid, sm_count[dev]), st, 1, ga,
+                              dev_status[dev]);
     }
   }
   const int P = g_combine_positions.load() == 2 ? 2 : 1;
@@ -2714,7 +2735,8 @@ int batch_launch(fmm_batch* b, cudaStream_t st, int n_ps, int n_pc, const bool t
         (unsigned)std::min<long long>(ba.units, (long long)sm_count[b->dev] * fmmt::TileShape<64, 64>::CTAS);
     ProfScope pf(K_PRODUCTS_BATCH, st);
     const int rc = launch_dependent(tma[ph] ? fmmt::fmm_products_batch_kernel<false> : fmmt::fmm_products_batch_kernel<true>,
-                                    dim3(grid), fmmt::NT, fmmt::ProdShape<64>::SMEM, st, 1, ba);
+                                    dim3(grid), fmmt::NT,
+                                    spread_smem(fmmt::ProdShape<64>::SMEM, grid, sm_count[b->dev]), st, 1, ba);
     if (rc != FMM_OK) return rc;
   }
   return FMM_OK;
