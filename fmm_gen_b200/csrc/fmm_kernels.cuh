@@ -990,6 +990,7 @@ struct PresumSide {
   const int* first;        // per product its first term (R + 1 entries)
   const PTerm* terms;
   int nout;
+  int brows, bcols;        // block grid of the operand (fmm_presum_staged_kernel)
   int pad;
 };
 
@@ -1152,6 +1153,119 @@ __global__ void __launch_bounds__(PS_THREADS) fmm_presum_kernel(const __grid_con
     const int j0 = (int)((long long)a.nout * blockIdx.y / gridDim.y), j1 = (int)((long long)a.nout * (blockIdx.y + 1) / gridDim.y);
     const long long nc = presum_chunks(a);
     if (j0 < j1 && c0 < nc) presum_side(a, ptab, g.cap, j0, j1, c0, gridDim.x);
+    // go on where this side's round robin ended
+    c0 = (c0 + gridDim.x - nc % gridDim.x) % gridDim.x;
+  }
+}
+
+// The same sums with the operand's blocks staged in shared memory: a thread copies its pair of
+// positions of every block (cp.async, slots of its own, so that no barrier is needed) and then
+// walks one flat list of all terms, which marks where a sum begins and where it is stored.  A
+// gather of the kernel above is an L1 or L2 access, and of many blocks' values few are still in
+// L1 (222-1 x 333-1: 540 terms of 36 blocks a side).  Bound by HBM where blocks are few (222-2 8192^3
+// 5.9 TB/s), at 36 blocks by the latency of the shared memory reads that 256 threads an SM can
+// hide: reading ahead over the sums' ends is what a list gives over a loop per sum (16384^3 6.0
+// against 7.7 ms), and two CTAs as the launch bound leave ptxas the registers for it (40 registers:
+// 6.8 ms).  Same additions in the same order.  Measured on B200 against the gathers: 222-1
+// 2048^3 39 -> 35 us, 8192^3 454 -> 404; 222-2 3600 x 4200 x 2900 (odd blocks: 8-byte copies) 194 -> 144,
+// 8192^3 935 -> 750; 222-1 x 333-1 2016^3 127 -> 84, 14400^2 x 480 210 -> 146, 16384^3 7.7 -> 6.0 ms.
+constexpr int PSS_THREADS = 128;
+constexpr int PSS_UNROLL = 8;
+struct PresumOp {
+  unsigned off;    // of the term's block in a thread's slots
+  unsigned flags;  // PSS_FIRST, PSS_STORE
+  double coef;
+};
+constexpr unsigned PSS_FIRST = 1, PSS_STORE = 2;
+__host__ __device__ constexpr size_t presum_staged_smem(int nblk, int cap) {
+  return (size_t)nblk * PSS_THREADS * 16 + sizeof(PresumOp) * (size_t)(cap + PSS_UNROLL);
+}
+
+__global__ void __launch_bounds__(PSS_THREADS, 2) fmm_presum_staged_kernel(const __grid_constant__ PresumArgs g) {
+  extern __shared__ __align__(16) unsigned char pss[];
+  const int tid = threadIdx.x;
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  if (blockIdx.y == 0)
+    for (long long q = (long long)blockIdx.x * PSS_THREADS + tid; q < g.nzero; q += (long long)gridDim.x * PSS_THREADS)
+      g.zero[q] = 0;
+  long long c0 = blockIdx.x;
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    const PresumSide& a = g.s[s];
+    if (a.nout == 0) continue;
+    const int hr = a.orows / 2;
+    const long long total = (long long)hr * a.ocols, nc = (total + PSS_THREADS - 1) / PSS_THREADS;
+    const int j0 = (int)((long long)a.nout * blockIdx.y / gridDim.y), j1 = (int)((long long)a.nout * (blockIdx.y + 1) / gridDim.y);
+    if (j0 < j1 && c0 < nc) {
+      // the terms of products r0 .. r1 in one list: a term of coefficient 0 pads it to whole steps, and
+      // products without a slot are summed and not stored
+      PresumOp* ops = reinterpret_cast<PresumOp*>(pss + (size_t)a.brows * a.bcols * PSS_THREADS * 16);
+      const int r0 = a.plist ? __ldg(a.plist + j0) : j0, r1 = a.plist ? __ldg(a.plist + j1 - 1) : j1 - 1;
+      const int t0 = __ldg(a.first + r0), nt = __ldg(a.first + r1 + 1) - t0;
+      const int ntp = (nt + PSS_UNROLL - 1) / PSS_UNROLL * PSS_UNROLL;
+      __syncthreads();  // the other side's list is no longer read
+      for (int t = tid; t < ntp; t += PSS_THREADS) {
+        PresumOp op{0u, PSS_FIRST, 0.0};
+        if (t < nt) {
+          const PTerm tm = a.terms[t0 + t];
+          op = PresumOp{(unsigned)(tm.row * a.bcols + tm.col) * (PSS_THREADS * 16), 0u, tm.coef};
+        }
+        ops[t] = op;
+      }
+      __syncthreads();
+      for (int r = r0 + tid; r <= r1; r += PSS_THREADS)
+        if (__ldg(a.first + r) - t0 < nt) ops[__ldg(a.first + r) - t0].flags = PSS_FIRST;
+      __syncthreads();
+      for (int q = j0 + tid; q < j1; q += PSS_THREADS)
+        ops[__ldg(a.first + (a.plist ? __ldg(a.plist + q) : q) + 1) - 1 - t0].flags |= PSS_STORE;
+      __syncthreads();
+      const unsigned char* mine = pss + tid * 16;
+      // pairs are 16-byte aligned and whole: even strides, base aligned, even row count
+      const bool vec = ((reinterpret_cast<uintptr_t>(a.X) & 15) == 0) && ((a.ldx | a.blk_row_stride | a.rows) & 1) == 0;
+      for (long long ch = c0; ch < nc; ch += gridDim.x) {
+        const long long e = ch * PSS_THREADS + tid;
+        if (e >= total) continue;
+        const long long c = e / hr;
+        const int i = 2 * (int)(e - c * hr);
+        const bool v0 = c < a.cols && i < a.rows, v1 = c < a.cols && i + 1 < a.rows;
+        const double* x = a.X + (v0 ? i + c * a.ldx : 0);  // what is not copied still names an address
+        unsigned dst = smem_u32(mine);
+        for (int br = 0; br < a.brows; ++br)
+          for (int bc = 0; bc < a.bcols; ++bc, dst += PSS_THREADS * 16) {
+            const double* xb = v0 ? x + (long long)br * a.blk_row_stride + (long long)bc * a.blk_col_stride * a.ldx : x;
+            if (vec) {
+              cp_async16(dst, xb, v1 ? 16 : 0);
+            } else {
+              cp_async8(dst, xb, v0 ? 8 : 0);
+              cp_async8(dst + 8, v1 ? xb + 1 : xb, v1 ? 8 : 0);
+            }
+          }
+        cp_async_commit();
+        cp_async_wait<0>();
+        double* o = a.out + i + c * a.ldo + j0 * a.out_stride;
+        double2 v = make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int t = 0; t < ntp; t += PSS_UNROLL) {
+          PresumOp op[PSS_UNROLL];
+          double2 xv[PSS_UNROLL];
+#pragma unroll
+          for (int q = 0; q < PSS_UNROLL; ++q) op[q] = ops[t + q];
+#pragma unroll
+          for (int q = 0; q < PSS_UNROLL; ++q) xv[q] = *reinterpret_cast<const double2*>(mine + op[q].off);
+#pragma unroll
+          for (int q = 0; q < PSS_UNROLL; ++q) {
+            if (op[q].flags & PSS_FIRST) v = make_double2(0.0, 0.0);
+            v.x = fma(op[q].coef, xv[q].x, v.x);
+            v.y = fma(op[q].coef, xv[q].y, v.y);
+            if (op[q].flags & PSS_STORE) {
+              *reinterpret_cast<double2*>(o) = v;
+              o += a.out_stride;
+            }
+          }
+        }
+      }
+    }
     // go on where this side's round robin ended
     c0 = (c0 + gridDim.x - nc % gridDim.x) % gridDim.x;
   }

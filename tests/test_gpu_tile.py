@@ -99,6 +99,23 @@ def test_fmm_edges(lib, alg, shape, pack, pad, off):
     plan.close()
 
 
+@pytest.mark.parametrize("algs,shape", [(["222"], (416, 400, 400)), (["222"], (413, 399, 401)), (["222"], (850, 402, 398)),
+                                        (["222", "333"], (846, 852, 858)), (["222", "333"], (845, 851, 849))], ids=str)
+@pytest.mark.parametrize("pad,off", [(0, 0), (1, 0), (0, 1)])
+@pytest.mark.parametrize("pack", ["abc", "naive"])
+def test_staged_operand_sums(lib, algs, shape, pad, off, pack):
+    """Operand sums from staged blocks (at least one 128-pair chunk per SM): even and odd blocks, aligned
+    and unaligned operands, only the sums or every product's operands."""
+    plan = rt.Plan.from_levels(algs, [1] * len(algs))
+    A, B, C0 = operands(*shape, pad, off, sum(shape))
+    _, _, C = operands(*shape, pad, off, sum(shape))
+    rt.fmm_gemm(plan, A, B, C, pack)
+    torch.cuda.synchronize()
+    assert lib.fmm_device_status(1) == 0
+    check(A, B, C0, C, algebra.error_bound(plan.algebra, *shape, 1.0, 1.0, 1.0))
+    plan.close()
+
+
 @pytest.mark.parametrize("side", [2, 66, 336, 338])
 def test_combine_units(lib, side):
     """36 C blocks in five groups: a group per unit below three tiles of 256 positions per SM (blocks of
