@@ -43,9 +43,10 @@ METRIC = "effective TFLOPS (2mnk/t), 222-1x333-1 abc FP64"
 UNIT = "TFLOP/s"
 # DRAM traffic of the FMM products kernel per executed core flop, from a one-pass ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum) of the products launch of a smaller case of
-# the same algorithm, 222-1 x 333-1 at 6144^3: 11.62 GB over 3.46e11 executed flops (its
-# algorithmic bytes: 11.4 GB).  roofline.traffic scales it to the average products launch.
-TRAFFIC_BYTES_PER_FLOP = 11.62e9 / 3.46e11
+# the same algorithm, 222-1 x 333-1 at 6144^3 (products stored): 4.16 GB over 3.46e11 executed flops.
+# roofline.traffic scales it to the average products launch (16384^3, where C blocks are updated,
+# has 0.0127 algorithmic bytes per flop against 0.0120 here).
+TRAFFIC_BYTES_PER_FLOP = 4.16e9 / 3.46e11
 TRAFFIC_SOURCE = "scaled by executed flops from one capture of the 222-1x333-1 6144^3 products launch"
 
 

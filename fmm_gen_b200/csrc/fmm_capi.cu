@@ -1442,8 +1442,8 @@ int device_status(bool clear) {
 // device and device-to-host copies run at the same time).  Before the first kernel only
 // A[I_0, :], B[:, J_0] and C[I_0, J_0] are copied: with two row panels half of A instead of
 // all of it (16384^3: 1.8 instead of 3.2 GB).  Row and column edges fall on multiples of 128 x
-// (block rows / columns of the plan), so every block's sub-blocks are whole 128-row tiles
-// where the size allows.
+// (block rows / columns of the plan), so every block's sub-blocks are whole tiles where the
+// size allows.
 #ifndef FMM_HOST_PANELS
 #define FMM_HOST_PANELS 4
 #endif

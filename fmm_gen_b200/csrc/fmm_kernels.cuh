@@ -7,7 +7,7 @@
 //
 // Mapping of the reference's CPU design (fmm-gen):
 //   * BLIS packing with fused sums (meta/abc_gen_mix.py:171-251, packA/B_add_stra_abc<r>)
-//     -> fmm_presum_kernel (operand sums formed in HBM; S_Add / T_Add of
+//     -> fmm_presum_staged_kernel, fmm_presum_kernel (operand sums formed in HBM; S_Add / T_Add of
 //        meta/naive_gen_mix.py:60-137 too), or the folding GEMM's producer warps (cp.async /
 //        TMA of every U/V term tile, folded into the operand stage).
 //   * AVX 8x4 micro-kernel (common/kernels/bl_dgemm_asm_8x4.c)

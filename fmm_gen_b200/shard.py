@@ -13,7 +13,7 @@ error bound).  No reduction is needed; the exchange is one all-gather per operan
     an all-gather over grid column j assembles B[:, J_j].
 
 Row and column ranges fall on multiples of a unit (128 x the plan's block rows / columns), so
-every local FMM call's sub-blocks are whole 128-row tiles where the size allows.  Every rank
+every local FMM call's sub-blocks are whole tiles where the size allows.  Every rank
 takes the same collective steps in the same order (group creation included).  With NCCL the
 gathered panels land in each GPU's own memory; the local call then reads only local memory.
 """

@@ -6,15 +6,17 @@ counts, per product, the nonzeros of U, V, W; meta/model_gen.py:65-102 turns the
 time = actual_flops * tau + memops * alpha for its CPU blocking MC/KC/NC).  The same
 structure is re-derived here for this implementation on B200:
 
-  * compute: every product of a job is a sub-GEMM tiled 128 x 128 with k steps of 8.
+  * compute: every product of a job is counted in 128 x 128 tiles with k steps of 8 (the
+    kernels' own tiles are 64 x 64 or 32 x 32; the constants below were fitted to earlier
+    128 x 128 kernels, and the measurements decide).
     A k step costs `kstep_s` on one SM at the plain kernel's rate.  A product whose
     operand sums are folded while staging costs `1 + fold_per_term * (T - 1)` times that
     (T = the larger of its A and B term counts) on whole tiles; pre-summed products (and
-    classical jobs) run in the direct kernel variant, cost 1, and their edge tiles count
+    classical jobs) cost 1, and their edge tiles count
     only the 16-row / 32-column fragments they compute.
   * memory: the pre-sum pass reads every U/V term and writes each summed operand once
     (HBM bytes / bandwidth, a separate pass).  The multi-destination epilogue reads and
-    writes one C tile per W nonzero: in the direct variant it overlaps the products'
+    writes one C tile per W nonzero: after pre-summed products it overlaps the products'
     MMAs (the job takes the longer of the two, the C traffic counted `c_direct` times its
     HBM time); in the folded kernel it does not (`c_exposed` times, added).
   * partition: the same fringe split as the library (algebra.partition); the strips
@@ -27,8 +29,9 @@ latency.
 
 The tuner takes the model's best candidate per problem, then measures the whole batch
 and re-assigns groups of problems (by the model's choice and margin) while that makes the
-measured batch faster.  The only tile shape of the FP64 kernel is 128 x 128; the other
-scheduling parameter, products per work unit, is chosen by the batch itself.
+measured batch faster.  The scheduling parameter of a batch, products per work unit, is
+chosen by the batch itself; a problem's tile height is accepted and changes nothing (every
+unit is a 64 x 64 tile).
 """
 from __future__ import annotations
 
@@ -52,7 +55,7 @@ class B200Model:
     plain FP64 kernel 34.5 TFLOP/s; folded 222-1 products at 1.7x a plain k step; 6.5 TB/s
     copy bandwidth; `c_exposed` fitted to the folded kernel (the epilogue on the consumer
     warps, 1.5 x its HBM time); `c_direct`, `wave_unit_s` and `launch_s` fitted to 17
-    single-problem measurements of the direct variant (222-1, 222-2, 222-1 x 333-1 and
+    single-problem measurements of the 128 x 128 pre-summed kernel (222-1, 222-2, 222-1 x 333-1 and
     classical, 1024^3 to 16384^3 and the rank-k shapes): `model_time_single` is within
     9 % RMS (log ratio) of them, 3-5 % on the large shapes."""
 
@@ -110,7 +113,7 @@ def _tiles(ms: int, ns: int) -> int:
 
 
 def _tile_work(ms: int, ns: int) -> float:
-    """Tiles of an ms x ns sub-block in the direct variant, an edge tile counted by the
+    """Tiles of an ms x ns sub-block of pre-summed products, an edge tile counted by the
     fragments it computes: 16-row fragments at the bottom edge, 32-column groups at the
     right edge, the cheaper of the two at the corner."""
     fr, rr = divmod(ms, TILE)
@@ -297,9 +300,9 @@ class BatchTuner:
             if not improved:
                 break
         rep.choices = list(choices)
-        # tile height: 64-row tiles halve a problem's unit length (twice the units); they help
-        # where a problem's units are long and few, so the batch's last units finish late.  The
-        # model ranks problems by unit length over unit count; the measurement decides.
+        # tile height: 64 instead of 128 rows for problems whose units are long and few, by the
+        # model's unit length over unit count; kept only if measured faster (both heights run the
+        # same 64 x 64 units today).
         rep.tiles = [TILE] * len(shapes)
         order = sorted(range(len(shapes)), key=lambda i: -self.tile_pressure(choices[i], shapes[i]))
         for frac in (0.05, 0.25, 1.0):
