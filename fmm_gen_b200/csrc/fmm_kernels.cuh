@@ -966,7 +966,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fmm_gemm_kernel(const __grid_cons
 // which come from L1 and L2.  A CTA takes chunks of element positions (a row pair a thread) and
 // walks all its outputs for each, so that the blocks' values at those positions stay close;
 // the terms' offsets and coefficients and the outputs' places among them are in shared
-// memory, made once per CTA.  Measured on B200 at four CTAs per SM (the registers' limit) against
+// memory, made once per CTA.  For calls of less than a chunk per SM and plans whose blocks or terms do not fit
+// the staged kernel below.  Measured on B200 at four CTAs per SM (the registers' limit) against
 // one chunk per CTA, tables per chunk and masked groups of four terms: 222-1 2048^3 50 -> 39 us,
 // 8192^3 644 -> 455 us; 222-2 8192^3 1050 -> 936 us; 222-1 x 333-1 16384^3 8.0 -> 7.7 ms.  One to
 // three CTAs per SM, whose positions would fit L1, took 1.1 to 2.3 times as long, two
