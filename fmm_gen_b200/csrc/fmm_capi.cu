@@ -637,14 +637,19 @@ int configure_kernel(int* dev_out) {
       return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)std::max(bytes, kSpreadSmem));
     };
-    FMM_CUDA_TRY(smem(fmmt::fmm_tile_gemm_kernel<64, 64>, fmmt::TileShape<64, 64>::SMEM));
-    FMM_CUDA_TRY(smem(fmmt::fmm_tile_gemm_kernel<32, 32>, fmmt::TileShape<32, 32>::SMEM));
+    for (auto kernel : {fmmt::fmm_tile_gemm_kernel<64, 64, false>, fmmt::fmm_tile_gemm_kernel<64, 64, true>})
+      FMM_CUDA_TRY(smem(kernel, fmmt::TileShape<64, 64>::SMEM));
+    for (auto kernel : {fmmt::fmm_tile_gemm_kernel<32, 32, false>, fmmt::fmm_tile_gemm_kernel<32, 32, true>})
+      FMM_CUDA_TRY(smem(kernel, fmmt::TileShape<32, 32>::SMEM));
     FMM_CUDA_TRY(smem(fmm::fmm_presum_staged_kernel, kPsStagedSmem));
-    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<64, false>, fmmt::ProdShape<64>::SMEM));
-    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<64, true>, fmmt::ProdShape<64>::SMEM));
-    FMM_CUDA_TRY(smem(fmmt::fmm_products_kernel<32, false>, fmmt::ProdShape<32>::SMEM));
-    FMM_CUDA_TRY(smem(fmmt::fmm_products_batch_kernel<false>, fmmt::ProdShape<64>::SMEM));
-    FMM_CUDA_TRY(smem(fmmt::fmm_products_batch_kernel<true>, fmmt::ProdShape<64>::SMEM));
+    for (auto kernel : {fmmt::fmm_products_kernel<64, false, false>, fmmt::fmm_products_kernel<64, false, true>,
+                        fmmt::fmm_products_kernel<64, true, false>, fmmt::fmm_products_kernel<64, true, true>})
+      FMM_CUDA_TRY(smem(kernel, fmmt::ProdShape<64>::SMEM));
+    for (auto kernel : {fmmt::fmm_products_kernel<32, false, false>, fmmt::fmm_products_kernel<32, false, true>})
+      FMM_CUDA_TRY(smem(kernel, fmmt::ProdShape<32>::SMEM));
+    for (auto kernel : {fmmt::fmm_products_batch_kernel<false, false>, fmmt::fmm_products_batch_kernel<false, true>,
+                        fmmt::fmm_products_batch_kernel<true, false>, fmmt::fmm_products_batch_kernel<true, true>})
+      FMM_CUDA_TRY(smem(kernel, fmmt::ProdShape<64>::SMEM));
     if (!g_encode_tiled) {
       cudaDriverEntryPointQueryResult q;
       void* fn = nullptr;
@@ -780,6 +785,31 @@ void classical_parts(int m, int n, int k, int* S, int* d) {
   *d = s == 1 ? k : depth(s);
 }
 
+// Depth of the parts in which a sum over k is formed (consume_k) for nprod products of m x n x k:
+// k / S for the S below, in whole stages.  On random operands one chain over k has a relative error of about
+// 0.3 * 2^-53 sqrt(k), S parts have 1 / sqrt(S) of that.  S is the k split that launches of few 128 x 128 units
+// had when splitting was what filled the SMs (waves of 148 units, parts of at least 16 steps of eight k, four
+// steps of overhead per unit): results of those sizes are as accurate as they were.  Measured relative
+// error against 80-bit sums, one chain / parts: plain 2048^3 1.51e-15 / 7.6e-16, 1024 x 2048 x 4096
+// 2.13e-15 / 7.6e-16, 222-1 2048^3 2.13e-15 / 1.52e-15, 1501 x 1203 x 999 1.47e-15 / 8.5e-16; us: plain 2048^3 497 /
+// 525 (D = 448 506), 1024 x 2048 x 4096 536 / 545, 222-1 2048^3 510 / 519, 1501 x 1203 x 999 168 / 172, the
+// 512-problem batch 0.4 % more.  Parts of an eighth of k at every size cost 2 to 5 %.
+int sum_depth(int m, int n, int k, int nprod) {
+  constexpr int kWave = 148, kStepOverhead = 4, kMinSteps = 16;
+  const long long units = tiles_of(m, n, 128) * nprod;
+  const int steps = k / 8;
+  if (k % 8 != 0 || units >= 8LL * kWave) return k;
+  auto cost = [&](int S) { return (double)((units * S + kWave - 1) / kWave) * (steps / S + kStepOverhead); };
+  int best = 1;
+  for (int S = 2; S <= 8; ++S)
+    if (steps % S == 0 && steps / S >= kMinSteps && cost(S) < 0.97 * cost(best)) best = S;
+  return best == 1 ? k : (k / best + fmmt::BK - 1) / fmmt::BK * fmmt::BK;
+}
+int product_depth(const fmm_plan* plan, int ms, int ns, int ks) {
+  const int kk = (ks + 7) / 8 * 8;  // of the slots; the same whether or not the products read slots
+  return (long long)ms * ns >= (1LL << 17) || plan->rank == 1 ? sum_depth(ms, ns, kk, plan->rank) : kk;
+}
+
 // One classical update of a tile_gemm launch.
 struct GemmJob {
   int m, n, k;
@@ -795,6 +825,7 @@ template <int T>
 int launch_tile_gemm(const GemmJob* jobs, int njob, int nsm, unsigned* status, cudaStream_t st) {
   fmmt::TileArgs g{};
   int cluster = 1;
+  bool parts = false;
   for (int q = 0; q < njob; ++q) {
     fmmt::TileJob& J = g.job[q];
     classical_parts(jobs[q].m, jobs[q].n, jobs[q].k, &J.S, &J.d);
@@ -821,6 +852,8 @@ int launch_tile_gemm(const GemmJob* jobs, int njob, int nsm, unsigned* status, c
     J.m = b.m;
     J.n = b.n;
     J.k = b.k;
+    J.depth = sum_depth(b.m, b.n, b.k, 1);
+    parts = parts || J.depth < J.d;
     J.tiles_m = (b.m + T - 1) / T;
     J.tiles_n = (b.n + T - 1) / T;
     J.a_tma = make_a_map(&J.tmA, b.A, b.m, b.k, b.lda);
@@ -834,7 +867,7 @@ int launch_tile_gemm(const GemmJob* jobs, int njob, int nsm, unsigned* status, c
   g.njob = njob;
   g.status = status;
   ProfScope ps(K_TILE_GEMM, st);
-  return launch_dependent(fmmt::fmm_tile_gemm_kernel<T, T>, dim3((unsigned)first), fmmt::NT,
+  return launch_dependent(parts ? fmmt::fmm_tile_gemm_kernel<T, T, true> : fmmt::fmm_tile_gemm_kernel<T, T, false>, dim3((unsigned)first), fmmt::NT,
                           cluster > 1 ? fmmt::TileShape<T, T>::SMEM : spread_smem(fmmt::TileShape<T, T>::SMEM, first, nsm),
                           st, cluster, g);
 }
@@ -908,8 +941,8 @@ ProdLaunch plan_products(const int grid_dims[3], int nprod, int mode, int ms, in
 // the operands' own); counter: the launch's work-unit counter and then its tickets, zeroed.
 int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int grid_dims[3], int nprod, int mode,
                     const double* A, long long lda, const double* B, long long ldb, const PresumOps& ps, double* C,
-                    long long ldc, double* M, int ms, int ns, int ks, int kk, const ProdLaunch& L, int* counter,
-                    cudaStream_t st) {
+                    long long ldc, double* M, int ms, int ns, int ks, int kk, int depth, const ProdLaunch& L,
+                    int* counter, cudaStream_t st) {
   int dev = 0;
   int rc = configure_kernel(&dev);
   if (rc != FMM_OK) return rc;
@@ -927,6 +960,7 @@ int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int gr
   a.ms = ms;
   a.ns = ns;
   a.ks = kk;
+  a.depth = depth;
   a.nprod = nprod;
   a.tiles_m = (ms + L.tile - 1) / L.tile;
   a.tiles_n = (ns + L.tile - 1) / L.tile;
@@ -956,11 +990,14 @@ int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int gr
   const int per_sm = L.tile == 64 ? fmmt::TileShape<64, 64>::CTAS : fmmt::TileShape<32, 32>::CTAS;
   const unsigned grid = (unsigned)std::min<long long>(claims, (long long)nsm * per_sm);
   ProfScope pf(K_PRODUCTS, st);
-  if (L.tile == 64)
-    return launch_dependent(tail > 0 ? fmmt::fmm_products_kernel<64, true> : fmmt::fmm_products_kernel<64, false>,
-                            dim3(grid), fmmt::NT, spread_smem(fmmt::ProdShape<64>::SMEM, grid, nsm), st, 1, a);
-  return launch_dependent(fmmt::fmm_products_kernel<32, false>, dim3(grid), fmmt::NT,
-                          spread_smem(fmmt::ProdShape<32>::SMEM, grid, nsm), st, 1, a);
+  const bool parts = depth < kk;
+  if (L.tile == 64) {
+    auto kernel = tail > 0 ? (parts ? fmmt::fmm_products_kernel<64, true, true> : fmmt::fmm_products_kernel<64, true, false>)
+                           : (parts ? fmmt::fmm_products_kernel<64, false, true> : fmmt::fmm_products_kernel<64, false, false>);
+    return launch_dependent(kernel, dim3(grid), fmmt::NT, spread_smem(fmmt::ProdShape<64>::SMEM, grid, nsm), st, 1, a);
+  }
+  return launch_dependent(parts ? fmmt::fmm_products_kernel<32, false, true> : fmmt::fmm_products_kernel<32, false, false>,
+                          dim3(grid), fmmt::NT, spread_smem(fmmt::ProdShape<32>::SMEM, grid, nsm), st, 1, a);
 }
 
 const int kUnitGrid[3] = {1, 1, 1};
@@ -1298,7 +1335,7 @@ int run_presum_groups(const fmm_plan* plan, const DevTables& d, const double* A,
     if (rc == FMM_OK) rc = ksplit_tables(plan, BASE_GROUP, g0, &gp, &gt, g1);
     if (rc == FMM_OK)
       rc = launch_products(gp, gt, plan->dims, n, fmm::MODE_ACCUM_C, A, lda, B, ldb, ps, C, ldc, nullptr, ms, ns, ks,
-                           kk, L, counter, st);
+                           kk, product_depth(plan, ms, ns, ks), L, counter, st);
   }
   cudaError_t fe = cudaFreeAsync(ws, st);
   return rc == FMM_OK ? cuda_status(fe) : rc;
@@ -1367,7 +1404,7 @@ int run_core(const fmm_plan* plan, int pack, const double* A, long long lda, con
     rc = cuda_status(cudaMemsetAsync(counter + 1, g_ticket_fill, sizeof(int) * L.tickets, st));
   if (rc == FMM_OK)
     rc = launch_products(pp.all ? d->prods_all : d->prods_ps, pp.all ? d->terms_all : d->terms_ps, plan->dims, R, mode, A,
-                         lda, B, ldb, ps, C, ldc, M, ms, ns, ks, pp.kk, L, counter, st);
+                         lda, B, ldb, ps, C, ldc, M, ms, ns, ks, pp.kk, product_depth(plan, ms, ns, ks), L, counter, st);
   if (rc == FMM_OK && stored && combine_fits(plan)) {
     rc = launch_combine(plan, *d, C, ldc, ms, ns, M, ms, (long long)ms * ns, st);
   } else if (rc == FMM_OK && stored) {
@@ -2380,6 +2417,8 @@ struct fmm_batch {
     size_t ws_off;                 // byte offset of S (then T) in the workspace
     int chunks, tiles_m, tiles_n, units;
     int S, d;                      // classical jobs: the k parts a single call makes (classical_parts)
+    int depth;                     // of the parts of a product's sums (sum_depth)
+    bool parts;                    // more than one of them
     const fmm::Prod* vprods;       // their tables when S > 1
     const fmm::Term* vterms;
     size_t ticket_off;             // int offset into the ticket array
@@ -2448,6 +2487,7 @@ void batch_add_job(fmm_batch* b, int phase, int prob, const fmm_plan* plan, int 
     classical_parts(ms, ns, ks, &j.S, &j.d);
     nprod = j.S;
     depth = j.d;
+    j.depth = sum_depth(ms, ns, ks, 1);
     j.chunks = 1;  // one unit adds all its parts, in order
   } else {
     // operands with an odd row count or k get slots throughout, so that no pitch copy of them
@@ -2461,8 +2501,10 @@ void batch_add_job(fmm_batch* b, int phase, int prob, const fmm_plan* plan, int 
     b->max_presum_chunks = std::max(b->max_presum_chunks, (std::max(ca, cb) + kPsChunk - 1) / kPsChunk);
     b->n_presum += (j.pp.nA > 0) + (j.pp.nB > 0);
     depth = j.pp.kk;
+    j.depth = product_depth(plan, ms, ns, ks);
     j.chunks = batch_chunks(nprod, depth);
   }
+  j.parts = j.depth < depth;
   j.tiles_m = (ms + 63) / 64;
   j.tiles_n = (ns + 63) / 64;
   j.units = j.tiles_m * j.tiles_n * j.chunks;
@@ -2620,6 +2662,7 @@ bool batch_fill(fmm_batch* b, int ph, const double* const* A, const long* lda, c
     a.ms = j.ms;
     a.ns = j.ns;
     a.ks = j.d;
+    a.depth = j.depth;
     a.kcap = j.grid[1] * j.ks;
     a.nprod = j.plan->rank;
     a.tiles_m = j.tiles_m;
@@ -2757,8 +2800,10 @@ int batch_launch(fmm_batch* b, cudaStream_t st, int n_ps, int n_pc, const bool t
     const unsigned grid =
         (unsigned)std::min<long long>(ba.units, (long long)sm_count[b->dev] * fmmt::TileShape<64, 64>::CTAS);
     ProfScope pf(K_PRODUCTS_BATCH, st);
-    const int rc = launch_dependent(tma[ph] ? fmmt::fmm_products_batch_kernel<false> : fmmt::fmm_products_batch_kernel<true>,
-                                    dim3(grid), fmmt::NT,
+    const bool parts = std::any_of(b->jobs[ph].begin(), b->jobs[ph].end(), [](const fmm_batch::Job& j) { return j.parts; });
+    auto kernel = tma[ph] ? (parts ? fmmt::fmm_products_batch_kernel<false, true> : fmmt::fmm_products_batch_kernel<false, false>)
+                          : (parts ? fmmt::fmm_products_batch_kernel<true, true> : fmmt::fmm_products_batch_kernel<true, false>);
+    const int rc = launch_dependent(kernel, dim3(grid), fmmt::NT,
                                     spread_smem(fmmt::ProdShape<64>::SMEM, grid, sm_count[b->dev]), st, 1, ba);
     if (rc != FMM_OK) return rc;
   }

@@ -48,6 +48,7 @@ struct TileJob {
   int m, n, k;
   int tiles_m, tiles_n;
   int S, d;
+  int depth;         // of the parts of a CTA's sum (consume_k)
   int first;         // first CTA of the job, a multiple of the launch's cluster size
   int units;         // CTAs
   int a_tma, b_tma;  // 0: per-lane copies (odd leading dimension or unaligned base)
@@ -298,6 +299,52 @@ __device__ __forceinline__ void zero_acc(double (&acc)[TileShape<TM, TN>::NI][Ti
       for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
 }
 
+// The sum over k into acc.  PARTS: in parts of `depth` (a multiple of BK, or k): a part is summed
+// from zero and the parts before it are added, so rounding grows with the parts' depth and their number and
+// not with k.  The part loop and the earlier parts' sums cost 64-row tiles 1 to 3 % (three parts of
+// 168 against one: 222-1 1501 x 1203 x 999 167.4 -> 172 us; kernels without it keep their time), about half of it
+// for the first boundary and half for the additions; folding fragment by fragment under the next one's DMMAs took
+// 1 % longer in batches.
+template <int TM, int TN, bool PARTS>
+__device__ __forceinline__ void consume_k(const unsigned char* smem, unsigned full0, unsigned empty0, unsigned* status, int k,
+                                          int depth, double (&acc)[TileShape<TM, TN>::NI][TileShape<TM, TN>::NJ][4],
+                                          int row, int col, int lane, int im, int jn, int& slot, unsigned& ph) {
+  using S = TileShape<TM, TN>;
+  if constexpr (!PARTS) {
+    zero_acc<TM, TN>(acc);
+    consume<TM, TN>(smem, full0, empty0, status, k, acc, row, col, lane, im, jn, slot, ph);
+  } else {
+    double2 sum[S::NI][S::NJ][2];
+    // in local memory: left to ptxas, these values and the k loop's competed for registers (2 to 3 %)
+    if constexpr (TM == 64) asm volatile("" ::"l"(&sum[0][0][0]) : "memory");
+#pragma unroll 1
+    for (int left = k; left > 0; left -= depth) {
+      zero_acc<TM, TN>(acc);
+      consume<TM, TN>(smem, full0, empty0, status, min(left, depth), acc, row, col, lane, im, jn, slot, ph);
+      if (left < k) {
+#pragma unroll
+        for (int i = 0; i < S::NI; ++i)
+#pragma unroll
+          for (int j = 0; j < S::NJ; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const double2 v = sum[i][j][e];
+              acc[i][j][2 * e] += v.x;
+              acc[i][j][2 * e + 1] += v.y;
+            }
+      }
+      if (left > depth) {
+#pragma unroll
+        for (int i = 0; i < S::NI; ++i)
+#pragma unroll
+          for (int j = 0; j < S::NJ; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) sum[i][j][e] = make_double2(acc[i][j][2 * e], acc[i][j][2 * e + 1]);
+      }
+    }
+  }
+}
+
 // Fragments of this warp inside a block of which vr x vc elements lie right and below the warp
 // tile's corner: i < im, j < jn.
 template <int TM, int TN>
@@ -379,7 +426,8 @@ __device__ __forceinline__ void grid_launch() { asm volatile("griddepcontrol.lau
 // One CTA per (tile, part) of up to three independent classical updates C += A * B: the plain
 // GEMM and the fringe strips.  The parts of a tile are the CTAs of a cluster, which leave their
 // sums in shared memory and then add every part, in order, to their share of the tile.
-template <int TM, int TN>
+// PARTS: some CTA's sum is made of parts of its own (consume_k).
+template <int TM, int TN, bool PARTS>
 __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_kernel(const __grid_constant__ TileArgs g) {
   using S = TileShape<TM, TN>;
   extern __shared__ unsigned char smem_raw[];
@@ -416,12 +464,12 @@ __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_k
     __syncwarp();
   } else {
     double acc[S::NI][S::NJ][4];
-    zero_acc<TM, TN>(acc);
     const int vr = J.m - m0 - wm * S::WM, vc = J.n - n0 - wn * S::WN;
     int im, jn, slot = 0;
     unsigned ph = 0;
     frag_counts<TM, TN>(vr, vc, im, jn);
-    consume<TM, TN>(smem, full0, empty0, g.status, kend - kbeg, acc, wm * S::WM, wn * S::WN, lane, im, jn, slot, ph);
+    consume_k<TM, TN, PARTS>(smem, full0, empty0, g.status, kend - kbeg, J.depth, acc, wm * S::WM, wn * S::WN, lane, im, jn,
+                             slot, ph);
     if (J.S == 1) {
       update_c<TM, TN, false>(J.C + (m0 + wm * S::WM) + (long long)(n0 + wn * S::WN) * J.ldc, J.ldc, vr, vc, vec, 1.0, acc,
                               g4, t4);
@@ -501,7 +549,8 @@ struct ProdArgs {
   int a_tma, b_tma;
   int tail, claims;       // fmm_products_kernel: units from `tail` on are cut into row strips (only in launches
                           // without tickets), and the claims that makes
-  int pad[2];
+  int depth;              // of the parts of a product's sum (consume_k)
+  int pad[1];
 };
 static_assert(sizeof(ProdArgs) % 64 == 0, "tensor maps in a job table start on 64 bytes");
 
@@ -685,7 +734,7 @@ __device__ __forceinline__ void prod_producer(const Src& src, const fmm::UnitRin
     fmm::mbar_wait_drain(full0 + 8 * (int)(k % S::STAGES), (unsigned)((k / S::STAGES) & 1));
 }
 
-template <int T, bool STRIPS, class Src>
+template <int T, bool STRIPS, bool PARTS, class Src>
 __device__ __forceinline__ void prod_consumer(const Src& src, const fmm::UnitRing& q, const unsigned char* smem,
                                               unsigned full0, unsigned empty0, int warp, int lane) {
   using S = TileShape<T, T>;
@@ -710,8 +759,7 @@ __device__ __forceinline__ void prod_consumer(const Src& src, const fmm::UnitRin
     const bool ordered = a.mode == fmm::MODE_ACCUM_C && a.chunks > 1;
 #pragma unroll 1
     for (int r = w.r0; r < w.r1; ++r) {
-      zero_acc<T, T>(acc);
-      consume<T, T>(smem, full0, empty0, src.status(), a.ks, acc, wrow, wcol, lane, im, jn, slot, ph);
+      consume_k<T, T, PARTS>(smem, full0, empty0, src.status(), a.ks, a.depth, acc, wrow, wcol, lane, im, jn, slot, ph);
       const long long row = w.m0 + wrow, col = w.n0 + wcol;
       if (a.mode == fmm::MODE_STORE_M) {
         update_c<T, T, true>(a.M + (long long)r * a.m_stride + row + col * a.ms, a.ms, vr, vc,
@@ -752,8 +800,9 @@ __device__ __forceinline__ void prod_consumer(const Src& src, const fmm::UnitRin
   }
 }
 
-// LANES: some operands are read by per-lane copies; STRIPS: the last units run as row strips (not with LANES).
-template <int T, bool LANES, bool STRIPS, class Src>
+// LANES: some operands are read by per-lane copies; STRIPS: the last units run as row strips (not with LANES);
+// PARTS: some products' sums are made of parts (consume_k).
+template <int T, bool LANES, bool STRIPS, bool PARTS, class Src>
 __device__ __forceinline__ void prod_cta(const Src& src) {
   using S = TileShape<T, T>;
   static_assert(!(LANES && STRIPS), "per-lane copies fill whole tiles");
@@ -776,18 +825,18 @@ __device__ __forceinline__ void prod_cta(const Src& src) {
   if (warp == NC / 32)
     prod_producer<T, LANES, STRIPS>(src, q, s0, full0, empty0, lane);
   else
-    prod_consumer<T, STRIPS>(src, q, smem, full0, empty0, warp, lane);
+    prod_consumer<T, STRIPS, PARTS>(src, q, smem, full0, empty0, warp, lane);
 }
 
-template <int T, bool STRIPS>
+template <int T, bool STRIPS, bool PARTS>
 __global__ void __launch_bounds__(NT, (TileShape<T, T>::CTAS)) fmm_products_kernel(const __grid_constant__ ProdArgs a) {
-  prod_cta<T, false, STRIPS>(OneProd{a});
+  prod_cta<T, false, STRIPS, PARTS>(OneProd{a});
 }
 
-template <bool LANES>
+template <bool LANES, bool PARTS>
 __global__ void __launch_bounds__(NT, (TileShape<64, 64>::CTAS))
     fmm_products_batch_kernel(const __grid_constant__ ProdBatchArgs b) {
-  prod_cta<64, LANES, false>(ProdBatch{b});
+  prod_cta<64, LANES, false, PARTS>(ProdBatch{b});
 }
 
 }  // namespace fmmt
