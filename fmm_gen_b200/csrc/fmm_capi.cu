@@ -1170,7 +1170,8 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
 //     1.08 max(t_mma, t_store); storing must gain 3 %.  Measured ms direct / stored: 222-1 x
 //     333-1 4000 x 16000 x 2000 8.83 / 7.81, 222-1 8192 x 8192 x 512 2.12 / 2.22, 8192^3 27.7 /
 //     28.0.
-// The product workspace (8 R ms ns bytes) must fit the workspace cap.  It is the reference's
+// The product workspace (8 R ms ns bytes) must fit the workspace cap, and so must the operand sums
+// (run_core: deep k makes them large where the products are few and small).  It is the reference's
 // own trade between its ABC and AB variants (meta/model_gen.py:87-95 counts the C memory
 // operations of each).  Both schedules give the same bits.
 bool prefer_stored_products(const fmm_plan* plan, int ms, int ns, int ks, int nsm) {
@@ -1375,9 +1376,12 @@ int run_core(const fmm_plan* plan, int pack, const double* A, long long lda, con
   const bool in_place = make_a_map(&probe, A, (long long)plan->dims[0] * ms, (long long)plan->dims[1] * ks, lda) &&
                         make_b_map(&probe, B, (long long)plan->dims[1] * ks, (long long)plan->dims[2] * ns, ldb, 64);
   const PresumPlan pp = presum_plan(plan, ms, ns, ks, pack == FMM_PACK_NAIVE || !in_place);
-  const bool stored = pack != FMM_PACK_ABC || (g_ticket_fill == 0 && combine_fits(plan) && prefer_stored_products(plan, ms, ns, ks, nsm));
-  if (!stored && (long long)presum_bytes(pp) > g_ws_limit.load())
-    return run_presum_groups(plan, *d, A, lda, B, ldb, C, ldc, ms, ns, ks, nsm, st);  // workspace within the limit
+  // an ABC call whose operand sums exceed the workspace cap runs in groups, whatever its C traffic
+  const bool capped = pack == FMM_PACK_ABC && (long long)presum_bytes(pp) > g_ws_limit.load();
+  const bool stored = pack != FMM_PACK_ABC ||
+                      (!capped && g_ticket_fill == 0 && combine_fits(plan) && prefer_stored_products(plan, ms, ns, ks, nsm));
+  if (capped)
+    return run_presum_groups(plan, *d, A, lda, B, ldb, C, ldc, ms, ns, ks, nsm, st);
   const int mode = stored ? fmm::MODE_STORE_M : fmm::MODE_ACCUM_C;
   const ProdLaunch L = plan_products(plan->dims, R, mode, ms, ns, nsm);
   const size_t tk = (sizeof(int) * (1 + L.tickets) + 255) & ~(size_t)255;
