@@ -1017,14 +1017,16 @@ struct PresumPos {
   bool v0, v1;
 };
 
+// Ordinary loads: these kernels may start while the operand's last writer (C of the call before) still
+// runs, which loads for read-only memory do not allow.
 template <bool VEC>
 __device__ __forceinline__ double2 presum_load(const PresumPos& p, long long off) {
   double2 x = make_double2(0.0, 0.0);
   if (VEC) {
-    if (p.v1) x = __ldg(reinterpret_cast<const double2*>(p.x + off));
+    if (p.v1) x = __ldca(reinterpret_cast<const double2*>(p.x + off));
   } else {
-    if (p.v0) x.x = __ldg(p.x + off);
-    if (p.v1) x.y = __ldg(p.x + off + 1);
+    if (p.v0) x.x = __ldca(p.x + off);
+    if (p.v1) x.y = __ldca(p.x + off + 1);
   }
   return x;
 }

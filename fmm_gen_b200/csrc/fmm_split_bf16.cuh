@@ -582,7 +582,7 @@ __host__ __device__ constexpr size_t plane_smem_bytes(int tr, int np, int nblk, 
 // TR rows x 32 NP k, 16 threads per row: thread q of a row makes the k pairs 2 q + 32 h, h < NP.
 template <int TR, int NP>
 __global__ void __launch_bounds__(16 * TR) fmm_split_planes_kernel(const __grid_constant__ PlaneArgs g) {
-  constexpr int NTH = 16 * TR, TK = 32 * NP, LD = plane_ld(NP), EL = 2 * NP;
+  constexpr int NTH = 16 * TR, TK = 32 * NP, LD = plane_ld(NP), EL = 2 * NP, STEP = 2 * NP;
   extern __shared__ __align__(16) unsigned char psm[];
   fmmt::grid_wait();
   fmmt::grid_launch();
@@ -609,23 +609,34 @@ __global__ void __launch_bounds__(16 * TR) fmm_split_planes_kernel(const __grid_
   }
   for (int r = tid; r <= a.nprod; r += NTH) tf[r] = a.first[r];
   __syncthreads();
-  // the blocks' tiles, zeros outside the block; lanes along the operand's contiguous direction
+  // the blocks' tiles, zeros outside the block; lanes along the operand's contiguous direction.  Ordinary
+  // loads (the kernel may start while the operand's last writer still runs), which only an explicit step keeps
+  // ahead of the stores: planes of 222-1 1021 x 3007 x 1530 47.7 us without, 45.0 with
   const int lr = a.side == 0 ? tid % TR : tid / TK, lk = a.side == 0 ? tid / TR : tid % TK;
   const int dr = a.side == 0 ? 0 : NTH / TK, dk = a.side == 0 ? 16 : 0;
   const long long sr = a.side == 0 ? 1 : a.ldx, sk = a.side == 0 ? a.ldx : 1;
-  for (int kq = 0; kq < nkt; ++kq) {
-    const int k0 = (kt0 + kq) * TK + lk;
-    const float* xk = a.X + (row0 + lr) * sr + k0 * sk;
-    float* xs = x + ((size_t)kq * a.nblk * TR + lr) * LD + lk;
-    bool in[EL];
+  const float* xk = a.X + (row0 + lr) * sr + (kt0 * TK + lk) * sk;
+  float* xs = x + lr * LD + lk;
+  const int items = nkt * a.nblk;  // staged tiles: block b of k tile kq
+  int kq = 0, b = 0;
+  for (int t0 = 0; t0 < items; t0 += STEP) {
+    float v[STEP][EL];  // all of a step's loads are issued before its stores
 #pragma unroll
-    for (int e = 0; e < EL; ++e) in[e] = row0 + lr + e * dr < a.rows && k0 + e * dk < a.ks;
-#pragma unroll 4
-    for (int b = 0; b < a.nblk; ++b) {
-      const float* xb = xk + bo[b];
+    for (int u = 0; u < STEP; ++u) {
+      const float* xb = xk + (long long)kq * TK * sk + (t0 + u < items ? bo[b] : 0);
 #pragma unroll
-      for (int e = 0; e < EL; ++e) xs[(b * TR + e * dr) * LD + e * dk] = in[e] ? __ldg(xb + e * (dr * sr + dk * sk)) : 0.0f;
+      for (int e = 0; e < EL; ++e) {
+        const bool in = t0 + u < items && row0 + lr + e * dr < a.rows && (kt0 + kq) * TK + lk + e * dk < a.ks;
+        v[u][e] = in ? __ldca(xb + e * (dr * sr + dk * sk)) : 0.0f;
+      }
+      if (++b == a.nblk) b = 0, ++kq;
     }
+#pragma unroll
+    for (int u = 0; u < STEP; ++u)
+      if (t0 + u < items) {
+#pragma unroll
+        for (int e = 0; e < EL; ++e) xs[((t0 + u) * TR + e * dr) * LD + e * dk] = v[u][e];
+      }
   }
   __syncthreads();
   const int q = tid % 16, row = tid / 16;
