@@ -30,7 +30,6 @@
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr int kBatchCounters = 2;  // a batch's per-phase work-unit counters, ahead of its tickets
 constexpr int kMR = 8;  // register-tile granularity of the FMM/fringe split (bl_config.h:16-17)
 constexpr int kNR = 4;
 
@@ -2432,18 +2431,30 @@ struct fmm_batch {
   int dev = 0;
   std::vector<int> m, n, k;
   std::vector<const fmm_plan*> plans;
-  std::vector<Job> jobs[2];        // phase 0: FMM cores and disjoint strips; phase 1: k strips
-  std::vector<int> unit_start[2];
+  // One products launch and, before it, the launch of its operand sums: usually one group of all FMM cores and
+  // disjoint strips (several, which use the same workspace in turn, where their sums together are too
+  // large), then the k strips.
+  struct Group {
+    int job0 = 0, njob = 0;        // its jobs
+    int start0 = 0, units = 0;     // its njob + 1 entries of unit_start
+    int ps0 = 0, nps = 0;          // its tasks of the operand sums
+    bool parts = false;            // some job's products are summed in parts
+    bool tma = true;               // this call's operands: all read by tensor copies
+  };
+  std::vector<Job> jobs;           // by group
+  std::vector<Group> groups;
+  bool k_strips = false;           // the last group holds the k strips
+  std::vector<int> unit_start;
   int max_slots = 0, presum_cap = 1;
   long long max_presum_chunks = 1;
   int n_presum = 0;
-  size_t n_tickets = 0, ws_bytes = 0;
-  fmmt::ProdArgs* d_jobs[2] = {nullptr, nullptr};
-  int* d_start[2] = {nullptr, nullptr};
-  fmmt::ProdArgs* h_jobs[2] = {nullptr, nullptr};  // pinned staging of the job tables
+  size_t n_tickets = 0, ws_bytes = 0, max_job_ws = 0;
+  fmmt::ProdArgs* d_jobs = nullptr;
+  int* d_start = nullptr;
+  fmmt::ProdArgs* h_jobs = nullptr;  // pinned staging of the job tables
   fmm::PresumSide* d_ps = nullptr;
   fmm::PresumSide* h_ps = nullptr;
-  int* d_tickets = nullptr;        // kBatchCounters work-unit counters (one per phase), then the tickets
+  int* d_tickets = nullptr;        // a work-unit counter per group, then the tickets
   char* d_ws = nullptr;
   // Even-pitch copies of A / B for problems whose row count is odd (a dense operand then
   // has an odd leading dimension, which tensor copies cannot stage): byte offsets into
@@ -2468,7 +2479,7 @@ int batch_chunks(int nprod, int ks) {
   return (int)c;
 }
 
-void batch_add_job(fmm_batch* b, int phase, int prob, const fmm_plan* plan, int ms, int ns, int ks, int a_r, int a_c,
+void batch_add_job(fmm_batch* b, std::vector<fmm_batch::Job>& jobs, int prob, const fmm_plan* plan, int ms, int ns, int ks, int a_r, int a_c,
                    int b_r, int b_c, int c_r, int c_c) {
   if (ms <= 0 || ns <= 0 || ks <= 0) return;
   fmm_batch::Job j{};
@@ -2497,13 +2508,10 @@ void batch_add_job(fmm_batch* b, int phase, int prob, const fmm_plan* plan, int 
     // operands with an odd row count or k get slots throughout, so that no pitch copy of them
     // is needed for the core
     j.pp = presum_plan(plan, ms, ns, ks, (b->m[prob] & 1) || (b->k[prob] & 1));
-    j.ws_off = b->ws_bytes;
-    b->ws_bytes += presum_bytes(j.pp);
     b->max_slots = std::max(b->max_slots, std::max(j.pp.nA, j.pp.nB));
     b->presum_cap = std::max(b->presum_cap, presum_cap(plan));
     const long long ca = j.pp.nA ? (j.pp.ldS / 2) * j.pp.kk : 0, cb = j.pp.nB ? (j.pp.ldT / 2) * ns : 0;
     b->max_presum_chunks = std::max(b->max_presum_chunks, (std::max(ca, cb) + kPsChunk - 1) / kPsChunk);
-    b->n_presum += (j.pp.nA > 0) + (j.pp.nB > 0);
     depth = j.pp.kk;
     j.depth = product_depth(plan, ms, ns, ks);
     j.chunks = batch_chunks(nprod, depth);
@@ -2515,15 +2523,73 @@ void batch_add_job(fmm_batch* b, int phase, int prob, const fmm_plan* plan, int 
   j.ticket_off = b->n_tickets;
   if (j.chunks > 1) b->n_tickets += 4 * (size_t)j.tiles_m * j.tiles_n;
   j.cost = (double)nprod / j.chunks * ((depth + 7) / 8);
-  b->jobs[phase].push_back(j);
+  jobs.push_back(j);
+}
+
+// Append `jobs` to the batch, longest units first (the persistent grid takes units in order, so the short
+// ones fill in at the end), in groups whose operand sums take at most `budget` bytes (one job's at least).
+// A group has at most kMaxPresumTasks tasks, the z extent of their launch.
+constexpr int kMaxPresumTasks = 65535;
+int batch_group(fmm_batch* b, std::vector<fmm_batch::Job>& jobs, long long budget) {
+  std::stable_sort(jobs.begin(), jobs.end(),
+                   [](const fmm_batch::Job& x, const fmm_batch::Job& y) { return x.cost > y.cost; });
+  fmm_batch::Group g{};
+  size_t ws = 0;
+  long long units = 0;
+  auto close = [&] {
+    if (g.njob == 0) return;
+    b->unit_start.push_back((int)units);
+    g.units = (int)units;
+    b->groups.push_back(g);
+  };
+  for (fmm_batch::Job& j : jobs) {
+    const size_t need = presum_bytes(j.pp);
+    const int tasks = (j.pp.nA > 0) + (j.pp.nB > 0);
+    if (g.njob == 0 || (need > 0 && (long long)(ws + need) > budget) || g.nps + tasks > kMaxPresumTasks) {
+      close();
+      g = fmm_batch::Group{};
+      g.job0 = (int)b->jobs.size();
+      g.start0 = (int)b->unit_start.size();
+      g.ps0 = b->n_presum;
+      ws = 0;
+      units = 0;
+    }
+    j.ws_off = ws;
+    ws += need;
+    b->ws_bytes = std::max(b->ws_bytes, ws);
+    b->max_job_ws = std::max(b->max_job_ws, need);
+    g.nps += tasks;
+    b->n_presum += tasks;
+    g.parts = g.parts || j.parts;
+    ++g.njob;
+    b->unit_start.push_back((int)units);
+    units += j.units;
+    if (units > INT32_MAX) return FMM_E_UNSUPPORTED;
+    DevTables* d = nullptr;
+    int rc = device_tables(j.plan, &d);
+    if (rc == FMM_OK && j.S > 1) rc = ksplit_tables(j.plan, BASE_SPLIT, j.S, &j.vprods, &j.vterms);
+    if (rc != FMM_OK) return rc;
+    b->jobs.push_back(j);
+  }
+  close();
+  return FMM_OK;
+}
+
+// Operand sums a batch holds at a time: four times a single call's cap.  A batch of large problems keeps the
+// one launch that its balance rests on (the 512-problem batch has 7 GB of sums), one of many small two-level
+// problems, whose sums are up to 4.5 times their operands, stays runnable.
+long long batch_budget() { return 4 * g_ws_limit.load(); }
+
+// After an allocation of the batch failed: a budget of half its sums, or 0 when they are one job's already.
+long long batch_smaller(const fmm_batch* b) {
+  cudaGetLastError();
+  return b->ws_bytes > b->max_job_ws ? (long long)(b->ws_bytes / 2) : 0;
 }
 
 void batch_free(fmm_batch* b) {
-  for (int ph = 0; ph < 2; ++ph) {
-    if (b->d_jobs[ph]) cudaFree(b->d_jobs[ph]);
-    if (b->d_start[ph]) cudaFree(b->d_start[ph]);
-    if (b->h_jobs[ph]) cudaFreeHost(b->h_jobs[ph]);
-  }
+  if (b->d_jobs) cudaFree(b->d_jobs);
+  if (b->d_start) cudaFree(b->d_start);
+  if (b->h_jobs) cudaFreeHost(b->h_jobs);
   if (b->d_ps) cudaFree(b->d_ps);
   if (b->h_ps) cudaFreeHost(b->h_ps);
   if (b->d_tickets) cudaFree(b->d_tickets);
@@ -2535,11 +2601,11 @@ void batch_free(fmm_batch* b) {
   delete b;
 }
 
-// The host side of a batch: jobs per phase in scheduling order, unit ranges, and the sizes
-// of the tickets and workspaces.  Allocates no device memory (the plans' tables are
+// The host side of a batch: jobs per group in scheduling order, unit ranges, and the sizes
+// of the tickets and workspaces (operand sums of at most `budget` bytes).  Allocates no device memory (the plans' tables are
 // uploaded on first use by device_tables).
-int batch_build(int count, const fmm_plan* const* plans, const int* m, const int* n, const int* k, fmm_batch** out,
-                const int* tile_m = nullptr) {
+int batch_build(int count, const fmm_plan* const* plans, const int* m, const int* n, const int* k, long long budget,
+                fmm_batch** out, const int* tile_m = nullptr) {
   if (!out || count <= 0 || !m || !n || !k) return FMM_E_INVALID;
   for (int i = 0; i < count; ++i) {
     if (m[i] < 0 || n[i] < 0 || k[i] < 0) return FMM_E_INVALID;
@@ -2556,6 +2622,7 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
   b->n.assign(n, n + count);
   b->k.assign(k, k + count);
   const fmm_plan* cls = classical_plan();
+  std::vector<fmm_batch::Job> main, strips;  // strips: the k strips, which update their core's C
   for (int i = 0; i < count; ++i) {
     const fmm_plan* p = (plans && plans[i]) ? plans[i] : nullptr;
     b->plans.push_back(p);
@@ -2569,7 +2636,7 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
     b->pitch_b.push_back(live && (k[i] & 1) ? reserve(k[i], n[i]) : SIZE_MAX);
     if (!live) continue;
     if (!p || is_classical(p)) {
-      batch_add_job(b, 0, i, cls, m[i], n[i], k[i], 0, 0, 0, 0, 0, 0);
+      batch_add_job(b, main, i, cls, m[i], n[i], k[i], 0, 0, 0, 0, 0, 0);
       continue;
     }
     // same partition and fringe regions as the single-problem path (run_fmm + peel)
@@ -2577,35 +2644,17 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
     const int mr = m[i] % pm, kr = k[i] % pk, nr = n[i] % pn;
     const int md = m[i] - mr, kd = k[i] - kr, nd = n[i] - nr;
     if (md > 0 && nd > 0 && kd > 0)
-      batch_add_job(b, 0, i, p, md / p->dims[0], nd / p->dims[2], kd / p->dims[1], 0, 0, 0, 0, 0, 0);
-    if (kr > 0 && md > 0 && nd > 0) batch_add_job(b, 1, i, cls, md, nd, kr, 0, kd, kd, 0, 0, 0);
-    if (nr > 0) batch_add_job(b, 0, i, cls, m[i], nr, k[i], 0, 0, 0, nd, 0, nd);
-    if (mr > 0 && nd > 0) batch_add_job(b, 0, i, cls, mr, nd, k[i], md, 0, 0, 0, md, 0);
+      batch_add_job(b, main, i, p, md / p->dims[0], nd / p->dims[2], kd / p->dims[1], 0, 0, 0, 0, 0, 0);
+    if (kr > 0 && md > 0 && nd > 0) batch_add_job(b, strips, i, cls, md, nd, kr, 0, kd, kd, 0, 0, 0);
+    if (nr > 0) batch_add_job(b, main, i, cls, m[i], nr, k[i], 0, 0, 0, nd, 0, nd);
+    if (mr > 0 && nd > 0) batch_add_job(b, main, i, cls, mr, nd, k[i], md, 0, 0, 0, md, 0);
   }
-  // Longest units first: the persistent grid takes units in order, so the short ones
-  // fill in at the end.
-  for (int ph = 0; ph < 2; ++ph) {
-    std::stable_sort(b->jobs[ph].begin(), b->jobs[ph].end(),
-                     [](const fmm_batch::Job& x, const fmm_batch::Job& y) { return x.cost > y.cost; });
-    long long acc = 0;
-    for (auto& j : b->jobs[ph]) {
-      b->unit_start[ph].push_back((int)acc);
-      acc += j.units;
-    }
-    if (acc > INT32_MAX) {
-      batch_free(b);
-      return FMM_E_UNSUPPORTED;
-    }
-    b->unit_start[ph].push_back((int)acc);
-    for (auto& j : b->jobs[ph]) {
-      DevTables* d = nullptr;
-      rc = device_tables(j.plan, &d);
-      if (rc == FMM_OK && j.S > 1) rc = ksplit_tables(j.plan, BASE_SPLIT, j.S, &j.vprods, &j.vterms);
-      if (rc != FMM_OK) {
-        batch_free(b);
-        return rc;
-      }
-    }
+  rc = batch_group(b, main, budget);
+  if (rc == FMM_OK) rc = batch_group(b, strips, budget);
+  b->k_strips = !strips.empty();
+  if (rc != FMM_OK) {
+    batch_free(b);
+    return rc;
   }
   *out = b;
   return FMM_OK;
@@ -2613,47 +2662,48 @@ int batch_build(int count, const fmm_plan* const* plans, const int* m, const int
 
 int batch_create(int count, const fmm_plan* const* plans, const int* m, const int* n, const int* k, fmm_batch** out,
                  const int* tile_m = nullptr) {
-  fmm_batch* b = nullptr;
-  int rc = batch_build(count, plans, m, n, k, &b, tile_m);
-  if (rc != FMM_OK) return rc;
-  auto fail = [&](cudaError_t e) {
+  for (long long budget = batch_budget(); budget > 0;) {
+    fmm_batch* b = nullptr;
+    const int rc = batch_build(count, plans, m, n, k, budget, &b, tile_m);
+    if (rc != FMM_OK) return rc;
+    cudaError_t e = cudaSuccess;
+    const size_t nj = b->jobs.size(), ns = b->unit_start.size();
+    if (nj > 0) {
+      e = cudaMalloc((void**)&b->d_jobs, sizeof(fmmt::ProdArgs) * nj);
+      if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_start, sizeof(int) * ns);
+      if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_jobs, sizeof(fmmt::ProdArgs) * nj);
+      if (e == cudaSuccess) e = cudaMemcpy(b->d_start, b->unit_start.data(), sizeof(int) * ns, cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess && b->n_presum > 0) {
+      e = cudaMalloc((void**)&b->d_ps, sizeof(fmm::PresumSide) * b->n_presum);
+      if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_ps, sizeof(fmm::PresumSide) * b->n_presum);
+    }
+    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_tickets, sizeof(int) * (b->groups.size() + b->n_tickets + 1));
+    if (e == cudaSuccess && b->pitch_bytes > 0) {
+      e = cudaMalloc((void**)&b->d_pitch, b->pitch_bytes);
+      if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_pc, sizeof(fmm::PitchCopy) * 2 * count);
+      if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_pc, sizeof(fmm::PitchCopy) * 2 * count);
+    }
+    if (e == cudaSuccess && b->ws_bytes > 0) e = cudaMalloc((void**)&b->d_ws, b->ws_bytes);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->staged, cudaEventDisableTiming);
+    if (e == cudaSuccess) {
+      *out = b;
+      return FMM_OK;
+    }
+    budget = e == cudaErrorMemoryAllocation ? batch_smaller(b) : 0;
     batch_free(b);
-    return cuda_status(e);
-  };
-  cudaError_t e = cudaSuccess;
-  for (int ph = 0; ph < 2 && e == cudaSuccess; ++ph) {
-    const size_t nj = b->jobs[ph].size();
-    if (nj == 0) continue;
-    e = cudaMalloc((void**)&b->d_jobs[ph], sizeof(fmmt::ProdArgs) * nj);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_start[ph], sizeof(int) * (nj + 1));
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_jobs[ph], sizeof(fmmt::ProdArgs) * nj);
-    if (e == cudaSuccess)
-      e = cudaMemcpy(b->d_start[ph], b->unit_start[ph].data(), sizeof(int) * (nj + 1), cudaMemcpyHostToDevice);
+    if (budget == 0) return cuda_status(e);
   }
-  if (e == cudaSuccess && b->n_presum > 0) {
-    e = cudaMalloc((void**)&b->d_ps, sizeof(fmm::PresumSide) * b->n_presum);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_ps, sizeof(fmm::PresumSide) * b->n_presum);
-  }
-  if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_tickets, sizeof(int) * (kBatchCounters + b->n_tickets));
-  if (e == cudaSuccess && b->ws_bytes > 0) e = cudaMalloc((void**)&b->d_ws, b->ws_bytes);
-  if (e == cudaSuccess && b->pitch_bytes > 0) {
-    e = cudaMalloc((void**)&b->d_pitch, b->pitch_bytes);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_pc, sizeof(fmm::PitchCopy) * 2 * count);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_pc, sizeof(fmm::PitchCopy) * 2 * count);
-  }
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->staged, cudaEventDisableTiming);
-  if (e != cudaSuccess) return fail(e);
-  *out = b;
-  return FMM_OK;
+  return FMM_E_NOMEM;
 }
 
-// Fill the job table of one phase for this call's operands; false if some operand cannot be
+// Fill the job table of one group for this call's operands; false if some operand cannot be
 // read by tensor copies (the launch then carries the per-lane copies).
-bool batch_fill(fmm_batch* b, int ph, const double* const* A, const long* lda, const double* const* B,
+bool batch_fill(fmm_batch* b, const fmm_batch::Group& g, const double* const* A, const long* lda, const double* const* B,
                 const long* ldb, double* const* C, const long* ldc, int* n_ps) {
   bool tma = true;
-  for (size_t q = 0; q < b->jobs[ph].size(); ++q) {
-    const fmm_batch::Job& j = b->jobs[ph][q];
+  for (int q = g.job0; q < g.job0 + g.njob; ++q) {
+    const fmm_batch::Job& j = b->jobs[q];
     const DevTables& d = j.plan->dev[b->dev];
     fmmt::ProdArgs a{};
     const long long la = lda[j.prob], lb = ldb[j.prob], lc = ldc[j.prob];
@@ -2673,7 +2723,7 @@ bool batch_fill(fmm_batch* b, int ph, const double* const* A, const long* lda, c
     a.tiles_n = j.tiles_n;
     a.chunks = j.chunks;
     a.mode = fmm::MODE_ACCUM_C;
-    a.tickets = j.chunks > 1 ? b->d_tickets + kBatchCounters + j.ticket_off : nullptr;
+    a.tickets = j.chunks > 1 ? b->d_tickets + b->groups.size() + j.ticket_off : nullptr;
     a.status = dev_status[b->dev];
     const PresumPlan& pp = j.pp;
     double* S = reinterpret_cast<double*>(b->d_ws + j.ws_off);
@@ -2702,14 +2752,14 @@ bool batch_fill(fmm_batch* b, int ph, const double* const* A, const long* lda, c
     if (pp.nA > 0) ok = make_a_map(&a.tmAw, S, j.ms, (long long)pp.nA * pp.kk, pp.ldS);
     if (pp.nB > 0) ok = ok && make_b_map(&a.tmBw, T, pp.kk, (long long)pp.nB * j.ns, pp.ldT, 64);
     tma = tma && ok && a.a_tma && a.b_tma;
-    b->h_jobs[ph][q] = a;
+    b->h_jobs[q] = a;
   }
   return tma;
 }
 
 void batch_prepare(fmm_batch* b, const double* const* A, const long* lda, const double* const* B, const long* ldb,
-                   double* const* C, const long* ldc, int* n_ps_out, int* n_pc_out, bool tma[2]);
-int batch_launch(fmm_batch* b, cudaStream_t st, int n_ps, int n_pc, const bool tma[2]);
+                   double* const* C, const long* ldc, int* n_pc_out);
+int batch_launch(fmm_batch* b, cudaStream_t st, int n_pc);
 
 int batch_run(fmm_batch* b, const double* const* A, const long* lda, const double* const* B, const long* ldb,
               double* const* C, const long* ldc, cudaStream_t st) {
@@ -2727,25 +2777,23 @@ int batch_run(fmm_batch* b, const double* const* A, const long* lda, const doubl
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   FMM_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
   if (cap == cudaStreamCaptureStatusNone) FMM_CUDA_TRY(cudaEventSynchronize(b->staged));
-  int n_ps = 0, n_pc = 0;
-  bool tma[2] = {true, true};
-  batch_prepare(b, A, lda, B, ldb, C, ldc, &n_ps, &n_pc, tma);
-  for (int ph = 0; ph < 2; ++ph)
-    if (!b->jobs[ph].empty())
-      FMM_CUDA_TRY(cudaMemcpyAsync(b->d_jobs[ph], b->h_jobs[ph], sizeof(fmmt::ProdArgs) * b->jobs[ph].size(),
-                                   cudaMemcpyHostToDevice, st));
-  if (n_ps > 0)
-    FMM_CUDA_TRY(cudaMemcpyAsync(b->d_ps, b->h_ps, sizeof(fmm::PresumSide) * n_ps, cudaMemcpyHostToDevice, st));
+  int n_pc = 0;
+  batch_prepare(b, A, lda, B, ldb, C, ldc, &n_pc);
+  if (!b->jobs.empty())
+    FMM_CUDA_TRY(cudaMemcpyAsync(b->d_jobs, b->h_jobs, sizeof(fmmt::ProdArgs) * b->jobs.size(), cudaMemcpyHostToDevice,
+                                 st));
+  if (b->n_presum > 0)
+    FMM_CUDA_TRY(cudaMemcpyAsync(b->d_ps, b->h_ps, sizeof(fmm::PresumSide) * b->n_presum, cudaMemcpyHostToDevice, st));
   if (n_pc > 0)
     FMM_CUDA_TRY(cudaMemcpyAsync(b->d_pc, b->h_pc, sizeof(fmm::PitchCopy) * n_pc, cudaMemcpyHostToDevice, st));
   if (cap == cudaStreamCaptureStatusNone) FMM_CUDA_TRY(cudaEventRecord(b->staged, st));
-  return batch_launch(b, st, n_ps, n_pc, tma);
+  return batch_launch(b, st, n_pc);
 }
 
 // This call's job tables (host staging): even-pitch copies for odd leading dimensions,
 // per-job arguments and tensor maps, pre-sum tasks.
 void batch_prepare(fmm_batch* b, const double* const* A, const long* lda, const double* const* B, const long* ldb,
-                   double* const* C, const long* ldc, int* n_ps_out, int* n_pc_out, bool tma[2]) {
+                   double* const* C, const long* ldc, int* n_pc_out) {
   // Operands with an odd leading dimension and a reserved even-pitch copy are staged
   // through it (rows + 1 pitch); the others are used in place.
   std::vector<const double*> eA(A, A + b->count), eB(B, B + b->count);
@@ -2766,47 +2814,44 @@ void batch_prepare(fmm_batch* b, const double* const* A, const long* lda, const 
     }
   }
   int n_ps = 0;
-  for (int ph = 0; ph < 2; ++ph)
-    if (!b->jobs[ph].empty())
-      tma[ph] = batch_fill(b, ph, eA.data(), elda.data(), eB.data(), eldb.data(), C, ldc, &n_ps);
-  *n_ps_out = n_ps;
+  for (fmm_batch::Group& g : b->groups) g.tma = batch_fill(b, g, eA.data(), elda.data(), eB.data(), eldb.data(), C, ldc, &n_ps);
   *n_pc_out = n_pc;
 }
 
 // Enqueue the launches of a prepared batch whose tables are (being) copied to the device.
-int batch_launch(fmm_batch* b, cudaStream_t st, int n_ps, int n_pc, const bool tma[2]) {
-  // the phases' work-unit counters and every ticket start at zero
-  FMM_CUDA_TRY(cudaMemsetAsync(b->d_tickets, 0, sizeof(int) * (kBatchCounters + b->n_tickets), st));
+int batch_launch(fmm_batch* b, cudaStream_t st, int n_pc) {
+  // the groups' work-unit counters and every ticket start at zero
+  FMM_CUDA_TRY(cudaMemsetAsync(b->d_tickets, 0, sizeof(int) * (b->groups.size() + b->n_tickets), st));
   if (n_pc > 0) {
     ProfScope pf(K_PITCH_COPY, st);
     fmm::fmm_pitch_copy_kernel<<<dim3(256, (unsigned)n_pc), 256, 0, st>>>(b->d_pc);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     FMM_CUDA_TRY(cudaGetLastError());
   }
-  if (n_ps > 0) {
-    ProfScope pf(K_PRESUM_BATCH, st);
-    const long long nc = std::min<long long>(b->max_presum_chunks, 1 << 16);
-    fmm::fmm_presum_batch_kernel<<<dim3((unsigned)nc, presum_ranges(nc * n_ps, b->max_slots, sm_count[b->dev]),
-                                        (unsigned)n_ps),
-                                   fmm::PS_THREADS, fmm::presum_smem_bytes(b->presum_cap), st>>>(b->d_ps, b->presum_cap);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    FMM_CUDA_TRY(cudaGetLastError());
-  }
-  for (int ph = 0; ph < 2; ++ph) {
-    if (b->jobs[ph].empty()) continue;
+  for (size_t q = 0; q < b->groups.size(); ++q) {
+    const fmm_batch::Group& g = b->groups[q];
+    if (g.nps > 0) {
+      ProfScope pf(K_PRESUM_BATCH, st);
+      const long long nc = std::min<long long>(b->max_presum_chunks, 1 << 16);
+      fmm::fmm_presum_batch_kernel<<<dim3((unsigned)nc, presum_ranges(nc * g.nps, b->max_slots, sm_count[b->dev]),
+                                          (unsigned)g.nps),
+                                     fmm::PS_THREADS, fmm::presum_smem_bytes(b->presum_cap), st>>>(b->d_ps + g.ps0,
+                                                                                                   b->presum_cap);
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+      FMM_CUDA_TRY(cudaGetLastError());
+    }
     fmmt::ProdBatchArgs ba{};
-    ba.jobs = b->d_jobs[ph];
-    ba.unit_start = b->d_start[ph];
-    ba.njobs = (int)b->jobs[ph].size();
-    ba.units = b->unit_start[ph].back();
+    ba.jobs = b->d_jobs + g.job0;
+    ba.unit_start = b->d_start + g.start0;
+    ba.njobs = g.njob;
+    ba.units = g.units;
     ba.status = dev_status[b->dev];
-    ba.counter = b->d_tickets + ph;
+    ba.counter = b->d_tickets + q;
     const unsigned grid =
         (unsigned)std::min<long long>(ba.units, (long long)sm_count[b->dev] * fmmt::TileShape<64, 64>::CTAS);
     ProfScope pf(K_PRODUCTS_BATCH, st);
-    const bool parts = std::any_of(b->jobs[ph].begin(), b->jobs[ph].end(), [](const fmm_batch::Job& j) { return j.parts; });
-    auto kernel = tma[ph] ? (parts ? fmmt::fmm_products_batch_kernel<false, true> : fmmt::fmm_products_batch_kernel<false, false>)
-                          : (parts ? fmmt::fmm_products_batch_kernel<true, true> : fmmt::fmm_products_batch_kernel<true, false>);
+    auto kernel = g.tma ? (g.parts ? fmmt::fmm_products_batch_kernel<false, true> : fmmt::fmm_products_batch_kernel<false, false>)
+                        : (g.parts ? fmmt::fmm_products_batch_kernel<true, true> : fmmt::fmm_products_batch_kernel<true, false>);
     const int rc = launch_dependent(kernel, dim3(grid), fmmt::NT,
                                     spread_smem(fmmt::ProdShape<64>::SMEM, grid, sm_count[b->dev]), st, 1, ba);
     if (rc != FMM_OK) return rc;
@@ -2835,7 +2880,10 @@ int fmm_batch_dgemm(fmm_batch* batch, const double* const* A, const long* lda, c
 
 int fmm_batch_units(const fmm_batch* batch, int phase) {
   if (!batch || phase < 0 || phase > 1) return FMM_E_INVALID;
-  return batch->unit_start[phase].empty() ? 0 : batch->unit_start[phase].back();
+  const size_t main = batch->groups.size() - (batch->k_strips ? 1 : 0);
+  long long units = 0;
+  for (size_t q = phase == 0 ? 0 : main; q < (phase == 0 ? main : batch->groups.size()); ++q) units += batch->groups[q].units;
+  return (int)std::min<long long>(units, INT32_MAX);
 }
 
 int fmm_batch_destroy(fmm_batch* batch) {
@@ -2897,47 +2945,38 @@ int batch_submit(int count, const fmm_plan* const* plans, const int* m, const in
     if (rc != FMM_OK) return rc;
   }
   fmm_batch* b = nullptr;
-  int rc = batch_build(count, plans, m, n, k, &b);
-  if (rc != FMM_OK) return rc;
-  // table block (identical layout in pinned staging and on the device)
-  size_t off = 0, o_jobs[2], o_start[2];
-  for (int ph = 0; ph < 2; ++ph) {
-    off = align_up(off, 64);
-    o_jobs[ph] = off;
-    off += sizeof(fmmt::ProdArgs) * b->jobs[ph].size();
-  }
-  for (int ph = 0; ph < 2; ++ph) {
-    off = align_up(off, 16);
-    o_start[ph] = off;
-    off += sizeof(int) * b->unit_start[ph].size();
-  }
-  off = align_up(off, 64);
-  const size_t o_ps = off;
-  off += sizeof(fmm::PresumSide) * b->n_presum;
-  off = align_up(off, 64);
-  const size_t o_pc = off;
-  off += sizeof(fmm::PitchCopy) * 2 * count;
-  const size_t table_bytes = align_up(off, 256);
-  const size_t o_tk = table_bytes;
-  const size_t o_ws = align_up(o_tk + sizeof(int) * (kBatchCounters + b->n_tickets), 256);
-  const size_t o_pt = align_up(o_ws + b->ws_bytes, 256);
-  const size_t dev_bytes = o_pt + b->pitch_bytes;
-  char* stage = nullptr;
+  size_t o_jobs = 0, o_start, o_ps, o_pc, table_bytes, o_tk, o_ws, o_pt;
+  char *stage = nullptr, *blk = nullptr;
   cudaEvent_t stage_ev = nullptr;
+  int rc = FMM_E_NOMEM;
+  for (long long budget = batch_budget(); budget > 0;) {
+    rc = batch_build(count, plans, m, n, k, budget, &b);
+    if (rc != FMM_OK) return rc;
+    // table block (identical layout in pinned staging and on the device)
+    o_start = align_up(o_jobs + sizeof(fmmt::ProdArgs) * b->jobs.size(), 16);
+    o_ps = align_up(o_start + sizeof(int) * b->unit_start.size(), 64);
+    o_pc = align_up(o_ps + sizeof(fmm::PresumSide) * b->n_presum, 64);
+    table_bytes = align_up(o_pc + sizeof(fmm::PitchCopy) * 2 * count, 256);
+    o_tk = table_bytes;
+    o_ws = align_up(o_tk + sizeof(int) * (b->groups.size() + b->n_tickets), 256);
+    o_pt = align_up(o_ws + b->ws_bytes, 256);
+    rc = cuda_status(cudaMallocAsync((void**)&blk, o_pt + b->pitch_bytes, st));
+    if (rc == FMM_OK) break;
+    budget = rc == FMM_E_NOMEM ? batch_smaller(b) : 0;
+    batch_free(b);
+    b = nullptr;
+  }
+  if (rc != FMM_OK) return rc;
   rc = ring_acquire(b->dev, table_bytes, &stage, &stage_ev);
-  char* blk = nullptr;
-  if (rc == FMM_OK) rc = cuda_status(cudaMallocAsync((void**)&blk, dev_bytes, st));
   if (rc != FMM_OK) {
+    cudaFreeAsync(blk, st);
     batch_free(b);
     return rc;
   }
-  for (int ph = 0; ph < 2; ++ph) {
-    b->h_jobs[ph] = reinterpret_cast<fmmt::ProdArgs*>(stage + o_jobs[ph]);
-    b->d_jobs[ph] = reinterpret_cast<fmmt::ProdArgs*>(blk + o_jobs[ph]);
-    b->d_start[ph] = reinterpret_cast<int*>(blk + o_start[ph]);
-    if (!b->unit_start[ph].empty())
-      std::memcpy(stage + o_start[ph], b->unit_start[ph].data(), sizeof(int) * b->unit_start[ph].size());
-  }
+  b->h_jobs = reinterpret_cast<fmmt::ProdArgs*>(stage + o_jobs);
+  b->d_jobs = reinterpret_cast<fmmt::ProdArgs*>(blk + o_jobs);
+  b->d_start = reinterpret_cast<int*>(blk + o_start);
+  if (!b->unit_start.empty()) std::memcpy(stage + o_start, b->unit_start.data(), sizeof(int) * b->unit_start.size());
   b->h_ps = reinterpret_cast<fmm::PresumSide*>(stage + o_ps);
   b->d_ps = reinterpret_cast<fmm::PresumSide*>(blk + o_ps);
   b->h_pc = reinterpret_cast<fmm::PitchCopy*>(stage + o_pc);
@@ -2945,16 +2984,15 @@ int batch_submit(int count, const fmm_plan* const* plans, const int* m, const in
   b->d_tickets = reinterpret_cast<int*>(blk + o_tk);
   b->d_ws = b->ws_bytes ? blk + o_ws : nullptr;
   b->d_pitch = b->pitch_bytes ? blk + o_pt : nullptr;
-  int n_ps = 0, n_pc = 0;
-  bool tma[2] = {true, true};
-  batch_prepare(b, A, lda, B, ldb, C, ldc, &n_ps, &n_pc, tma);
+  int n_pc = 0;
+  batch_prepare(b, A, lda, B, ldb, C, ldc, &n_pc);
   rc = cuda_status(cudaMemcpyAsync(blk, stage, table_bytes, cudaMemcpyHostToDevice, st));
   if (rc == FMM_OK) rc = cuda_status(cudaEventRecord(stage_ev, st));
-  if (rc == FMM_OK) rc = batch_launch(b, st, n_ps, n_pc, tma);
+  if (rc == FMM_OK) rc = batch_launch(b, st, n_pc);
   cudaError_t fe = cudaFreeAsync(blk, st);
   if (rc == FMM_OK) rc = cuda_status(fe);
   // the buffers belong to the pool and the ring: detach them before freeing the host side
-  for (int ph = 0; ph < 2; ++ph) b->h_jobs[ph] = nullptr, b->d_jobs[ph] = nullptr, b->d_start[ph] = nullptr;
+  b->h_jobs = nullptr, b->d_jobs = nullptr, b->d_start = nullptr;
   b->h_ps = nullptr, b->d_ps = nullptr, b->h_pc = nullptr, b->d_pc = nullptr;
   b->d_tickets = nullptr, b->d_ws = nullptr, b->d_pitch = nullptr;
   batch_free(b);

@@ -198,7 +198,10 @@ int fmm_split_gemm_dev(const fmm_plan *plan, int m, int n, int k, const float *A
  * fmm_dgemm_dev partitions it (FMM core plus fringe strips), so results are identical
  * to calling fmm_dgemm_dev per problem.  A second launch handles the k-fringe strips
  * (they update the same C region as their core), and a launch before them forms the
- * pre-summed operands of the FMM problems.
+ * pre-summed operands of the FMM problems.  Where those would take more than four times the
+ * workspace cap (fmm_set_workspace_limit, read when the batch is formed), more memory than there is, or more
+ * than 65535 sums, the problems run in groups, a launch pair each, whose sums use one workspace in turn;
+ * results are unchanged.
  *
  * fmm_batch_create fixes the shapes and plans and allocates (cudaMalloc) the job tables,
  * tickets and workspaces; the plans must outlive the batch.  fmm_batch_dgemm takes this
