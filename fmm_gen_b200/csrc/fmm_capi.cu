@@ -1291,6 +1291,28 @@ int launch_presum(const fmm_plan* plan, const fmm::PresumSide& a, const fmm::Pre
 // Bytes of the pre-summed workspace of one call.
 size_t presum_bytes(const PresumPlan& pp) { return pp.s_bytes + pp.t_bytes; }
 
+// C_l += sum_r W[l,r] M_r for stored products (product r at M + r ms ns).
+int apply_stored(const fmm_plan* plan, const DevTables& d, double* C, long long ldc, int ms, int ns, const double* M,
+                 cudaStream_t st) {
+  if (combine_fits(plan)) return launch_combine(plan, d, C, ldc, ms, ns, M, ms, (long long)ms * ns, st);
+  fmm::ScatterArgs sa{};
+  sa.C = C;
+  sa.ldc = ldc;
+  sa.ms = ms;
+  sa.ns = ns;
+  sa.M = M;
+  sa.ldm = ms;
+  sa.m_stride = (long long)ms * ns;
+  sa.cblk = d.cblk;
+  sa.ent_r = d.ent_r;
+  sa.ent_w = d.ent_w;
+  const dim3 gs((unsigned)grid_for(sa.m_stride, 256), (unsigned)plan->n_cblk);
+  ProfScope pf(K_SCATTER, st);
+  fmm::fmm_scatter_kernel<<<gs, 256, 0, st>>>(sa);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cuda_status(cudaGetLastError());
+}
+
 // Pre-summed products in groups, when one call's whole operand workspace would exceed the
 // workspace limit: the R products run as groups of G consecutive products, each group's
 // operand sums (one slot per product, k extent padded to whole k groups) formed in the one
@@ -1299,22 +1321,36 @@ size_t presum_bytes(const PresumPlan& pp) { return pp.s_bytes + pp.t_bytes; }
 // products launches all the same, and twice the groups read A and B twice as often: 16384^3
 // 222-1 x 333-1 200.6 ms.)  Groups run in product order, so every C element still receives its
 // products' updates in order r = 0..R-1 (results are those of the ungrouped call).  Workspace
-// G (ms + ns) kk 8 bytes, within the limit for G >= 1.
+// G (ms + ns) kk 8 bytes, within the limit for G >= 1, and less where it cannot be allocated.  stored (the
+// ab pack type): the products go to a workspace of their own and W is applied at the end.
 int run_presum_groups(const fmm_plan* plan, const DevTables& d, const double* A, long long lda, const double* B,
-                      long long ldb, double* C, long long ldc, int ms, int ns, int ks, int nsm, cudaStream_t st) {
+                      long long ldb, double* C, long long ldc, int ms, int ns, int ks, int nsm, bool stored,
+                      cudaStream_t st) {
   const int R = plan->rank;
   const int kk = (ks + 7) / 8 * 8;
   const long long ldS = (ms + 1) / 2 * 2;
   const size_t sb = sizeof(double) * (size_t)ldS * kk, tb = sizeof(double) * (size_t)kk * ns;
   long long G = g_ws_limit.load() / (long long)(sb + tb);
   G = std::max<long long>(1, std::min<long long>(G, R));
-  const int ng = (int)((R + G - 1) / G);
-  G = (R + ng - 1) / ng;  // even groups
-  const ProdLaunch L = plan_products(plan->dims, (int)G, fmm::MODE_ACCUM_C, ms, ns, nsm);
-  const size_t tk = (sizeof(int) * (1 + L.tickets) + 255) & ~(size_t)255;
+  const int mode = stored ? fmm::MODE_STORE_M : fmm::MODE_ACCUM_C;
+  const size_t mb = stored ? sizeof(double) * (size_t)ms * ns * R : 0;
+  ProdLaunch L;
+  size_t tk = 0;
   char* ws = nullptr;
-  FMM_CUDA_TRY(cudaMallocAsync((void**)&ws, G * (sb + tb) + tk, st));
+  for (;;) {
+    const int ng = (int)((R + G - 1) / G);
+    G = (R + ng - 1) / ng;  // even groups
+    L = plan_products(plan->dims, (int)G, mode, ms, ns, nsm);
+    tk = (sizeof(int) * (1 + L.tickets) + 255) & ~(size_t)255;
+    const size_t sums = ((size_t)G * (sb + tb) + 255) & ~(size_t)255;
+    const cudaError_t e = cudaMallocAsync((void**)&ws, tk + sums + mb, st);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation || G == 1) return cuda_status(e);
+    cudaGetLastError();
+    G = G / 2;
+  }
   t_last_ws = (long long)(G * (sb + tb));
+  double* M = stored ? reinterpret_cast<double*>(ws + tk + (((size_t)G * (sb + tb) + 255) & ~(size_t)255)) : nullptr;
   int* counter = reinterpret_cast<int*>(ws);
   int rc = FMM_OK;
   for (int g0 = 0; g0 < R && rc == FMM_OK; g0 += (int)G) {
@@ -1334,9 +1370,11 @@ int run_presum_groups(const fmm_plan* plan, const DevTables& d, const double* A,
     const fmm::Term* gt = nullptr;
     if (rc == FMM_OK) rc = ksplit_tables(plan, BASE_GROUP, g0, &gp, &gt, g1);
     if (rc == FMM_OK)
-      rc = launch_products(gp, gt, plan->dims, n, fmm::MODE_ACCUM_C, A, lda, B, ldb, ps, C, ldc, nullptr, ms, ns, ks,
-                           kk, product_depth(plan, ms, ns, ks), L, counter, st);
+      rc = launch_products(gp, gt, plan->dims, n, mode, A, lda, B, ldb, ps, C, ldc,
+                           stored ? M + (long long)g0 * ms * ns : nullptr, ms, ns, ks, kk, product_depth(plan, ms, ns, ks),
+                           L, counter, st);
   }
+  if (rc == FMM_OK && stored) rc = apply_stored(plan, d, C, ldc, ms, ns, M, st);
   cudaError_t fe = cudaFreeAsync(ws, st);
   return rc == FMM_OK ? cuda_status(fe) : rc;
 }
@@ -1379,14 +1417,18 @@ int run_core(const fmm_plan* plan, int pack, const double* A, long long lda, con
   const bool capped = pack == FMM_PACK_ABC && (long long)presum_bytes(pp) > g_ws_limit.load();
   const bool stored = pack != FMM_PACK_ABC ||
                       (!capped && g_ticket_fill == 0 && combine_fits(plan) && prefer_stored_products(plan, ms, ns, ks, nsm));
-  if (capped)
-    return run_presum_groups(plan, *d, A, lda, B, ldb, C, ldc, ms, ns, ks, nsm, st);
+  if (capped) return run_presum_groups(plan, *d, A, lda, B, ldb, C, ldc, ms, ns, ks, nsm, false, st);
   const int mode = stored ? fmm::MODE_STORE_M : fmm::MODE_ACCUM_C;
   const ProdLaunch L = plan_products(plan->dims, R, mode, ms, ns, nsm);
   const size_t tk = (sizeof(int) * (1 + L.tickets) + 255) & ~(size_t)255;
   const size_t mb = stored ? sizeof(double) * (size_t)ms * ns * R : 0;
   char* ws = nullptr;
-  FMM_CUDA_TRY(cudaMallocAsync((void**)&ws, tk + presum_bytes(pp) + mb, st));
+  const cudaError_t ae = cudaMallocAsync((void**)&ws, tk + presum_bytes(pp) + mb, st);
+  if (ae == cudaErrorMemoryAllocation && pack != FMM_PACK_NAIVE) {  // no room: a group's sums at a time
+    cudaGetLastError();
+    return run_presum_groups(plan, *d, A, lda, B, ldb, C, ldc, ms, ns, ks, nsm, pack == FMM_PACK_AB, st);
+  }
+  FMM_CUDA_TRY(ae);
   t_last_ws = (long long)presum_bytes(pp);
   int* counter = reinterpret_cast<int*>(ws);
   double* M = stored ? reinterpret_cast<double*>(ws + tk + presum_bytes(pp)) : nullptr;
@@ -1408,28 +1450,7 @@ int run_core(const fmm_plan* plan, int pack, const double* A, long long lda, con
   if (rc == FMM_OK)
     rc = launch_products(pp.all ? d->prods_all : d->prods_ps, pp.all ? d->terms_all : d->terms_ps, plan->dims, R, mode, A,
                          lda, B, ldb, ps, C, ldc, M, ms, ns, ks, pp.kk, product_depth(plan, ms, ns, ks), L, counter, st);
-  if (rc == FMM_OK && stored && combine_fits(plan)) {
-    rc = launch_combine(plan, *d, C, ldc, ms, ns, M, ms, (long long)ms * ns, st);
-  } else if (rc == FMM_OK && stored) {
-    fmm::ScatterArgs sa{};
-    sa.C = C;
-    sa.ldc = ldc;
-    sa.ms = ms;
-    sa.ns = ns;
-    sa.M = M;
-    sa.ldm = ms;
-    sa.m_stride = (long long)ms * ns;
-    sa.cblk = d->cblk;
-    sa.ent_r = d->ent_r;
-    sa.ent_w = d->ent_w;
-    const dim3 gs((unsigned)grid_for(sa.m_stride, 256), (unsigned)plan->n_cblk);
-    {
-      ProfScope pf(K_SCATTER, st);
-      fmm::fmm_scatter_kernel<<<gs, 256, 0, st>>>(sa);
-    }
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    rc = cuda_status(cudaGetLastError());
-  }
+  if (rc == FMM_OK && stored) rc = apply_stored(plan, *d, C, ldc, ms, ns, M, st);
   cudaError_t fe = cudaFreeAsync(ws, st);
   return rc == FMM_OK ? cuda_status(fe) : rc;
 }

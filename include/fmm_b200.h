@@ -119,8 +119,8 @@ int fmm_device_status(int clear);
  * products in groups, one group's sums in the workspace at a time; results are unchanged.
  * The groups' workspace is G (ms + ns) kk 8 bytes for groups of G >= 1 products (kk: the k
  * extent per product rounded up to 8), so a cap below one product's sums is exceeded by that
- * much.  Returns
- * the previous cap.
+ * much.  A call of the abc or ab pack type whose workspace cannot be allocated runs in
+ * groups too, of as many products as there is room for.  Returns the previous cap.
  * fmm_last_workspace_bytes: pre-summed workspace bytes of the calling thread's last
  * fmm_dgemm_dev / host call (0 when it used none).  The stored products of a call whose C
  * traffic the library routes through one combine pass (8 R ms ns bytes) are not capped. */

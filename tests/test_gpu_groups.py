@@ -1,4 +1,4 @@
-"""Operand sums in groups: batches whose sums together exceed what may be, or can be, allocated run
+"""Operand sums in groups: batches and calls whose sums together exceed what may be, or can be, allocated run
 their products a group at a time, with the results of the ungrouped call."""
 import subprocess
 import sys
@@ -109,8 +109,12 @@ filler = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, dev
 if form == "batch":
     batch = rt.Batch([shape] * count, [plan] * count)
     batch.run(As, Bs, Cs)
-else:
+elif form == "submit":
     rt.batch_submit([plan] * count, As, Bs, Cs)
+else:
+    for a, b, c in zip(As, Bs, Cs):
+        rt.fmm_gemm(plan, a, b, c, form)
+        assert 0 < rt.last_workspace_bytes() < room + (256 << 20)
 torch.cuda.synchronize()
 assert lib.fmm_device_status(1) == 0
 for w, c in zip(want, Cs):
@@ -120,9 +124,11 @@ print("equal")
 
 
 @pytest.mark.parametrize("form,algs,shape,count,room", [
+    ("ab", (["222"], [2]), (512, 512, 100000), 1, 1 << 30),             # 2.2 GB of sums, 0.05 GB a product
+    ("abc", (["222"], [2]), (512, 512, 100000), 1, 1 << 30),
     ("batch", (["222", "333"], [1, 1]), (360, 360, 30000), 4, 2 << 30),  # 0.8 GB of sums a problem
     ("submit", (["222", "333"], [1, 1]), (360, 360, 30000), 4, 2 << 30),
-], ids=["batch", "submit"])
+], ids=["ab", "abc", "batch", "submit"])
 def test_sums_larger_than_the_free_memory(form, algs, shape, count, room):
     """A card that is almost full (in a process of its own, whose pools are empty)."""
     code = FULL.format(form=form, algs=algs, shape=shape, count=count, room=room)
