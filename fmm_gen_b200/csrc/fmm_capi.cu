@@ -636,9 +636,11 @@ int configure_kernel(int* dev_out) {
       return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)std::max(bytes, kSpreadSmem));
     };
-    for (auto kernel : {fmmt::fmm_tile_gemm_kernel<64, 64, false>, fmmt::fmm_tile_gemm_kernel<64, 64, true>})
+    for (auto kernel : {fmmt::fmm_tile_gemm_kernel<64, 64, false>, fmmt::fmm_tile_gemm_kernel<64, 64, true>,
+                        fmmt::fmm_tile_gemm_kernel<64, 64, false, true>})
       FMM_CUDA_TRY(smem(kernel, fmmt::TileShape<64, 64>::SMEM));
-    for (auto kernel : {fmmt::fmm_tile_gemm_kernel<32, 32, false>, fmmt::fmm_tile_gemm_kernel<32, 32, true>})
+    for (auto kernel : {fmmt::fmm_tile_gemm_kernel<32, 32, false>, fmmt::fmm_tile_gemm_kernel<32, 32, true>,
+                        fmmt::fmm_tile_gemm_kernel<32, 32, false, true>})
       FMM_CUDA_TRY(smem(kernel, fmmt::TileShape<32, 32>::SMEM));
     FMM_CUDA_TRY(smem(fmm::fmm_presum_staged_kernel, kPsStagedSmem));
     for (auto kernel : {fmmt::fmm_products_kernel<64, false, false>, fmmt::fmm_products_kernel<64, false, true>,
@@ -809,6 +811,12 @@ int product_depth(const fmm_plan* plan, int ms, int ns, int ks) {
   return (long long)ms * ns >= (1LL << 17) || plan->rank == 1 ? sum_depth(ms, ns, kk, plan->rank) : kk;
 }
 
+// Plain updates up to this deep are bound by their C traffic and run the kernel's SHALLOW form; in columns that do
+// not all start on 16 bytes (two accesses a row pair) up to the second.  Measured us without / with: 12000 x
+// 12000 x 8 634 / 456, x 40 734 / 633, x 64 853 / 869; 4000 x 4000 x 16 75 / 59; odd 12001 x 12001 x 8 830 / 600,
+// x 96 1192 / 1088, x 256 2328 / 2335.
+constexpr int kShallowDepth = 48, kShallowDepthOdd = 128;
+
 // One classical update of a tile_gemm launch.
 struct GemmJob {
   int m, n, k;
@@ -865,8 +873,17 @@ int launch_tile_gemm(const GemmJob* jobs, int njob, int nsm, unsigned* status, c
   }
   g.njob = njob;
   g.status = status;
+  bool shallow = cluster == 1 && !parts;
+  for (int q = 0; q < njob; ++q) {
+    const bool vec = (reinterpret_cast<uintptr_t>(jobs[q].C) & 15) == 0 && (jobs[q].ldc & 1) == 0;
+    shallow = shallow && jobs[q].k <= (vec ? kShallowDepth : kShallowDepthOdd);
+  }
+  g.ahead = nsm;  // half a round to two rounds of the CTAs took 1 to 5 % longer
   ProfScope ps(K_TILE_GEMM, st);
-  return launch_dependent(parts ? fmmt::fmm_tile_gemm_kernel<T, T, true> : fmmt::fmm_tile_gemm_kernel<T, T, false>, dim3((unsigned)first), fmmt::NT,
+  auto kernel = shallow ? fmmt::fmm_tile_gemm_kernel<T, T, false, true>
+                : parts ? fmmt::fmm_tile_gemm_kernel<T, T, true>
+                        : fmmt::fmm_tile_gemm_kernel<T, T, false>;
+  return launch_dependent(kernel, dim3((unsigned)first), fmmt::NT,
                           cluster > 1 ? fmmt::TileShape<T, T>::SMEM : spread_smem(fmmt::TileShape<T, T>::SMEM, first, nsm),
                           st, cluster, g);
 }
@@ -885,6 +902,16 @@ int tile_gemm(const GemmJob* jobs, int njob, cudaStream_t st) {
     todo[n++] = jobs[q];
   }
   if (n == 0) return FMM_OK;
+  // a strip that fills the SMs several times (the k strip of a large C) has a launch of its own shape: with the thin
+  // strips' 32 x 32 tiles, 222-1 12000 x 12000 x 17 took 2987 us instead of 2860
+  for (int q = 0; n > 1 && q < n; ++q)
+    if (tiles_of(todo[q].m, todo[q].n, 64) >= 8LL * fmmt::TileShape<64, 64>::CTAS * sm_count[dev]) {
+      const GemmJob big = todo[q];
+      const int r = tile_gemm(&big, 1, st);
+      if (r != FMM_OK) return r;
+      todo[q] = todo[n - 1];
+      return tile_gemm(todo, n - 1, st);
+    }
   if (n == 1 && S == 1 && tile_side(tiles_of(todo[0].m, todo[0].n, 64), tiles_of(todo[0].m, todo[0].n, 32), sm_count[dev]) == 64)
     return launch_tile_gemm<64>(todo, n, sm_count[dev], dev_status[dev], st);
   return launch_tile_gemm<32>(todo, n, sm_count[dev], dev_status[dev], st);

@@ -57,6 +57,7 @@ struct TileJob {
 struct TileArgs {
   TileJob job[MAX_JOBS];
   int njob;
+  int ahead;  // distance of prefetch_update, in CTAs
   unsigned* status;
 };
 
@@ -179,9 +180,39 @@ __device__ __forceinline__ void tma_stage_b(unsigned st, const CUtensorMap* map,
   for (int h = 0; h < 2; ++h) fmm::tma_load_2d(st + h * TN * 64, map, x + 8 * h, y, fb);
 }
 
+// A C tile of which m x n elements exist to L2, 128-byte lines spread over the warp.
+template <int TM, int TN>
+__device__ __forceinline__ void prefetch_tile(const double* C, long long ldc, int m, int n, int lane) {
+  for (int l = lane; l < (TM / 16) * TN; l += 32) {
+    const int r = (l % (TM / 16)) * 16, c = l / (TM / 16);
+    if (r < m && c < n) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(C + r + (long long)c * ldc));
+  }
+}
+
+// Tiles in groups of 16 tile rows: concurrent CTAs share operand panels in L2.
+template <int TM, int TN>
+__device__ __forceinline__ void tile_origin(int bid, int tiles_m, int tiles_n, int& m0, int& n0) {
+  constexpr int G = 16;
+  const int per = G * tiles_n, first_m = (bid / per) * G;
+  const int rows = min(tiles_m - first_m, G), in = bid % per;
+  m0 = (first_m + in % rows) * TM;
+  n0 = (in / rows) * TN;
+}
+
+// Updates of few stages wait for C and for little else: the CTA of tile t brings the C tile of tile t + ahead to
+// L2, those of the first round their own too.  With streaming stores 12000 x 12000 x 8 takes 456 us (5.05 TB/s),
+// without both 634; x 2 took 467, in groups of 64 or 256 tile rows instead of 16 about 500.
+template <int TM, int TN>
+__device__ __forceinline__ void prefetch_update(const TileJob& J, int m0, int n0, int t, int ahead, int lane) {
+  if (J.first + t < ahead) prefetch_tile<TM, TN>(J.C + m0 + (long long)n0 * J.ldc, J.ldc, J.m - m0, J.n - n0, lane);
+  if (t + ahead >= J.units) return;
+  tile_origin<TM, TN>(t + ahead, J.tiles_m, J.tiles_n, m0, n0);
+  prefetch_tile<TM, TN>(J.C + m0 + (long long)n0 * J.ldc, J.ldc, J.m - m0, J.n - n0, lane);
+}
+
 template <int TM, int TN>
 __device__ __forceinline__ void produce(const TileJob& J, unsigned s0, unsigned full0, unsigned empty0, unsigned* status,
-                                        int m0, int n0, int kbeg, int kend, int lane) {
+                                        int m0, int n0, int kbeg, int kend, int pre, int ahead, int lane) {
   using S = TileShape<TM, TN>;
   const int nst = (kend - kbeg + BK - 1) / BK;
   const bool at = J.a_tma != 0, bt = J.b_tma != 0;
@@ -209,6 +240,7 @@ __device__ __forceinline__ void produce(const TileJob& J, unsigned s0, unsigned 
       cp_async_arrive(fb);
     }
   }
+  if (pre >= 0) prefetch_update<TM, TN>(J, m0, n0, pre, ahead, lane);
   // copies still in flight (only on an error path) land before the CTA exits
   for (int q = max(0, s - S::STAGES); q < s; ++q)
     fmm::mbar_wait_drain(full0 + 8 * (q % S::STAGES), (unsigned)((q / S::STAGES) & 1));
@@ -356,8 +388,8 @@ __device__ __forceinline__ void frag_counts(int vr, int vc, int& im, int& jn) {
 // C += w acc (or C = acc) for a warp's fragments; C at the warp tile's first element of an
 // m x n remainder.  Rows 2 g, 2 g + 1 of a column are one 16-byte access where the columns
 // allow it (vec), and a warp access covers 128 bytes of four columns; a fragment row's loads
-// are all issued before its stores.
-template <int TM, int TN, bool STORE>
+// are all issued before its stores.  STREAM: the stores leave L2 first (an update that C's traffic bounds).
+template <int TM, int TN, bool STORE, bool STREAM = false>
 __device__ __forceinline__ void update_c(double* C, long long ldc, int m, int n, bool vec, double w,
                                          const double (&acc)[TileShape<TM, TN>::NI][TileShape<TM, TN>::NJ][4], int g,
                                          int t4) {
@@ -394,10 +426,13 @@ __device__ __forceinline__ void update_c(double* C, long long ldc, int m, int n,
         const double x = STORE ? acc[i][j][q] : fma(w, acc[i][j][q], cv[j][q].x);
         const double y = STORE ? acc[i][j][2 + q] : fma(w, acc[i][j][2 + q], cv[j][q].y);
         if (two) {
-          *reinterpret_cast<double2*>(cp) = make_double2(x, y);
+          if (STREAM)
+            __stcs(reinterpret_cast<double2*>(cp), make_double2(x, y));
+          else
+            *reinterpret_cast<double2*>(cp) = make_double2(x, y);
         } else {
-          if (rr < m) cp[0] = x;
-          if (rr + 1 < m) cp[1] = y;
+          if (rr < m) STREAM ? __stcs(cp, x) : (void)(cp[0] = x);
+          if (rr + 1 < m) STREAM ? __stcs(cp + 1, y) : (void)(cp[1] = y);
         }
       }
   }
@@ -405,17 +440,6 @@ __device__ __forceinline__ void update_c(double* C, long long ldc, int m, int n,
 
 __device__ __forceinline__ bool vec_ok(const double* C, long long ldc) {
   return ((reinterpret_cast<uintptr_t>(C) & 15) == 0) && ((ldc & 1) == 0);
-}
-
-// Tiles in groups of eight (sixteen for 32-row tiles) tile rows: concurrent CTAs share operand
-// panels in L2.
-template <int TM, int TN>
-__device__ __forceinline__ void tile_origin(int bid, int tiles_m, int tiles_n, int& m0, int& n0) {
-  constexpr int G = TM == 64 ? 16 : 16;
-  const int per = G * tiles_n, first_m = (bid / per) * G;
-  const int rows = min(tiles_m - first_m, G), in = bid % per;
-  m0 = (first_m + in % rows) * TM;
-  n0 = (in / rows) * TN;
 }
 
 // Wait for the launch's predecessors (programmatic dependent launch): nothing before this
@@ -426,8 +450,9 @@ __device__ __forceinline__ void grid_launch() { asm volatile("griddepcontrol.lau
 // One CTA per (tile, part) of up to three independent classical updates C += A * B: the plain
 // GEMM and the fringe strips.  The parts of a tile are the CTAs of a cluster, which leave their
 // sums in shared memory and then add every part, in order, to their share of the tile.
-// PARTS: some CTA's sum is made of parts of its own (consume_k).
-template <int TM, int TN, bool PARTS>
+// PARTS: some CTA's sum is made of parts of its own (consume_k).  SHALLOW: C's traffic bounds the launch, whose
+// jobs have one part each.
+template <int TM, int TN, bool PARTS, bool SHALLOW = false>
 __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_kernel(const __grid_constant__ TileArgs g) {
   using S = TileShape<TM, TN>;
   extern __shared__ unsigned char smem_raw[];
@@ -459,7 +484,7 @@ __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_k
   const int g4 = lane >> 2, t4 = lane & 3, wm = (warp >> 1) & 1, wn = warp & 1;
   const bool vec = vec_ok(J.C, J.ldc);
   if (warp == NC / 32) {
-    produce<TM, TN>(J, s0, full0, empty0, g.status, m0, n0, kbeg, kend, lane);
+    produce<TM, TN>(J, s0, full0, empty0, g.status, m0, n0, kbeg, kend, SHALLOW ? t : -1, g.ahead, lane);
     if (J.S == 1) return;
     __syncwarp();
   } else {
@@ -471,8 +496,11 @@ __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_k
     consume_k<TM, TN, PARTS>(smem, full0, empty0, g.status, kend - kbeg, J.depth, acc, wm * S::WM, wn * S::WN, lane, im, jn,
                              slot, ph);
     if (J.S == 1) {
-      update_c<TM, TN, false>(J.C + (m0 + wm * S::WM) + (long long)(n0 + wn * S::WN) * J.ldc, J.ldc, vr, vc, vec, 1.0, acc,
-                              g4, t4);
+      double* C = J.C + (m0 + wm * S::WM) + (long long)(n0 + wn * S::WN) * J.ldc;
+      if (SHALLOW && !vec)  // code without the wide accesses
+        update_c<TM, TN, false, SHALLOW>(C, J.ldc, vr, vc, false, 1.0, acc, g4, t4);
+      else
+        update_c<TM, TN, false, SHALLOW>(C, J.ldc, vr, vc, vec, 1.0, acc, g4, t4);
       return;
     }
     fmm::named_bar_sync(1, NC);  // every consumer warp is done with the stages
