@@ -947,12 +947,14 @@ struct ProdLaunch {
   int tile = 64;
   size_t tickets = 0;
   int nbt = 0, nbc = 0;
+  bool by_tiles = false;  // a unit per tile with all its products (no tickets)
 };
 
-ProdLaunch plan_products(const int grid_dims[3], int nprod, int mode, int ms, int ns, int nsm) {
+ProdLaunch plan_products(const int grid_dims[3], int nprod, int mode, int ms, int ns, int nsm, bool by_tiles = false) {
   ProdLaunch L;
-  L.tile = product_tile(ms, ns, nprod, nsm);
-  if (mode == fmm::MODE_ACCUM_C && nprod > 1) {
+  L.tile = by_tiles ? 64 : product_tile(ms, ns, nprod, nsm);
+  L.by_tiles = by_tiles;
+  if (mode == fmm::MODE_ACCUM_C && nprod > 1 && !by_tiles) {
     const long long ntiles = tiles_of(ms, ns, L.tile);
     if (ntiles <= kResident64 * (long long)nsm) {
       L.nbt = grid_dims[0] * grid_dims[2];
@@ -990,7 +992,7 @@ int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int gr
   a.nprod = nprod;
   a.tiles_m = (ms + L.tile - 1) / L.tile;
   a.tiles_n = (ns + L.tile - 1) / L.tile;
-  a.chunks = nprod;
+  a.chunks = L.by_tiles ? 1 : nprod;
   a.mode = mode;
   a.status = dev_status[dev];
   a.counter = counter;
@@ -998,9 +1000,9 @@ int launch_products(const fmm::Prod* prods, const fmm::Term* terms, const int gr
   a.nbt = L.nbt;
   a.nbc = L.nbc;
   a.a_tma = a.b_tma = 1;
-  const long long units = (long long)a.tiles_m * a.tiles_n * nprod;
+  const long long units = (long long)a.tiles_m * a.tiles_n * a.chunks;
   const int nsm = sm_count[dev];
-  const bool cut = L.tile == 64 && L.tickets == 0 && kk >= kTailDepth && cut_tail((double)units / nsm);
+  const bool cut = !L.by_tiles && L.tile == 64 && L.tickets == 0 && kk >= kTailDepth && cut_tail((double)units / nsm);
   const long long tail = cut ? units % nsm : 0;
   const long long claims = units + (64 / fmmt::TAIL_ROWS - 1) * tail;
   if (claims > INT32_MAX) return FMM_E_UNSUPPORTED;
@@ -1182,36 +1184,45 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
   return cuda_status(cudaGetLastError());
 }
 
-// ABC schedule: the multi-destination epilogue (C_l += W[l,r] M_r straight from each product
-// tile, ordered by tickets) or the products stored to a workspace and one combine pass (every
-// M_r and C element crossing HBM once).
-//   * Few tiles: when a product has no more tiles than CTAs run at a time, the units of one
-//     tile run together and their ordered C updates form a chain; storing has none.  Measured
-//     us direct / stored: 222-1 1024^3 119 / 97, 2048^3 542 / 544; 222-2 1024^3 189 / 112, 4096^3
-//     3484 / 3456; 222-1 x 333-1 528^3 200 / 67, 2016^3 1165 / 673, 4128^3 4248 / 3982.
-//   * C traffic: the epilogue moves 16 nnz(W) ms ns bytes of C while the DMMAs run, the stored
-//     schedule 8 R ms ns while they run and 8 (R + 2 blocks) ms ns in the combine.  Model
-//     (products 35 TFLOP/s, epilogue C traffic 4.6 TB/s, product stores 6 TB/s, combine 2.6
-//     TB/s): the direct launch takes max(t_mma, t_epi) + 1.05 min^2 / max, the storing launch
-//     1.08 max(t_mma, t_store); storing must gain 3 %.  Measured ms direct / stored: 222-1 x
-//     333-1 4000 x 16000 x 2000 8.83 / 7.81, 222-1 8192 x 8192 x 512 2.12 / 2.22, 8192^3 27.7 /
-//     28.0.
+// ABC schedule of a call (all give the same bits).
+//   STORED: the products stored to a workspace and one combine pass (every M_r and C element crossing HBM once).
+//   DIRECT: the multi-destination epilogue, C_l += W[l,r] M_r straight from each product tile, a unit per tile and
+//     product, ordered by tickets.
+//   DIRECT_TILES: the same, a unit per tile with all its products: its C tiles stay in L2 from update to update.
+// The lines between them, measured on B200 (us stored / direct / direct by tiles):
+//   * Few tiles: when a product has no more tiles than CTAs run at a time, the units of one tile run together
+//     and their ordered C updates form a chain: stored.  222-1 1024^3 97 / 119; 222-2 1024^3 112 / 189;
+//     222-1 x 333-1 2016^3 673 / 1165.
+//   * C traffic: the epilogue moves 16 nnz(W) ms ns bytes of C, at 3 TB/s where nothing else bounds it, the stored
+//     schedule 8 R ms ns and, after the products, 8 (R + 2 blocks) ms ns.  The model below (products at 35
+//     TFLOP/s) picks the faster of the two at 196 of 196 sizes from 4000^2 to 14400^2, block depth 4 to 2048,
+//     five plans: 222-1 12000^2 x 128 1825 / 2562, x 512 4484 / 4494, x 1024 8092 / 7836; 222-1 x 333-1 12000^2 x
+//     1008 8269 / 13900.
+//   * By tiles, where the tiles fill the SMs eight times and the C tiles of a CTA's few blocks stay in L2, up to
+//     2.5 times as long for the products as for C (222-1 12000^2: x 128 1833, x 512 4293, x 1024 7776, x 2048
+//     15011 against 14991; 4000^2 x 512, 1024 tiles, 578; 222-2, 16 blocks, 12000^2 x 512 7557 against 4644), and
+//     against stored with at most four blocks and products that take at least 0.6 of its C updates' time (222-1 x 64
+//     1532, 232-1 x 504 4618 against 4848), in aligned columns (222-1 8001^2 x 128 1002 against 880).
 // The product workspace (8 R ms ns bytes) must fit the workspace cap, and so must the operand sums
 // (run_core: deep k makes them large where the products are few and small).  It is the reference's
 // own trade between its ABC and AB variants (meta/model_gen.py:87-95 counts the C memory
-// operations of each).  Both schedules give the same bits.
-bool prefer_stored_products(const fmm_plan* plan, int ms, int ns, int ks, int nsm) {
+// operations of each).
+enum AbcSchedule : int { ABC_STORED = 0, ABC_DIRECT = 1, ABC_DIRECT_TILES = 2 };
+AbcSchedule abc_schedule(const fmm_plan* plan, int ms, int ns, int ks, bool vec, int nsm) {
   const double mn = (double)ms * ns;
   const int nblk = plan->dims[0] * plan->dims[2];
-  if (plan->rank < 2 || 8.0 * plan->rank * mn > (double)g_ws_limit.load()) return false;
-  if (tiles_of(ms, ns, 64) <= kResident64 * (long long)nsm) return true;
+  const long long ntiles = tiles_of(ms, ns, 64), resident = kResident64 * (long long)nsm;
+  const bool room = plan->rank > 1 && combine_fits(plan) && 8.0 * plan->rank * mn <= (double)g_ws_limit.load();
+  if (room && ntiles <= resident) return ABC_STORED;
   const double t_mma = 2.0 * plan->rank * mn * ks / 35e12;
-  const double t_epi = 16.0 * plan->n_cterms * mn / 4.6e12;
-  const double t_store = 8.0 * plan->rank * mn / 6.0e12;
-  const double t_comb = 8.0 * (plan->rank + 2.0 * nblk) * mn / 2.6e12;
+  const double t_epi = 16.0 * plan->n_cterms * mn / 3e12;
+  const double t_store = 8.0 * plan->rank * mn / 5e12;
+  const double t_comb = 8.0 * (plan->rank + 2.0 * nblk) * mn / 4e12;
+  const bool by_tiles = plan->rank > 1 && nblk <= 9 && ntiles >= 8 * resident && t_mma < 2.5 * t_epi;
+  if (by_tiles && nblk <= 4 && vec && t_mma > 0.35 * t_epi) return ABC_DIRECT_TILES;  // C updates by tiles: 5.2 TB/s
   const double hi = std::max(t_mma, t_epi), lo = std::min(t_mma, t_epi);
-  const double t_direct = hi + 1.05 * lo * lo / hi;
-  return 1.08 * std::max(t_mma, t_store) + t_comb < 0.97 * t_direct;
+  if (room && 0.98 * std::max(t_mma, t_store) + t_comb < hi + 0.7 * lo * lo / hi) return ABC_STORED;
+  return by_tiles ? ABC_DIRECT_TILES : ABC_DIRECT;
 }
 
 // The pre-summed form of one call: which operands get slots, the tables the products kernel
@@ -1442,11 +1453,13 @@ int run_core(const fmm_plan* plan, int pack, const double* A, long long lda, con
   const PresumPlan pp = presum_plan(plan, ms, ns, ks, pack == FMM_PACK_NAIVE || !in_place);
   // an ABC call whose operand sums exceed the workspace cap runs in groups, whatever its C traffic
   const bool capped = pack == FMM_PACK_ABC && (long long)presum_bytes(pp) > g_ws_limit.load();
-  const bool stored = pack != FMM_PACK_ABC ||
-                      (!capped && g_ticket_fill == 0 && combine_fits(plan) && prefer_stored_products(plan, ms, ns, ks, nsm));
+  const bool vec = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc & 1) == 0;
+  AbcSchedule sched = pack != FMM_PACK_ABC ? ABC_STORED : abc_schedule(plan, ms, ns, ks, vec, nsm);
+  if (pack == FMM_PACK_ABC && g_ticket_fill != 0) sched = ABC_DIRECT;  // the schedule with tickets
+  const bool stored = sched == ABC_STORED;
   if (capped) return run_presum_groups(plan, *d, A, lda, B, ldb, C, ldc, ms, ns, ks, nsm, false, st);
   const int mode = stored ? fmm::MODE_STORE_M : fmm::MODE_ACCUM_C;
-  const ProdLaunch L = plan_products(plan->dims, R, mode, ms, ns, nsm);
+  const ProdLaunch L = plan_products(plan->dims, R, mode, ms, ns, nsm, sched == ABC_DIRECT_TILES);
   const size_t tk = (sizeof(int) * (1 + L.tickets) + 255) & ~(size_t)255;
   const size_t mb = stored ? sizeof(double) * (size_t)ms * ns * R : 0;
   char* ws = nullptr;
