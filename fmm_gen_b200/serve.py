@@ -69,6 +69,26 @@ class Request:
         return None if self.done is None else self.done - self.arrival
 
 
+def operand_sum_bytes(plan, m: int, n: int, k: int) -> int:
+    """Device bytes of a batch problem's operand sums: a slot per sum, or per product where m, k or the
+    blocks' k is odd or no multiple of eight (the k extent then rounded up to eight)."""
+    p = tuner.algebra.partition(m, n, k, plan.dims)
+    if min(p.ms, p.ns, p.ks) <= 0:
+        return 0
+    every = p.ks % 8 != 0 or (m | k) & 1
+    kk = -(-p.ks // 8) * 8 if every else p.ks
+
+    def slots(M):
+        # a single term with a power of two as its coefficient is read in place
+        single = (np.count_nonzero(M, axis=0) == 1) & (np.frexp(np.abs(M).sum(axis=0))[0] == 0.5)
+        return plan.rank if every else int((~single).sum())
+
+    def padded(nbytes):
+        return -(-nbytes // 256) * 256
+
+    return padded(8 * slots(plan.U) * (p.ms + p.ms % 2) * kk) + padded(8 * slots(plan.V) * (kk + kk % 2) * p.ns)
+
+
 def request_bytes(kind: str, shape: Sequence[int], algorithm: str) -> int:
     """Device bytes a request holds while admitted: operands, C and workspaces."""
     m, n, k = shape
@@ -80,14 +100,8 @@ def request_bytes(kind: str, shape: Sequence[int], algorithm: str) -> int:
         kpad = -(-ks // 64) * 64
         mws = 8 * R * ms * ns if R > 1 else 0  # product tiles before the combine pass
         return 4 * (m * k + k * n) + 8 * m * n + 6 * R * (ms + ns) * kpad + mws
-    ws = 0
     plan = tuner.plan_of(algorithm)
-    if plan is not None:
-        p = tuner.algebra.partition(m, n, k, plan.dims)
-        if tuner._presummed(plan, p.ms, p.ns, p.ks):
-            nu = np.count_nonzero(plan.U, axis=0)
-            nv = np.count_nonzero(plan.V, axis=0)
-            ws = 8 * (int((nu > 1).sum()) * p.ms * p.ks + int((nv > 1).sum()) * (p.ks + 1) * p.ns)
+    ws = operand_sum_bytes(plan, m, n, k) if plan is not None else 0
     pitch = 8 * ((m + 1) * k if m & 1 else 0) + 8 * ((k + 1) * n if k & 1 else 0)
     return 8 * (m * k + k * n + m * n) + ws + pitch
 
