@@ -104,7 +104,8 @@ def model_counts(plan: algebra.FMMPlan) -> List[int]:
 
 
 def _presummed(plan: algebra.FMMPlan, ms: int, ns: int, ks: int) -> bool:
-    """The library's rule for forming operand sums in HBM before the products."""
+    """Blocks whose sums the model counts as formed in HBM before the products; smaller ones as folded while
+    staging, as the kernels that the constants were fitted to did (the library forms all sums in HBM today)."""
     return plan.rank > 1 and ms * ns >= (1 << 17) and ks >= 64
 
 
@@ -301,9 +302,11 @@ class BatchTuner:
                 break
         rep.choices = list(choices)
         # tile height: 64 instead of 128 rows for problems whose units are long and few, by the
-        # model's unit length over unit count; kept only if measured faster (both heights run the
-        # same 64 x 64 units today).
+        # model's unit length over unit count; kept only if measured faster.  Not for a measurement
+        # whose heights run alike (batch_timer's: the library's units are 64 x 64 either way).
         rep.tiles = [TILE] * len(shapes)
+        if not getattr(measure, "tile_heights", True):
+            return rep
         order = sorted(range(len(shapes)), key=lambda i: -self.tile_pressure(choices[i], shapes[i]))
         for frac in (0.05, 0.25, 1.0):
             sel = order[:max(1, int(round(frac * len(order))))]
@@ -370,6 +373,7 @@ def batch_timer(runtime, shapes, As, Bs, Cs, reps: int = 3, warmup: int = 1):
             b.close()
 
     measure.plans = plans
+    measure.tile_heights = False
     return measure
 
 
