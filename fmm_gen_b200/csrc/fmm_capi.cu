@@ -760,7 +760,10 @@ bool cut_tail(double units_per_sm) {
 // partly filled round in quarters where it runs as strips (half a unit for 32 x 32), the small
 // tile at 6 % lower rate.  Measured us with 64 / 32: products of 222-1 1024^3 70 / 76, 1100^3 93 / 95,
 // 1488 x 1200 x 998 116 / 124, 1900 x 1800 x 2200 415 / 444, 2500^3 827 / 872, of 222-1 x 333-1 1200^3
-// 116 / 116, 2016^3 406 / 431 (blocks of 336: partial tiles cost their fragments, not whole tiles).
+// 116 / 116, 2016^3 406 / 431 (blocks of 336: partial tiles cost their fragments, not whole tiles).  Launches
+// without strips (k below kTailDepth, updates of C) are priced alike: their last round in whole units instead
+// chose better at 222-1 1088^2 x 200 (40.5 / 36.8 us a call) and worse at 1600^2 x 200 (59.0 / 63.7), 333-1 1100^2 x 200
+// (52.5 / 57.3), 222-2 1000^2 x 192 (55.0 / 58.6).
 int product_tile(long long m, long long n, int nprod, int nsm) {
   const double work = (double)((m + 15) / 16 * 16) * (double)((n + 7) / 8 * 8) * nprod / nsm;
   const double u64 = work / 4096, whole = std::floor(u64), f = u64 - whole;
@@ -918,11 +921,10 @@ int tile_gemm(const GemmJob* jobs, int njob, cudaStream_t st) {
 }
 
 // Workspaces of pre-summed operands: slot j of S is ms x kslot, of T kslot x ns (block
-// columns); nslot = 0: every operand of that side is a block of A / B.
+// columns), kslot the products' depth; nslot = 0: every operand of that side is a block of A / B.
 struct PresumOps {
   const int* plistA = nullptr;  // products of the slots (device)
   const int* plistB = nullptr;
-  int kslot = 0;                // columns per S slot and rows per T slot
   double* S = nullptr;
   long long ldS = 0;
   int nslotA = 0;
@@ -1394,7 +1396,6 @@ int run_presum_groups(const fmm_plan* plan, const DevTables& d, const double* A,
   for (int g0 = 0; g0 < R && rc == FMM_OK; g0 += (int)G) {
     const int g1 = (int)std::min<long long>(R, g0 + G), n = g1 - g0;
     PresumOps ps;
-    ps.kslot = kk;
     ps.S = reinterpret_cast<double*>(ws + tk);
     ps.ldS = ldS;
     ps.nslotA = n;
@@ -1475,7 +1476,6 @@ int run_core(const fmm_plan* plan, int pack, const double* A, long long lda, con
   PresumOps ps;
   ps.plistA = pp.all ? d->plist_all : d->plistA;
   ps.plistB = pp.all ? d->plist_all : d->plistB;
-  ps.kslot = pp.kk;
   ps.S = reinterpret_cast<double*>(ws + tk);
   ps.ldS = pp.ldS;
   ps.nslotA = pp.nA;

@@ -12,10 +12,12 @@
 // 128 x 128 CTA per SM, 64-bit fragment loads with 4-way conflicts, a separate epilogue
 // group): plain 4096^3 33.9 -> 35.6 TFLOP/s (cuBLAS 35.5), 2048^3 32.7 -> 34.7, 1024^3 25 ->
 // 30; plain 701 x 503 x 615 108 -> 26 us; whole calls (with the operand sums and combine as they are
-// now) 222-1 240^3 126 -> 17.5 us, 1501 x 1203 x 999 421 -> 168 us, 2048^3 568 -> 510 us; 222-1 x 333-1
-// 16384^3 205.6 -> 196.1 ms; the 512-problem batch 96.8 -> 88.7 ms.  A 64 x 64 tile reads twice the operand bytes of a 128 x 128 one (16 bytes
+// now) 222-1 240^3 126 -> 17.6 us, 1501 x 1203 x 999 421 -> 174 us, 2048^3 568 -> 519 us; 222-1 x 333-1
+// 16384^3 205.6 -> 196.1 ms; the 512-problem batch 96.8 -> 88.9 ms (sums in k parts, which cost 2 to 3 % where there
+// are any, included: consume_k).  A 64 x 64 tile reads twice the operand bytes of a 128 x 128 one (16 bytes
 // per cycle and SM from L2), which costs nothing measurable, and wastes a quarter as much on
-// partial tiles and a launch's last round.
+// partial tiles and a launch's last round.  Three 64 x 64 CTAs leave a thread 128 registers: the plain kernel fits,
+// the products kernels spill 88 to 148 bytes of their units' state (16384^3 runs at 0.95 of the pipe all the same).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -464,7 +466,9 @@ __global__ void __launch_bounds__(NT, (TileShape<TM, TN>::CTAS)) fmm_tile_gemm_k
     if (q < g.njob && (int)blockIdx.x >= g.job[q].first) ji = q;
   const TileJob& J = g.job[ji];
   const int u = (int)blockIdx.x - J.first;
-  if (u >= J.units) return;  // padding to whole clusters (only in jobs of one part)
+  // Padding to whole clusters, where the launch's cluster is larger than this job's part count.  The cluster's
+  // barriers do not count threads that have exited, and a tile's parts never address another tile's CTAs.
+  if (u >= J.units) return;
   const int part = u % J.S, t = u / J.S;
   int m0, n0;
   tile_origin<TM, TN>(t, J.tiles_m, J.tiles_n, m0, n0);
@@ -566,8 +570,7 @@ struct ProdArgs {
   int* tickets;           // per warp tile (4 per tile) and, nbt > 0, per C block: updates done, in
                           // product order; zeroed before the launch
   unsigned* status;
-  int* counter;           // work units claimed so far, zeroed before the launch; nullptr: CTA b
-                          // takes units b, b + grid, ... (launches without tickets)
+  int* counter;           // work units claimed so far, zeroed before the launch
   int ms, ns, ks;         // product sizes
   int kcap;               // k extent of A and B (a k split's last part may end early)
   int nprod, tiles_m, tiles_n;
@@ -696,7 +699,7 @@ __device__ __forceinline__ void prod_producer(const Src& src, const fmm::UnitRin
       const int e = n % fmm::UQ_DEPTH;
       fmm::mbar_wait(q.empty(e), (unsigned)(((n / fmm::UQ_DEPTH) & 1) ^ 1), src.status());
       if ((*(volatile unsigned*)src.status() & fmm::STATUS_WAIT_TIMEOUT) == 0u) {
-        u = src.counter() ? atomicAdd(src.counter(), 1) : (int)(blockIdx.x + (unsigned)n * gridDim.x);
+        u = atomicAdd(src.counter(), 1);
         if (u >= src.claims()) u = -1;
       }
       fmm::st_shared_s32(q.entry(e), u);
