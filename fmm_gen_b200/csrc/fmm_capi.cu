@@ -1197,14 +1197,14 @@ int launch_combine(const fmm_plan* plan, const DevTables& d, double* C, long lon
 //     222-1 x 333-1 2016^3 673 / 1165.
 //   * C traffic: the epilogue moves 16 nnz(W) ms ns bytes of C, at 3 TB/s where nothing else bounds it, the stored
 //     schedule 8 R ms ns and, after the products, 8 (R + 2 blocks) ms ns.  The model below (products at 35
-//     TFLOP/s) picks the faster of the two at 196 of 196 sizes from 4000^2 to 14400^2, block depth 4 to 2048,
+//     TFLOP/s) picks the faster of the two at all of 204 sizes from 4000^2 to 14400^2, block depth 4 to 2048,
 //     five plans: 222-1 12000^2 x 128 1825 / 2562, x 512 4484 / 4494, x 1024 8092 / 7836; 222-1 x 333-1 12000^2 x
 //     1008 8269 / 13900.
 //   * By tiles, where the tiles fill the SMs eight times and the C tiles of a CTA's few blocks stay in L2, up to
 //     2.5 times as long for the products as for C (222-1 12000^2: x 128 1833, x 512 4293, x 1024 7776, x 2048
 //     15011 against 14991; 4000^2 x 512, 1024 tiles, 578; 222-2, 16 blocks, 12000^2 x 512 7557 against 4644), and
 //     against stored with at most four blocks and products that take at least 0.6 of its C updates' time (222-1 x 64
-//     1532, 232-1 x 504 4618 against 4848), in aligned columns (222-1 8001^2 x 128 1002 against 880).
+//     1532 against 1448, 232-1 x 504 4618 against 4848), in aligned columns (222-1 8001^2 x 128 1002 against 880).
 // The product workspace (8 R ms ns bytes) must fit the workspace cap, and so must the operand sums
 // (run_core: deep k makes them large where the products are few and small).  It is the reference's
 // own trade between its ABC and AB variants (meta/model_gen.py:87-95 counts the C memory

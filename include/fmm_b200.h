@@ -112,7 +112,7 @@ int fmm_dgemm_host(const fmm_plan *plan, int pack_type, int m, int n, int k, con
  * synchronous host entry points check it themselves. */
 int fmm_device_status(int clear);
 
-/* Workspace of the pre-summed operands (the ABC pack type's large products) -- the
+/* Workspace of the pre-summed operands (the ABC pack type) -- the
  * reference's counterpart is its packing pool (common/dgemm/bl_dgemm_util.c:375-394),
  * sized by the first call and never bounded.  One call's workspace is capped at `bytes`
  * (default 8 GiB; bytes <= 0 restores it): a call whose sums would need more runs its
@@ -122,8 +122,8 @@ int fmm_device_status(int clear);
  * much.  A call of the abc or ab pack type whose workspace cannot be allocated runs in
  * groups too, of as many products as there is room for.  Returns the previous cap.
  * fmm_last_workspace_bytes: pre-summed workspace bytes of the calling thread's last
- * fmm_dgemm_dev / host call (0 when it used none).  The stored products of a call whose C
- * traffic the library routes through one combine pass (8 R ms ns bytes) are not capped. */
+ * fmm_dgemm_dev / host call (0 when it used none).  Products that a call stores (8 R ms ns bytes)
+ * are not counted; an ABC call stores them only where they fit the cap on their own. */
 long long fmm_set_workspace_limit(long long bytes);
 long long fmm_last_workspace_bytes(void);
 
@@ -132,7 +132,7 @@ long long fmm_last_workspace_bytes(void);
  *     device, in ns (default 4e9; value <= 0 restores the default).
  *   FMM_DEBUG_TICKET_FILL: byte written into every ticket of a single-problem FMM launch
  *     before it runs (default 0).  While it is set, ABC calls of any size take the schedule
- *     whose products wait on tickets (else small ones store their products).  0xFF starts every ticket at -1, which no launch ever
+ *     whose products wait on tickets (else their size decides).  0xFF starts every ticket at -1, which no launch ever
  *     releases, so the launch's first ticket waits run out: the kernel records
  *     FMM_E_TIMEOUT after the limit, stops waiting for tickets, and finishes (its result
  *     is then unreliable); fmm_device_status() reports it.  Lets a test check the
