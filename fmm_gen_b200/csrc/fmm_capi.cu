@@ -733,12 +733,18 @@ std::atomic<int> g_force_ksplit{0};  // fmm_debug_set FMM_DEBUG_KSPLIT: S for ev
 
 long long tiles_of(int m, int n, int t) { return (long long)((m + t - 1) / t) * ((n + t - 1) / t); }
 
+constexpr int kResident64 = fmmt::TileShape<64, 64>::CTAS;  // 64 x 64 CTAs per SM
+
 // Tile side of a plain update with u64 units of 64 x 64 or u32 of 32 x 32: the modelled time,
 // SM-seconds over the SMs plus half a unit for the last, partly filled round, the small tile at
 // 6 % lower rate (more shared-memory reads per DMMA, twice the operand bytes).  Measured us with
-// 64 / 32: 1024^3 77.1 / 75.8, 1200^3 139 / 124, 2048^3 503 / 528, 4096^3 3857 / 4022.
+// 64 / 32: 1024^3 77.1 / 75.8, 1200^3 139 / 124, 2048^3 503 / 528, 4096^3 3857 / 4022.  Two or three units an SM
+// run at the same time and end together: 1088 x 1088 x 1200 90.6 / 99.4, 1344 x 1280 x 3936 431 / 454 (one alone does
+// not reach the rate: 768 x 768 x 1200 58.8 / 55.0).
 int tile_side(long long u64, long long u32, int nsm) {
-  const double c64 = ((double)u64 / nsm + 0.5) * 4096, c32 = ((double)u32 / nsm + 0.5) * 1024 * 1.06;
+  const double n64 = (double)u64 / nsm;
+  const double c64 = (n64 > 1 && n64 <= kResident64 ? std::ceil(n64) : n64 + 0.5) * 4096;
+  const double c32 = ((double)u32 / nsm + 0.5) * 1024 * 1.06;
   return c64 <= c32 ? 64 : 32;
 }
 
@@ -776,13 +782,23 @@ int product_tile(long long m, long long n, int nprod, int nsm) {
 // [s d, min(k, (s + 1) d)).  The result of an update depends on S (each part is summed on its
 // own and added to C in order), so S is a function of the sizes alone and batches use the
 // same one.
+// Launches that fill the SMs a few times run deep k in two parts all the same: half as long units, whose last round
+// costs half as much (us with 1 / 2 parts: 1408 x 1408 x 3936 524 / 502, 1280 x 1216 x 8000 844 / 788, 2112 x 2112
+// x 2048 567 / 560; 1600 x 1600 x 1504 246 / 251, and 1344 x 1344 x 3936 431 / 449, whose 64 x 64 units
+// end together).  The lines are those of a 148-SM chip.
 constexpr int kMinPartDepth = 64;
 constexpr int kPartCtas = 460;
+constexpr int kTwoPartDepth = 2048, kTwoPartSms = 148;
 void classical_parts(int m, int n, int k, int* S, int* d) {
   auto depth = [&](int s) { return ((k + s - 1) / s + 7) / 8 * 8; };
   const long long t32 = tiles_of(m, n, 32);
   int s = 1;
   while (2 * s <= fmmt::MAX_SPLIT && t32 * 2 * s <= kPartCtas && k >= 2 * s * kMinPartDepth) s *= 2;
+  if (s == 1 && k >= kTwoPartDepth) {
+    const long long t64 = tiles_of(m, n, 64);
+    const bool together = t64 <= kResident64 * kTwoPartSms && tile_side(t64, t32, kTwoPartSms) == 64;
+    if (t64 <= 8 * kTwoPartSms && !together) s = 2;
+  }
   const int forced = g_force_ksplit.load();
   if (forced > 0 && (long long)(forced - 1) * depth(forced) < k) s = forced;
   *S = s;
@@ -939,8 +955,6 @@ struct PresumOps {
 bool whole_k_steps(const fmm_plan* plan, int ks) {
   return ks % 8 == 0 || (plan->rank == 1 && plan->dims[0] == 1 && plan->dims[1] == 1 && plan->dims[2] == 1);
 }
-
-constexpr int kResident64 = fmmt::TileShape<64, 64>::CTAS;  // 64 x 64 CTAs per SM
 
 // Tile side of a products launch and its tickets: per (tile, C block) where a product has no
 // more tiles than CTAs run at a time (the units of one tile then run together, and one ticket
