@@ -13,7 +13,7 @@
 // group): plain 4096^3 33.9 -> 35.6 TFLOP/s (cuBLAS 35.5), 2048^3 32.7 -> 34.7, 1024^3 25 ->
 // 30; plain 701 x 503 x 615 108 -> 26 us; whole calls (with the operand sums and combine as they are
 // now) 222-1 240^3 126 -> 17.6 us, 1501 x 1203 x 999 421 -> 174 us, 2048^3 568 -> 519 us; 222-1 x 333-1
-// 16384^3 205.6 -> 196.1 ms; the 512-problem batch 96.8 -> 88.9 ms (sums in k parts, which cost 2 to 3 % where there
+// 16384^3 205.6 -> 196.1 ms; the 512-problem batch 96.8 -> 89.1 ms (sums in k parts, which cost 2 to 3 % where there
 // are any, included: consume_k).  A 64 x 64 tile reads twice the operand bytes of a 128 x 128 one (16 bytes
 // per cycle and SM from L2), which costs nothing measurable, and wastes a quarter as much on
 // partial tiles and a launch's last round.  Three 64 x 64 CTAs leave a thread 128 registers: the plain kernel fits,
